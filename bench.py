@@ -1177,15 +1177,15 @@ def main():
     except Exception:
         pass
     peak = peaks.get("bf16_tflops", 1900.0)
-    # algorithmic tensor work of the amplitude GEMM: digit products x 2 B N_up N_F
+    # algorithmic tensor work of the amplitude GEMM: products (one per modulus) x 2 B N_up N_F
     NF = int(inp["infl"][1].Ntot[GF])
-    prods2 = st["slices2"] * (st["slices2"] + 1) // 2
+    prods2 = st["products2"]
     alg2 = prods2 * 2.0 * B * NU * NF
     g2ms = float(np.median(g2))
     achieved = alg2 / (g2ms * 1e-3) / 1e12
     traffic = None
     try:
-        traffic = json.load(open(os.path.join(ROOT, "profiles", "roofline_traffic.json")))["gemm2_bytes_per_launch"]
+        traffic = json.load(open(os.path.join(ROOT, "profiles", "roofline_traffic.json")))["residue_gemm2_bytes_per_launch"]
     except Exception:
         pass
 
@@ -1200,14 +1200,14 @@ def main():
                "config": {"workload": WORKLOAD + ("" if args.rule == "c4" else f", symmetrisation {args.rule}"),
                           "symmetrisation": args.rule, "lower_states": B, "upper_states": NU, "N_v": inp["nv"],
                           "lower_dim": int(inp["infl"][0].Ntot[GI]), "upper_dim": NF,
-                          "l2": "inputs larger than L2 (BF16 digits of the upper vectors ~2 GB per step)",
+                          "l2": "inputs larger than L2 (BF16 residues of the upper vectors ~4 GB per step)",
                           "parallelism": f"replicas by lower-state range x{ws}",
-                          "precision": f"Ozaki digits: GEMM1 beta={st['beta1']} x{st['slices1']}, "
-                                       f"GEMM2 beta={st['beta2']} x{st['slices2']} chunks={st['chunks2']}; "
-                                       "exact FP32 accumulation, FP64 recombination + refinement"},
+                          "precision": f"Ozaki residues: GEMM1 {st['slices1']} moduli, GEMM2 {st['slices2']} moduli in "
+                                       f"{st['chunks2']} chunks; exact FP32 accumulation, exact reconstruction, "
+                                       "FP64 refinement"},
                "roofline": {"bound": "tensor", "achieved": achieved, "peak": peak, "unit": "TFLOP/s",
                             "frac": achieved / peak, "traffic": traffic,
-                            "kernel": "k_digit_gemm (amplitude GEMM)", "kernel_ms": g2ms,
+                            "kernel": "k_residue_gemm (amplitude GEMM)", "kernel_ms": g2ms,
                             "algorithmic_flops": alg2, "peak_source": "MEASURED_PEAKS.json bf16_tflops (burst)"},
                "cpu_baseline": cpu,
                "e2e": {"value": ws * transitions / (e2e_step * 1e-3), "unit": UNIT, "ms_per_step": e2e_step,

@@ -23,6 +23,7 @@
 #include <cstdlib>
 
 #include "gain_internal.h"
+#include "residue.h"
 #include "split.h"
 
 namespace gain {
@@ -214,7 +215,9 @@ struct PairLayout {
     std::vector<std::pair<int, int>> fblocks;   // padded [start, end) of each upper K block
     DevArray<int> d_colposI, d_i_sym, d_i_prim, d_colposF, d_f_sym, d_f_prim, d_band_k0, d_band_len;
     DevArray<double> d_i_coef, d_f_coef, band;
-    int beta1 = 0, s1 = 0, c1 = 0;
+    std::array<int, 4> dig = {0, 0, 0, 0};   // the band digits' beta, slices, chunks and bits (0: none)
+    template <class P>
+    bool digits_are(const P& p) const { return dig == std::array<int, 4>{p.beta, p.slices, p.chunks, p.bits}; }
     DevArray<__nv_bfloat16> bandDig;
     StatsDev bandStats;
     CUtensorMap tmBand, tmBandPair;   // 128-row boxes; 64-row boxes for a CTA pair
@@ -351,6 +354,8 @@ struct gain_engine_s {
     gain::DevArray<int> err;
     gain::DevArray<gain::split::Tile> tiles1, tiles2;
     gain::DevArray<gain::split::Prod> prods1, prods2;
+    gain::DevArray<gain::split::ResTile> rtiles1, rtiles2;
+    gain::DevArray<uint16_t> res;   // residues of one panel of a residue GEMM's outputs
     gain::DevArray<double> lineS, lineA, lineI, eIdev, eFdev;
     gain::DevArray<unsigned char> lineKeep;
     gain::DevArray<uint32_t> textLens;
@@ -606,8 +611,21 @@ gain_status run_plain_pieces(gain_engine e, const gain_pair_job* j, int dI, int 
 }
 
 // ------------------------------------------------------------------ split path
+// Operand planes of a split-precision GEMM: balanced digits (bits = 0: `slices` digits of
+// `beta` bits), or residues (residue.h: `slices` moduli, integers of `bits` fraction bits).
 struct SplitParams {
     int beta, slices, chunks;
+    int bits = 0;
+    int tab = 0;   // residue form: the plane constants' table (operand A: 0, operand B: slices)
+    SplitParams as_b() const {
+        SplitParams p = *this;
+        p.tab = bits ? slices : 0;
+        return p;
+    }
+    int stat_chunks() const { return bits ? 1 : chunks; }   // row-statistics entries per row
+    bool same(const SplitParams& o) const {
+        return beta == o.beta && slices == o.slices && chunks == o.chunks && bits == o.bits;
+    }
 };
 
 // Digits and chunking from the inner length K of the exact accumulations: the Cauchy-Schwarz
@@ -705,8 +723,8 @@ void row_grouped(std::vector<split::Tile>& t, int mstep) {
 // list, and the digits of each then come from DRAM).  The jobs (tile groups) with the
 // costliest tiles go first, so that cheap tiles even out the end.  The list is laid out so
 // that unit u runs entries u, u + units, ... (empty slots: group -1).
-std::vector<split::Tile> list_schedule(const std::vector<split::Tile>& tiles, const std::vector<double>& cost,
-                                       int units) {
+template <class T>
+std::vector<T> list_schedule(const std::vector<T>& tiles, const std::vector<double>& cost, int units) {
     std::map<int, double> job_cost;
     for (size_t i = 0; i < tiles.size(); ++i) job_cost[tiles[i].group] = std::max(job_cost[tiles[i].group], cost[i]);
     std::vector<int> order(tiles.size());
@@ -726,10 +744,10 @@ std::vector<split::Tile> list_schedule(const std::vector<split::Tile>& tiles, co
     }
     size_t depth = 0;
     for (auto& v : per) depth = std::max(depth, v.size());
-    split::Tile empty;
+    T empty;
     memset(&empty, 0, sizeof empty);
     empty.group = -1;
-    std::vector<split::Tile> out(depth * units, empty);
+    std::vector<T> out(depth * units, empty);
     for (int u = 0; u < units; ++u)
         for (size_t k = 0; k < per[u].size(); ++k) out[k * units + u] = tiles[per[u][k]];
     return out;
@@ -954,9 +972,7 @@ gain_status build_layout(gain_engine e, const gain_pair_job* j, int dI, int dF, 
     GAIN_TRY(L.d_band_len.upload(L.band_len));
     GAIN_TRY(L.band.alloc((size_t)L.fpad * L.W));
     GAIN_TRY(launch_layout_band(e, j));
-    L.beta1 = 0;
-    L.s1 = 0;
-    L.c1 = 0;
+    L.dig = {};
     std::copy(key, key + 6, L.key);
     L.dip_version = e->dip_version;
     L.wig_version = wv;
@@ -1045,7 +1061,9 @@ split::SliceArgs slice_args(const double* src, long ld, const int* src_rows, int
     a.grid_limit = grid_limit;
     a.col_inv = col_inv;
     const int nkb = kpad / split::BK;
-    for (int c = 0; c <= p.chunks; ++c) {
+    a.bits = p.bits;
+    a.tab = p.tab;
+    for (int c = 0; c <= p.chunks && !p.bits; ++c) {
         const int dest0 = c == p.chunks ? kpad : (int)(((long)c * nkb) / p.chunks) * split::BK;
         int s0;
         if (c == p.chunks) s0 = ncols;
@@ -1064,8 +1082,8 @@ split::SliceArgs slice_args(const double* src, long ld, const int* src_rows, int
     a.digits = dig + (size_t)row0 * kpad;
     a.slices = p.slices;
     a.beta = p.beta;
-    a.nchunks = p.chunks;
-    a.st = stv.view(with_inerr, (size_t)row0, p.chunks);
+    a.nchunks = p.stat_chunks();
+    a.st = stv.view(with_inerr, (size_t)row0, p.stat_chunks());
     a.inerr2_prev = inerr_prev ? inerr_prev + row0 : nullptr;
     a.e_prev = e_prev ? e_prev + row0 : nullptr;
     return a;
@@ -1086,19 +1104,19 @@ gain_status slice(gain_engine e, const double* src, long ld, const int* src_rows
 // The band digits of layout L for the first GEMM's digit configuration p1 (kept until the
 // configuration or the band changes) and their tensor maps.
 gain_status layout_band_digits(gain_engine e, PairLayout& L, const SplitParams& p1, cudaStream_t st) {
-    if (L.beta1 != p1.beta || L.s1 != p1.slices || L.c1 != p1.chunks) {
+    if (!L.digits_are(p1)) {
         GAIN_TRY(L.bandDig.alloc((size_t)p1.slices * L.fpad * L.W));
-        GAIN_TRY(L.bandDig.zero(st, (size_t)p1.slices * L.fpad * L.W));
-        GAIN_TRY(L.bandStats.alloc(L.fpad, p1.chunks, false));
-        GAIN_TRY(L.bandStats.zero(st, L.fpad, p1.chunks, false));
-        GAIN_TRY(slice(e, L.band.p, L.W, nullptr, L.fpad, L.W, nullptr, nullptr, L.W, L.fpad, L.bandDig.p, p1,
+        GAIN_TRY(L.bandStats.alloc(L.fpad, p1.stat_chunks(), false));
+        if (!p1.bits) {   // every row and column of the residue planes is written
+            GAIN_TRY(L.bandDig.zero(st, (size_t)p1.slices * L.fpad * L.W));
+            GAIN_TRY(L.bandStats.zero(st, L.fpad, p1.chunks, false));
+        }
+        GAIN_TRY(slice(e, L.band.p, L.W, nullptr, L.fpad, L.W, nullptr, nullptr, L.W, L.fpad, L.bandDig.p, p1.as_b(),
                        L.bandStats, false, nullptr, nullptr, st));
         if (!split::make_digit_map(&L.tmBand, L.bandDig.p, L.W, L.fpad, p1.slices) ||
             !split::make_digit_map(&L.tmBandPair, L.bandDig.p, L.W, L.fpad, p1.slices, split::BN / 2))
             return set_error(GAIN_ERR_CUDA, "cuTensorMapEncodeTiled failed for the band digits");
-        L.beta1 = p1.beta;
-        L.s1 = p1.slices;
-        L.c1 = p1.chunks;
+        L.dig = {p1.beta, p1.slices, p1.chunks, p1.bits};
     }
     return GAIN_OK;
 }
@@ -1128,10 +1146,141 @@ SplitParams gemm1_params(const PairLayout& L, const gain_split_opts* opts) {
     return p1x;
 }
 
+// Residue form of a GEMM of inner length K at `bits` fraction bits (slices 0: no set of moduli
+// holds it).  beta is the bits a modulus holds, rounded down.
+SplitParams residue_params(int bits, int K) {
+    SplitParams p;
+    p.bits = bits;
+    p.beta = 8;
+    p.slices = split::residue_moduli(bits, K);
+    p.chunks = (K + split::kChunkK - 1) / split::kChunkK;
+    return p;
+}
+
+// First GEMM in residue form.  Its certificate (every H entry within the FP64 bound of its dot
+// product) needs 53 - log2(W + 64) + 6 bits as the digits do; the moduli that holds are then
+// filled: the fraction bits that the same number of moduli still holds, at most 52 (beyond
+// that the FP64 output's own rounding is all that is left).  At W = 3072: 49 bits, 13 moduli.
+SplitParams residue_params1(const PairLayout& L) {
+    int bits = (int)std::ceil(53.0 - std::log2((double)L.W + 64.0) + 6.0);
+    bits = std::max(46, std::min(52, bits));
+    if (const char* b1 = getenv("GAINLS_GEMM1_BITS"))
+        return residue_params(std::max(40, std::min(split::kResMaxBits, atoi(b1))), L.W);
+    SplitParams p = residue_params(bits, L.W);
+    while (p.slices && bits < 52 && split::residue_moduli(bits + 1, L.W) == p.slices) p = residue_params(++bits, L.W);
+    return p;
+}
+
+// Second GEMM in residue form: 48 bits, as the digits keep, with no product dropped.
+SplitParams residue_params2(int K2) { return residue_params(48, K2); }
+
+// The residue form serves runs that leave the digit configuration open.
+bool residues_wanted(const gain_split_opts* o) { return !(o && (o->beta || o->slices || o->kchunks)); }
+
 bool digits_supported(const SplitParams& p1, const SplitParams& p2) {
+    if (p1.bits || p2.bits) return p1.bits && p2.bits && p1.slices && p2.slices;
     return !(p1.slices * p1.beta > 62 || p2.slices * p2.beta > 62 || p1.slices > split::MAX_SLICES ||
              p2.slices > split::MAX_SLICES || p1.beta < 2 || p1.beta > 8 || p2.beta < 2 || p2.beta > 8 ||
              2 * (p2.slices - 1) * p2.beta > 126 || 2 * (p1.slices - 1) * p1.beta > 126);
+}
+
+// Columns [n0, n1) of a GEMM that share their inner range (k-blocks [a_k0 / BK, + nkb) of A).
+struct ColumnRange {
+    int n0, n1, a_k0, nkb;
+};
+
+// Tiles of `rows` output rows over the column ranges, column by column: 256 columns wide on CTA
+// pairs (where a range has them), 128 otherwise.
+void residue_tiles(const std::vector<ColumnRange>& cols, int rows, int mstep, bool wide, std::vector<split::ResTile>& out) {
+    for (const ColumnRange& c : cols)
+        for (int n = c.n0; n < c.n1;) {
+            const int nc = wide && c.n1 - n >= 256 ? 256 : 128;
+            for (int m0 = 0; m0 < rows; m0 += mstep) {
+                split::ResTile t;
+                memset(&t, 0, sizeof t);
+                t.m0 = m0;
+                t.n0 = n;
+                t.a_k0 = c.a_k0;
+                t.nkb = c.nkb;
+                t.ncols = nc;
+                out.push_back(t);
+            }
+            n += nc;
+        }
+}
+
+// 256-column tiles where they still give every unit several (tile, modulus) items; smaller
+// problems take 128-column tiles, twice as many items.
+bool residue_wide(const std::vector<ColumnRange>& cols, int row_tiles, int nmod, int units) {
+    long w = 0;
+    for (const ColumnRange& c : cols) w += (c.n1 - c.n0 + 255) / 256;
+    return w * row_tiles * nmod >= 4L * units;
+}
+
+// Output rows per launch of a residue GEMM and its reconstruction: the residues of one such
+// panel (2 bytes per modulus and output) are the workspace, and its rows' A planes stay in L2
+// across the columns.
+int residue_panel(int mstep) { return kRowGroup * mstep; }
+
+// Panel by panel: the residue GEMM over `parts` (column ranges; before part p > 0 the stream
+// waits for `waits[p]`), then the reconstruction of all columns from `crt` (res, plane, row0
+// and rows are set here).  Returns the MMA flops through *flops.
+gain_status residue_gemm(gain_engine e, const CUtensorMap& tmA, const CUtensorMap& tmB,
+                         const std::vector<std::vector<ColumnRange>>& parts, const cudaEvent_t* waits, int B, int Bpad,
+                         bool pair, split::CrtArgs crt, DevArray<split::ResTile>& d_tiles, cudaEvent_t ev_done,
+                         double* flops) {
+    cudaStream_t st = e->st;
+    const int mstep = pair ? 2 * split::BM : split::BM, panel = residue_panel(mstep);
+    const int units = pair ? e->num_sms / 2 : e->num_sms;
+    std::vector<split::ResTile> all;
+    struct Span { int first, count; };
+    std::vector<std::array<Span, 2>> spans(parts.size());   // tiles of a full panel and of the last one
+    const int rows0 = std::min(Bpad, panel), rows1 = Bpad % panel;
+    double f = 0.0;
+    for (size_t p = 0; p < parts.size(); ++p) {
+        const bool wide = pair && residue_wide(parts[p], rows0 / mstep, crt.nmod, units);
+        const int a0 = (int)all.size();
+        residue_tiles(parts[p], rows0, mstep, wide, all);
+        const int a1 = (int)all.size();
+        spans[p][0] = spans[p][1] = {a0, a1 - a0};
+        if (Bpad > panel && rows1) {
+            residue_tiles(parts[p], rows1, mstep, wide, all);
+            spans[p][1] = {a1, (int)all.size() - a1};
+        }
+        for (const ColumnRange& c : parts[p]) f += 2.0 * Bpad * (c.n1 - c.n0) * (double)c.nkb * split::BK * crt.nmod;
+    }
+    if (flops) *flops += f;
+    if (!all.empty()) GAIN_TRY(d_tiles.upload(all));
+    split::ResGemmArgs g;
+    memset(&g, 0, sizeof g);
+    g.nmod = crt.nmod;
+    g.res = e->res.p;
+    g.ldr = crt.ldr;
+    g.plane = (long)rows0 * crt.ldr;
+    g.err = e->err.p;
+    for (int m0 = 0; m0 < Bpad; m0 += panel) {
+        const bool last = m0 + panel >= Bpad;
+        g.m_base = m0;
+        for (size_t p = 0; p < parts.size(); ++p) {
+            const Span& sp = spans[p][last && m0 > 0 && rows1 ? 1 : 0];
+            if (p > 0 && m0 == 0 && waits) GAIN_CUDA(cudaStreamWaitEvent(st, waits[p], 0));
+            if (!sp.count) continue;
+            g.tiles = d_tiles.p + sp.first;
+            g.ntiles = sp.count;
+            GAIN_CUDA(split::launch_residue_gemm(tmA, tmB, g, e->num_sms, st, pair));
+            ++e->launches;
+        }
+        if (last && ev_done) GAIN_CUDA(cudaEventRecord(ev_done, st));
+        crt.res = e->res.p;
+        crt.plane = g.plane;
+        crt.row0 = m0;
+        crt.rows = std::min(panel, B - m0);
+        if (crt.rows > 0) {
+            GAIN_CUDA(split::launch_crt(crt, st));
+            ++e->launches;
+        }
+    }
+    return GAIN_OK;
 }
 
 gain_status run_split(gain_engine e, const gain_pair_job* j, int dI, int dF, const gain_split_opts* opts,
@@ -1159,23 +1308,47 @@ gain_status run_split(gain_engine e, const gain_pair_job* j, int dI, int dF, con
     // through ||dH||_2 ||u||_2; every entry must certify FP64-grade), see gemm1_params.
     // Second GEMM: 48 bits (8-bit digits in up to MAX_CHUNKS chunks, else 7 x 7 bits);
     // options (beta, slices, kchunks) apply to it.
-    const SplitParams p1x = gemm1_params(L, opts);
+    // Both GEMMs take the residue form (residue.h: 13 products each at these precisions, against
+    // 28 and 21 digit products) unless the options name a digit configuration or the device
+    // cannot hold its planes (26 bytes per operand entry, the digits' 12 to 16).  Residues
+    // against digits on GB300: 7.8 / 13.5 ms at 2000 x 12 000 of 11 000 x 12 000 functions, 0.27 /
+    // 0.40 ms at 550 x 1200, 0.17 / 0.33 ms at 50 x 600; errors against FP64 1.8e-14 / 6.3e-14.
     const int K2 = L.general ? L.ntpad : L.fpad;   // inner dimension of the second GEMM
-    const SplitParams p2 = choose_params(K2, opts, 48, 8);
+    const int B = j->nlower;
+    const char* pair_env = getenv("GAINLS_GEMM_PAIR");
+    // CTA pairs whenever the lower states fill more than one 128-row block; GAINLS_GEMM_PAIR=0
+    // keeps single-CTA tiles
+    const bool pair = B > split::BM && !(pair_env && pair_env[0] == '0');
+    const int mstep = pair ? 2 * split::BM : split::BM;
+    const int Bpad = round_up(B, mstep);
+    const int Nu = j->nupper, Nupad = round_up(Nu, split::BN);
+    SplitParams p1x, p2;
+    bool res = residues_wanted(opts);
+    if (res) {
+        p1x = residue_params1(L);
+        p2 = residue_params2(K2);
+        res = digits_supported(p1x, p2);
+        const size_t panel = (size_t)std::min(Bpad, residue_panel(mstep));
+        if (res && (e->Vdig.alloc((size_t)p1x.slices * Bpad * L.kpadI) || e->Hdig.alloc((size_t)p2.slices * Bpad * K2) ||
+                    e->Udig.alloc((size_t)p2.slices * Nupad * K2) || L.bandDig.alloc((size_t)p1x.slices * L.fpad * L.W) ||
+                    e->res.alloc(std::max(panel * L.fpad * p1x.slices, panel * Nupad * p2.slices)))) {
+            (void)cudaGetLastError();
+            clear_error();
+            e->res.release();
+            L.dig = {};
+            res = false;
+        }
+    }
+    if (!res) {
+        p1x = gemm1_params(L, opts);
+        p2 = choose_params(K2, opts, 48, 8);
+    }
     if (!digits_supported(p1x, p2)) return set_error(GAIN_ERR_INVALID_ARG, "unsupported digit configuration");
 
     // band digits (cached per digit configuration)
     auto band_digits = [&]() -> gain_status { return layout_band_digits(e, L, p1x, st); };
     GAIN_TRY(band_digits());
 
-    // CTA pairs (256 x 128 tiles) whenever the lower states fill more than one 128-row block;
-    // GAINLS_GEMM_PAIR=0 keeps single-CTA tiles
-    const int B = j->nlower;
-    const char* pair_env = getenv("GAINLS_GEMM_PAIR");
-    const bool pair = B > split::BM && !(pair_env && pair_env[0] == '0');
-    const int mstep = pair ? 2 * split::BM : split::BM;
-    const int Bpad = round_up(B, mstep);
-    const int Nu = j->nupper, Nupad = round_up(Nu, split::BN);
     // While the upper vectors are still arriving in two parts, the upper side runs in two
     // halves: the first half's digits and amplitude GEMM start when the first part lands.
     int Nu2 = 0;
@@ -1216,25 +1389,30 @@ gain_status run_split(gain_engine e, const gain_pair_job* j, int dI, int dF, con
     const size_t hdig = (size_t)p2.slices * Bpad * K2;
     const size_t udig = (size_t)p2.slices * Nupad * K2;
     GAIN_TRY(e->Vdig.alloc(vdig));
-    GAIN_TRY(e->Vst.alloc(Bpad, p1x.chunks, false));
+    GAIN_TRY(e->Vst.alloc(Bpad, p1x.stat_chunks(), false));
     GAIN_TRY(e->Hdig.alloc(hdig));
-    GAIN_TRY(e->Hst.alloc(Bpad, p2.chunks, true));
+    GAIN_TRY(e->Hst.alloc(Bpad, p2.stat_chunks(), true));
     GAIN_TRY(e->Udig.alloc(udig));
-    GAIN_TRY(e->Ust.alloc(Nupad, p2.chunks, false));
+    GAIN_TRY(e->Ust.alloc(Nupad, p2.stat_chunks(), false));
+    if (res) {   // the residue slicing writes whole rows, and padding rows reach no output that is read
+        e->zkey_V.clear();
+        e->zkey_H.clear();
+        e->zkey_U.clear();
+    }
     const std::vector<long> kV = {lkey, p1x.slices, p1x.beta, p1x.chunks, B, Bpad, (long)(uintptr_t)e->Vdig.p};
     const std::vector<long> kH = {lkey, p2.slices, p2.chunks, B, Bpad, (long)(uintptr_t)e->Hdig.p};
     const std::vector<long> kU = {lkey, p2.slices, p2.chunks, Nu, Nupad, (long)(uintptr_t)e->Udig.p};
-    if (e->zkey_V != kV) {
+    if (!res && e->zkey_V != kV) {
         GAIN_TRY(e->Vdig.zero(st, vdig));
         GAIN_TRY(e->Vst.zero(st, Bpad, p1x.chunks, false));
         e->zkey_V = kV;
     }
-    if (e->zkey_H != kH) {
+    if (!res && e->zkey_H != kH) {
         GAIN_TRY(e->Hdig.zero(st, hdig));
         GAIN_TRY(e->Hst.zero(st, Bpad, p2.chunks, true));
         e->zkey_H = kH;
     }
-    if (e->zkey_U != kU) {
+    if (!res && e->zkey_U != kU) {
         GAIN_TRY(e->Udig.zero(st, udig));
         GAIN_TRY(e->Ust.zero(st, Nupad, p2.chunks, false));
         e->zkey_U = kU;
@@ -1279,9 +1457,10 @@ gain_status run_split(gain_engine e, const gain_pair_job* j, int dI, int dF, con
         return set_error(GAIN_ERR_CUDA, "cuTensorMapEncodeTiled failed (lower digits)");
 
     // ---- GEMM 1: H = V M (one pass per dipole piece)
-    const int fuse1 = gemm1_fuse(L, p1x);
-    const std::vector<split::Prod> pr1 = make_prods(p1x, fuse1);
-    GAIN_TRY(e->prods1.upload(pr1));
+    const int fuse1 = res ? 1 : gemm1_fuse(L, p1x);
+    const std::vector<split::Prod> pr1 = res ? std::vector<split::Prod>() : make_prods(p1x, fuse1);
+    if (!res) GAIN_TRY(e->prods1.upload(pr1));
+    double res_flops = 0.0;
     GAIN_TRY(e->H.alloc((size_t)Bpad * L.fpad));
     GAIN_TRY(e->rowerr.alloc(Bpad));
     GAIN_TRY(e->rowerr.zero(st, Bpad));
@@ -1304,12 +1483,13 @@ gain_status run_split(gain_engine e, const gain_pair_job* j, int dI, int dF, con
             GAIN_TRY(load_piece(e, piece));
             GAIN_TRY(launch_layout_band(e, j));
             L.dip_version = e->dip_version;
-            L.beta1 = 0;
+            L.dig = {};
             GAIN_TRY(band_digits());
             GAIN_CUDA(cudaMemsetAsync(e->counters.p, 0, sizeof(unsigned int), st));
         }
         if (npieces > 1) GAIN_CUDA(cudaMemsetAsync(e->H.p, 0, sizeof(double) * (size_t)Bpad * L.fpad, st));
         t1.clear();
+        std::vector<ColumnRange> cols1;
         for (auto& fb : L.fblocks)
             for (int n0 = fb.first; n0 < fb.second; n0 += split::BN) {
                 if (npieces > 1) {   // only column tiles holding an upper function of this piece
@@ -1325,6 +1505,11 @@ gain_status run_split(gain_engine e, const gain_pair_job* j, int dI, int dF, con
                     }
                     if (!any) continue;
                 }
+                if (res) {   // consecutive column blocks of one upper K block share their band
+                    if (!cols1.empty() && cols1.back().n1 == n0 && n0 > fb.first) cols1.back().n1 = n0 + split::BN;
+                    else cols1.push_back({n0, n0 + split::BN, L.band_k0[n0], L.band_len[n0] / split::BK});
+                    continue;
+                }
                 for (int m0 = 0; m0 < Bpad; m0 += mstep) {
                     split::Tile t;
                     memset(&t, 0, sizeof t);
@@ -1337,7 +1522,7 @@ gain_status run_split(gain_engine e, const gain_pair_job* j, int dI, int dF, con
                 }
             }
         row_grouped(t1, mstep);
-        {   // band tiles of the edge K blocks are shorter: dealt in list order to the unit that
+        if (!res) {   // band tiles of the edge K blocks are shorter: dealt in list order to the unit that
             // frees up first, no unit runs a tile more than the rest (a static round robin of
             // the list left the last units up to two thirds of a tile behind)
             const double per_kb = (double)pr1.size() / p1x.chunks;
@@ -1345,7 +1530,7 @@ gain_status run_split(gain_engine e, const gain_pair_job* j, int dI, int dF, con
             for (size_t i = 0; i < t1.size(); ++i) c1[i] = t1[i].nkb * per_kb + 2.0 * (double)pr1.size();
             t1 = list_schedule(t1, c1, pair ? e->num_sms / 2 : e->num_sms);
         }
-        GAIN_TRY(e->tiles1.upload(t1));
+        if (!res) GAIN_TRY(e->tiles1.upload(t1));
         split::GemmArgs g1;
         memset(&g1, 0, sizeof g1);
         g1.tiles = e->tiles1.p;
@@ -1372,19 +1557,48 @@ gain_status run_split(gain_engine e, const gain_pair_job* j, int dI, int dF, con
         g1.err = e->err.p;
         g1.fuse = fuse1;
         if (piece == 0) GAIN_CUDA(cudaEventRecord(e->ev[2], st));
-        if (!t1.empty()) {
-            GAIN_CUDA(split::launch_gemm(tmV, pair ? L.tmBandPair : L.tmBand, g1, e->num_sms, st, pair));
-            ++e->launches;
+        if (res) {
+            split::CrtArgs c1;
+            memset(&c1, 0, sizeof c1);
+            c1.ldr = L.fpad;
+            c1.nmod = p1x.slices;
+            c1.bits = p1x.bits;
+            c1.cols = c1.cols_valid = L.fpad;
+            c1.A = g1.A;
+            c1.B = g1.B;
+            c1.out = g1.out;
+            c1.ldo = g1.ldo;
+            c1.c_f64 = g1.c_f64;
+            c1.tol = g1.tol;
+            c1.flag_mode = g1.flag_mode;
+            c1.rowerr2 = g1.rowerr2;
+            c1.flags = g1.flags;
+            c1.nflags = g1.nflags;
+            c1.max_flags = max_flags;
+            split::crt_constants(&c1);
+            // columns outside the piece are not computed: their residues are zero
+            if (npieces > 1)
+                GAIN_CUDA(cudaMemsetAsync(e->res.p, 0,
+                                          sizeof(uint16_t) * (size_t)std::min(Bpad, residue_panel(mstep)) * L.fpad *
+                                              p1x.slices, st));
+            GAIN_TRY(residue_gemm(e, tmV, L.tmBandPair, {cols1}, nullptr, B, Bpad, pair, c1, e->rtiles1,
+                                  piece == npieces - 1 ? e->ev[3] : nullptr, &res_flops));
+        } else {
+            if (!t1.empty()) {
+                GAIN_CUDA(split::launch_gemm(tmV, pair ? L.tmBandPair : L.tmBand, g1, e->num_sms, st, pair));
+                ++e->launches;
+            }
+            if (piece == npieces - 1) GAIN_CUDA(cudaEventRecord(e->ev[3], st));
         }
-        if (piece == npieces - 1) GAIN_CUDA(cudaEventRecord(e->ev[3], st));
         if (piece == 0) {
             // ---- upper vectors -> digits on the low-priority second stream (rows [r0, r1))
             auto slice_upper = [&](int r0, int r1) -> gain_status {
                 if (L.general)   // symmetric functions in their own order
                     return slice(e, EF.d.p, EF.nsize, e->d_upper.p + r0, r1 - r0, L.nsymF, nullptr, nullptr, K2, Nupad,
-                                 e->Udig.p, p2, e->Ust, false, nullptr, nullptr, e->st2, nullptr, 0, r0);
+                                 e->Udig.p, p2.as_b(), e->Ust, false, nullptr, nullptr, e->st2, nullptr, 0, r0);
                 return slice(e, EF.d.p, EF.nsize, e->d_upper.p + r0, r1 - r0, EF.nsize, L.d_colposF.p, &L.colposF,
-                             L.fpad, Nupad, e->Udig.p, p2, e->Ust, false, nullptr, nullptr, e->st2, L.d_f_sym.p, 0, r0);
+                             L.fpad, Nupad, e->Udig.p, p2.as_b(), e->Ust, false, nullptr, nullptr, e->st2, L.d_f_sym.p,
+                             0, r0);
             };
             GAIN_CUDA(cudaStreamWaitEvent(e->st2, e->ev[6], 0));
             if (Nu2 > 0) {
@@ -1440,12 +1654,12 @@ gain_status run_split(gain_engine e, const gain_pair_job* j, int dI, int dF, con
     // the upper digits the (first) amplitude GEMM reads
     GAIN_CUDA(cudaStreamWaitEvent(st, Nu2 > 0 ? e->ev[9] : e->ev[7], 0));
     if (!split::make_digit_map(&tmH, e->Hdig.p, K2, Bpad, p2.slices) ||
-        !split::make_digit_map(&tmU, e->Udig.p, K2, Nupad, p2.slices, pair ? split::BN / 2 : split::BM))
+        !split::make_digit_map(&tmU, e->Udig.p, K2, Nupad, p2.slices, pair || res ? split::BN / 2 : split::BM))
         return set_error(GAIN_ERR_CUDA, "cuTensorMapEncodeTiled failed (second GEMM digits)");
 
     // ---- GEMM 2: amp = H U^T
     std::vector<split::Tile> t2;
-    for (int n0 = 0; n0 < Nupad; n0 += split::BN)
+    for (int n0 = 0; n0 < Nupad && !res; n0 += split::BN)
         for (int m0 = 0; m0 < Bpad; m0 += mstep) {
             split::Tile t;
             memset(&t, 0, sizeof t);
@@ -1457,9 +1671,11 @@ gain_status run_split(gain_engine e, const gain_pair_job* j, int dI, int dF, con
             t2.push_back(t);
         }
     row_grouped(t2, mstep, [&](const split::Tile& t) { return Nu2 > 0 && t.n0 >= Nu2 ? 1 : 0; });
-    const std::vector<split::Prod> pr2 = make_prods(p2);
-    GAIN_TRY(e->tiles2.upload(t2));
-    GAIN_TRY(e->prods2.upload(pr2));
+    const std::vector<split::Prod> pr2 = res ? std::vector<split::Prod>() : make_prods(p2);
+    if (!res) {
+        GAIN_TRY(e->tiles2.upload(t2));
+        GAIN_TRY(e->prods2.upload(pr2));
+    }
     GAIN_TRY(e->amp.alloc((size_t)Bpad * Nupad));
     GAIN_TRY(e->ampbnd.alloc((size_t)Bpad * Nupad));
     split::GemmArgs g2;
@@ -1490,7 +1706,34 @@ gain_status run_split(gain_engine e, const gain_pair_job* j, int dI, int dF, con
     g2.bnd = e->ampbnd.p;
     g2.ldb = Nupad;
     GAIN_CUDA(cudaEventRecord(e->ev[4], st));
-    if (Nu2 > 0) {
+    if (res) {
+        split::CrtArgs c2;
+        memset(&c2, 0, sizeof c2);
+        c2.ldr = Nupad;
+        c2.nmod = p2.slices;
+        c2.bits = p2.bits;
+        c2.cols = Nupad;
+        c2.cols_valid = Nu;
+        c2.A = g2.A;
+        c2.B = g2.B;
+        c2.out = g2.out;
+        c2.ldo = g2.ldo;
+        c2.bnd = g2.bnd;
+        c2.ldb = g2.ldb;
+        c2.c_f64 = g2.c_f64;
+        c2.tol = g2.tol;
+        c2.flag_mode = g2.flag_mode;
+        c2.absmax = g2.absmax;
+        c2.flags = g2.flags;
+        c2.nflags = g2.nflags;
+        c2.max_flags = max_flags;
+        split::crt_constants(&c2);
+        std::vector<std::vector<ColumnRange>> parts;
+        if (Nu2 > 0) parts = {{{0, Nu2, 0, K2 / split::BK}}, {{Nu2, Nupad, 0, K2 / split::BK}}};
+        else parts = {{{0, Nupad, 0, K2 / split::BK}}};
+        const cudaEvent_t waits[2] = {nullptr, e->ev[7]};
+        GAIN_TRY(residue_gemm(e, tmH, tmU, parts, waits, B, Bpad, pair, c2, e->rtiles2, e->ev[5], &res_flops));
+    } else if (Nu2 > 0) {
         // tiles are upper-block-major: those of the first half (n0 < Nu2) come first
         int n1 = 0;
         while (n1 < (int)t2.size() && t2[n1].n0 < Nu2) ++n1;
@@ -1506,7 +1749,7 @@ gain_status run_split(gain_engine e, const gain_pair_job* j, int dI, int dF, con
         GAIN_CUDA(split::launch_gemm(tmH, tmU, g2, e->num_sms, st, pair));
         ++e->launches;
     }
-    GAIN_CUDA(cudaEventRecord(e->ev[5], st));
+    if (!res) GAIN_CUDA(cudaEventRecord(e->ev[5], st));
     split::RefineAmpArgs ra;
     ra.flags = e->flags2.p;
     ra.nflags = e->counters.p + 1;
@@ -1578,10 +1821,10 @@ gain_status run_split(gain_engine e, const gain_pair_job* j, int dI, int dF, con
         stats->beta2 = p2.beta;
         stats->slices2 = p2.slices;
         stats->chunks2 = p2.chunks;
-        stats->products1 = (int)pr1.size();
-        stats->products2 = (int)pr2.size();
+        stats->products1 = res ? p1x.slices : (int)pr1.size();
+        stats->products2 = res ? p2.slices : (int)pr2.size();
         stats->kernel_launches = e->launches - launches0;
-        double f = 0;
+        double f = res_flops;
         // a tile covers mstep rows (256 for CTA pairs); t1 holds the last piece's tiles
         for (auto& t : t1) f += 2.0 * mstep * split::BN * split::BK * (double)t.nkb * pr1.size() / p1x.chunks;
         for (auto& t : t2) f += 2.0 * mstep * split::BN * split::BK * (double)t.nkb * pr2.size() / p2.chunks;
@@ -3250,6 +3493,15 @@ struct gain_plan_s {
     int ntiles1 = 0, ntiles2 = 0, real1 = 0, real2 = 0;
     int s1max = 1, c1max = 1, s2max = 1, c2max = 1;
     double flops = 0.0;
+    // residue form (residue.h) of both grouped launches: operands and items, the reconstruction
+    // of every job's outputs, and the residues' workspace (both GEMMs use it in turn)
+    bool residues = false, residues_failed = false, residues_unsupported = false;
+    DevArray<split::ResGroup> rgroups1, rgroups2;
+    DevArray<split::ResTile> rtiles1, rtiles2;
+    DevArray<split::CrtArgs> crt1, crt2;
+    DevArray<int> crt1_offs, crt2_offs;
+    int crt1_blocks = 0, crt2_blocks = 0;
+    DevArray<uint16_t> res;
     // the plan's digit slicings, one launch per slicing kernel: the eigenvectors (before the
     // first GEMM) and H (before the second)
     struct SliceBatch {
@@ -3311,17 +3563,20 @@ gain_status plan_prepare_job(gain_plan P, PlanJob& J) {
     J.L = e->layouts.at(akey);
     PairLayout& L = *J.L;
     const gain_split_opts* opts = P->has_opts ? &P->opts : nullptr;
-    J.p1 = gemm1_params(L, opts);
     J.K2 = L.general ? L.ntpad : L.fpad;
+    J.p1 = P->residues ? residue_params1(L) : gemm1_params(L, opts);
     gain_split_opts o2 = P->has_opts ? P->opts : gain_split_opts{};
     if (J.beta2) {
         o2.beta = J.beta2;
         o2.slices = J.slices2;
         o2.kchunks = 0;
     }
-    J.p2 = choose_params(J.K2, &o2, 48, 8);
+    J.p2 = P->residues ? residue_params2(J.K2) : choose_params(J.K2, &o2, 48, 8);
     J.klass = k2_class(J.K2);
-    if (!digits_supported(J.p1, J.p2)) return set_error(GAIN_ERR_INVALID_ARG, "unsupported digit configuration");
+    if (!digits_supported(J.p1, J.p2)) {
+        P->residues_unsupported = P->residues;
+        return set_error(GAIN_ERR_INVALID_ARG, "unsupported digit configuration");
+    }
     GAIN_TRY(layout_band_digits(e, L, J.p1, st));
     const Basis& bI = e->bases[j->jindI];
     const Eig& EI = *e->eig[{j->jindI, j->gammaI}];
@@ -3348,8 +3603,7 @@ gain_status plan_prepare_job(gain_plan P, PlanJob& J) {
         if (Q.get() == &J) break;
         const PairLayout& QL = *Q->L;
         if (Q->job.jindF == j->jindF && Q->job.gammaF == j->gammaF && Q->upper == J.upper && Q->K2 == J.K2 &&
-            Q->p2.beta == J.p2.beta && Q->p2.slices == J.p2.slices && Q->p2.chunks == J.p2.chunks &&
-            QL.general == L.general && QL.colposF == L.colposF && QL.f_sym == L.f_sym && QL.nsymF == L.nsymF &&
+            Q->p2.same(J.p2) && QL.general == L.general && QL.colposF == L.colposF && QL.f_sym == L.f_sym && QL.nsymF == L.nsymF &&
             Q->uowner < 0) {
             J.uowner = (int)(&Q - &P->jobs[0]);
             break;
@@ -3364,8 +3618,7 @@ gain_status plan_prepare_job(gain_plan P, PlanJob& J) {
             if (Q.get() == &J) break;
             const PairLayout& QL = *Q->L;
             if (Q->job.jindI == j->jindI && Q->job.gammaI == j->gammaI && Q->lower == J.lower && Q->Bpad == J.Bpad &&
-                Q->p1.beta == J.p1.beta && Q->p1.slices == J.p1.slices && Q->p1.chunks == J.p1.chunks &&
-                !QL.general && QL.kpadI == L.kpadI && QL.colposI == L.colposI && QL.i_sym == L.i_sym &&
+                Q->p1.same(J.p1) && !QL.general && QL.kpadI == L.kpadI && QL.colposI == L.colposI && QL.i_sym == L.i_sym &&
                 Q->lowner < 0) {
                 J.lowner = (int)(&Q - &P->jobs[0]);
                 break;
@@ -3376,22 +3629,28 @@ gain_status plan_prepare_job(gain_plan P, PlanJob& J) {
     const size_t udig = J.uowner < 0 ? (size_t)J.p2.slices * J.Nupad * J.K2 : 0;
     if (J.lowner < 0) {
         GAIN_TRY(J.Vdig.alloc(vdig));
-        GAIN_TRY(J.Vdig.zero(st, vdig));
-        GAIN_TRY(J.Vst.alloc(J.Bpad, J.p1.chunks, false));
-        GAIN_TRY(J.Vst.zero(st, J.Bpad, J.p1.chunks, false));
+        GAIN_TRY(J.Vst.alloc(J.Bpad, J.p1.stat_chunks(), false));
+        if (!P->residues) {   // (residue planes and the statistics that are read are written whole)
+            GAIN_TRY(J.Vdig.zero(st, vdig));
+            GAIN_TRY(J.Vst.zero(st, J.Bpad, J.p1.chunks, false));
+        }
     } else {   // not this job's: release what an earlier preparation left
         J.Vdig.release();
         J.Vst = StatsDev();
     }
     GAIN_TRY(J.Hdig.alloc(hdig));
-    GAIN_TRY(J.Hdig.zero(st, hdig));
-    GAIN_TRY(J.Hst.alloc(J.Bpad, J.p2.chunks, true));
-    GAIN_TRY(J.Hst.zero(st, J.Bpad, J.p2.chunks, true));
+    GAIN_TRY(J.Hst.alloc(J.Bpad, J.p2.stat_chunks(), true));
+    if (!P->residues) {
+        GAIN_TRY(J.Hdig.zero(st, hdig));
+        GAIN_TRY(J.Hst.zero(st, J.Bpad, J.p2.chunks, true));
+    }
     if (J.uowner < 0) {
         GAIN_TRY(J.Udig.alloc(udig));
-        GAIN_TRY(J.Udig.zero(st, udig));
-        GAIN_TRY(J.Ust.alloc(J.Nupad, J.p2.chunks, false));
-        GAIN_TRY(J.Ust.zero(st, J.Nupad, J.p2.chunks, false));
+        GAIN_TRY(J.Ust.alloc(J.Nupad, J.p2.stat_chunks(), false));
+        if (!P->residues) {
+            GAIN_TRY(J.Udig.zero(st, udig));
+            GAIN_TRY(J.Ust.zero(st, J.Nupad, J.p2.chunks, false));
+        }
     } else {   // not this job's: release what an earlier preparation left
         J.Udig.release();
         J.Ust = StatsDev();
@@ -3411,16 +3670,23 @@ gain_status plan_prepare_job(gain_plan P, PlanJob& J) {
         GAIN_TRY(J.iota.upload(io));
         GAIN_TRY(J.Hsym.alloc((size_t)J.Bpad * J.K2));
     }
-    J.fuse1 = gemm1_fuse(L, J.p1);
-    const std::vector<split::Prod> pr1 = make_prods(J.p1, J.fuse1), pr2 = make_prods(J.p2);
-    GAIN_TRY(J.prods1.upload(pr1));
-    GAIN_TRY(J.prods2.upload(pr2));
-    J.nprods1 = (int)pr1.size();
-    J.nprods2 = (int)pr2.size();
+    if (P->residues) {
+        J.fuse1 = 1;
+        J.nprods1 = J.p1.slices;
+        J.nprods2 = J.p2.slices;
+    } else {
+        J.fuse1 = gemm1_fuse(L, J.p1);
+        const std::vector<split::Prod> pr1 = make_prods(J.p1, J.fuse1), pr2 = make_prods(J.p2);
+        GAIN_TRY(J.prods1.upload(pr1));
+        GAIN_TRY(J.prods2.upload(pr2));
+        J.nprods1 = (int)pr1.size();
+        J.nprods2 = (int)pr2.size();
+    }
     if ((J.lowner < 0 && !split::make_digit_map(&J.tmV, J.Vdig.p, L.kpadI, J.Bpad, J.p1.slices)) ||
         !split::make_digit_map(&J.tmH, J.Hdig.p, J.K2, J.Bpad, J.p2.slices) ||
         (J.uowner < 0 &&
-         !split::make_digit_map(&J.tmU, J.Udig.p, J.K2, J.Nupad, J.p2.slices, P->pair ? split::BN / 2 : split::BM)))
+         !split::make_digit_map(&J.tmU, J.Udig.p, J.K2, J.Nupad, J.p2.slices,
+                                P->pair || P->residues ? split::BN / 2 : split::BM)))
         return set_error(GAIN_ERR_CUDA, "cuTensorMapEncodeTiled failed (plan job digits)");
     J.vI = EI.d.p;
     J.vF = EF.d.p;
@@ -3468,7 +3734,7 @@ gain_status plan_build_slices(gain_plan P) {
                                     J.Vdig.p, J.p1, J.Vst, false, nullptr, nullptr, L.d_i_sym.p));
             if (J.uowner < 0)
                 s1.push_back(slice_args(EF.d.p, EF.nsize, J.d_upper.p, J.Nu, L.nsymF, nullptr, nullptr, J.K2, J.Nupad,
-                                        J.Udig.p, J.p2, J.Ust, false, nullptr, nullptr));
+                                        J.Udig.p, J.p2.as_b(), J.Ust, false, nullptr, nullptr));
         } else {
             if (J.lowner < 0)
                 s1.push_back(slice_args(EI.d.p, EI.nsize, J.d_lower.p, J.B, EI.nsize, L.d_colposI.p, &L.colposI,
@@ -3476,7 +3742,7 @@ gain_status plan_build_slices(gain_plan P) {
                                         L.d_i_sym.p));
             if (J.uowner < 0)
                 s1.push_back(slice_args(EF.d.p, EF.nsize, J.d_upper.p, J.Nu, EF.nsize, L.d_colposF.p, &L.colposF,
-                                        L.fpad, J.Nupad, J.Udig.p, J.p2, J.Ust, false, nullptr, nullptr,
+                                        L.fpad, J.Nupad, J.Udig.p, J.p2.as_b(), J.Ust, false, nullptr, nullptr,
                                         L.d_f_sym.p));
         }
         const PlanJob& JL = J.lowner < 0 ? J : *P->jobs[J.lowner];   // the lower digits' owner
@@ -3504,8 +3770,149 @@ gain_status plan_launch_slices(const std::vector<gain_plan_s::SliceBatch>& batch
     return GAIN_OK;
 }
 
+// The residue form of plan_build_groups: per job and GEMM an operand group, its (tile, modulus)
+// items and the reconstruction of its outputs.
+gain_status plan_build_residue_groups(gain_plan P) {
+    gain_engine e = P->e;
+    const int mstep = P->pair ? 2 * split::BM : split::BM;
+    P->units = P->pair ? e->num_sms / 2 : e->num_sms;
+    const int nj = (int)P->jobs.size();
+    const double tol = (P->has_opts && P->opts.tol > 0) ? P->opts.tol : 4.5e-9;
+    P->flops = 0.0;
+    std::vector<size_t> off(nj + 1, 0);   // each job's residues in the workspace
+    for (int q = 0; q < nj; ++q) {
+        const PlanJob& J = *P->jobs[q];
+        off[q + 1] = off[q] + (size_t)J.Bpad * std::max((size_t)J.L->fpad * J.p1.slices, (size_t)J.Nupad * J.p2.slices);
+    }
+    GAIN_TRY(P->res.alloc(off[nj]));
+    std::vector<split::ResGroup> g1(nj), g2(nj);
+    std::vector<split::CrtArgs> a1(nj), a2(nj);
+    std::vector<int> o1(nj + 1, 0), o2(nj + 1, 0);
+    std::vector<split::ResTile> t1, t2;
+    std::vector<double> c1, c2;
+    // items of one job in its launch's order: row group, modulus, column, row
+    auto items = [&](int q, const PlanJob& J, const std::vector<ColumnRange>& cols, int nmod,
+                     std::vector<split::ResTile>& out, std::vector<double>& cost) {
+        const int panel = residue_panel(mstep);
+        const bool wide = P->pair && residue_wide(cols, J.Bpad / mstep, nmod, P->units);
+        for (int m0 = 0; m0 < J.Bpad; m0 += panel) {
+            std::vector<split::ResTile> t;
+            residue_tiles(cols, std::min(panel, J.Bpad - m0), mstep, wide, t);
+            for (int i = 0; i < nmod; ++i)
+                for (split::ResTile x : t) {
+                    x.m0 += m0;
+                    x.group = q;
+                    x.mod = i;
+                    out.push_back(x);
+                    // an item's k-blocks (a 256-column MMA takes twice a 128-column one) and its
+                    // fixed part: the last drain and the residues' stores
+                    cost.push_back((x.nkb + 4.0) * (x.ncols / 128));
+                }
+        }
+        for (const ColumnRange& c : cols) P->flops += 2.0 * J.Bpad * (c.n1 - c.n0) * (double)c.nkb * split::BK * nmod;
+    };
+    auto crt = [&](const PlanJob& J, const SplitParams& p, int ldr, int cols_valid) {
+        split::CrtArgs a;
+        memset(&a, 0, sizeof a);
+        a.ldr = ldr;
+        a.plane = (long)J.Bpad * ldr;
+        a.nmod = p.slices;
+        a.bits = p.bits;
+        a.rows = J.B;
+        a.cols = ldr;
+        a.cols_valid = cols_valid;
+        a.ldo = ldr;
+        a.tol = (float)tol;
+        split::crt_constants(&a);
+        return a;
+    };
+    for (int q = 0; q < nj; ++q) {
+        PlanJob& J = *P->jobs[q];
+        PairLayout& L = *J.L;
+        PlanJob& JL = J.lowner < 0 ? J : *P->jobs[J.lowner];   // the lower planes' owner
+        PlanJob& JU = J.uowner < 0 ? J : *P->jobs[J.uowner];   // the upper planes' owner
+        memset(&g1[q], 0, sizeof g1[q]);
+        memset(&g2[q], 0, sizeof g2[q]);
+        g1[q].tmA = JL.tmV;
+        g1[q].tmB = L.tmBandPair;
+        g2[q].tmA = J.tmH;
+        g2[q].tmB = JU.tmU;
+        a1[q] = crt(J, J.p1, L.fpad, L.fpad);
+        a2[q] = crt(J, J.p2, J.Nupad, J.Nu);
+        for (auto g : {&g1[q], &g2[q]}) {
+            const split::CrtArgs& a = g == &g1[q] ? a1[q] : a2[q];
+            g->res = P->res.p + off[q];
+            g->plane = a.plane;
+            g->ldr = a.ldr;
+        }
+        a1[q].res = a2[q].res = P->res.p + off[q];
+        a1[q].A = JL.Vst.view(false);
+        a1[q].B = L.bandStats.view(false);
+        a1[q].out = J.H.p;
+        a1[q].c_f64 = (float)((double)(L.W + 64) * std::ldexp(1.0, -53) * 1.01);
+        a1[q].rowerr2 = J.rowerr.p;
+        a1[q].flag_mode = 2;
+        a1[q].flags = J.flags1.p;
+        a1[q].nflags = P->counters.p + 2 * q;
+        a1[q].max_flags = J.cap1;
+        a2[q].A = J.Hst.view(false);
+        a2[q].B = JU.Ust.view(false);
+        a2[q].out = J.amp.p;
+        a2[q].c_f64 = (float)((double)((L.general ? L.nsymF : L.nF) + 64) * std::ldexp(1.0, -53) * 1.01);
+        a2[q].absmax = P->ull.p + 4 * q + 2;
+        a2[q].flag_mode = 1;
+        a2[q].flags = J.flags2.p;
+        a2[q].nflags = P->counters.p + 2 * q + 1;
+        a2[q].max_flags = J.cap2;
+        a2[q].bnd = J.ampbnd.p;
+        a2[q].ldb = J.Nupad;
+        o1[q + 1] = o1[q] + split::crt_blocks(a1[q]);
+        o2[q + 1] = o2[q] + split::crt_blocks(a2[q]);
+        std::vector<ColumnRange> cols;
+        for (auto& fb : L.fblocks)
+            cols.push_back({fb.first, fb.second, L.band_k0[fb.first], L.band_len[fb.first] / split::BK});
+        items(q, J, cols, J.p1.slices, t1, c1);
+        items(q, J, {{0, J.Nupad, 0, J.K2 / split::BK}}, J.p2.slices, t2, c2);
+    }
+    P->real1 = (int)t1.size();
+    P->real2 = (int)t2.size();
+    const std::vector<split::ResTile> s1 = list_schedule(t1, c1, P->units), s2 = list_schedule(t2, c2, P->units);
+    P->ntiles1 = (int)s1.size();
+    P->ntiles2 = (int)s2.size();
+    P->crt1_blocks = o1[nj];
+    P->crt2_blocks = o2[nj];
+    GAIN_TRY(P->rgroups1.upload(g1));
+    GAIN_TRY(P->rgroups2.upload(g2));
+    GAIN_TRY(P->rtiles1.upload(s1));
+    GAIN_TRY(P->rtiles2.upload(s2));
+    GAIN_TRY(P->crt1.upload(a1));
+    GAIN_TRY(P->crt2.upload(a2));
+    GAIN_TRY(P->crt1_offs.upload(o1));
+    GAIN_TRY(P->crt2_offs.upload(o2));
+    return GAIN_OK;
+}
+
+// One grouped residue GEMM and the reconstruction of its outputs (between them: ev).
+gain_status plan_residue_gemm(gain_plan P, const split::ResGroup* groups, const split::ResTile* tiles, int ntiles,
+                              const split::CrtGroups& crt, cudaEvent_t ev0, cudaEvent_t ev1) {
+    cudaStream_t st = P->e->st;
+    split::ResGemmArgs g;
+    memset(&g, 0, sizeof g);
+    g.groups = groups;
+    g.tiles = tiles;
+    g.ntiles = ntiles;
+    g.nmod = 1;
+    g.err = P->err.p;
+    GAIN_CUDA(cudaEventRecordWithFlags(ev0, st, cudaEventRecordExternal));
+    GAIN_CUDA(split::launch_residue_gemm_grouped(g, P->units, st, P->pair));
+    GAIN_CUDA(cudaEventRecordWithFlags(ev1, st, cudaEventRecordExternal));
+    GAIN_CUDA(split::launch_crt_grouped(crt, st));
+    return GAIN_OK;
+}
+
 // Groups and schedules of both grouped launches.
 gain_status plan_build_groups(gain_plan P) {
+    if (P->residues) return plan_build_residue_groups(P);
     gain_engine e = P->e;
     const int mstep = P->pair ? 2 * split::BM : split::BM;
     P->units = P->pair ? e->num_sms / 2 : e->num_sms;
@@ -3686,9 +4093,14 @@ gain_status plan_enqueue(gain_plan P) {
     ga.groups = P->groups1.p;
     ga.tiles = P->tiles1.p;
     ga.ntiles = P->ntiles1;
-    GAIN_CUDA(cudaEventRecordWithFlags(P->ev[1], st, cudaEventRecordExternal));
-    GAIN_CUDA(split::launch_gemm_grouped(ga, P->units, P->s1max, P->c1max, st, P->pair));
-    GAIN_CUDA(cudaEventRecordWithFlags(P->ev[2], st, cudaEventRecordExternal));
+    if (P->residues) {
+        GAIN_TRY(plan_residue_gemm(P, P->rgroups1.p, P->rtiles1.p, P->ntiles1,
+                                   {P->crt1.p, P->crt1_offs.p, nj, P->crt1_blocks}, P->ev[1], P->ev[2]));
+    } else {
+        GAIN_CUDA(cudaEventRecordWithFlags(P->ev[1], st, cudaEventRecordExternal));
+        GAIN_CUDA(split::launch_gemm_grouped(ga, P->units, P->s1max, P->c1max, st, P->pair));
+        GAIN_CUDA(cudaEventRecordWithFlags(P->ev[2], st, cudaEventRecordExternal));
+    }
     // ---- stage 3: FP64 refinement of H, contraction (mixing expansions), digits of H
     GAIN_TRY(fork());
     for (int q = 0; q < nj; ++q) {
@@ -3729,9 +4141,14 @@ gain_status plan_enqueue(gain_plan P) {
     ga.groups = P->groups2.p;
     ga.tiles = P->tiles2.p;
     ga.ntiles = P->ntiles2;
-    GAIN_CUDA(cudaEventRecordWithFlags(P->ev[3], st, cudaEventRecordExternal));
-    GAIN_CUDA(split::launch_gemm_grouped(ga, P->units, P->s2max, P->c2max, st, P->pair));
-    GAIN_CUDA(cudaEventRecordWithFlags(P->ev[4], st, cudaEventRecordExternal));
+    if (P->residues) {
+        GAIN_TRY(plan_residue_gemm(P, P->rgroups2.p, P->rtiles2.p, P->ntiles2,
+                                   {P->crt2.p, P->crt2_offs.p, nj, P->crt2_blocks}, P->ev[3], P->ev[4]));
+    } else {
+        GAIN_CUDA(cudaEventRecordWithFlags(P->ev[3], st, cudaEventRecordExternal));
+        GAIN_CUDA(split::launch_gemm_grouped(ga, P->units, P->s2max, P->c2max, st, P->pair));
+        GAIN_CUDA(cudaEventRecordWithFlags(P->ev[4], st, cudaEventRecordExternal));
+    }
     // ---- stage 5: FP64 refinement of the amplitudes
     GAIN_TRY(fork());
     for (int q = 0; q < nj; ++q) {
@@ -3777,12 +4194,33 @@ gain_status plan_build(gain_plan P) {
     gain_engine e = P->e;
     P->drop_graph();
     const int nj = (int)P->jobs.size();
-    for (auto& J : P->jobs) GAIN_TRY(plan_prepare_job(P, *J));
-    GAIN_TRY(P->counters.alloc(2 * nj));
-    GAIN_TRY(P->ull.alloc(4 * nj));
-    GAIN_TRY(P->err.alloc(1));
-    GAIN_TRY(plan_build_groups(P));
-    GAIN_TRY(plan_build_slices(P));
+    auto prepare = [&]() -> gain_status {
+        for (auto& J : P->jobs) GAIN_TRY(plan_prepare_job(P, *J));
+        GAIN_TRY(P->counters.alloc(2 * nj));
+        GAIN_TRY(P->ull.alloc(4 * nj));
+        GAIN_TRY(P->err.alloc(1));
+        GAIN_TRY(plan_build_groups(P));
+        return plan_build_slices(P);
+    };
+    // the residue form unless the options (or the autotuner) name digits, or its planes and
+    // residues do not fit the device
+    P->residues = !P->residues_failed && residues_wanted(P->has_opts ? &P->opts : nullptr);
+    for (auto& J : P->jobs) P->residues = P->residues && !J->beta2;
+    gain_status ps = prepare();
+    if (ps != GAIN_OK && P->residues && (ps == GAIN_ERR_OOM || P->residues_unsupported)) {
+        (void)cudaGetLastError();
+        P->residues_failed = true;
+        P->residues = false;
+        P->res.release();
+        for (auto& J : P->jobs) {   // what the residue planes took
+            J->Vdig.release();
+            J->Hdig.release();
+            J->Udig.release();
+        }
+        clear_error();
+        ps = prepare();
+    }
+    GAIN_TRY(ps);
     if (!P->rb) GAIN_CUDA(cudaMallocHost(&P->rb, 40 * (size_t)nj + 64));
     GAIN_CUDA(split::prepare_device());   // kernel attributes are set outside the capture
     GAIN_CUDA(cudaStreamSynchronize(e->st));
@@ -3830,7 +4268,7 @@ bool plan_current(gain_plan P) {
         if (iI == e->eig.end() || iF == e->eig.end()) return false;
         if (iI->second->d.p != J->vI || iF->second->d.p != J->vF || J->L->bandDig.p != J->band) return false;
         if (iI->second->nlevels != J->nlevI || iF->second->nlevels != J->nlevF) return false;
-        if (J->L->beta1 != J->p1.beta || J->L->s1 != J->p1.slices || J->L->c1 != J->p1.chunks) return false;
+        if (!J->L->digits_are(J->p1)) return false;
     }
     return true;
 }
@@ -3950,7 +4388,7 @@ gain_status plan_autotune(gain_plan P, TuneChoice* out) {
     }
     if (best >= 1e300) return set_error(GAIN_ERR_TOL_NOT_MET, "autotuner: no candidate configuration ran");
     bool present[4] = {false, false, false, false};
-    for (auto& J : P->jobs) present[k2_class(J->K2)] = true;
+    for (auto& J : P->jobs) present[k2_class(J->K2)] = !P->residues;   // the residue form leaves no digits to choose
     for (int k = 0; k < 4; ++k) {
         if (!present[k]) continue;
         TuneChoice c = best_c;

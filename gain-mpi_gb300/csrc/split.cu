@@ -7,6 +7,8 @@
 #include <cuda_bf16.h>
 
 #include "gain_internal.h"
+#include "residue.h"
+#include "tcgen05.cuh"
 
 namespace gain {
 namespace split {
@@ -31,197 +33,7 @@ constexpr uint32_t COLSTAT_BYTES = 5 * BN * 4;
 constexpr uint32_t GARGS_OFF = COLSTAT_OFF + COLSTAT_BYTES;
 constexpr uint32_t GARGS_BYTES = (sizeof(GemmArgs) + 15) / 16 * 16;
 constexpr uint32_t TMEM_COLS = 512;         // acc0 [0,128) acc1 [128,256) hi [256,384) lo [384,512)
-constexpr unsigned long long kWaitNs = 2000000000ull;   // 2 s per wait before giving up
 
-// ------------------------------------------------------------------- PTX wrappers
-__device__ __forceinline__ uint32_t smem_u32(const void* p) {
-    return (uint32_t)__cvta_generic_to_shared(p);
-}
-__device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
-}
-__device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes)
-                 : "memory");
-}
-__device__ __forceinline__ void mbar_arrive(uint32_t bar) {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
-}
-// Probe with a zero suspend-time hint: the caller loops (with its own time limit), and a
-// probe that does not offer to suspend costs the MMA-issuing thread less time per stage.
-__device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
-    uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}\n"
-        : "=r"(ok)
-        : "r"(bar), "r"(parity), "r"(0)
-        : "memory");
-    return ok != 0;
-}
-__device__ __forceinline__ unsigned long long globaltimer() {
-    unsigned long long t;
-    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-    return t;
-}
-// Bounded wait on a barrier phase.  Gives up when another role raised the CTA abort flag
-// (unless ignore_abort) or after kWaitNs, raising the flag and the device error word.
-__device__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag, int* err,
-                          int code, bool ignore_abort = false, unsigned long long limit_ns = kWaitNs) {
-    if (mbar_try_wait(bar, parity)) return true;
-    const unsigned long long t0 = globaltimer();
-    for (uint32_t it = 1;; ++it) {
-        if (mbar_try_wait(bar, parity)) return true;
-        if ((it & 127u) == 0) {
-            if (!ignore_abort && *abort_flag) return false;
-            if (globaltimer() - t0 > limit_ns) {
-                *abort_flag = 1;
-                atomicCAS(err, 0, code);
-                return false;
-            }
-        }
-    }
-}
-__device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* map, uint32_t bar,
-                                            int c0, int c1, int c2) {
-    asm volatile(
-        "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes"
-        " [%0], [%1, {%3, %4, %5}], [%2];" ::"r"(dst),
-        "l"((unsigned long long)map), "r"(bar), "r"(c0), "r"(c1), "r"(c2)
-        : "memory");
-}
-// ---- CTA-pair (cta_group::2) forms: the two CTAs of a cluster share each MMA (M = 256)
-__device__ __forceinline__ uint32_t cluster_rank() {
-    uint32_t r;
-    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-    return r;
-}
-__device__ __forceinline__ uint32_t cluster_map(uint32_t addr, uint32_t rank) {   // peer's address
-    uint32_t r;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
-    return r;
-}
-__device__ __forceinline__ void cluster_sync_all() {
-    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-__device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar_cluster) {
-    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar_cluster) : "memory");
-}
-__device__ __forceinline__ void tma_load_3d_pair(uint32_t dst, const CUtensorMap* map, uint32_t bar_cluster, int c0,
-                                                 int c1, int c2) {
-    asm volatile(
-        "cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes"
-        " [%0], [%1, {%3, %4, %5}], [%2];" ::"r"(dst),
-        "l"((unsigned long long)map), "r"(bar_cluster), "r"(c0), "r"(c1), "r"(c2)
-        : "memory");
-}
-__device__ __forceinline__ void tmem_alloc_pair(uint32_t dst_smem, uint32_t ncols) {
-    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(dst_smem), "r"(ncols)
-                 : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
-}
-__device__ __forceinline__ void tmem_dealloc_pair(uint32_t taddr, uint32_t ncols) {
-    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
-}
-__device__ __forceinline__ void mma_bf16_pair(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
-                                              uint32_t accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(d_tmem),
-        "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-        : "memory");
-}
-// arrive on the barrier at this offset in each CTA of mask (bit r = cluster rank r)
-__device__ __forceinline__ void mma_commit_pair(uint32_t bar, uint16_t mask) {
-    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
-                 ::"r"(bar), "h"(mask)
-                 : "memory");
-}
-__device__ __forceinline__ void tmem_alloc(uint32_t dst_smem, uint32_t ncols) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(dst_smem),
-                 "r"(ncols)
-                 : "memory");
-}
-__device__ __forceinline__ void tmem_relinquish() {
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-}
-__device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t ncols) {
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols)
-                 : "memory");
-}
-__device__ __forceinline__ void tc_fence_before() {
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-}
-__device__ __forceinline__ void tc_fence_after() {
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-}
-__device__ __forceinline__ void mma_bf16(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc,
-                                         uint32_t idesc, uint32_t accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(d_tmem),
-        "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-        : "memory");
-}
-__device__ __forceinline__ void mma_commit(uint32_t bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar)
-                 : "memory");
-}
-__device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
-__device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
-
-#define GAIN_R8(b) "=r"(r[b + 0]), "=r"(r[b + 1]), "=r"(r[b + 2]), "=r"(r[b + 3]), \
-                   "=r"(r[b + 4]), "=r"(r[b + 5]), "=r"(r[b + 6]), "=r"(r[b + 7])
-#define GAIN_W8(b) "r"(r[b + 0]), "r"(r[b + 1]), "r"(r[b + 2]), "r"(r[b + 3]), \
-                   "r"(r[b + 4]), "r"(r[b + 5]), "r"(r[b + 6]), "r"(r[b + 7])
-
-// 32 consecutive 32-bit TMEM columns of this thread's lane
-__device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-        "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
-        "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
-        : GAIN_R8(0), GAIN_R8(8), GAIN_R8(16), GAIN_R8(24)
-        : "r"(taddr));
-}
-__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
-        "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
-        : GAIN_R8(0), GAIN_R8(8)
-        : "r"(taddr));
-}
-__device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&r)[32]) {
-    asm volatile(
-        "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
-        "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, "
-        "%17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31, %32};" ::"r"(taddr),
-        GAIN_W8(0), GAIN_W8(8), GAIN_W8(16), GAIN_W8(24)
-        : "memory");
-}
-__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16]) {
-    asm volatile(
-        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], "
-        "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};" ::"r"(taddr),
-        GAIN_W8(0), GAIN_W8(8)
-        : "memory");
-}
-
-// Shared-memory matrix descriptor of a K-major tile written by TMA with 128-byte swizzle:
-// rows of 128 bytes, 8-row groups 1024 bytes apart (SBO), base 1024-byte aligned.
-__device__ __forceinline__ uint64_t smem_desc(uint32_t addr) {
-    uint64_t d = 0;
-    d |= (uint64_t)((addr & 0x3FFFFu) >> 4);       // start address
-    d |= (uint64_t)1 << 16;                        // leading byte offset (unused for SW128 K-major)
-    d |= (uint64_t)(1024 >> 4) << 32;              // stride byte offset
-    d |= (uint64_t)1 << 46;                        // descriptor version
-    d |= (uint64_t)2 << 61;                        // 128-byte swizzle
-    return d;
-}
 // Instruction descriptor: BF16 x BF16 -> F32, A and B K-major, M = BM, N = BN.
 constexpr uint32_t kIdesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) |
                             ((uint32_t)(BM >> 4) << 24);
@@ -229,13 +41,6 @@ constexpr uint32_t kIdesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN 
 constexpr uint32_t kIdescPair = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) |
                                 ((uint32_t)((2 * BM) >> 4) << 24);
 
-__device__ __forceinline__ float pow2f(int e) {   // exact 2^e for -126 <= e <= 127
-    return __int_as_float((e + 127) << 23);
-}
-__device__ __forceinline__ double pow2d(int e) {
-    if (e >= -1022 && e <= 1023) return __longlong_as_double((long long)(e + 1023) << 52);
-    return ldexp(1.0, e);
-}
 // Bits of the double nearest (ties to even) to run 2^E, by integer operations only (the FP64
 // units are slow on this part); *mag = |run| 2^-kFixTotal as a float, truncated.  Results
 // outside the normal range take the FP64 route.
@@ -777,10 +582,8 @@ __device__ __forceinline__ unsigned long long rne_shr(unsigned long long m, int 
     return (rem > half || (rem == half && (q & 1ull))) ? q + 1ull : q;
 }
 
-// Rows of at most kShortRow destination columns are sliced by 128 threads (flag
-// kShortRowKernel in the kernel code), longer ones by 256.
-constexpr int kShortRow = 4096;
-constexpr int kShortRowKernel = 16;
+// Flags of the kernel code: a short row (kShortRow), the residue form.
+constexpr int kShortRowKernel = 16, kResidueKernel = 32;
 
 // The slicing of output row `flat` of a grouped launch: the block copies that slicing's
 // arguments to shared memory (in global memory any digit store might alias them, and copies
@@ -1388,7 +1191,10 @@ static cudaError_t set_attributes_once() {
     return cudaSuccess;
 }
 
-cudaError_t prepare_device() { return set_attributes_once(); }
+cudaError_t prepare_device() {
+    const cudaError_t e = set_attributes_once();
+    return e != cudaSuccess ? e : prepare_residue();
+}
 
 cudaError_t launch_gemm(const CUtensorMap& tmA, const CUtensorMap& tmB, const GemmArgs& a, int num_sms,
                         cudaStream_t st, bool pair) {
@@ -1476,6 +1282,7 @@ bool make_digit_map(CUtensorMap* map, void* base, int kpad, int rows_pad, int sl
 
 cudaError_t launch_slice(const SliceArgs& a, cudaStream_t st) {
     if (a.nrows <= 0) return cudaSuccess;
+    if (a.bits > 0) return launch_residue_slice(a, st);
     cudaError_t e = set_attributes_once();
     if (e != cudaSuccess) return e;
     const int grid = (a.grid_limit > 0 && a.grid_limit < a.nrows) ? a.grid_limit : a.nrows;
@@ -1501,12 +1308,13 @@ cudaError_t launch_slice(const SliceArgs& a, cudaStream_t st) {
 int slice_kernel_of(const SliceArgs& a) {
     // the four-column kernel needs the destination map (or the identity) and whole k-blocks
     const bool four = (a.col_inv || !a.col_map) && (a.kpad % BK) == 0;
-    const int k = four && a.slices >= 6 && a.slices <= 8 ? a.slices : 0;
+    const int k = a.bits > 0 ? kResidueKernel : four && a.slices >= 6 && a.slices <= 8 ? a.slices : 0;
     return a.kpad <= kShortRow ? (k | kShortRowKernel) : k;
 }
 
 cudaError_t launch_slice_grouped(const SliceGroups& g, int kernel, cudaStream_t st) {
     if (g.rows <= 0 || g.n <= 0) return cudaSuccess;
+    if (kernel & kResidueKernel) return launch_residue_slice_grouped(g, (kernel & kShortRowKernel) != 0, st);
     cudaError_t e = set_attributes_once();
     if (e != cudaSuccess) return e;
     if (kernel & kShortRowKernel) {

@@ -152,7 +152,12 @@ struct SliceArgs {
     const float* inerr2_prev;  // optional: squared row error in units of 2^{2 e_prev}
     const int* e_prev;         // exponent those units refer to
     int grid_limit;            // CTAs at most (0: one per row)
+    // residue form (residue.h) when bits > 0: X = round(x 2^(bits - e)), `slices` moduli, tab the
+    // digit constants' table (0: the A operand, slices: the B operand); needs col_inv or no map
+    int bits, tab;
 };
+// Rows of at most kShortRow destination columns are sliced by 128 threads, longer ones by 256.
+constexpr int kShortRow = 4096;
 cudaError_t launch_slice(const SliceArgs& a, cudaStream_t st);
 // Several slicings in one launch: args[g] (device memory) produces the rows
 // offs[g] <= r < offs[g + 1] of the flat row range [0, rows); all use the same kernel.

@@ -207,12 +207,16 @@ typedef struct gain_pair_job {
  * amplitude (second GEMM) within max(tol |amp|, that FP64 bound).  Outputs that fail (or
  * whose exact-accumulation certificate fails) are recomputed in FP64.  Every amplitude is
  * therefore within tol or within the reference FP64 method's own worst-case bound. */
+/* With beta, slices and kchunks all 0 both GEMMs run in residue form (one BF16 product per
+ * modulus, the exact product of operands rounded to 48 bits, 49 to 52 in the first GEMM;
+ * Ozaki scheme II), unless the device cannot hold its operand planes; naming any of the three
+ * takes balanced digits (Ozaki scheme I). */
 typedef struct gain_split_opts {
     double tol;       /* relative tolerance on each amplitude (0 -> 4.5e-9, so that
                          S = amp^2 meets 1e-8) */
-    int slices;       /* digits per operand of the amplitude GEMM (0 -> 49 bits; the
-                         rotational-dipole GEMM always keeps 56 bits) */
-    int beta;         /* bits per digit, 2..8 (0 -> 7) */
+    int slices;       /* digits per operand of the amplitude GEMM (0 -> 48 bits; the
+                         rotational-dipole GEMM keeps 46 to 56 bits by its inner length) */
+    int beta;         /* bits per digit, 2..8 (0 -> 8) */
     int kchunks;      /* inner-dimension chunks for exact FP32 accumulation (0 -> auto) */
     double s_floor;   /* certification domain: lines with S >= s_floor * S_max must meet tol
                          (0 -> 1e-10, the domain of the headline accuracy requirement) */
@@ -231,7 +235,9 @@ typedef struct gain_stats {
     double amp_max;             /* split path: largest |amplitude| of the run */
     int beta1, slices1, chunks1;  /* first GEMM (lower vectors x rotational-dipole matrix) */
     int beta2, slices2, chunks2;  /* second GEMM (half line strengths x upper vectors) */
-    int products1, products2;   /* BF16 digit products per GEMM */
+    int products1, products2;   /* BF16 products per GEMM (digit pairs, or moduli).  In residue form
+                                   slices is the number of moduli, beta the bits each holds
+                                   (rounded down) and chunks the exact accumulations per product */
     int kernel_launches;        /* kernels launched by the last run */
     double gemm1_ms, gemm2_ms;  /* device time of the two tensor-core GEMMs */
     double tensor_flops;        /* BF16 MMA flops issued by the two GEMMs (whole tiles, padding

@@ -1,0 +1,109 @@
+"""The residue form of the split path (the default): one BF16 GEMM per modulus, reconstructed
+exactly.  Sizes at the edges of its row and column tiles (128, 256), of its exact-accumulation
+chunks (384 inner elements) and of the reconstruction's blocks, on CTA pairs and single CTAs."""
+import os
+import re
+
+import numpy as np
+import pytest
+
+JMAX = 11
+
+
+def test_moduli_are_coprime_and_chunks_stay_exact():
+    """Pairwise coprime moduli; a chunk of products of balanced residues plus the running
+    residue stays below 2^24; residues are exact in BF16 (8 significant bits)."""
+    import math
+    src = open(os.path.join(os.path.dirname(__file__), "..", "gain-mpi_gb300", "csrc", "residue.h")).read()
+    mods = [int(x) for x in re.search(r"kModuli\[kMaxMod\] = \{([^}]*)\}", src).group(1).split(",")]
+    blocks = int(re.search(r"kChunkBlocks = (\d+)", src).group(1))
+    assert all(math.gcd(a, b) == 1 for i, a in enumerate(mods) for b in mods[:i])
+    for m in mods:
+        v = np.arange(-(1 << 24) + 1, 1 << 24, 7, dtype=np.int64)
+        q = np.rint(v.astype(np.float64) * np.float64(np.float32(1.0) / np.float32(m)))
+        r = np.abs(v - q.astype(np.int64) * m).max()     # the kernel's reduction, exact in binary64
+        assert r <= 256 and 64 * blocks * r * r + r < 1 << 24, (m, r)
+
+
+@pytest.fixture(scope="module")
+def problems(built_lib):
+    import gainls
+    import synth
+    out = {}
+    for name, (rule, nv, jv) in {"c4": ("c4", 120, (5, 6)), "c4r": ("c4r", 130, (2, 3)), "full": ("full", 48, (3, 4)),
+                                 "c4m": ("c4m", 75, (3, 4))}.items():
+        g = (0, 0) if rule == "full" else (0, 1)
+        p = synth.make_problem(nv, list(jv), rule, blocks=[(jv[0], g[0]), (jv[1], g[1])])
+        eng = gainls.Engine(JMAX, p.nsym, 1)
+        gainls.upload_problem(eng, p)
+        out[name] = (p, eng, g)
+    return out
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("name", ["c4", "c4r", "full", "c4m"])
+@pytest.mark.parametrize("sizes", [(1, 1), (5, 127), (128, 128), (129, 129), (127, 257), (256, 256), (257, 391), (10**6, 10**6)])
+@pytest.mark.parametrize("pair", ["1", "0"])
+def test_residue_form_matches_plain_fp64(problems, name, sizes, pair, monkeypatch):
+    """|amp - plain| against the rounding of the operands: each operand row is rounded to 48
+    bits of its largest entry (a relative 2^-48 sqrt(N) of its norm, twice), each H entry is
+    within the FP64 bound (W + 64) 2^-53 of its rows' norms, and the plain path adds N 2^-53."""
+    import gainls
+    p, eng, (gI, gF) = problems[name]
+    vI, vF = p.blocks[(0, gI)].vecs, p.blocks[(1, gF)].vecs
+    lo = np.arange(min(sizes[0], vI.shape[0]), dtype=np.int32)
+    up = np.arange(min(sizes[1], vF.shape[0]), dtype=np.int32)[::-1].copy()
+    monkeypatch.setenv("GAINLS_GEMM_PAIR", pair)
+    eng.run_pair(0, gI, 1, gF, lo, np.arange(vF.shape[0], dtype=np.int32), gainls.PATH_PLAIN_FP64)
+    full = eng.fetch_amp().copy()      # every upper state: an orthonormal set, so the rows' norms are those of H
+    st = eng.run_pair(0, gI, 1, gF, lo, up, gainls.PATH_SPLIT)
+    assert st["status"] == gainls.OK and st["products2"] == st["slices2"] == 13
+    amp = eng.fetch_amp()
+    N, W = vF.shape[1], 2 * vI.shape[1] + 128
+    h = np.linalg.norm(full, axis=1).max()
+    mrow = np.sqrt(15.0) * np.sqrt((p.dipole ** 2).sum(axis=(0, 1))).max()     # a row of M: at most 5 of each (K, tau)
+    tol = (4 * np.sqrt(N) * 2.0 ** -48 + (N + 64) * 2.0 ** -52) * h + np.sqrt(N) * (W + 64) * 2.0 ** -53 * mrow
+    assert np.max(np.abs(amp - full[:, up])) <= tol
+
+
+@pytest.mark.gpu
+def test_several_row_panels_equal_one_run(problems, monkeypatch):
+    """More output rows than one panel (1024 on single CTAs): every row equals its own run's bits."""
+    import gainls
+    p, eng, (gI, gF) = problems["c4"]
+    n = p.blocks[(0, gI)].vecs.shape[0]
+    up = np.arange(200, dtype=np.int32)
+    many = np.tile(np.arange(n, dtype=np.int32), 4)[:2 * 1024 + 130]
+    eng.run_pair(0, gI, 1, gF, np.arange(n, dtype=np.int32), up, gainls.PATH_SPLIT)
+    one = eng.fetch_amp().copy()
+    for pair in ("1", "0"):
+        monkeypatch.setenv("GAINLS_GEMM_PAIR", pair)
+        eng.run_pair(0, gI, 1, gF, many, up, gainls.PATH_SPLIT)
+        np.testing.assert_array_equal(eng.fetch_amp(), one[many])
+
+
+@pytest.mark.gpu
+def test_scales_and_zero_rows(built_lib):
+    """Rows of very different scales, subnormal rows and all-zero rows: amplitudes scale with
+    their rows exactly (powers of two) and zero rows give exact zeros."""
+    import gainls
+    import synth
+    p = synth.make_problem(24, [2, 3], "c4", blocks=[(2, 0), (3, 1)])
+    vI, vF = p.blocks[(0, 0)].vecs, p.blocks[(1, 1)].vecs
+    lo, up = np.arange(vI.shape[0]), np.arange(vF.shape[0])
+    eng = gainls.Engine(JMAX, p.nsym, 1)
+    gainls.upload_problem(eng, p)
+    eng.run_pair(0, 0, 1, 1, lo, up, gainls.PATH_SPLIT)
+    ref = eng.fetch_amp().copy()
+    e = np.resize([0, -40, 300, -300, 7], vI.shape[0])
+    v2 = np.ldexp(vI, e[:, None])
+    v2[3] = 0.0
+    eng.upload_eigvecs(0, 0, v2)
+    eng.run_pair(0, 0, 1, 1, lo, up, gainls.PATH_SPLIT)
+    want = np.ldexp(ref, e[:, None])
+    want[3] = 0.0
+    np.testing.assert_array_equal(eng.fetch_amp(), want)
+    eng.upload_eigvecs(0, 0, np.ldexp(vI, -1060))     # subnormal entries, rounded by the input itself
+    eng.run_pair(0, 0, 1, 1, lo, up, gainls.PATH_SPLIT)
+    got = eng.fetch_amp()
+    assert np.max(np.abs(got - np.ldexp(ref, -1060))) <= 2.0 ** -1074 * 64 * vI.shape[1]
