@@ -28,13 +28,132 @@ __device__ __forceinline__ void rot_factor(int kI, int kF, int tauI, int tauF, i
 }
 
 // ---------------------------------------------------------------------------------------
-// Drop-in K-block kernel.  One thread per upper primitive of the K block; lower functions
-// of the three neighbouring K blocks are staged through shared memory 128 at a time.  Each
-// output is accumulated in ascending lower index with one fused multiply-add per term, the
-// same operation sequence as the reference kernel, so results agree bit for bit.
-constexpr int kDropTile = 128;
+// K-block half line strengths: the sum of one upper primitive F over the lower functions I of
+// the three neighbouring K blocks, one fused multiply-add per term in ascending I, as the
+// reference kernel accumulates it, so results agree with it bit for bit.
+//
+// What bounds these kernels is the FP64 pipe (about 1.7 lane operations per clock and SM) and,
+// where a launch has few outputs, the serial chain of each.  The reference multiplies every
+// (F, I) term by the integer rotational coefficient and by the parity sign before the
+// fused multiply-add; both depend on F only through the parity tau_F (0 or 1), so the block
+// forms each lower function's coefficient once for both parities and the inner loop is one
+// FP64 operation per term instead of three.  Lower functions whose weight is zero (the
+// reference skips them: the other symmetry classes' primitives) are left out of the list.
+// Measured (GB300): the drop-in kernel 526 -> 60 us for 1200 outputs of 900 non-zero terms each
+// (32 outputs per block instead of 128, and the dipole loads run ahead of the chain), the plain
+// path's 480 -> 88 us for 8 x 3000 outputs of 1200 terms (53 us at the FP64 rate).
+struct HlsTerm {
+    double v;    // weight: vector x 1/sqrt(2) x 3j x coefficient x sign
+    long off;    // the lower function's row of the dipole component it couples through
+};
 
-__global__ void __launch_bounds__(kDropTile)
+// Lower function `ir` of block kI for upper block kF: its terms for tau_F = 0 and 1; false
+// where the reference skips it.
+__device__ __forceinline__ bool hls_terms(double vec, int t, int icor, int kI, int kF, double sq, double f3j, int ncontrF,
+                                          long stride, HlsTerm (&term)[2]) {
+    double l = vec;
+    if (kF != kI) l = __dmul_rn(l, sq);
+    l = __dmul_rn(l, f3j);
+    if (l == 0.0) return false;
+    const double sg = parity_sign((kI % 3) * t + kI);
+    const long off = (long)icor * ncontrF;
+#pragma unroll
+    for (int tF = 0; tF < 2; ++tF) {
+        int didx, c;
+        rot_factor(kI, kF, t, tF, &didx, &c);
+        // c = +-1 (the usual case of two parities) and the sign only flip bits
+        const double ls = c == 1 ? l : (c == -1 ? -l : __dmul_rn(l, (double)c));
+        term[tF].v = sg < 0.0 ? -ls : ls;
+        term[tF].off = off + didx * stride;
+    }
+    return true;
+}
+
+// Terms of the lower functions [0, count) of block kI, in order, appended to the list segment
+// by segment; `sum` consumes a full list.  source(i) gives function i's vector entry, tau and
+// vibrational index.  A thread forms kHlsEach functions at once (their loads overlap).
+constexpr int kHlsEach = 4, kHlsList = 1024;
+struct HlsLists {
+    HlsTerm term[2][kHlsList];
+    int cnt[kHlsEach][4];
+};
+template <int NT, class Source, class Sum>
+__device__ __forceinline__ void hls_block(HlsLists& L, int count, int kI, int kF, double sq, double f3j, int ncontrF,
+                                          long stride, Source source, Sum sum) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    int n = 0;
+    for (int base = 0; base < count; base += NT * kHlsEach) {
+        double v[kHlsEach];
+        int t[kHlsEach], ic[kHlsEach];
+#pragma unroll
+        for (int e = 0; e < kHlsEach; ++e) {
+            const int i = base + e * NT + threadIdx.x;
+            v[e] = 0.0;
+            t[e] = ic[e] = 0;
+            if (i < count) source(i, v[e], t[e], ic[e]);
+        }
+        HlsTerm term[kHlsEach][2];
+        unsigned int mask[kHlsEach];
+#pragma unroll
+        for (int e = 0; e < kHlsEach; ++e) {
+            const bool keep = hls_terms(v[e], t[e], ic[e], kI, kF, sq, f3j, ncontrF, stride, term[e]);
+            mask[e] = __ballot_sync(0xffffffffu, keep);
+            if (lane == 0) L.cnt[e][warp] = __popc(mask[e]);
+        }
+        __syncthreads();
+#pragma unroll
+        for (int e = 0; e < kHlsEach; ++e) {
+            int pos = n + __popc(mask[e] & ((1u << lane) - 1u));
+#pragma unroll
+            for (int w = 0; w < NT / 32; ++w) {
+                if (w < warp) pos += L.cnt[e][w];
+                n += L.cnt[e][w];
+            }
+            if ((mask[e] >> lane) & 1u) {
+                L.term[0][pos] = term[e][0];
+                L.term[1][pos] = term[e][1];
+            }
+        }
+        __syncthreads();
+        if (n + NT * kHlsEach > kHlsList || base + NT * kHlsEach >= count) {
+            sum(n);
+            __syncthreads();
+            n = 0;
+        }
+    }
+}
+
+// acc += the n listed terms against the dipole column at mu, in order.  The dipole comes from L2
+// (several hundred clocks): the next group's loads are in flight under this group's chain.
+__device__ __forceinline__ double hls_sum(double acc, const HlsTerm* list, int n, const double* __restrict__ mu) {
+    constexpr int G = 16;
+    double m[G];
+#pragma unroll
+    for (int k = 0; k < G; ++k) m[k] = k < n ? __ldg(mu + list[k].off) : 0.0;
+    for (int i = 0; i < n; i += G) {
+        double next[G];
+#pragma unroll
+        for (int k = 0; k < G; ++k) next[k] = i + G + k < n ? __ldg(mu + list[i + G + k].off) : 0.0;
+        if (i + G <= n) {
+#pragma unroll
+            for (int k = 0; k < G; ++k) acc = __fma_rn(list[i + k].v, m[k], acc);
+        } else {
+#pragma unroll
+            for (int k = 0; k < G; ++k)
+                if (i + k < n) acc = __fma_rn(list[i + k].v, m[k], acc);
+        }
+#pragma unroll
+        for (int k = 0; k < G; ++k) m[k] = next[k];
+    }
+    return acc;
+}
+
+// Drop-in K-block kernel: kDropF upper primitives per block of kDropThreads threads.  A launch
+// has one K block's primitives (a few thousand at most): small blocks spread their chains over
+// the SMs, the block's other threads share in forming the terms.
+constexpr int kDropThreads = 128, kDropF = 32;
+
+__global__ void __launch_bounds__(kDropThreads)
 k_hls_kblock(int dimenF, int dimenI, int jI, int jF, int kF, const int* __restrict__ tauI,
              const int* __restrict__ tauF, const int* __restrict__ icorrI,
              const int* __restrict__ icorrF, int startF_idx, int startI_idx, int startFblock,
@@ -42,21 +161,17 @@ k_hls_kblock(int dimenF, int dimenI, int jI, int jF, int kF, const int* __restri
              const double* __restrict__ dipole_me, const double* __restrict__ vector,
              const double* __restrict__ threej, double* __restrict__ half_ls, int jmax,
              int dip_stride) {
-    __shared__ double s_lsf[kDropTile];
-    __shared__ double s_sgn[kDropTile];
-    __shared__ int s_tau[kDropTile];
-    __shared__ long s_off[kDropTile];
-
-    const int f = blockIdx.x * kDropTile + threadIdx.x;
+    __shared__ HlsLists L;
+    const int f = blockIdx.x * kDropF + threadIdx.x;
     const int irootF = startF_idx + f;
-    const bool inF = f < dimenF;
+    const bool inF = (int)threadIdx.x < kDropF && f < dimenF;
     int icF = 0, tF = 0;
     if (inF) {
         icF = icorrF[irootF];
         tF = tauF[irootF] & 1;
     }
     const bool valid = inF && icF >= startFblock && icF < endFblock;
-    icF -= startFblock;
+    const double* mu = dipole_me + (valid ? icF - startFblock : 0);
     const long stride = (long)ncontrF * dip_stride;
     double acc = 0.0;
     int startI = startI_idx;
@@ -64,44 +179,16 @@ k_hls_kblock(int dimenF, int dimenI, int jI, int jF, int kF, const int* __restri
         const int kbs = kblock_size[kI];
         const double sq = (kI * kF != 0) ? kSqrt2Ref : 1.0;
         const double f3j = threej[threej_index(jI, kI, jF, kF, jmax)];
-        int didx_same, c_same, didx_flip, c_flip;   // tau_I == tau_F and tau_I != tau_F cases
-        rot_factor(kI, kF, tF, tF, &didx_same, &c_same);
-        rot_factor(kI, kF, tF ^ 1, tF, &didx_flip, &c_flip);
-        for (int base = 0; base < kbs; base += kDropTile) {
-            const int loc = base + threadIdx.x;
-            double lsf = 0.0, sg = 1.0;
-            int ti = 0;
-            long off = 0;
-            if (loc < kbs) {
-                const int ir = startI + loc;
-                ti = tauI[ir];
-                off = (long)icorrI[ir] * ncontrF;
-                sg = parity_sign((kI % 3) * ti + kI);
-                double ls = vector[ir];
-                if (kF != kI) ls = __dmul_rn(ls, sq);
-                lsf = __dmul_rn(ls, f3j);
-            }
-            __syncthreads();
-            s_lsf[threadIdx.x] = lsf;
-            s_sgn[threadIdx.x] = sg;
-            s_tau[threadIdx.x] = ti;
-            s_off[threadIdx.x] = off;
-            __syncthreads();
-            const int n = min(kDropTile, kbs - base);
-            if (valid) {
-                for (int i = 0; i < n; ++i) {
-                    const double l = s_lsf[i];
-                    if (l == 0.0) continue;
-                    const int t = s_tau[i];
-                    int didx, c;
-                    if (t == tF) { didx = didx_same; c = c_same; }
-                    else if (t == (tF ^ 1)) { didx = didx_flip; c = c_flip; }
-                    else rot_factor(kI, kF, t, tF, &didx, &c);
-                    const double ls = __dmul_rn(l, (double)c);
-                    acc = __fma_rn(__dmul_rn(ls, s_sgn[i]), dipole_me[icF + s_off[i] + didx * stride], acc);
-                }
-            }
-        }
+        hls_block<kDropThreads>(
+            L, kbs, kI, kF, sq, f3j, ncontrF, stride,
+            [&](int i, double& v, int& t, int& ic) {
+                v = vector[startI + i];
+                t = tauI[startI + i];
+                ic = icorrI[startI + i];
+            },
+            [&](int n) {
+                if (valid) acc = hls_sum(acc, L.term[tF], n, mu);
+            });
         startI += kbs;
         if (startI >= dimenI) break;
     }
@@ -157,10 +244,7 @@ k_hls_needed(const HlsCta* __restrict__ ctas, const int* __restrict__ f_list, in
              int startFblock, int endFblock, int ncontrF, const double* __restrict__ dipole_me,
              int dip_stride, const double* __restrict__ prim_vec, long ld_prim,
              const double* __restrict__ threej, int jmax, double* __restrict__ half_ls, long ld_h) {
-    __shared__ double s_lsf[kHlsTile];
-    __shared__ double s_sgn[kHlsTile];
-    __shared__ int s_tau[kHlsTile];
-    __shared__ long s_off[kHlsTile];
+    __shared__ HlsLists L;
     // blockIdx.y: lower state of the batch
     prim_vec += (long)blockIdx.y * ld_prim;
     half_ls += (long)blockIdx.y * ld_h;
@@ -174,45 +258,24 @@ k_hls_needed(const HlsCta* __restrict__ ctas, const int* __restrict__ f_list, in
         tF = tauF[irootF] & 1;
     }
     const bool valid = inF && icF >= startFblock && icF < endFblock;
-    icF -= startFblock;
+    const double* mu = dipole_me + (valid ? icF - startFblock : 0);
     const long stride = (long)ncontrF * dip_stride;
     double acc = 0.0;
     for (int kI = max(kF - 1, 0); kI < kF + 2 && kI < jI + 1; ++kI) {
         const int s0 = sup_start[kI], ns = sup_start[kI + 1] - s0;
         const double sq = (kI * kF != 0) ? kSqrt2Ref : 1.0;
         const double f3j = threej[threej_index(jI, kI, jF, kF, jmax)];
-        for (int base = 0; base < ns; base += kHlsTile) {
-            const int loc = base + threadIdx.x;
-            double lsf = 0.0, sg = 1.0;
-            int ti = 0;
-            long off = 0;
-            if (loc < ns) {
-                const int ir = sup_list[s0 + loc];
-                ti = tauI[ir];
-                off = (long)icorrI[ir] * ncontrF;
-                sg = parity_sign((kI % 3) * ti + kI);
-                double ls = prim_vec[ir];
-                if (kF != kI) ls = __dmul_rn(ls, sq);
-                lsf = __dmul_rn(ls, f3j);
-            }
-            __syncthreads();
-            s_lsf[threadIdx.x] = lsf;
-            s_sgn[threadIdx.x] = sg;
-            s_tau[threadIdx.x] = ti;
-            s_off[threadIdx.x] = off;
-            __syncthreads();
-            const int n = min(kHlsTile, ns - base);
-            if (valid) {
-                for (int i = 0; i < n; ++i) {
-                    const double l = s_lsf[i];
-                    if (l == 0.0) continue;
-                    int didx, c;
-                    rot_factor(kI, kF, s_tau[i], tF, &didx, &c);
-                    const double ls = __dmul_rn(l, (double)c);
-                    acc = __fma_rn(__dmul_rn(ls, s_sgn[i]), dipole_me[icF + s_off[i] + didx * stride], acc);
-                }
-            }
-        }
+        hls_block<kHlsTile>(
+            L, ns, kI, kF, sq, f3j, ncontrF, stride,
+            [&](int i, double& v, int& t, int& ic) {
+                const int ir = sup_list[s0 + i];
+                v = prim_vec[ir];
+                t = tauI[ir];
+                ic = icorrI[ir];
+            },
+            [&](int n) {
+                if (valid) acc = hls_sum(acc, L.term[tF], n, mu);
+            });
     }
     if (valid) half_ls[irootF] = __dmul_rn(acc, parity_sign((kF % 3) * tF));
     else if (inF) half_ls[irootF] = 0.0;
@@ -438,7 +501,7 @@ cudaError_t launch_hls_kblock(int dimenF, int dimenI, int jI, int jF, int kF, co
                               const double* vector, const double* threej, double* half_ls,
                               int jmax, int dip_stride, cudaStream_t st) {
     if (dimenF <= 0) return cudaSuccess;
-    k_hls_kblock<<<(dimenF + kDropTile - 1) / kDropTile, kDropTile, 0, st>>>(
+    k_hls_kblock<<<(dimenF + kDropF - 1) / kDropF, kDropThreads, 0, st>>>(
         dimenF, dimenI, jI, jF, kF, tauI, tauF, icorrI, icorrF, startF_idx, startI_idx,
         startFblock, endFblock, ncontrF, kblock_size, dipole_me, vector, threej, half_ls, jmax,
         dip_stride);

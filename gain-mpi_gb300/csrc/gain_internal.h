@@ -93,7 +93,7 @@ struct HlsCta {
     int f_count;   // <= kHlsTile
     int pad;
 };
-constexpr int kHlsTile = 128;
+constexpr int kHlsTile = 64;
 
 // half_ls restricted to the needed upper primitives (F list), summing over the lower
 // support lists per K block. Writes half_ls[F] (primitive index) for every listed F.
