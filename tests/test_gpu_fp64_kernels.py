@@ -51,3 +51,25 @@ def test_kblock_lists_bit_exact_vs_oracle(built_lib, nv, JI, JF, zeros):
     assert np.array_equal(np.isnan(got), np.isnan(ref))
     keep = ~np.isnan(ref)
     assert np.array_equal(got[keep].view(np.uint64), ref[keep].view(np.uint64))
+
+
+@pytest.mark.parametrize("n", [0, 1, 1024, 4095, 4096, 4097, 8192, 8193, 32768 + 5, 1000003])
+def test_dot_one_block_and_cluster(built_lib, n):
+    """Any n against the double-double sum, within the bound of an FP64 sum of n products; the
+    same inputs give the same bits again, on another stream too."""
+    import torch
+    import gainls
+    import oracle
+    rng = np.random.default_rng(n)
+    x, y = rng.standard_normal(max(n, 1)), rng.standard_normal(max(n, 1))
+    dx, dy = _dev(x), _dev(y)
+    res = torch.full((3,), np.nan, dtype=torch.float64, device="cuda")
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    gainls.dot(n, dx.data_ptr(), dy.data_ptr(), res.data_ptr(), torch.cuda.current_stream().cuda_stream)
+    gainls.dot(n, dx.data_ptr(), dy.data_ptr(), res[1:].data_ptr(), side.cuda_stream)
+    torch.cuda.synchronize()
+    got = res.cpu().numpy()
+    assert got[0] == got[1] and np.isnan(got[2])
+    ref = oracle.dot(x[:n], y[:n], oracle.DD) if n else 0.0
+    assert abs(got[0] - ref) <= (n + 1) * 2.0 ** -53 * np.sum(np.abs(x[:n] * y[:n]))
