@@ -3500,7 +3500,7 @@ struct gain_plan_s {
     DevArray<split::ResTile> rtiles1, rtiles2;
     DevArray<split::CrtArgs> crt1, crt2;
     DevArray<int> crt1_offs, crt2_offs;
-    int crt1_blocks = 0, crt2_blocks = 0;
+    int crt1_blocks = 0, crt2_blocks = 0, crt1_nmod = 0, crt2_nmod = 0;   // nmod 0: jobs differ
     DevArray<uint16_t> res;
     // the plan's digit slicings, one launch per slicing kernel: the eigenvectors (before the
     // first GEMM) and H (before the second)
@@ -3881,6 +3881,13 @@ gain_status plan_build_residue_groups(gain_plan P) {
     P->ntiles2 = (int)s2.size();
     P->crt1_blocks = o1[nj];
     P->crt2_blocks = o2[nj];
+    auto common = [](const std::vector<split::CrtArgs>& v) {
+        for (const auto& a : v)
+            if (a.nmod != v[0].nmod) return 0;
+        return v[0].nmod;
+    };
+    P->crt1_nmod = common(a1);
+    P->crt2_nmod = common(a2);
     GAIN_TRY(P->rgroups1.upload(g1));
     GAIN_TRY(P->rgroups2.upload(g2));
     GAIN_TRY(P->rtiles1.upload(s1));
@@ -4095,7 +4102,7 @@ gain_status plan_enqueue(gain_plan P) {
     ga.ntiles = P->ntiles1;
     if (P->residues) {
         GAIN_TRY(plan_residue_gemm(P, P->rgroups1.p, P->rtiles1.p, P->ntiles1,
-                                   {P->crt1.p, P->crt1_offs.p, nj, P->crt1_blocks}, P->ev[1], P->ev[2]));
+                                   {P->crt1.p, P->crt1_offs.p, nj, P->crt1_blocks, P->crt1_nmod}, P->ev[1], P->ev[2]));
     } else {
         GAIN_CUDA(cudaEventRecordWithFlags(P->ev[1], st, cudaEventRecordExternal));
         GAIN_CUDA(split::launch_gemm_grouped(ga, P->units, P->s1max, P->c1max, st, P->pair));
@@ -4143,7 +4150,7 @@ gain_status plan_enqueue(gain_plan P) {
     ga.ntiles = P->ntiles2;
     if (P->residues) {
         GAIN_TRY(plan_residue_gemm(P, P->rgroups2.p, P->rtiles2.p, P->ntiles2,
-                                   {P->crt2.p, P->crt2_offs.p, nj, P->crt2_blocks}, P->ev[3], P->ev[4]));
+                                   {P->crt2.p, P->crt2_offs.p, nj, P->crt2_blocks, P->crt2_nmod}, P->ev[3], P->ev[4]));
     } else {
         GAIN_CUDA(cudaEventRecordWithFlags(P->ev[3], st, cudaEventRecordExternal));
         GAIN_CUDA(split::launch_gemm_grouped(ga, P->units, P->s2max, P->c2max, st, P->pair));

@@ -103,6 +103,7 @@ struct CrtGroups {
     const CrtArgs* args;
     const int* offs;
     int n, blocks;
+    int nmod;              // every group's moduli (0: they differ)
 };
 cudaError_t launch_crt_grouped(const CrtGroups& g, cudaStream_t st);
 

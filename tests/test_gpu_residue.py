@@ -67,19 +67,44 @@ def test_residue_form_matches_plain_fp64(problems, name, sizes, pair, monkeypatc
 
 
 @pytest.mark.gpu
-def test_several_row_panels_equal_one_run(problems, monkeypatch):
-    """More output rows than one panel (1024 on single CTAs): every row equals its own run's bits."""
+@pytest.mark.parametrize("nup", [200, 780])
+def test_several_row_panels_equal_one_run(problems, nup, monkeypatch):
+    """More output rows than one panel (1024 on single CTAs), reconstructed one and four rows to a
+    block: every row equals its own run's bits."""
     import gainls
     p, eng, (gI, gF) = problems["c4"]
     n = p.blocks[(0, gI)].vecs.shape[0]
-    up = np.arange(200, dtype=np.int32)
-    many = np.tile(np.arange(n, dtype=np.int32), 4)[:2 * 1024 + 130]
+    up = np.arange(nup, dtype=np.int32) % p.blocks[(1, gF)].vecs.shape[0]
+    many = np.arange(2 * 1024 + 130, dtype=np.int32) % n
     eng.run_pair(0, gI, 1, gF, np.arange(n, dtype=np.int32), up, gainls.PATH_SPLIT)
     one = eng.fetch_amp().copy()
     for pair in ("1", "0"):
         monkeypatch.setenv("GAINLS_GEMM_PAIR", pair)
         eng.run_pair(0, gI, 1, gF, many, up, gainls.PATH_SPLIT)
         np.testing.assert_array_equal(eng.fetch_amp(), one[many])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("bits,moduli", [(46, 12), (48, 13), (54, 14), (56, 14)])
+def test_other_numbers_of_moduli(problems, bits, moduli, monkeypatch):
+    """First-GEMM precisions that take fewer or more moduli than the usual 13: the amplitudes agree
+    within the rounding of the lower and band rows to that many bits (H entries that miss the
+    FP64 bound are recomputed)."""
+    import gainls
+    p, eng, (gI, gF) = problems["c4"]
+    lo = np.arange(p.blocks[(0, gI)].vecs.shape[0], dtype=np.int32)
+    up = np.arange(p.blocks[(1, gF)].vecs.shape[0], dtype=np.int32)
+    eng.run_pair(0, gI, 1, gF, lo, up, gainls.PATH_SPLIT)
+    ref = eng.fetch_amp().copy()
+    monkeypatch.setenv("GAINLS_GEMM1_BITS", str(bits))
+    st = eng.run_pair(0, gI, 1, gF, lo, up, gainls.PATH_SPLIT)
+    assert st["status"] == gainls.OK and st["slices1"] == moduli
+    N, W = up.size, 2 * lo.size + 128
+    mrow = np.sqrt(15.0) * np.sqrt((p.dipole ** 2).sum(axis=(0, 1))).max()
+    h = np.linalg.norm(ref, axis=1).max()
+    # two H errors (each within the FP64 bound of its rows) and two roundings of H to 48 bits
+    tol = 2 * (np.sqrt(N) * (W + 64) * 2.0 ** -53 * mrow + 2 * np.sqrt(N) * 2.0 ** -48 * h)
+    assert np.max(np.abs(eng.fetch_amp() - ref)) <= tol
 
 
 @pytest.mark.gpu
