@@ -40,7 +40,7 @@ constexpr int balanced(int r, int m) { return 2 * r > m ? r - m : r; }
 struct ModTables {
     float digit[kMaxMod + 1][kMaxMod][4];
     float inv[kMaxMod], m[kMaxMod];
-    unsigned int frac[kMaxMod][3];   // floor(2^96 / m_i), low word first
+    unsigned int frac[kMaxMod][3];   // floor(2^80 / m_i): the low 16 bits, then two 32-bit words
 };
 constexpr ModTables make_tables() {
     ModTables t{};
@@ -48,9 +48,9 @@ constexpr ModTables make_tables() {
         const int m = kModuli[i];
         t.m[i] = (float)m;
         t.inv[i] = 1.0f / (float)m;
-        unsigned long long rem = 1;   // long division of 2^96 by m in base 2^32
+        unsigned long long rem = 1;   // long division of 2^80 by m, word by word
         for (int w = 2; w >= 0; --w) {
-            const unsigned long long cur = rem << 32;
+            const unsigned long long cur = rem << (w ? 32 : 16);
             t.frac[i][w] = (unsigned int)(cur / (unsigned)m);
             rem = cur % (unsigned)m;
         }
@@ -78,20 +78,34 @@ __device__ __forceinline__ float mod_balanced(float v, float inv, float neg_m) {
     return __fmaf_rn(neg_m, q, v);
 }
 
-// Two such reductions at once (packed FP32: half the issue slots, the same roundings).
-__device__ __forceinline__ void mod_balanced2(uint32_t& x, uint32_t& y, float inv, float neg_m) {
-    asm("{\n\t.reg .b64 v, i, m, g, h, q;\n\t"
-        "mov.b64 v, {%0, %1};\n\t"
-        "mov.b64 i, {%2, %2};\n\t"
-        "mov.b64 m, {%3, %3};\n\t"
-        "mov.b64 g, {%4, %4};\n\t"
-        "mov.b64 h, {%5, %5};\n\t"
-        "fma.rn.f32x2 q, v, i, g;\n\t"
-        "add.rn.f32x2 q, q, h;\n\t"
-        "fma.rn.f32x2 v, q, m, v;\n\t"
-        "mov.b64 {%0, %1}, v;\n\t}"
-        : "+r"(x), "+r"(y)
-        : "f"(inv), "f"(neg_m), "f"(kRoundMagic), "f"(-kRoundMagic));
+// Packed FP32 pairs: half the issue slots of the scalar operations, the same roundings.
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 pack2(float x, float y) {
+    f32x2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
+    return r;
+}
+__device__ __forceinline__ void unpack2(f32x2 v, uint32_t& x, uint32_t& y) {
+    asm("mov.b64 {%0, %1}, %2;" : "=r"(x), "=r"(y) : "l"(v));
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+    f32x2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f32x2 mod_balanced2(f32x2 v, f32x2 inv, f32x2 neg_m) {
+    const f32x2 q = add2(fma2(v, inv, pack2(kRoundMagic, kRoundMagic)), pack2(-kRoundMagic, -kRoundMagic));
+    return fma2(neg_m, q, v);
 }
 
 // ------------------------------------------------------------------- the GEMM
@@ -413,7 +427,10 @@ k_residue_gemm(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
 #pragma unroll
                         for (int k = 0; k < 2; ++k)
 #pragma unroll
-                            for (int j = 0; j < 32; j += 2) mod_balanced2(v[k][j], v[k][j + 1], inv, -m);
+                            for (int j = 0; j < 32; j += 2)
+                                unpack2(mod_balanced2(pack2(__uint_as_float(v[k][j]), __uint_as_float(v[k][j + 1])),
+                                                      pack2(inv, inv), pack2(-m, -m)),
+                                        v[k][j], v[k][j + 1]);
                         if (last) {
                             pack(v, m, o + 16 * p);
                         } else {
@@ -452,11 +469,11 @@ k_residue_gemm(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
 
 // ------------------------------------------------------------------- residue planes
 // One row per block iteration: the scale exponent from the largest |x| (integer compares on
-// the IEEE bits), then four destination columns per thread: X = round(x 2^(bits - e)) in
-// integer arithmetic, its four digits as floats, and per modulus the residue (seven FP32
-// operations), stored as four BF16 (a residue's float is exact in BF16: its upper half).
-// Row statistics: e, non-zero count, ||x^||_2 rounded up.
-template <bool G, int NT>
+// the IEEE bits), then COLS destination columns per thread: X = round(x 2^(bits - e)) in
+// integer arithmetic, its four digits as floats, and per modulus the residue (seven packed FP32
+// operations per two columns), stored as BF16 (a residue's float is exact in BF16: its upper
+// half).  Row statistics: e, non-zero count, ||x^||_2 rounded up.
+template <bool G, int NT, int COLS>
 __device__ __forceinline__ void residue_rows(const SliceArgs& a0, const SliceGroups& gs) {
     const int tid = threadIdx.x;
     __shared__ unsigned long long red_u[NT / 32];
@@ -482,11 +499,36 @@ __device__ __forceinline__ void residue_rows(const SliceArgs& a0, const SliceGro
         const SliceArgs& a = G ? sa : a0;
         const long srow = a.src_rows ? (long)a.src_rows[row] : (long)row;
         const unsigned long long* src = (const unsigned long long*)(a.src + srow * a.ld_src);
+        const int* map = a.col_inv;   // source column of each destination column, -1: padding
         unsigned long long mx = 0;
-#pragma unroll 4
-        for (int c = tid; c < a.ncols; c += NT) {
-            const unsigned long long b = src[c] & 0x7FFFFFFFFFFFFFFFull;
+        auto top = [&](unsigned long long b) {
+            b &= 0x7FFFFFFFFFFFFFFFull;
             mx = b > mx ? b : mx;
+        };
+        if (((uintptr_t)src & 15) == 0) {   // 16-byte loads
+            const ulonglong2* s2 = reinterpret_cast<const ulonglong2*>(src);
+            const int n2 = a.ncols >> 1;
+            int c = tid;
+            for (; c + 7 * NT < n2; c += 8 * NT) {
+                ulonglong2 v[8];
+#pragma unroll
+                for (int u = 0; u < 8; ++u) v[u] = __ldg(s2 + c + u * NT);
+#pragma unroll
+                for (int u = 0; u < 8; ++u) {
+                    top(v[u].x);
+                    top(v[u].y);
+                }
+            }
+#pragma unroll 4
+            for (; c < n2; c += NT) {
+                const ulonglong2 v = __ldg(s2 + c);
+                top(v.x);
+                top(v.y);
+            }
+            if ((a.ncols & 1) && tid == 0) top(src[a.ncols - 1]);
+        } else {
+#pragma unroll 8
+            for (int c = tid; c < a.ncols; c += NT) top(__ldg(src + c));
         }
         for (int o = 16; o > 0; o >>= 1) {
             const unsigned long long y = __shfl_xor_sync(0xffffffffu, mx, o);
@@ -500,59 +542,84 @@ __device__ __forceinline__ void residue_rows(const SliceArgs& a0, const SliceGro
         const int Emax = (int)(mx >> 52);
         const bool zero_row = (mx == 0);
         const int e = zero_row ? 0 : (Emax > 0 ? Emax - 1022 : -1022);
-        const int bits_e = a.bits - e, nmod = a.slices, tab = a.tab;
+        const int nmod = a.slices, tab = a.tab;
+        const int r0 = 1085 - a.bits + e;   // a column's shift is r0 - max(E, 1)
         const float scale = pow2f(-a.bits);
         const long sstride = a.slice_stride;
         __nv_bfloat16* drow = a.digits + (long)row * a.kpad;
         int nnz = 0;
         float l2sq = 0.0f;
-        for (int dc = 4 * tid; dc < a.kpad; dc += 4 * NT) {
-            float d[4][4];
+        for (int dc = COLS * tid; dc < a.kpad; dc += COLS * NT) {
+            f32x2 d[COLS / 2][4];
+            unsigned long long cur[COLS];
+            int sc[COLS];
+            if (map) {
 #pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                const int col = dc + u;
-                const int sc = a.col_inv ? a.col_inv[col] : (col < a.ncols ? col : -1);
-                const unsigned long long bits = sc >= 0 ? src[sc] : 0ull;
-                const unsigned long long ab = bits & 0x7FFFFFFFFFFFFFFFull;
-                long long I = 0;
-                if (ab != 0 && ab < 0x7FF0000000000000ull) {
-                    const int E = (int)(ab >> 52);
-                    const unsigned long long mant = E > 0 ? (ab & 0xFFFFFFFFFFFFFull) | (1ull << 52) : ab;
-                    const int sh = (E > 0 ? E - 1075 : -1074) + bits_e;
-                    unsigned long long m;
-                    if (sh >= 0) m = mant << sh;
-                    else m = sh >= -54 ? (mant + (1ull << (-sh - 1))) >> -sh : 0ull;   // to nearest, ties up in |x|
-                    I = (bits >> 63) ? -(long long)m : (long long)m;
-                    ++nnz;
+                for (int u = 0; u < COLS; u += 4) {
+                    const int4 q = __ldg(reinterpret_cast<const int4*>(map + dc + u));
+                    sc[u] = q.x;
+                    sc[u + 1] = q.y;
+                    sc[u + 2] = q.z;
+                    sc[u + 3] = q.w;
                 }
-                // digits of I offset to be non-negative: 15-bit fields of I + 2^14 (1 + 2^15 + 2^30 + 2^45)
-                const unsigned long long f = (unsigned long long)(I + ((1ll << 14) + (1ll << 29) + (1ll << 44) + (1ll << 59)));
-                const uint32_t flo = (uint32_t)f, fhi = (uint32_t)(f >> 32);
-                const float off = 8388608.0f + 16384.0f;
-                d[u][0] = __uint_as_float(0x4B000000u | (flo & 0x7FFFu)) - off;
-                d[u][1] = __uint_as_float(0x4B000000u | ((flo >> 15) & 0x7FFFu)) - off;
-                d[u][2] = __uint_as_float(0x4B000000u | (__funnelshift_r(flo, fhi, 30) & 0x7FFFu)) - off;
-                d[u][3] = __uint_as_float(0x4B000000u | (fhi >> 13)) - off;
-                // x^ to a few FP32 roundings (the row norm's slack covers them)
-                const float xv = __fmaf_rn(__fmaf_rn(__fmaf_rn(d[u][3], 32768.0f, d[u][2]), 32768.0f, d[u][1]), 32768.0f,
-                                           d[u][0]) * scale;
-                l2sq = __fmaf_ru(xv, xv, l2sq);
+            } else {
+#pragma unroll
+                for (int u = 0; u < COLS; ++u) sc[u] = dc + u < a.ncols ? dc + u : -1;
             }
-#pragma unroll 2
+#pragma unroll
+            for (int u = 0; u < COLS; ++u) cur[u] = sc[u] >= 0 ? __ldg(src + sc[u]) : 0ull;
+#pragma unroll
+            for (int u = 0; u < COLS; u += 2) {
+                float dd[2][4];
+#pragma unroll
+                for (int w = 0; w < 2; ++w) {
+                    const unsigned long long bits = cur[u + w];
+                    const uint32_t blo = (uint32_t)bits, bhi = (uint32_t)(bits >> 32);
+                    const uint32_t E = (bhi >> 20) & 0x7FFu;
+                    // |x| = mant 2^(max(E, 1) - 1075); mant 2^10 shifted down by r >= 7 (bits <= 56), to
+                    // nearest, ties up
+                    uint32_t mhi = (bhi & 0xFFFFFu) | (E ? 0x100000u : 0u);
+                    const bool some = ((mhi | blo) != 0u) && E != 0x7FFu;   // not zero and finite
+                    nnz += some;
+                    const int r = min(r0 - max((int)E, 1), 64);
+                    unsigned long long m = ((unsigned long long)mhi << 32 | blo) << 10;
+                    m = some ? ((m >> (r - 1)) + 1ull) >> 1 : 0ull;
+                    const long long sgn = (long long)(int)bhi >> 31;
+                    const long long I = ((long long)m ^ sgn) - sgn;
+                    // digits of I offset to be non-negative: 15-bit fields of I + 2^14 (1 + 2^15 + 2^30 + 2^45)
+                    const unsigned long long f =
+                        (unsigned long long)(I + ((1ll << 14) + (1ll << 29) + (1ll << 44) + (1ll << 59)));
+                    const uint32_t flo = (uint32_t)f, fhi = (uint32_t)(f >> 32);
+                    const float off = 8388608.0f + 16384.0f;
+                    dd[w][0] = __uint_as_float(0x4B000000u | (flo & 0x7FFFu)) - off;
+                    dd[w][1] = __uint_as_float(0x4B000000u | ((flo >> 15) & 0x7FFFu)) - off;
+                    dd[w][2] = __uint_as_float(0x4B000000u | (__funnelshift_r(flo, fhi, 30) & 0x7FFFu)) - off;
+                    dd[w][3] = __uint_as_float(0x4B000000u | (fhi >> 13)) - off;
+                    // x^ to a few FP32 roundings (the row norm's slack covers them)
+                    const float xv = __fmaf_rn(__fmaf_rn(__fmaf_rn(dd[w][3], 32768.0f, dd[w][2]), 32768.0f, dd[w][1]),
+                                               32768.0f, dd[w][0]) * scale;
+                    l2sq = __fmaf_ru(xv, xv, l2sq);
+                }
+#pragma unroll
+                for (int k = 0; k < 4; ++k) d[u / 2][k] = pack2(dd[0][k], dd[1][k]);
+            }
+#pragma unroll 1
             for (int i = 0; i < nmod; ++i) {
                 const float k0 = c_tab.digit[tab][i][0], k1 = c_tab.digit[tab][i][1], k2 = c_tab.digit[tab][i][2],
                             k3 = c_tab.digit[tab][i][3], inv = c_tab.inv[i], neg_m = -c_tab.m[i];
-                uint32_t r[4];
+                const f32x2 q0 = pack2(k0, k0), q1 = pack2(k1, k1), q2 = pack2(k2, k2), q3 = pack2(k3, k3),
+                            inv2 = pack2(inv, inv), neg_m2 = pack2(neg_m, neg_m);
+                uint32_t o[COLS / 2];
 #pragma unroll
-                for (int u = 0; u < 4; ++u) {
-                    float t = __fmul_rn(d[u][0], k0);
-                    t = __fmaf_rn(d[u][1], k1, t);
-                    t = __fmaf_rn(d[u][2], k2, t);
-                    t = __fmaf_rn(d[u][3], k3, t);
-                    r[u] = __float_as_uint(mod_balanced(t, inv, neg_m));
+                for (int u = 0; u < COLS / 2; ++u) {
+                    uint32_t x, y;
+                    const f32x2 t = fma2(d[u][3], q3, fma2(d[u][2], q2, fma2(d[u][1], q1, mul2(d[u][0], q0))));
+                    unpack2(mod_balanced2(t, inv2, neg_m2), x, y);
+                    o[u] = __byte_perm(x, y, 0x7632);
                 }
-                *reinterpret_cast<uint2*>(drow + i * sstride + dc) =
-                    make_uint2(__byte_perm(r[0], r[1], 0x7632), __byte_perm(r[2], r[3], 0x7632));
+                __nv_bfloat16* dst = drow + i * sstride + dc;
+                if constexpr (COLS == 8) *reinterpret_cast<uint4*>(dst) = make_uint4(o[0], o[1], o[2], o[3]);
+                else *reinterpret_cast<uint2*>(dst) = make_uint2(o[0], o[1]);
             }
         }
         for (int o = 16; o > 0; o >>= 1) {
@@ -588,11 +655,18 @@ __device__ __forceinline__ void residue_rows(const SliceArgs& a0, const SliceGro
     }
 }
 
+// Four blocks of 256 threads (eight of 128) to an SM.  Measured, 12 000 rows of 12 288 columns and 13
+// moduli (1.15 GB read, 3.8 GB written): 0.96 ms, 5.1 TB/s, where scalar loads and scalar FP32 took
+// 1.04.  Neither the stores (one plane stored instead of 13: 0.95), the residues' arithmetic (none:
+// 0.91) nor the search for the maximum (none: 0.88) bounds it alone; more loads in flight per
+// thread cost resident blocks and gained nothing (0.96 to 1.03 over 2 to 5 blocks).
 template <int NT>
-__global__ void __launch_bounds__(NT) k_residue_slice(const SliceArgs a) { residue_rows<false, NT>(a, SliceGroups{}); }
+__global__ void __launch_bounds__(NT, 1024 / NT) k_residue_slice(const SliceArgs a) {
+    residue_rows<false, NT, NT == 256 ? 8 : 4>(a, SliceGroups{});
+}
 template <int NT>
-__global__ void __launch_bounds__(NT) k_residue_slice_grouped(const SliceGroups gs) {
-    residue_rows<true, NT>(SliceArgs{}, gs);
+__global__ void __launch_bounds__(NT, 1024 / NT) k_residue_slice_grouped(const SliceGroups gs) {
+    residue_rows<true, NT, NT == 256 ? 8 : 4>(SliceArgs{}, gs);
 }
 
 // ------------------------------------------------------------------- reconstruction
@@ -603,59 +677,57 @@ __host__ __device__ __forceinline__ int crt_rows(const CrtArgs& a) {
     return (long)a.rows * ((a.cols + kCrtCols - 1) / kCrtCols) >= 4096 ? kCrtRows : 1;
 }
 
-// Bits of the double nearest to F 2^-96 M 2^E0 (F a signed 96-bit integer in three words, M =
-// m_mant 2^(m_exp - 63)); *mag = |F| 2^-96 M 2^(E0 - es) as a float, truncated, in units of
-// 2^es.  Integer operations: the FP64 units are slow on this part.
+// Bits of the double nearest (ties up) to F 2^-80 M 2^E0: F a signed 80-bit integer in three words
+// (w2, w1, 16 bits w0), M = m_mant 2^(m_exp - 63), E = m_exp - 126 + E0; *mag = |value| 2^-es as a
+// float, truncated.  Integer operations: the FP64 units are slow on this part.
 __device__ __forceinline__ unsigned long long crt_bits(uint32_t w0, uint32_t w1, uint32_t w2, unsigned long long m_mant,
                                                        int E, int es, float* mag) {
+    const uint32_t sgn = (uint32_t)((int)w2 >> 31);
     unsigned long long hi = ((unsigned long long)w2 << 32) | w1;
-    const unsigned long long sign = hi & (1ull << 63);
-    if (sign) {   // |F|
-        w0 = 0u - w0;
-        hi = ~hi + (w0 == 0u ? 1ull : 0ull);
+    uint32_t lo = w0 << 16;       // the word below hi
+    if (sgn) {                    // |F|
+        lo = 0u - lo;
+        hi = ~hi + (lo == 0u ? 1ull : 0ull);
     }
     *mag = 0.0f;
-    if ((hi | w0) == 0ull) return 0ull;
-    int p;                       // position of the leading bit of |F|
-    unsigned long long f;        // its leading 64 bits
-    if (hi) {
-        const int z = __clzll((long long)hi);
-        p = 95 - z;
-        f = z ? (hi << z) | (z < 32 ? (unsigned long long)(w0 >> (32 - z)) : (unsigned long long)w0 << (z - 32)) : hi;
-    } else {
-        const int z = __clz((int)w0);
-        p = 31 - z;
-        f = (unsigned long long)w0 << (32 + z);
+    if (hi == 0ull) {             // |F| below 2^16: one step down
+        hi = (unsigned long long)lo << 16;
+        lo = 0u;
+        E -= 48;
+        if (hi == 0ull) return 0ull;
     }
-    unsigned long long P = __umul64hi(f, m_mant);
-    int ex = p + E;              // value = P 2^ex, E = m_exp - 158 + E0
-    if (!(P >> 63)) {
-        P = (P << 1) | ((f * m_mant) >> 63);
-        --ex;
+    // leading 64 bits
+    int z = __clzll((long long)hi);
+    E -= z;
+    uint32_t a2 = (uint32_t)(hi >> 32), a1 = (uint32_t)hi, a0 = lo;
+    if (z >= 32) {
+        a2 = a1;
+        a1 = a0;
+        a0 = 0u;
+        z -= 32;
     }
-    // magnitude in units of 2^es
-    const int fe = 63 + ex - es;
-    if (fe >= -126 && fe <= 127) *mag = __uint_as_float(((unsigned)(fe + 127) << 23) | (unsigned)((P >> 40) & 0x7FFFFFull));
-    unsigned long long q = P >> 11;
-    const unsigned int rem = (unsigned int)(P & 0x7FFull);
-    q += (rem > 0x400u || (rem == 0x400u && (q & 1ull))) ? 1ull : 0ull;
-    int be = ex + 63 + 1023;
-    if (q >> 53) {
-        q >>= 1;
-        ++be;
-    }
-    if (be <= 0 || be >= 2047)   // outside the normal range: the FP64 route
-        return sign | (unsigned long long)__double_as_longlong(ldexp((double)P, ex));
-    return sign | ((unsigned long long)be << 52) | (q & 0xFFFFFFFFFFFFFull);
+    const unsigned long long f = ((unsigned long long)__funnelshift_l(a1, a2, z) << 32) | __funnelshift_l(a0, a1, z);
+    const unsigned long long P = __umul64hi(f, m_mant);   // 63 or 64 bits; value = P 2^(E + 63)
+    const int top = (int)(P >> 63);
+    const int ex = E + 62 + 63 + top;                     // exponent of the leading bit
+    const int fe = ex - es;
+    if (fe >= -126 && fe <= 127)
+        *mag = __uint_as_float(((unsigned)(fe + 127) << 23) | ((unsigned)(P >> (39 + top)) & 0x7FFFFFu));
+    const unsigned long long q = ((P >> (9 + top)) + 1ull) >> 1;   // 53 bits, or 2^53
+    const int be = ex + 1023;
+    const unsigned long long sign = (unsigned long long)(sgn & 0x80000000u) << 32;
+    if (be <= 0 || be >= 2046)    // outside the normal range: the FP64 route
+        return sign | (unsigned long long)__double_as_longlong(ldexp((double)P, E + 63));
+    return sign | (((unsigned long long)(be - 1) << 52) + q);   // q's leading bit, or its carry, adds to the exponent
 }
 
 // Four columns per thread, crt_rows rows per block.  Per output: C / M = sum_i r_i / m_i mod 1 as
-// a 96-bit fixed-point sum (one 32 x 32 -> 64-bit multiply-add per 32-bit word of each 1 / m_i,
-// carries combined at the end), then value, certified bound and flag.  Reads the residues once
+// an 80-bit fixed-point sum (three multiply-adds per modulus, carries combined at the end), then value, certified bound and flag.  Reads the residues once
 // (2 bytes per modulus) and writes 8 (12 with bounds) bytes per output.  NM: the number of
 // moduli, 0 for any; all of a row's residues are loaded before the first is used.
-// Measured: 24.6 M outputs 237 us (0.14 ms at the copy bandwidth; the rest is integer issue),
-// four loads at a time 330; 50 x 600 outputs 7 us, four rows to a block there 20.
+// Measured: 24.6 M outputs 220 us (0.14 ms at the copy bandwidth; the rest is integer issue),
+// 96-bit sums and 64-bit finalisation 237, four loads at a time 330; 50 x 600 outputs 7 us, four
+// rows to a block there 20.
 template <bool G, int NM>
 __global__ void __launch_bounds__(kCrtThreads) k_crt(const CrtArgs a0, const CrtGroups gs) {
     __shared__ CrtArgs sa;
@@ -696,15 +768,16 @@ __global__ void __launch_bounds__(kCrtThreads) k_crt(const CrtArgs a0, const Crt
         for (int lr = lr0; lr < lr1; ++lr) {
             const int r = a.row0 + lr;
             const uint2* src = reinterpret_cast<const uint2*>(a.res + (long)lr * a.ldr + c);
-            unsigned long long s0[4] = {0, 0, 0, 0}, s1[4] = {0, 0, 0, 0}, s2[4] = {0, 0, 0, 0};
+            uint32_t s0[4] = {0, 0, 0, 0}, s2[4] = {0, 0, 0, 0};   // s0: 16 x 25 bits; s2 wraps (mod 1)
+            unsigned long long s1[4] = {0, 0, 0, 0};
             auto add = [&](int i, uint2 v) {
                 const uint32_t f0 = c_tab.frac[i][0], f1 = c_tab.frac[i][1], f2 = c_tab.frac[i][2];
                 const uint32_t x[4] = {v.x & 0xFFFFu, v.x >> 16, v.y & 0xFFFFu, v.y >> 16};
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
-                    s0[j] += (unsigned long long)x[j] * f0;
+                    s0[j] += x[j] * f0;
                     s1[j] += (unsigned long long)x[j] * f1;
-                    s2[j] += (unsigned long long)x[j] * f2;
+                    s2[j] += x[j] * f2;
                 }
             };
             if (NM) {
@@ -724,28 +797,30 @@ __global__ void __launch_bounds__(kCrtThreads) k_crt(const CrtArgs a0, const Crt
             float rowerr2 = 0.0f;
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
-                const unsigned long long t1 = s1[j] + (s0[j] >> 32);
-                const unsigned long long t2 = s2[j] + (t1 >> 32);
+                const unsigned long long t1 = s1[j] + (s0[j] >> 16);
                 const int es = eA + eB[j];
                 float av;
-                unsigned long long vb = 0ull;
                 bout[j] = 0.0f;
                 vout[j] = 0.0;
                 if (l2A == 0.0f || l2B[j] == 0.0f) continue;   // an exact zero
-                vb = crt_bits((uint32_t)s0[j], (uint32_t)t1, (uint32_t)t2, a.m_mant, a.m_exp - 158 + es - 2 * a.bits, es,
-                              &av);
+                const unsigned long long vb = crt_bits(s0[j] & 0xFFFFu, (uint32_t)t1, s2[j] + (uint32_t)(t1 >> 32),
+                                                       a.m_mant, a.m_exp - 126 + es - 2 * a.bits, es, &av);
                 vout[j] = __longlong_as_double((long long)vb);
                 const float f64b = __fmul_ru(cf64A, l2B[j]);
                 const float limit = a.flag_mode == 1 ? fmaxf(a.tol * av, f64b) : f64b;
                 // |x^ y^ - X Y| <= ||x^ - X|| ||y^|| + ||X|| ||y^ - Y||
                 float bound = __fadd_ru(__fmaf_ru(dqA, l2B[j], __fmul_ru(l2A, dqB[j])), a.c_fix);
                 bound = __fmaf_ru(inA, l2B[j], bound);
-                bout[j] = es > 127 ? __int_as_float(0x7f800000) : __fmul_ru(bound, pow2f(max(es, -126)));
-                const float bb = __fmul_ru(bound, pow2f(max(-126, min(127, eB[j]))));
-                rowerr2 = __fmaf_ru(bb, bb, rowerr2);
+                if (a.bnd) bout[j] = es > 127 ? __int_as_float(0x7f800000) : __fmul_ru(bound, pow2f(max(es, -126)));
+                if (a.rowerr2) {
+                    const float bb = __fmul_ru(bound, pow2f(max(-126, min(127, eB[j]))));
+                    rowerr2 = __fmaf_ru(bb, bb, rowerr2);
+                }
                 if (c + j < a.cols_valid) {
-                    const unsigned long long ab = vb & 0x7FFFFFFFFFFFFFFFull;
-                    vmax = ab > vmax ? ab : vmax;
+                    if (a.absmax) {
+                        const unsigned long long ab = vb & 0x7FFFFFFFFFFFFFFFull;
+                        vmax = ab > vmax ? ab : vmax;
+                    }
                     if (bound > limit) {
                         const unsigned int idx = atomicAdd(a.nflags, 1u);
                         if ((int)idx < a.max_flags) a.flags[idx] = make_int2(r, c + j);
@@ -846,9 +921,10 @@ void crt_constants(CrtArgs* a) {
     }
     a->m_mant = mant;
     a->m_exp = top;
-    // each floor(2^96 / m_i) is short of 2^96 / m_i by less than one unit, times r_i < m_i;
-    // units of 2^{eA+eB}: M 2^-96 2^(-2 bits).  The final rounding is a relative 2^-53.
-    a->c_fix = (float)(std::ldexp(msum, top + 1 - 96 - 2 * a->bits) * 1.01);
+    // each floor(2^80 / m_i) is short of 2^80 / m_i by less than one unit, times r_i < m_i;
+    // units of 2^{eA+eB}: M 2^-80 2^(-2 bits) (2^-51 for 13 moduli at 48 bits).  The final
+    // rounding is a relative 2^-53.
+    a->c_fix = (float)(std::ldexp(msum, top + 1 - 80 - 2 * a->bits) * 1.01);
 }
 
 int crt_blocks(const CrtArgs& a) {
