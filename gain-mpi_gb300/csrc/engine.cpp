@@ -349,9 +349,16 @@ struct gain_engine_s {
     gain::DevArray<int> iota;
     gain::DevArray<float> rowerr;
     gain::DevArray<int2> flags1, flags2;
-    gain::DevArray<unsigned int> counters;      // [0] nflags1 [1] nflags2
-    gain::DevArray<unsigned long long> ull;     // [0] uncertified [1] nkeep
-    gain::DevArray<int> err;
+    // a run's counters, in one block that one copy reads back: refinement counts, sums, error word
+    gain::DevArray<unsigned long long> words;
+    unsigned int* counters() const { return (unsigned int*)words.p; }   // [0] nflags1 [1] nflags2
+    unsigned long long* ull() const { return words.p + 2; }   // [0] uncertified [2] amp max [3] uncertified weak
+    int* err() const { return (int*)(words.p + 6); }
+    // page-locked area the run's small uploads (level lists, tile lists) are read from by one
+    // kernel; stage_busy: a launched kernel may still be reading it
+    char* stage = nullptr;
+    size_t stage_cap = 0;
+    bool stage_busy = false;
     gain::DevArray<gain::split::Tile> tiles1, tiles2;
     gain::DevArray<gain::split::Prod> prods1, prods2;
     gain::DevArray<gain::split::ResTile> rtiles1, rtiles2;
@@ -374,6 +381,7 @@ namespace gain {
 namespace {
 
 constexpr int kMaxFlags = 1 << 22;
+constexpr int kRunWords = 8;
 
 gain_status check_engine(gain_engine e) {
     if (!e) return set_error(GAIN_ERR_INVALID_ARG, "engine is NULL");
@@ -1222,50 +1230,61 @@ bool residue_wide(const std::vector<ColumnRange>& cols, int row_tiles, int nmod,
 // across the columns.
 int residue_panel(int mstep) { return kRowGroup * mstep; }
 
-// Panel by panel: the residue GEMM over `parts` (column ranges; before part p > 0 the stream
-// waits for `waits[p]`), then the reconstruction of all columns from `crt` (res, plane, row0
-// and rows are set here).  Returns the MMA flops through *flops.
-gain_status residue_gemm(gain_engine e, const CUtensorMap& tmA, const CUtensorMap& tmB,
-                         const std::vector<std::vector<ColumnRange>>& parts, const cudaEvent_t* waits, int B, int Bpad,
-                         bool pair, split::CrtArgs crt, DevArray<split::ResTile>& d_tiles, cudaEvent_t ev_done,
-                         double* flops) {
-    cudaStream_t st = e->st;
+// The tiles of a residue GEMM over `parts` (lists of column ranges that are launched one after
+// the other): those of a full panel of rows and those of the last one.
+struct ResiduePlan {
+    std::vector<split::ResTile> tiles;
+    struct Span { int first, count; };
+    std::vector<std::array<Span, 2>> spans;   // per part
+    int rows0 = 0, rows1 = 0;                 // rows of a full panel; of a shorter last one (0: none)
+    double flops = 0.0;
+};
+ResiduePlan residue_plan(gain_engine e, const std::vector<std::vector<ColumnRange>>& parts, int Bpad, bool pair, int nmod) {
     const int mstep = pair ? 2 * split::BM : split::BM, panel = residue_panel(mstep);
     const int units = pair ? e->num_sms / 2 : e->num_sms;
-    std::vector<split::ResTile> all;
-    struct Span { int first, count; };
-    std::vector<std::array<Span, 2>> spans(parts.size());   // tiles of a full panel and of the last one
-    const int rows0 = std::min(Bpad, panel), rows1 = Bpad % panel;
-    double f = 0.0;
-    for (size_t p = 0; p < parts.size(); ++p) {
-        const bool wide = pair && residue_wide(parts[p], rows0 / mstep, crt.nmod, units);
-        const int a0 = (int)all.size();
-        residue_tiles(parts[p], rows0, mstep, wide, all);
-        const int a1 = (int)all.size();
-        spans[p][0] = spans[p][1] = {a0, a1 - a0};
-        if (Bpad > panel && rows1) {
-            residue_tiles(parts[p], rows1, mstep, wide, all);
-            spans[p][1] = {a1, (int)all.size() - a1};
+    ResiduePlan P;
+    P.rows0 = std::min(Bpad, panel);
+    P.rows1 = Bpad > panel ? Bpad % panel : 0;
+    for (const auto& cols : parts) {
+        const bool wide = pair && residue_wide(cols, P.rows0 / mstep, nmod, units);
+        const int a0 = (int)P.tiles.size();
+        residue_tiles(cols, P.rows0, mstep, wide, P.tiles);
+        const int a1 = (int)P.tiles.size();
+        std::array<ResiduePlan::Span, 2> sp;
+        sp[0] = sp[1] = {a0, a1 - a0};
+        if (P.rows1) {
+            residue_tiles(cols, P.rows1, mstep, wide, P.tiles);
+            sp[1] = {a1, (int)P.tiles.size() - a1};
         }
-        for (const ColumnRange& c : parts[p]) f += 2.0 * Bpad * (c.n1 - c.n0) * (double)c.nkb * split::BK * crt.nmod;
+        P.spans.push_back(sp);
+        for (const ColumnRange& c : cols) P.flops += 2.0 * Bpad * (c.n1 - c.n0) * (double)c.nkb * split::BK * nmod;
     }
-    if (flops) *flops += f;
-    if (!all.empty()) GAIN_TRY(d_tiles.upload(all));
+    return P;
+}
+
+// Panel by panel: the residue GEMM over P's parts (before part p > 0 the stream waits for
+// waits[p]), then the reconstruction of all columns from `crt` (res, plane, row0 and rows are
+// set here).  d_tiles: P.tiles on the device.
+gain_status residue_gemm(gain_engine e, const CUtensorMap& tmA, const CUtensorMap& tmB, const ResiduePlan& P,
+                         const split::ResTile* d_tiles, const cudaEvent_t* waits, int B, int Bpad, bool pair,
+                         split::CrtArgs crt, cudaEvent_t ev_done) {
+    cudaStream_t st = e->st;
+    const int panel = residue_panel(pair ? 2 * split::BM : split::BM);
     split::ResGemmArgs g;
     memset(&g, 0, sizeof g);
     g.nmod = crt.nmod;
     g.res = e->res.p;
     g.ldr = crt.ldr;
-    g.plane = (long)rows0 * crt.ldr;
-    g.err = e->err.p;
+    g.plane = (long)P.rows0 * crt.ldr;
+    g.err = e->err();
     for (int m0 = 0; m0 < Bpad; m0 += panel) {
         const bool last = m0 + panel >= Bpad;
         g.m_base = m0;
-        for (size_t p = 0; p < parts.size(); ++p) {
-            const Span& sp = spans[p][last && m0 > 0 && rows1 ? 1 : 0];
+        for (size_t p = 0; p < P.spans.size(); ++p) {
+            const ResiduePlan::Span& sp = P.spans[p][last && m0 > 0 && P.rows1 ? 1 : 0];
             if (p > 0 && m0 == 0 && waits) GAIN_CUDA(cudaStreamWaitEvent(st, waits[p], 0));
             if (!sp.count) continue;
-            g.tiles = d_tiles.p + sp.first;
+            g.tiles = d_tiles + sp.first;
             g.ntiles = sp.count;
             GAIN_CUDA(split::launch_residue_gemm(tmA, tmB, g, e->num_sms, st, pair));
             ++e->launches;
@@ -1282,6 +1301,60 @@ gain_status residue_gemm(gain_engine e, const CUtensorMap& tmA, const CUtensorMa
     }
     return GAIN_OK;
 }
+
+// A run's small uploads and clears as ONE kernel on the engine's stream, which reads the data
+// from page-locked host memory.  Each synchronous copy instead cost about 10 us of a small
+// run; an asynchronous one would queue in the host-to-device engine behind an eigenvector copy
+// still in flight and hold the run back until that ended.
+struct Staging {
+    StageArgs a{};
+    std::vector<const void*> src;
+    gain_status add(void* dst, const void* from, size_t bytes) {   // from NULL: zeros; whole words
+        if (!bytes) return GAIN_OK;
+        if (a.n == kStageSegs || bytes % 4 || bytes / 4 > 0x7FFFFFFFu)
+            return set_error(GAIN_ERR_INVALID_ARG, "staged uploads: too many or odd sizes");
+        a.seg[a.n].dst = (uint32_t*)dst;
+        a.seg[a.n].words = (unsigned int)(bytes / 4);
+        src.push_back(from);
+        ++a.n;
+        return GAIN_OK;
+    }
+    template <class T>
+    gain_status add(DevArray<T>& d, const T* from, size_t count) {
+        GAIN_TRY(d.alloc(count));
+        return add(d.p, from, sizeof(T) * count);
+    }
+    gain_status launch(gain_engine e, cudaStream_t st) {
+        size_t need = 0;
+        for (int k = 0; k < a.n; ++k)
+            if (src[k]) need += ((size_t)a.seg[k].words * 4 + 15) / 16 * 16;
+        if (e->stage_busy) {   // an earlier run stopped before it synchronised
+            GAIN_CUDA(cudaStreamSynchronize(st));
+            e->stage_busy = false;
+        }
+        if (need > e->stage_cap) {
+            if (e->stage) cudaFreeHost(e->stage);
+            e->stage = nullptr;
+            e->stage_cap = 0;
+            const size_t cap = std::max<size_t>(2 * need, 64 << 10);
+            GAIN_CUDA(cudaMallocHost((void**)&e->stage, cap));
+            e->stage_cap = cap;
+        }
+        size_t off = 0;
+        for (int k = 0; k < a.n; ++k) {
+            a.seg[k].src = nullptr;
+            if (!src[k]) continue;
+            const size_t bytes = (size_t)a.seg[k].words * 4;
+            memcpy(e->stage + off, src[k], bytes);
+            a.seg[k].src = (const uint32_t*)(e->stage + off);
+            off += (bytes + 15) / 16 * 16;
+        }
+        e->stage_busy = true;
+        GAIN_CUDA(launch_stage(a, st));
+        ++e->launches;
+        return GAIN_OK;
+    }
+};
 
 gain_status run_split(gain_engine e, const gain_pair_job* j, int dI, int dF, const gain_split_opts* opts,
                       gain_stats* stats) {
@@ -1365,16 +1438,30 @@ gain_status run_split(gain_engine e, const gain_pair_job* j, int dI, int dF, con
         for (int u = 0; u < cand && in_head; ++u) in_head = j->upper_levels[u] < EF.head_rows;
         if (in_head) Nu2 = cand;
     }
-    // Small uploads stay synchronous: an asynchronous copy on this stream would queue in the
-    // host-to-device engine behind an eigenvector copy still in flight and hold GEMM 1 back.
-    GAIN_TRY(e->d_lower.upload(j->lower_levels, B));
-    GAIN_TRY(e->d_upper.upload(j->upper_levels, Nu));
-    GAIN_TRY(e->counters.alloc(4));
-    GAIN_TRY(e->counters.zero(st, 4));
-    GAIN_TRY(e->ull.alloc(4));
-    GAIN_TRY(e->ull.zero(st, 4));
-    GAIN_TRY(e->err.alloc(1));
-    GAIN_TRY(e->err.zero(st, 1));
+    GAIN_TRY(e->words.alloc(kRunWords));
+    GAIN_TRY(e->rowerr.alloc(Bpad));
+    ResiduePlan rp1, rp2;
+    Staging up;
+    GAIN_TRY(up.add(e->d_lower, j->lower_levels, B));
+    GAIN_TRY(up.add(e->d_upper, j->upper_levels, Nu));
+    GAIN_TRY(up.add(e->words.p, nullptr, sizeof(unsigned long long) * kRunWords));
+    GAIN_TRY(up.add(e->rowerr.p, nullptr, sizeof(float) * Bpad));
+    if (res) {
+        if (npieces == 1) {
+            std::vector<ColumnRange> cols;
+            for (auto& fb : L.fblocks)
+                cols.push_back({fb.first, fb.second, L.band_k0[fb.first], L.band_len[fb.first] / split::BK});
+            rp1 = residue_plan(e, {cols}, Bpad, pair, p1x.slices);
+            GAIN_TRY(up.add(e->rtiles1, rp1.tiles.data(), rp1.tiles.size()));
+        }
+        const int nkb2 = K2 / split::BK;
+        std::vector<std::vector<ColumnRange>> parts;
+        if (Nu2 > 0) parts = {{{0, Nu2, 0, nkb2}}, {{Nu2, Nupad, 0, nkb2}}};
+        else parts = {{{0, Nupad, 0, nkb2}}};
+        rp2 = residue_plan(e, parts, Bpad, pair, p2.slices);
+        GAIN_TRY(up.add(e->rtiles2, rp2.tiles.data(), rp2.tiles.size()));
+    }
+    GAIN_TRY(up.launch(e, st));
     GAIN_TRY(e->flags1.alloc(kMaxFlags));
     GAIN_TRY(e->flags2.alloc(kMaxFlags));
     // capacity of the refinement lists (GAINLS_MAX_FLAGS lowers it, to exercise the overflow
@@ -1462,8 +1549,6 @@ gain_status run_split(gain_engine e, const gain_pair_job* j, int dI, int dF, con
     if (!res) GAIN_TRY(e->prods1.upload(pr1));
     double res_flops = 0.0;
     GAIN_TRY(e->H.alloc((size_t)Bpad * L.fpad));
-    GAIN_TRY(e->rowerr.alloc(Bpad));
-    GAIN_TRY(e->rowerr.zero(st, Bpad));
     if (npieces > 1) {
         GAIN_TRY(e->acc.alloc((size_t)Bpad * L.fpad));
         GAIN_TRY(e->acc.zero(st, (size_t)Bpad * L.fpad));
@@ -1477,7 +1562,7 @@ gain_status run_split(gain_engine e, const gain_pair_job* j, int dI, int dF, con
         if (piece > 0) {   // the next piece's band (the previous GEMM and refinement read theirs)
             GAIN_CUDA(cudaStreamSynchronize(st));
             unsigned int c0 = 0;
-            GAIN_CUDA(cudaMemcpy(&c0, e->counters.p, sizeof c0, cudaMemcpyDeviceToHost));
+            GAIN_CUDA(cudaMemcpy(&c0, e->counters(), sizeof c0, cudaMemcpyDeviceToHost));
             inexact_prev += c0;
             overflow_prev = overflow_prev || c0 > (unsigned)max_flags;
             GAIN_TRY(load_piece(e, piece));
@@ -1485,13 +1570,14 @@ gain_status run_split(gain_engine e, const gain_pair_job* j, int dI, int dF, con
             L.dip_version = e->dip_version;
             L.dig = {};
             GAIN_TRY(band_digits());
-            GAIN_CUDA(cudaMemsetAsync(e->counters.p, 0, sizeof(unsigned int), st));
+            GAIN_CUDA(cudaMemsetAsync(e->counters(), 0, sizeof(unsigned int), st));
         }
         if (npieces > 1) GAIN_CUDA(cudaMemsetAsync(e->H.p, 0, sizeof(double) * (size_t)Bpad * L.fpad, st));
         t1.clear();
         std::vector<ColumnRange> cols1;
         for (auto& fb : L.fblocks)
             for (int n0 = fb.first; n0 < fb.second; n0 += split::BN) {
+                if (res && npieces == 1) continue;   // planned above
                 if (npieces > 1) {   // only column tiles holding an upper function of this piece
                     bool any = false;
                     for (int r = n0; r < n0 + split::BN && r < L.fpad && !any; ++r) {
@@ -1550,11 +1636,11 @@ gain_status run_split(gain_engine e, const gain_pair_job* j, int dI, int dF, con
         g1.flag_mode = 2;   // every H entry FP64-grade, else recomputed in FP64
         g1.tol = (float)tol;
         g1.flags = e->flags1.p;
-        g1.nflags = e->counters.p + 0;
+        g1.nflags = e->counters() + 0;
         g1.max_flags = max_flags;
         g1.rows_valid = B;
         g1.cols_valid = L.fpad;
-        g1.err = e->err.p;
+        g1.err = e->err();
         g1.fuse = fuse1;
         if (piece == 0) GAIN_CUDA(cudaEventRecord(e->ev[2], st));
         if (res) {
@@ -1581,8 +1667,13 @@ gain_status run_split(gain_engine e, const gain_pair_job* j, int dI, int dF, con
                 GAIN_CUDA(cudaMemsetAsync(e->res.p, 0,
                                           sizeof(uint16_t) * (size_t)std::min(Bpad, residue_panel(mstep)) * L.fpad *
                                               p1x.slices, st));
-            GAIN_TRY(residue_gemm(e, tmV, L.tmBandPair, {cols1}, nullptr, B, Bpad, pair, c1, e->rtiles1,
-                                  piece == npieces - 1 ? e->ev[3] : nullptr, &res_flops));
+            if (npieces > 1) {
+                rp1 = residue_plan(e, {cols1}, Bpad, pair, p1x.slices);
+                GAIN_TRY(e->rtiles1.upload(rp1.tiles));
+            }
+            res_flops += rp1.flops;
+            GAIN_TRY(residue_gemm(e, tmV, L.tmBandPair, rp1, e->rtiles1.p, nullptr, B, Bpad, pair, c1,
+                                  piece == npieces - 1 ? e->ev[3] : nullptr));
         } else {
             if (!t1.empty()) {
                 GAIN_CUDA(split::launch_gemm(tmV, pair ? L.tmBandPair : L.tmBand, g1, e->num_sms, st, pair));
@@ -1613,7 +1704,7 @@ gain_status run_split(gain_engine e, const gain_pair_job* j, int dI, int dF, con
         // inexact first-GEMM entries recomputed in FP64
         split::RefineHArgs rh;
         rh.flags = e->flags1.p;
-        rh.nflags = e->counters.p + 0;
+        rh.nflags = e->counters() + 0;
         rh.max_flags = max_flags;
         rh.vecs = L.general ? e->primI.p : EI.d.p;
         rh.nsize = L.general ? bIs.dimen : EI.nsize;
@@ -1694,15 +1785,15 @@ gain_status run_split(gain_engine e, const gain_pair_job* j, int dI, int dF, con
     g2.c_fix = fix_const((int)pr2.size());
     g2.c_f64 = (float)((double)((L.general ? L.nsymF : L.nF) + 64) * std::ldexp(1.0, -53) * 1.01);
     g2.rowerr2 = nullptr;
-    g2.absmax = e->ull.p + 2;
+    g2.absmax = e->ull() + 2;
     g2.flag_mode = 1;
     g2.tol = (float)tol;
     g2.flags = e->flags2.p;
-    g2.nflags = e->counters.p + 1;
+    g2.nflags = e->counters() + 1;
     g2.max_flags = max_flags;
     g2.rows_valid = B;
     g2.cols_valid = Nu;
-    g2.err = e->err.p;
+    g2.err = e->err();
     g2.bnd = e->ampbnd.p;
     g2.ldb = Nupad;
     GAIN_CUDA(cudaEventRecord(e->ev[4], st));
@@ -1728,11 +1819,9 @@ gain_status run_split(gain_engine e, const gain_pair_job* j, int dI, int dF, con
         c2.nflags = g2.nflags;
         c2.max_flags = max_flags;
         split::crt_constants(&c2);
-        std::vector<std::vector<ColumnRange>> parts;
-        if (Nu2 > 0) parts = {{{0, Nu2, 0, K2 / split::BK}}, {{Nu2, Nupad, 0, K2 / split::BK}}};
-        else parts = {{{0, Nupad, 0, K2 / split::BK}}};
         const cudaEvent_t waits[2] = {nullptr, e->ev[7]};
-        GAIN_TRY(residue_gemm(e, tmH, tmU, parts, waits, B, Bpad, pair, c2, e->rtiles2, e->ev[5], &res_flops));
+        res_flops += rp2.flops;
+        GAIN_TRY(residue_gemm(e, tmH, tmU, rp2, e->rtiles2.p, waits, B, Bpad, pair, c2, e->ev[5]));
     } else if (Nu2 > 0) {
         // tiles are upper-block-major: those of the first half (n0 < Nu2) come first
         int n1 = 0;
@@ -1752,7 +1841,7 @@ gain_status run_split(gain_engine e, const gain_pair_job* j, int dI, int dF, con
     if (!res) GAIN_CUDA(cudaEventRecord(e->ev[5], st));
     split::RefineAmpArgs ra;
     ra.flags = e->flags2.p;
-    ra.nflags = e->counters.p + 1;
+    ra.nflags = e->counters() + 1;
     ra.max_flags = max_flags;
     ra.U = EF.d.p;
     ra.nsize = EF.nsize;
@@ -1767,10 +1856,10 @@ gain_status run_split(gain_engine e, const gain_pair_job* j, int dI, int dF, con
     ra.bnd = e->ampbnd.p;
     ra.ldb = Nupad;
     ra.tol = tol;
-    ra.absmax = e->ull.p + 2;
+    ra.absmax = e->ull() + 2;
     ra.amp_floor = std::sqrt((opts && opts->s_floor > 0) ? opts->s_floor : 1e-10);
-    ra.uncertified = e->ull.p;
-    ra.uncertified_weak = e->ull.p + 3;
+    ra.uncertified = e->ull();
+    ra.uncertified_weak = e->ull() + 3;
     GAIN_CUDA(split::launch_refine_amp(ra, 4 * e->num_sms, st));
     ++e->launches;
     GAIN_CUDA(cudaEventRecord(e->ev[1], st));
@@ -1781,13 +1870,12 @@ gain_status run_split(gain_engine e, const gain_pair_job* j, int dI, int dF, con
     {   // the run's counters through one page-locked area
         if (!e->readback) GAIN_CUDA(cudaMallocHost(&e->readback, 128));
         char* rb = (char*)e->readback;
-        GAIN_CUDA(cudaMemcpyAsync(rb, e->counters.p, sizeof cnt, cudaMemcpyDeviceToHost, st));
-        GAIN_CUDA(cudaMemcpyAsync(rb + 32, e->ull.p, sizeof unc, cudaMemcpyDeviceToHost, st));
-        GAIN_CUDA(cudaMemcpyAsync(rb + 64, e->err.p, sizeof errw, cudaMemcpyDeviceToHost, st));
+        GAIN_CUDA(cudaMemcpyAsync(rb, e->words.p, sizeof(unsigned long long) * kRunWords, cudaMemcpyDeviceToHost, st));
         GAIN_CUDA(cudaStreamSynchronize(st));
+        e->stage_busy = false;
         memcpy(cnt, rb, sizeof cnt);
-        memcpy(unc, rb + 32, sizeof unc);
-        memcpy(&errw, rb + 64, sizeof errw);
+        memcpy(unc, rb + 16, sizeof unc);
+        memcpy(&errw, rb + 48, sizeof errw);
     }
     e->amp_rows = B;
     e->amp_cols = Nu;
@@ -1931,6 +2019,7 @@ void destroy_engine(gain_engine e) {
     if (e->st2) cudaStreamDestroy(e->st2);
     if (e->st) cudaStreamDestroy(e->st);
     if (e->readback) cudaFreeHost(e->readback);
+    if (e->stage) cudaFreeHost(e->stage);
     delete e;
 }
 
@@ -2948,11 +3037,11 @@ gain_status gain_selftest_bounded_wait(gain_engine e, double limit_ms) {
     GAIN_TRY(check_engine(e));
     if (!(limit_ms > 0.0) || limit_ms > 1000.0)
         return set_error(GAIN_ERR_INVALID_ARG, "gain_selftest_bounded_wait: limit outside (0, 1000] ms");
-    GAIN_TRY(e->err.alloc(1));
-    GAIN_TRY(e->err.zero(e->st, 1));
-    GAIN_CUDA(split::launch_wait_selftest((unsigned long long)(limit_ms * 1e6), e->err.p, e->st));
+    GAIN_TRY(e->words.alloc(kRunWords));
+    GAIN_TRY(e->words.zero(e->st, kRunWords));
+    GAIN_CUDA(split::launch_wait_selftest((unsigned long long)(limit_ms * 1e6), e->err(), e->st));
     int code = 0;
-    GAIN_CUDA(cudaMemcpyAsync(&code, e->err.p, sizeof code, cudaMemcpyDeviceToHost, e->st));
+    GAIN_CUDA(cudaMemcpyAsync(&code, e->err(), sizeof code, cudaMemcpyDeviceToHost, e->st));
     GAIN_CUDA(cudaStreamSynchronize(e->st));
     if (code != 0)
         return set_error(GAIN_ERR_TIMEOUT, "bounded device wait gave up after %.3f ms (code %d)", limit_ms, code);
@@ -3112,15 +3201,23 @@ gain_status pair_lines(gain_engine e, const gain_line_params* prm, const double*
     const int rows = e->amp_rows, cols = e->amp_cols;
     const size_t n = (size_t)rows * cols;
     cudaStream_t st = e->st;
-    GAIN_TRY(e->eIdev.upload(energiesI, rows));
-    GAIN_TRY(e->eFdev.upload(energiesF, cols));
+    GAIN_TRY(e->lcnt.alloc(1));
+    if (async) {   // (nothing of this call may stay in the staging area once it returns)
+        GAIN_TRY(e->eIdev.upload(energiesI, rows));
+        GAIN_TRY(e->eFdev.upload(energiesF, cols));
+        GAIN_TRY(e->lcnt.zero(st, 1));
+    } else {
+        Staging up;
+        GAIN_TRY(up.add(e->eIdev, energiesI, rows));
+        GAIN_TRY(up.add(e->eFdev, energiesF, cols));
+        GAIN_TRY(up.add(e->lcnt.p, nullptr, sizeof(unsigned long long)));
+        GAIN_TRY(up.launch(e, st));
+    }
     GAIN_TRY(thresh_certify(e, prm, p, amp, ld));
     if (S) GAIN_TRY(e->lineS.alloc(n));
     if (A) GAIN_TRY(e->lineA.alloc(n));
     if (I) GAIN_TRY(e->lineI.alloc(n));
     if (keep) GAIN_TRY(e->lineKeep.alloc(n));
-    GAIN_TRY(e->lcnt.alloc(1));
-    GAIN_TRY(e->lcnt.zero(st, 1));
     // only the requested outputs are written
     GAIN_CUDA(launch_lines(rows, cols, amp, ld, e->eIdev.p, e->eFdev.p, p, S ? e->lineS.p : nullptr,
                            A ? e->lineA.p : nullptr, I ? e->lineI.p : nullptr, keep ? e->lineKeep.p : nullptr,
@@ -3150,6 +3247,7 @@ gain_status pair_lines(gain_engine e, const gain_line_params* prm, const double*
     if (I) GAIN_CUDA(cudaMemcpyAsync(I, e->lineI.p, sizeof(double) * n, cudaMemcpyDeviceToHost, st));
     if (keep) GAIN_CUDA(cudaMemcpyAsync(keep, e->lineKeep.p, n, cudaMemcpyDeviceToHost, st));
     GAIN_CUDA(cudaStreamSynchronize(st));
+    e->stage_busy = false;
     if (n_lines) *n_lines = (long long)nk;
     return GAIN_OK;
 }

@@ -427,6 +427,14 @@ __global__ void k_add(double* __restrict__ acc, const double* __restrict__ x, lo
         acc[i] += x[i];
 }
 
+__global__ void __launch_bounds__(256) k_stage(const StageArgs a) {
+    for (int k = 0; k < a.n; ++k) {
+        const StageArgs::Seg s = a.seg[k];
+        for (unsigned int i = blockIdx.x * 256 + threadIdx.x; i < s.words; i += gridDim.x * 256)
+            s.dst[i] = s.src ? s.src[i] : 0u;
+    }
+}
+
 // S / A / I of every amplitude (non-degenerate symmetries), Output.cpp:52-112.
 // Grid-stride over the rows x cols lines (each pass coalesced); the kept-line count is
 // reduced in the block and added once per block.
@@ -520,6 +528,14 @@ __global__ void k_patch(int n, const long long* __restrict__ pairs, const double
 }
 
 }  // namespace
+
+cudaError_t launch_stage(const StageArgs& a, cudaStream_t st) {
+    unsigned int most = 0;
+    for (int k = 0; k < a.n; ++k) most = std::max(most, a.seg[k].words);
+    if (!most) return cudaSuccess;
+    k_stage<<<std::min((most + 255) / 256, 128u), 256, 0, st>>>(a);
+    return cudaGetLastError();
+}
 
 cudaError_t launch_thresh_flag(int rows, int cols, const double* amp, long ld, const float* bnd, long ldb,
                                const double* eI, const double* eF, const LineParams& p, int2* list,

@@ -140,6 +140,19 @@ cudaError_t launch_contract_rowerr(int rows, const double* Hp, long ldp, int nco
 // acc[i] += x[i], i < n
 cudaError_t launch_add(double* acc, const double* x, long n, cudaStream_t st);
 
+// Small uploads and clears in one launch: seg[k] receives `words` 32-bit words from src (page-locked
+// host memory), or zeros (src NULL).
+constexpr int kStageSegs = 8;
+struct StageArgs {
+    struct Seg {
+        uint32_t* dst;
+        const uint32_t* src;
+        unsigned int words;
+    } seg[kStageSegs];
+    int n;
+};
+cudaError_t launch_stage(const StageArgs& a, cudaStream_t st);
+
 // S, A, I of a [rows x cols] amplitude block, Output.cpp:52-112
 constexpr int kMaxDegSlots = 9;   // degenerate component pairs of one line (maxdeg <= 3)
 struct LineParams {
