@@ -1217,12 +1217,23 @@ void residue_tiles(const std::vector<ColumnRange>& cols, int rows, int mstep, bo
         }
 }
 
-// 256-column tiles where they still give every unit several (tile, modulus) items; smaller
-// problems take 128-column tiles, twice as many items.
+// 256- or 128-column tiles: the shorter estimated launch, rounds of items per unit times an
+// item's clocks.  A 16-deep MMA of a CTA pair takes 128 clocks at 256 columns and (paced by shared
+// memory) about 100 at 128, an item about 2500 more (first loads, last drain, residue stores).
 bool residue_wide(const std::vector<ColumnRange>& cols, int row_tiles, int nmod, int units) {
-    long w = 0;
-    for (const ColumnRange& c : cols) w += (c.n1 - c.n0 + 255) / 256;
-    return w * row_tiles * nmod >= 4L * units;
+    double wide = 0.0, narrow = 0.0;
+    long nw = 0, nn = 0;
+    for (const ColumnRange& c : cols) {
+        const long w = (c.n1 - c.n0) / 256, n = (c.n1 - c.n0) / 128, k = 4L * c.nkb;
+        nw += w + (n & 1);
+        nn += n;
+        wide += w * (128.0 * k + 2500.0) + (n & 1) * (100.0 * k + 2500.0);
+        narrow += n * (100.0 * k + 2500.0);
+    }
+    if (!nn) return false;
+    const double items = (double)row_tiles * nmod;
+    const double rw = std::ceil(nw * items / units), rn = std::ceil(nn * items / units);
+    return rw * (wide / nw) <= rn * (narrow / nn);
 }
 
 // Output rows per launch of a residue GEMM and its reconstruction: the residues of one such
