@@ -1278,7 +1278,7 @@ ResiduePlan residue_plan(gain_engine e, const std::vector<std::vector<ColumnRang
 // set here).  d_tiles: P.tiles on the device.
 gain_status residue_gemm(gain_engine e, const CUtensorMap& tmA, const CUtensorMap& tmB, const ResiduePlan& P,
                          const split::ResTile* d_tiles, const cudaEvent_t* waits, int B, int Bpad, bool pair,
-                         split::CrtArgs crt, cudaEvent_t ev_done) {
+                         split::CrtArgs crt, int* err, cudaEvent_t ev_done) {
     cudaStream_t st = e->st;
     const int panel = residue_panel(pair ? 2 * split::BM : split::BM);
     split::ResGemmArgs g;
@@ -1287,7 +1287,7 @@ gain_status residue_gemm(gain_engine e, const CUtensorMap& tmA, const CUtensorMa
     g.res = e->res.p;
     g.ldr = crt.ldr;
     g.plane = (long)P.rows0 * crt.ldr;
-    g.err = e->err();
+    g.err = err;
     for (int m0 = 0; m0 < Bpad; m0 += panel) {
         const bool last = m0 + panel >= Bpad;
         g.m_base = m0;
@@ -1684,7 +1684,7 @@ gain_status run_split(gain_engine e, const gain_pair_job* j, int dI, int dF, con
             }
             res_flops += rp1.flops;
             GAIN_TRY(residue_gemm(e, tmV, L.tmBandPair, rp1, e->rtiles1.p, nullptr, B, Bpad, pair, c1,
-                                  piece == npieces - 1 ? e->ev[3] : nullptr));
+                                  e->err(), piece == npieces - 1 ? e->ev[3] : nullptr));
         } else {
             if (!t1.empty()) {
                 GAIN_CUDA(split::launch_gemm(tmV, pair ? L.tmBandPair : L.tmBand, g1, e->num_sms, st, pair));
@@ -1832,7 +1832,7 @@ gain_status run_split(gain_engine e, const gain_pair_job* j, int dI, int dF, con
         split::crt_constants(&c2);
         const cudaEvent_t waits[2] = {nullptr, e->ev[7]};
         res_flops += rp2.flops;
-        GAIN_TRY(residue_gemm(e, tmH, tmU, rp2, e->rtiles2.p, waits, B, Bpad, pair, c2, e->ev[5]));
+        GAIN_TRY(residue_gemm(e, tmH, tmU, rp2, e->rtiles2.p, waits, B, Bpad, pair, c2, e->err(), e->ev[5]));
     } else if (Nu2 > 0) {
         // tiles are upper-block-major: those of the first half (n0 < Nu2) come first
         int n1 = 0;
@@ -2459,23 +2459,128 @@ gain_status adjoint_split_chain(gain_engine e, const gain_pair_job* job, int dI,
     const WignerTab* wt = wigner_of(e, job->jindI, job->jindF);
     cudaStream_t st = e->st;
     const int B = job->nlower, Nu = job->nupper, NtF = iF.Ntot[job->gammaF];
-    const int Bpad = round_up(B, BM), Bk = round_up(B, BK);
+    const bool pair = B > BM;   // CTA pairs in the first product of the residue form
+    const int Bpad = round_up(B, pair ? 2 * BM : BM), Bk = round_up(B, BK);
     const int Nuk = round_up(Nu, BK), NtFpad = round_up(NtF, BN);
-    const SplitParams pA = choose_params(Nuk, nullptr, kAdjSplitBits, 8);
-    const SplitParams pB = choose_params(Bk, nullptr, kAdjSplitBits, 8);
+    // ---- the band layout over the expansions' supports, grouped by K
+    std::vector<int> fmap, imap, fstart(bF.J + 2, 0), istart(bI.J + 2, 0);
+    for (int k = 0; k <= bF.J; ++k) {
+        for (int q = mF->sup_start[k]; q < mF->sup_start[k + 1]; ++q) fmap.push_back(mF->support[q]);
+        while (fmap.size() % BM) fmap.push_back(-1);
+        fstart[k + 1] = (int)fmap.size();
+    }
+    for (int k = 0; k <= bI.J; ++k) {
+        for (int q = mI->sup_start[k]; q < mI->sup_start[k + 1]; ++q) imap.push_back(mI->support[q]);
+        while (imap.size() % BK) imap.push_back(-1);
+        istart[k + 1] = (int)imap.size();
+    }
+    const int Fpad = std::max((int)fmap.size(), BM), Ipad = (int)imap.size();
+    fmap.resize(Fpad, -1);
+    const int ldM = round_up(Ipad + BN, BN);
+    imap.resize(ldM, -1);
+    std::vector<int> blo(Fpad, 0), bhi(Fpad, 0);
+    for (int k = 0; k <= bF.J; ++k) {
+        int lo = 0, hi = Ipad;
+        if (!wt) {
+            const int klo = std::max(k - 1, 0), khi = std::min(k + 1, bI.J);
+            lo = klo <= khi ? istart[klo] : 0;
+            hi = klo <= khi ? istart[khi + 1] : 0;
+        }
+        for (int r = fstart[k]; r < fstart[k + 1] && hi > lo; ++r) {
+            blo[r] = lo;
+            bhi[r] = hi;
+        }
+    }
+    std::vector<int> umap(NtFpad, -1);
+    for (int f = 0; f < NtF; ++f) umap[f] = f;
+
+    // Operand planes: residues (residue.h: 13 products, exact for any operands) unless the
+    // device cannot hold them, else 48-bit digits.
+    SplitParams pA = residue_params(kAdjSplitBits, Nuk), pB = residue_params(kAdjSplitBits, Bk);
+    const int panel1 = std::min(Bpad, residue_panel(pair ? 2 * BM : BM)), panel2 = std::min(Fpad, residue_panel(BM));
+    bool res = pA.slices && pB.slices;
+    if (res && (e->adjs_dig[0].alloc((size_t)pA.slices * Bpad * Nuk) || e->adjs_dig[1].alloc((size_t)pA.slices * NtFpad * Nuk) ||
+                e->adjs_dig[2].alloc((size_t)pB.slices * Fpad * Bk) || e->adjs_dig[3].alloc((size_t)pB.slices * ldM * Bk) ||
+                e->res.alloc(std::max((size_t)panel1 * NtFpad * pA.slices, (size_t)panel2 * ldM * pB.slices)))) {
+        (void)cudaGetLastError();
+        clear_error();
+        e->res.release();
+        res = false;
+    }
+    if (!res) {
+        pA = choose_params(Nuk, nullptr, kAdjSplitBits, 8);
+        pB = choose_params(Bk, nullptr, kAdjSplitBits, 8);
+    }
     const int cap = kMaxFlags;
     GAIN_TRY(e->adjs_flags.alloc(cap));
     GAIN_TRY(e->adjs_cnt.alloc(2));
-    GAIN_TRY(e->adjs_cnt.zero(st, 2));
     GAIN_TRY(e->adjs_err.alloc(1));
-    GAIN_TRY(e->adjs_err.zero(st, 1));
+
+    // ---- small uploads and clears; the tiles of both products
+    const ResiduePlan rp = res ? residue_plan(e, {{{0, NtFpad, 0, Nuk / BK}}}, Bpad, pair, pA.slices) : ResiduePlan();
+    std::vector<split::ResTile> rt2;                    // 128 x 128 tiles of the band, row panel by row panel
+    std::vector<std::array<int, 4>> panels;             // first tile, tiles, first and end column
+    std::vector<split::Tile> t1, t2;
+    for (int n0 = 0; n0 < NtFpad && !res; n0 += BN)
+        for (int m0 = 0; m0 < Bpad; m0 += BM) {
+            split::Tile x;
+            memset(&x, 0, sizeof x);
+            x.m0 = m0;
+            x.n0 = n0;
+            x.nkb = Nuk / BK;
+            t1.push_back(x);
+        }
+    row_grouped(t1, BM);
+    for (int m0 = 0; m0 < Fpad; m0 += BM) {
+        if (m0 % panel2 == 0) panels.push_back({(int)rt2.size(), 0, ldM, 0});
+        for (int n0 = blo[m0]; n0 < bhi[m0]; n0 += BN) {
+            if (res) {
+                split::ResTile x;
+                memset(&x, 0, sizeof x);
+                x.m0 = m0 % panel2;
+                x.n0 = n0;
+                x.nkb = Bk / BK;
+                x.ncols = BN;
+                rt2.push_back(x);
+                ++panels.back()[1];
+                panels.back()[2] = std::min(panels.back()[2], n0);
+                panels.back()[3] = std::max(panels.back()[3], n0 + BN);
+            } else {
+                split::Tile x;
+                memset(&x, 0, sizeof x);
+                x.m0 = m0;
+                x.n0 = n0;
+                x.nkb = Bk / BK;
+                t2.push_back(x);
+            }
+        }
+    }
+    Staging up;
+    GAIN_TRY(up.add(e->adjs_cnt.p, nullptr, 2 * sizeof(unsigned int)));
+    GAIN_TRY(up.add(e->adjs_err.p, nullptr, sizeof(int)));
+    GAIN_TRY(up.add(e->adjs_umap, umap.data(), umap.size()));
+    GAIN_TRY(up.add(e->adjs_fmap, fmap.data(), fmap.size()));
+    GAIN_TRY(up.add(e->adjs_imap, imap.data(), imap.size()));
+    GAIN_TRY(up.add(e->adjs_blo, blo.data(), blo.size()));
+    GAIN_TRY(up.add(e->adjs_bhi, bhi.data(), bhi.size()));
+    std::vector<split::ResTile> rt = rp.tiles;
+    const int rt2_at = (int)rt.size();
+    rt.insert(rt.end(), rt2.begin(), rt2.end());
+    GAIN_TRY(up.add(e->rtiles1, rt.data(), rt.size()));
+    GAIN_TRY(up.launch(e, st));
     double fl = 0.0;
-    auto zero_dig = [&](int k, size_t n, size_t rows, int nch) -> gain_status {
+    // planes of nrows rows, laid out in buffer k
+    auto planes = [&](int k, const SplitParams& p, const double* src, long ld, int nrows, int ncols, int kpad,
+                      int rows_pad) -> gain_status {
+        const size_t n = (size_t)p.slices * rows_pad * kpad;
         GAIN_TRY(e->adjs_dig[k].alloc(n));
-        GAIN_TRY(e->adjs_dig[k].zero(st, n));
-        GAIN_TRY(e->adjs_st[k].alloc(rows, nch, false));
-        GAIN_TRY(e->adjs_st[k].zero(st, rows, nch, false));
-        return GAIN_OK;
+        GAIN_TRY(e->adjs_st[k].alloc(rows_pad, p.stat_chunks(), false));
+        if (!res) {
+            GAIN_TRY(e->adjs_dig[k].zero(st, n));
+            GAIN_TRY(e->adjs_st[k].zero(st, rows_pad, p.chunks, false));
+        }
+        return slice(e, src, ld, nullptr, nrows, ncols, nullptr, nullptr, kpad, rows_pad, e->adjs_dig[k].p,
+                     k & 1 ? p.as_b() : p, e->adjs_st[k], false, nullptr, nullptr, st);
     };
     // C = A B^T over the listed tiles from digit buffers ka (rowsA rows) and kb (rowsB rows),
     // inner length ldk; the flags of uncertified entries go to the list behind cnt
@@ -2515,32 +2620,41 @@ gain_status adjoint_split_chain(gain_engine e, const gain_pair_job* job, int dI,
         for (auto& t : tiles) fl += 2.0 * BM * BN * BK * t.nkb * (double)pr.size() / p.chunks;
         return GAIN_OK;
     };
+    // the residue form's reconstruction: values only (no operand is ever inexact)
+    auto crt_args = [&](int ka, int kb, const SplitParams& p, double* out, long ldo) {
+        split::CrtArgs c;
+        memset(&c, 0, sizeof c);
+        c.ldr = c.ldo = ldo;
+        c.nmod = p.slices;
+        c.bits = p.bits;
+        c.cols = (int)ldo;
+        c.A = e->adjs_st[ka].view(false);
+        c.B = e->adjs_st[kb].view(false);
+        c.out = out;
+        split::crt_constants(&c);
+        return c;
+    };
+    auto maps = [&](CUtensorMap* ta, CUtensorMap* tb, int ka, int kb, const SplitParams& p, int ldk, int rowsA,
+                    int rowsB) -> gain_status {
+        if (!split::make_digit_map(ta, e->adjs_dig[ka].p, ldk, rowsA, p.slices) ||
+            !split::make_digit_map(tb, e->adjs_dig[kb].p, ldk, rowsB, p.slices, BN / 2))
+            return set_error(GAIN_ERR_CUDA, "cuTensorMapEncodeTiled failed (adjoint residues)");
+        return GAIN_OK;
+    };
     // ---- dH = G U: A = G rows (inner: upper states), B = U^T rows (upper symmetric functions)
-    {
-        std::vector<int> umap(NtFpad, -1);
-        for (int f = 0; f < NtF; ++f) umap[f] = f;
-        GAIN_TRY(e->adjs_umap.upload(umap));
-        GAIN_TRY(e->adjs_UT.alloc((size_t)NtFpad * Nuk));
-        GAIN_CUDA(launch_gather_t(NtFpad, Nu, Nuk, EF.d.p, EF.nsize, e->d_upper.p, e->adjs_umap.p, e->adjs_UT.p, st));
-        GAIN_TRY(zero_dig(0, (size_t)pA.slices * Bpad * Nuk, Bpad, pA.chunks));
-        GAIN_TRY(zero_dig(1, (size_t)pA.slices * NtFpad * Nuk, NtFpad, pA.chunks));
-        GAIN_TRY(slice(e, G, Nu, nullptr, B, Nu, nullptr, nullptr, Nuk, Bpad, e->adjs_dig[0].p, pA, e->adjs_st[0],
-                       false, nullptr, nullptr, st));
-        GAIN_TRY(slice(e, e->adjs_UT.p, Nuk, nullptr, NtFpad, Nuk, nullptr, nullptr, Nuk, NtFpad, e->adjs_dig[1].p, pA,
-                       e->adjs_st[1], false, nullptr, nullptr, st));
-        std::vector<split::Tile> t;
-        for (int n0 = 0; n0 < NtFpad; n0 += BN)
-            for (int m0 = 0; m0 < Bpad; m0 += BM) {
-                split::Tile x;
-                memset(&x, 0, sizeof x);
-                x.m0 = m0;
-                x.n0 = n0;
-                x.nkb = Nuk / BK;
-                t.push_back(x);
-            }
-        row_grouped(t, BM);
-        GAIN_TRY(e->adjs_dH.alloc((size_t)Bpad * NtFpad));
-        GAIN_TRY(gemm(0, 1, pA, Nuk, Bpad, NtFpad, e->adjs_dH.p, NtFpad, B, NtF, t, e->adjs_tiles1, e->adjs_prods1,
+    GAIN_TRY(e->adjs_UT.alloc((size_t)NtFpad * Nuk));
+    GAIN_CUDA(launch_gather_t(NtFpad, Nu, Nuk, EF.d.p, EF.nsize, e->d_upper.p, e->adjs_umap.p, e->adjs_UT.p, st));
+    GAIN_TRY(planes(0, pA, G, Nu, B, Nu, Nuk, Bpad));
+    GAIN_TRY(planes(1, pA, e->adjs_UT.p, Nuk, NtFpad, Nuk, Nuk, NtFpad));
+    GAIN_TRY(e->adjs_dH.alloc((size_t)Bpad * NtFpad));
+    if (res) {
+        CUtensorMap ta, tb;
+        GAIN_TRY(maps(&ta, &tb, 0, 1, pA, Nuk, Bpad, NtFpad));
+        GAIN_TRY(residue_gemm(e, ta, tb, rp, e->rtiles1.p, nullptr, B, Bpad, pair, crt_args(0, 1, pA, e->adjs_dH.p, NtFpad),
+                              e->adjs_err.p, nullptr));
+        fl += rp.flops;
+    } else {
+        GAIN_TRY(gemm(0, 1, pA, Nuk, Bpad, NtFpad, e->adjs_dH.p, NtFpad, B, NtF, t1, e->adjs_tiles1, e->adjs_prods1,
                       e->adjs_cnt.p));
         GAIN_CUDA(launch_refine_rows(e->adjs_flags.p, e->adjs_cnt.p, cap, G, Nu, e->adjs_UT.p, Nuk, Nu, e->adjs_dH.p,
                                      NtFpad, 2 * e->num_sms, st));
@@ -2556,65 +2670,47 @@ gain_status adjoint_split_chain(gain_engine e, const gain_pair_job* job, int dI,
     GAIN_CUDA(launch_expand_levels(iI.dimen, job->gammaI, iI.maxcoeff, dI, iI.sdeg[job->gammaI], iI.Ntot[job->gammaI],
                                    iI.dijterms.p, iI.dicontr.p, iI.dN[job->gammaI]->p, iI.drepres[job->gammaI]->p,
                                    EI.d.p, EI.nsize, e->d_lower.p, vp, bI.dimen, B, st));
-    // ---- the band layout over the expansions' supports, grouped by K
-    std::vector<int> fmap, imap, fstart(bF.J + 2, 0), istart(bI.J + 2, 0);
-    for (int k = 0; k <= bF.J; ++k) {
-        for (int q = mF->sup_start[k]; q < mF->sup_start[k + 1]; ++q) fmap.push_back(mF->support[q]);
-        while (fmap.size() % BM) fmap.push_back(-1);
-        fstart[k + 1] = (int)fmap.size();
-    }
-    for (int k = 0; k <= bI.J; ++k) {
-        for (int q = mI->sup_start[k]; q < mI->sup_start[k + 1]; ++q) imap.push_back(mI->support[q]);
-        while (imap.size() % BK) imap.push_back(-1);
-        istart[k + 1] = (int)imap.size();
-    }
-    const int Fpad = std::max((int)fmap.size(), BM), Ipad = (int)imap.size();
-    fmap.resize(Fpad, -1);
-    const int ldM = round_up(Ipad + BN, BN);
-    imap.resize(ldM, -1);
-    std::vector<int> blo(Fpad, 0), bhi(Fpad, 0);
-    std::vector<split::Tile> t2;
-    for (int k = 0; k <= bF.J; ++k) {
-        if (fstart[k + 1] == fstart[k]) continue;
-        int lo = 0, hi = Ipad;
-        if (!wt) {
-            const int klo = std::max(k - 1, 0), khi = std::min(k + 1, bI.J);
-            if (klo > khi) continue;
-            lo = istart[klo];
-            hi = istart[khi + 1];
-        }
-        if (hi <= lo) continue;
-        for (int r = fstart[k]; r < fstart[k + 1]; ++r) {
-            blo[r] = lo;
-            bhi[r] = hi;
-        }
-        for (int m0 = fstart[k]; m0 < fstart[k + 1]; m0 += BM)
-            for (int n0 = lo; n0 < hi; n0 += BN) {
-                split::Tile x;
-                memset(&x, 0, sizeof x);
-                x.m0 = m0;
-                x.n0 = n0;
-                x.nkb = Bk / BK;
-                t2.push_back(x);
-            }
-    }
-    GAIN_TRY(e->adjs_fmap.upload(fmap));
-    GAIN_TRY(e->adjs_imap.upload(imap));
-    GAIN_TRY(e->adjs_blo.upload(blo));
-    GAIN_TRY(e->adjs_bhi.upload(bhi));
     // ---- dM = dh^T vp on the band: A = dh^T rows (upper positions), B = vp^T rows (lower)
     GAIN_TRY(e->adjs_dhT.alloc((size_t)Fpad * Bk));
     GAIN_TRY(e->adjs_vpT.alloc((size_t)ldM * Bk));
     GAIN_CUDA(launch_gather_t(Fpad, B, Bk, dh, bF.dimen, nullptr, e->adjs_fmap.p, e->adjs_dhT.p, st));
     GAIN_CUDA(launch_gather_t(ldM, B, Bk, vp, bI.dimen, nullptr, e->adjs_imap.p, e->adjs_vpT.p, st));
-    GAIN_TRY(zero_dig(2, (size_t)pB.slices * Fpad * Bk, Fpad, pB.chunks));
-    GAIN_TRY(zero_dig(3, (size_t)pB.slices * ldM * Bk, ldM, pB.chunks));
-    GAIN_TRY(slice(e, e->adjs_dhT.p, Bk, nullptr, Fpad, Bk, nullptr, nullptr, Bk, Fpad, e->adjs_dig[2].p, pB,
-                   e->adjs_st[2], false, nullptr, nullptr, st));
-    GAIN_TRY(slice(e, e->adjs_vpT.p, Bk, nullptr, ldM, Bk, nullptr, nullptr, Bk, ldM, e->adjs_dig[3].p, pB,
-                   e->adjs_st[3], false, nullptr, nullptr, st));
+    GAIN_TRY(planes(2, pB, e->adjs_dhT.p, Bk, Fpad, Bk, Bk, Fpad));
+    GAIN_TRY(planes(3, pB, e->adjs_vpT.p, Bk, ldM, Bk, Bk, ldM));
     GAIN_TRY(e->adjs_dM.alloc((size_t)Fpad * ldM));
-    if (!t2.empty()) {
+    if (res) {
+        CUtensorMap ta, tb;
+        GAIN_TRY(maps(&ta, &tb, 2, 3, pB, Bk, Fpad, ldM));
+        const split::CrtArgs c0 = crt_args(2, 3, pB, e->adjs_dM.p, ldM);
+        split::ResGemmArgs g;
+        memset(&g, 0, sizeof g);
+        g.nmod = pB.slices;
+        g.res = e->res.p;
+        g.ldr = ldM;
+        g.plane = (long)panel2 * ldM;
+        g.err = e->adjs_err.p;
+        for (size_t q = 0; q < panels.size(); ++q) {
+            const auto& pn = panels[q];
+            if (!pn[1]) continue;
+            g.m_base = (int)q * panel2;
+            g.tiles = e->rtiles1.p + rt2_at + pn[0];
+            g.ntiles = pn[1];
+            GAIN_CUDA(split::launch_residue_gemm(ta, tb, g, e->num_sms, st, false));
+            // the panel's columns (entries outside its rows' bands are never read)
+            split::CrtArgs c = c0;
+            c.res = g.res + pn[2];
+            c.plane = g.plane;
+            c.row0 = g.m_base;
+            c.rows = std::min(panel2, Fpad - g.m_base);
+            c.cols = pn[3] - pn[2];
+            c.B.e += pn[2];
+            c.B.l2 += pn[2];
+            c.B.dn += pn[2];
+            c.out += pn[2];
+            GAIN_CUDA(split::launch_crt(c, st));
+            fl += 2.0 * pn[1] * BM * BN * (double)Bk * pB.slices;
+        }
+    } else if (!t2.empty()) {
         GAIN_TRY(gemm(2, 3, pB, Bk, Fpad, ldM, e->adjs_dM.p, ldM, Fpad, ldM, t2, e->adjs_tiles2, e->adjs_prods2,
                       e->adjs_cnt.p + 1));
         GAIN_CUDA(launch_refine_rows(e->adjs_flags.p, e->adjs_cnt.p + 1, cap, e->adjs_dhT.p, Bk, e->adjs_vpT.p, Bk,
@@ -2657,6 +2753,7 @@ gain_status adjoint_split_chain(gain_engine e, const gain_pair_job* job, int dI,
     GAIN_CUDA(cudaMemcpyAsync(cnt, e->adjs_cnt.p, sizeof cnt, cudaMemcpyDeviceToHost, st));
     GAIN_CUDA(cudaMemcpyAsync(&errw, e->adjs_err.p, sizeof errw, cudaMemcpyDeviceToHost, st));
     GAIN_CUDA(cudaStreamSynchronize(st));
+    e->stage_busy = false;
     if (errw) return set_error(GAIN_ERR_TIMEOUT, "a bounded device wait of the adjoint GEMM gave up (code %d)", errw);
     if (cnt[0] > (unsigned)cap || cnt[1] > (unsigned)cap)
         return set_error(GAIN_ERR_TOL_NOT_MET, "adjoint: more uncertified products than the refinement list holds");
@@ -2708,8 +2805,10 @@ gain_status adjoint_run(gain_engine e, const gain_pair_job* job, const std::vect
         }
     };
     std::vector<int> kFlo, kFhi, kIlo, kIhi, tiles;
-    kranges(bF, true, kFlo, kFhi);
-    kranges(bI, false, kIlo, kIhi);
+    if (!tc) {   // (the SIMT chains' tiles)
+        kranges(bF, true, kFlo, kFhi);
+        kranges(bI, false, kIlo, kIhi);
+    }
     for (size_t tf = 0; tf < kFlo.size(); ++tf) {
         if (kFlo[tf] > kFhi[tf]) continue;   // no function of the piece
         for (size_t ti = 0; ti < kIlo.size(); ++ti) {

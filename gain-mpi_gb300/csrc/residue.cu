@@ -821,7 +821,7 @@ __global__ void __launch_bounds__(kCrtThreads) k_crt(const CrtArgs a0, const Crt
                         const unsigned long long ab = vb & 0x7FFFFFFFFFFFFFFFull;
                         vmax = ab > vmax ? ab : vmax;
                     }
-                    if (bound > limit) {
+                    if (a.flag_mode && bound > limit) {
                         const unsigned int idx = atomicAdd(a.nflags, 1u);
                         if ((int)idx < a.max_flags) a.flags[idx] = make_int2(r, c + j);
                     }

@@ -75,7 +75,7 @@ struct CrtArgs {
     int nmod, bits;
     int row0;              // output row of residue row 0
     int rows;              // residue rows to reconstruct
-    int cols;              // columns to reconstruct (a multiple of 128)
+    int cols;              // columns to reconstruct (a multiple of 4)
     int cols_valid;        // columns that are flagged and counted
     RowStats A, B;
     double* out;
@@ -85,7 +85,7 @@ struct CrtArgs {
     float c_fix;           // bound of the reconstruction, units of 2^{eA+eB}
     float c_f64;           // as GemmArgs
     float tol;
-    int flag_mode;         // 1: bound > max(tol |value|, FP64 bound) is flagged; 2: bound > FP64 bound
+    int flag_mode;         // 1: bound > max(tol |value|, FP64 bound) is flagged; 2: bound > FP64 bound; 0: none
     float* rowerr2;        // optional, as GemmArgs
     unsigned long long* absmax;   // optional, as GemmArgs
     int2* flags;
