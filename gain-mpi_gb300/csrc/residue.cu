@@ -117,7 +117,11 @@ constexpr uint32_t STA = KS * BOX_A, STB = KS * 2 * BOX_B;
 constexpr int EPI_WARPS = 8;
 constexpr int NTHREADS = 64 + 32 * EPI_WARPS;
 constexpr uint32_t ACC_COLS = 256;               // TMEM columns of one accumulator; two fill TMEM
-constexpr uint32_t kSmemBytes = NST * (STA + STB) + 256 + 1024;
+// after the stage ring and the barriers: 32 rows x 128 bytes per epilogue warp, in which the
+// residues are turned from a row per thread to whole lines per store
+constexpr uint32_t TURN_OFF = NST * (STA + STB) + 256;
+constexpr uint32_t kSmemBytes = TURN_OFF + EPI_WARPS * 4096 + 1024;
+static_assert(kSmemBytes <= 227 * 1024, "shared memory");
 
 __device__ __forceinline__ uint32_t idesc_of(bool pair, int ncols) {   // BF16 x BF16 -> F32, K-major
     return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(ncols >> 3) << 17) |
@@ -144,8 +148,8 @@ __device__ __forceinline__ uint32_t idesc_of(bool pair, int ncols) {   // BF16 x
 // Measured (GB300, 2000 x 12 000 outputs, inner length 12 288, 13 moduli): 4.18 ms, 1885
 // TFLOP/s, where the 21 products of 8-bit digits took 9.0 ms at 1340; the chip's power limit
 // bounds it (SM clock 1.9 GHz instead of 2.07, tensor pipe above 80 % of its cycles).  Band
-// GEMM of the same run (12 288 columns, up to 3072 deep): 1.14 ms, with 28 digit products 3.0.
-// 550 x 1200 outputs, inner length 1408: 54 us, with digits (30 tiles on 76 pairs) 167.
+// GEMM of the same run (12 288 columns, up to 3072 deep): 1.10 ms, with 28 digit products 3.0.
+// 550 x 1200 outputs, inner length 1408: 47 us, with digits (30 tiles on 76 pairs) 167.
 template <bool PAIR, bool GROUPED>
 __global__ void __launch_bounds__(NTHREADS, 1)
 k_residue_gemm(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const ResGemmArgs a) {
@@ -365,35 +369,52 @@ k_residue_gemm(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         // ---------------- epilogue: one TMEM lane (output row) per thread
         const int q = warp & 3;
         const int half = (warp - 2) >> 2;   // which half of the tile's columns
-        const int row = (int)rank * BM + q * 32 + lane;
         const uint32_t lane_off = (uint32_t)(q * 32) << 16;
-        // balanced residues of 64 columns to [0, m) and 16 bits (a float's low half over 2^23)
-        auto pack = [&](const uint32_t (&v)[2][32], float m, uint32_t* o) {
+        // balanced residues of 32 columns to [0, m) and 16 bits (a float's low half over 2^23)
+        auto pack = [&](const uint32_t (&v)[32], float m, uint32_t* o) {
 #pragma unroll
-            for (int k = 0; k < 2; ++k)
-#pragma unroll
-                for (int j = 0; j < 32; j += 2) {
-                    const float x = __uint_as_float(v[k][j]), y = __uint_as_float(v[k][j + 1]);
-                    o[16 * k + j / 2] =
-                        __byte_perm(__float_as_uint(__fadd_rn(x < 0.0f ? __fadd_rn(x, m) : x, 8388608.0f)),
-                                    __float_as_uint(__fadd_rn(y < 0.0f ? __fadd_rn(y, m) : y, 8388608.0f)), 0x5410);
-                }
+            for (int j = 0; j < 32; j += 2) {
+                const float x = __uint_as_float(v[j]), y = __uint_as_float(v[j + 1]);
+                o[j / 2] = __byte_perm(__float_as_uint(__fadd_rn(x < 0.0f ? __fadd_rn(x, m) : x, 8388608.0f)),
+                                       __float_as_uint(__fadd_rn(y < 0.0f ? __fadd_rn(y, m) : y, 8388608.0f)), 0x5410);
+            }
         };
-        // this thread's packed residues (ncols / 2 columns) of an item
+        // the warp's packed residues (32 rows, ncols / 2 columns each) of an item, 64 columns at a
+        // time through shared memory: eight threads then store one row's 128 bytes.  (A row per
+        // thread took 32 lines per store instruction: about 5 us an item, as long as the MMAs of
+        // an inner length of 1200.)
+        char* turn = reinterpret_cast<char*>(smem) + TURN_OFF + (warp - 2) * 4096;
+        auto ld_of = [&](const ResTile& tl) { return GROUPED ? a.groups[tl.group].ldr : a.ldr; };
+        auto rows_of = [&](const ResTile& tl) {   // the warp's first row, its half of the columns
+            return (GROUPED ? a.groups[tl.group].res : a.res) +
+                   (long)tl.mod * (GROUPED ? a.groups[tl.group].plane : a.plane) +
+                   (long)(tl.m0 + (int)rank * BM + q * 32) * ld_of(tl) + tl.n0 + half * (tl.ncols / 2);
+        };
         auto store = [&](const ResTile& tl, const uint32_t (&o)[64]) {
-            uint16_t* res = GROUPED ? a.groups[tl.group].res : a.res;
-            const long plane = GROUPED ? a.groups[tl.group].plane : a.plane;
-            const long ldr = GROUPED ? a.groups[tl.group].ldr : a.ldr;
-            uint4* dst = reinterpret_cast<uint4*>(res + (long)tl.mod * plane + (long)(tl.m0 + row) * ldr + tl.n0 +
-                                                  half * (tl.ncols / 2));
+            uint16_t* dst = rows_of(tl);
+            const long ldr = ld_of(tl);
 #pragma unroll
-            for (int g = 0; g < 16; ++g)
-                if (g < tl.ncols / 16) dst[g] = make_uint4(o[4 * g], o[4 * g + 1], o[4 * g + 2], o[4 * g + 3]);
+            for (int h = 0; h < 2; ++h) {
+                if (h < tl.ncols / 128) {
+                    __syncwarp();
+#pragma unroll
+                    for (int c = 0; c < 8; ++c)
+                        *reinterpret_cast<uint4*>(turn + lane * 128 + ((c ^ (lane & 7)) * 16)) =
+                            make_uint4(o[32 * h + 4 * c], o[32 * h + 4 * c + 1], o[32 * h + 4 * c + 2], o[32 * h + 4 * c + 3]);
+                    __syncwarp();
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) {
+                        const int r = 4 * i + (lane >> 3), c = lane & 7;
+                        *reinterpret_cast<uint4*>(dst + (long)r * ldr + 64 * h + 8 * c) =
+                            *reinterpret_cast<const uint4*>(turn + r * 128 + ((c ^ (r & 7)) * 16));
+                    }
+                }
+            }
         };
         auto load_chunks = [&](Stream& x) {   // items without an inner range: zeros
             for (load_item(x); x.it < nitems && x.tl.nkb <= 0; load_item(x)) {
-                const uint32_t z[64] = {};
-                store(x.tl, z);
+                uint4* d = reinterpret_cast<uint4*>(rows_of(x.tl) + (long)lane * ld_of(x.tl));
+                for (int g = 0; g < x.tl.ncols / 16; ++g) d[g] = make_uint4(0u, 0u, 0u, 0u);
                 x.it += 2 * nunits;
             }
         };
@@ -418,25 +439,18 @@ k_residue_gemm(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                 const bool last = x.kb >= x.tl.nkb;
                 uint32_t o[64];   // (last chunk) packed residues: stored after the accumulator is released
 #pragma unroll
-                for (int p = 0; p < 4; p += 2) {   // 64 columns at a time
+                for (int p = 0; p < 4; ++p) {   // 32 columns at a time
                     if (p < npc) {
-                        uint32_t v[2][32];
-                        tmem_ld32(t0 + p * 32, v[0]);
-                        tmem_ld32(t0 + p * 32 + 32, v[1]);
+                        uint32_t v[32];
+                        tmem_ld32(t0 + p * 32, v);
                         tmem_wait_ld();
 #pragma unroll
-                        for (int k = 0; k < 2; ++k)
-#pragma unroll
-                            for (int j = 0; j < 32; j += 2)
-                                unpack2(mod_balanced2(pack2(__uint_as_float(v[k][j]), __uint_as_float(v[k][j + 1])),
-                                                      pack2(inv, inv), pack2(-m, -m)),
-                                        v[k][j], v[k][j + 1]);
-                        if (last) {
-                            pack(v, m, o + 16 * p);
-                        } else {
-                            tmem_st32(t0 + p * 32, v[0]);
-                            tmem_st32(t0 + p * 32 + 32, v[1]);
-                        }
+                        for (int j = 0; j < 32; j += 2)
+                            unpack2(mod_balanced2(pack2(__uint_as_float(v[j]), __uint_as_float(v[j + 1])),
+                                                  pack2(inv, inv), pack2(-m, -m)),
+                                    v[j], v[j + 1]);
+                        if (last) pack(v, m, o + 16 * p);
+                        else tmem_st32(t0 + p * 32, v);
                     }
                 }
                 if (!last) tmem_wait_st();
