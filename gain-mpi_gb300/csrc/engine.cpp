@@ -3661,7 +3661,8 @@ struct PlanJob {
     int B = 0, Bpad = 0, Nu = 0, Nupad = 0, K2 = 0, cap1 = 0, cap2 = 0, klass = 0;
     DevArray<int> d_lower, d_upper, iota;
     DevArray<double> primI, H, Hsym, amp;
-    DevArray<float> rowerr, ampbnd;
+    DevArray<float> ampbnd;
+    float* rowerr = nullptr;      // the job's part of the plan's row errors
     DevArray<__nv_bfloat16> Vdig, Hdig, Udig;
     StatsDev Vst, Hst, Ust;
     DevArray<int2> flags1, flags2;
@@ -3718,6 +3719,10 @@ struct gain_plan_s {
         DevArray<int> offs;
     };
     std::vector<SliceBatch> slices1, slices3;
+    DevArray<float> rowerr;                 // every job's row errors
+    size_t nrowerr = 0;
+    DevArray<split::RefineHArgs> refine1;   // every job's refinement of H and of the amplitudes
+    DevArray<split::RefineAmpArgs> refine2;
     DevArray<unsigned int> counters;        // [2 * njobs]: GEMM1 / GEMM2 refinement counts
     DevArray<unsigned long long> ull;       // [4 * njobs]: uncertified, -, amp max, uncertified weak
     DevArray<int> err;
@@ -3864,7 +3869,6 @@ gain_status plan_prepare_job(gain_plan P, PlanJob& J) {
         J.Ust = StatsDev();
     }
     GAIN_TRY(J.H.alloc((size_t)J.Bpad * L.fpad));
-    GAIN_TRY(J.rowerr.alloc(J.Bpad));
     GAIN_TRY(J.amp.alloc((size_t)J.Bpad * J.Nupad));
     GAIN_TRY(J.ampbnd.alloc((size_t)J.Bpad * J.Nupad));
     GAIN_TRY(J.flags1.alloc(J.cap1));
@@ -3955,7 +3959,7 @@ gain_status plan_build_slices(gain_plan P) {
         }
         const PlanJob& JL = J.lowner < 0 ? J : *P->jobs[J.lowner];   // the lower digits' owner
         s3.push_back(slice_args(L.general ? J.Hsym.p : J.H.p, J.K2, nullptr, J.B, L.general ? L.nsymF : L.fpad,
-                                nullptr, nullptr, J.K2, J.Bpad, J.Hdig.p, J.p2, J.Hst, true, J.rowerr.p,
+                                nullptr, nullptr, J.K2, J.Bpad, J.Hdig.p, J.p2, J.Hst, true, J.rowerr,
                                 JL.Vst.e.p));
     }
     GAIN_TRY(plan_slice_batches(s1, P->slices1));
@@ -4058,7 +4062,7 @@ gain_status plan_build_residue_groups(gain_plan P) {
         a1[q].B = L.bandStats.view(false);
         a1[q].out = J.H.p;
         a1[q].c_f64 = (float)((double)(L.W + 64) * std::ldexp(1.0, -53) * 1.01);
-        a1[q].rowerr2 = J.rowerr.p;
+        a1[q].rowerr2 = J.rowerr;
         a1[q].flag_mode = 2;
         a1[q].flags = J.flags1.p;
         a1[q].nflags = P->counters.p + 2 * q;
@@ -4074,8 +4078,6 @@ gain_status plan_build_residue_groups(gain_plan P) {
         a2[q].max_flags = J.cap2;
         a2[q].bnd = J.ampbnd.p;
         a2[q].ldb = J.Nupad;
-        o1[q + 1] = o1[q] + split::crt_blocks(a1[q]);
-        o2[q + 1] = o2[q] + split::crt_blocks(a2[q]);
         std::vector<ColumnRange> cols;
         for (auto& fb : L.fblocks)
             cols.push_back({fb.first, fb.second, L.band_k0[fb.first], L.band_len[fb.first] / split::BK});
@@ -4087,6 +4089,12 @@ gain_status plan_build_residue_groups(gain_plan P) {
     const std::vector<split::ResTile> s1 = list_schedule(t1, c1, P->units), s2 = list_schedule(t2, c2, P->units);
     P->ntiles1 = (int)s1.size();
     P->ntiles2 = (int)s2.size();
+    split::crt_set_rows(a1.data(), nj);
+    split::crt_set_rows(a2.data(), nj);
+    for (int q = 0; q < nj; ++q) {
+        o1[q + 1] = o1[q] + split::crt_blocks(a1[q]);
+        o2[q + 1] = o2[q] + split::crt_blocks(a2[q]);
+    }
     P->crt1_blocks = o1[nj];
     P->crt2_blocks = o2[nj];
     auto common = [](const std::vector<split::CrtArgs>& v) {
@@ -4158,7 +4166,7 @@ gain_status plan_build_groups(gain_plan P) {
         a1.B = L.bandStats.view(false);
         a1.c_fix = fix_const(J.nprods1);
         a1.c_f64 = (float)((double)(L.W + 64) * std::ldexp(1.0, -53) * 1.01);
-        a1.rowerr2 = J.rowerr.p;
+        a1.rowerr2 = J.rowerr;
         a1.flag_mode = 2;
         a1.tol = (float)tol;
         a1.flags = J.flags1.p;
@@ -4255,6 +4263,61 @@ gain_status plan_build_groups(gain_plan P) {
     return GAIN_OK;
 }
 
+// Every job's FP64 refinement of H and of the amplitudes, for one launch each.
+gain_status plan_build_refinement(gain_plan P) {
+    gain_engine e = P->e;
+    const int nj = (int)P->jobs.size();
+    std::vector<split::RefineHArgs> r1(nj);
+    std::vector<split::RefineAmpArgs> r2(nj);
+    for (int q = 0; q < nj; ++q) {
+        PlanJob& J = *P->jobs[q];
+        PairLayout& L = *J.L;
+        const gain_pair_job* j = &J.job;
+        const Eig& EI = *e->eig[{j->jindI, j->gammaI}];
+        const Eig& EF = *e->eig[{j->jindF, j->gammaF}];
+        split::RefineHArgs& rh = r1[q];
+        rh.flags = J.flags1.p;
+        rh.nflags = P->counters.p + 2 * q;
+        rh.max_flags = J.cap1;
+        rh.vecs = L.general ? J.primI.p : EI.d.p;
+        rh.nsize = L.general ? e->bases[j->jindI].dimen : EI.nsize;
+        rh.row_level = L.general ? J.iota.p : J.d_lower.p;
+        rh.i_sym = L.d_i_sym.p;
+        rh.band_k0 = L.d_band_k0.p;
+        rh.band_len = L.d_band_len.p;
+        rh.band = L.band.p;
+        rh.W = L.W;
+        rh.H = J.H.p;
+        rh.ldh = L.fpad;
+        rh.eA = (J.lowner < 0 ? J : *P->jobs[J.lowner]).Vst.e.p;
+        rh.rowerr2 = J.rowerr;
+        split::RefineAmpArgs& ra = r2[q];
+        ra.flags = J.flags2.p;
+        ra.nflags = P->counters.p + 2 * q + 1;
+        ra.max_flags = J.cap2;
+        ra.U = EF.d.p;
+        ra.nsize = EF.nsize;
+        ra.col_level = J.d_upper.p;
+        ra.colpos = L.general ? L.d_ident.p : L.d_colposF.p;
+        ra.H = L.general ? J.Hsym.p : J.H.p;
+        ra.ldh = J.K2;
+        ra.h_inerr = J.Hst.inerr.p;
+        ra.eH = J.Hst.e.p;
+        ra.amp = J.amp.p;
+        ra.lda = J.Nupad;
+        ra.bnd = J.ampbnd.p;
+        ra.ldb = J.Nupad;
+        ra.tol = (P->has_opts && P->opts.tol > 0) ? P->opts.tol : 4.5e-9;
+        ra.absmax = P->ull.p + 4 * q + 2;
+        ra.amp_floor = std::sqrt((P->has_opts && P->opts.s_floor > 0) ? P->opts.s_floor : 1e-10);
+        ra.uncertified = P->ull.p + 4 * q;
+        ra.uncertified_weak = P->ull.p + 4 * q + 3;
+    }
+    GAIN_TRY(P->refine1.upload(r1));
+    GAIN_TRY(P->refine2.upload(r2));
+    return GAIN_OK;
+}
+
 // The plan's work on the engine's stream (and its side streams), to be captured.
 gain_status plan_enqueue(gain_plan P) {
     gain_engine e = P->e;
@@ -4276,10 +4339,13 @@ gain_status plan_enqueue(gain_plan P) {
     GAIN_CUDA(cudaMemsetAsync(P->counters.p, 0, sizeof(unsigned int) * 2 * nj, st));
     GAIN_CUDA(cudaMemsetAsync(P->ull.p, 0, sizeof(unsigned long long) * 4 * nj, st));
     GAIN_CUDA(cudaMemsetAsync(P->err.p, 0, sizeof(int), st));
+    GAIN_CUDA(cudaMemsetAsync(P->rowerr.p, 0, sizeof(float) * P->nrowerr, st));
+    bool any_general = false;
+    for (auto& J : P->jobs) any_general = any_general || J->L->general;
     GAIN_CUDA(cudaEventRecordWithFlags(P->ev[0], st, cudaEventRecordExternal));
     // ---- stage 1: expansions of mixing lower vectors (per job, on the branches), then the
     // digits of every job's lower and upper eigenvectors (one launch per slicing kernel)
-    GAIN_TRY(fork());
+    if (any_general) GAIN_TRY(fork());
     for (int q = 0; q < nj; ++q) {
         PlanJob& J = *P->jobs[q];
         PairLayout& L = *J.L;
@@ -4293,9 +4359,8 @@ gain_status plan_enqueue(gain_plan P) {
                                            iI.dijterms.p, iI.dicontr.p, iI.dN[j->gammaI]->p, iI.drepres[j->gammaI]->p,
                                            EI.d.p, EI.nsize, J.d_lower.p, J.primI.p, bI.dimen, J.B, sq));
         }
-        GAIN_CUDA(cudaMemsetAsync(J.rowerr.p, 0, sizeof(float) * J.Bpad, sq));
     }
-    GAIN_TRY(join());
+    if (any_general) GAIN_TRY(join());
     cudaStream_t streams[kPlanStreams];
     for (int k = 0; k < kPlanStreams; ++k) streams[k] = stream_of(k);
     GAIN_TRY(fork());
@@ -4317,38 +4382,20 @@ gain_status plan_enqueue(gain_plan P) {
         GAIN_CUDA(cudaEventRecordWithFlags(P->ev[2], st, cudaEventRecordExternal));
     }
     // ---- stage 3: FP64 refinement of H, contraction (mixing expansions), digits of H
-    GAIN_TRY(fork());
-    for (int q = 0; q < nj; ++q) {
-        PlanJob& J = *P->jobs[q];
-        PairLayout& L = *J.L;
-        const gain_pair_job* j = &J.job;
-        cudaStream_t sq = stream_of(q);
-        const Eig& EI = *e->eig[{j->jindI, j->gammaI}];
-        const Basis& bI = e->bases[j->jindI];
-        split::RefineHArgs rh;
-        rh.flags = J.flags1.p;
-        rh.nflags = P->counters.p + 2 * q;
-        rh.max_flags = J.cap1;
-        rh.vecs = L.general ? J.primI.p : EI.d.p;
-        rh.nsize = L.general ? bI.dimen : EI.nsize;
-        rh.row_level = L.general ? J.iota.p : J.d_lower.p;
-        rh.i_sym = L.d_i_sym.p;
-        rh.band_k0 = L.d_band_k0.p;
-        rh.band_len = L.d_band_len.p;
-        rh.band = L.band.p;
-        rh.W = L.W;
-        rh.H = J.H.p;
-        rh.ldh = L.fpad;
-        rh.eA = (J.lowner < 0 ? J : *P->jobs[J.lowner]).Vst.e.p;
-        rh.rowerr2 = J.rowerr.p;
-        GAIN_CUDA(split::launch_refine_h(rh, std::min(2 * e->num_sms, std::max(1, J.cap1 / 8)), sq));
-        if (L.general) {
-            GAIN_CUDA(launch_contract_rowerr(J.B, J.H.p, L.fpad, L.fpad, J.rowerr.p, J.Vst.e.p, L.sigmaF, L.gamF, sq));
+    GAIN_CUDA(split::launch_refine_h_grouped(P->refine1.p, nj, 2 * e->num_sms, st));
+    if (any_general) {
+        GAIN_TRY(fork());
+        for (int q = 0; q < nj; ++q) {
+            PlanJob& J = *P->jobs[q];
+            PairLayout& L = *J.L;
+            cudaStream_t sq = stream_of(q);
+            if (!L.general) continue;
+            GAIN_CUDA(launch_contract_rowerr(J.B, J.H.p, L.fpad, L.fpad, J.rowerr, J.Vst.e.p, L.sigmaF, L.gamF, sq));
             GAIN_CUDA(launch_contract(L.nsymF, L.d_cF_ptr.p, L.d_cF_col.p, L.d_cF_val.p, J.H.p, L.fpad, J.Hsym.p, J.K2,
                                       J.B, sq));
         }
+        GAIN_TRY(join());
     }
-    GAIN_TRY(join());
     GAIN_TRY(fork());
     GAIN_TRY(plan_launch_slices(P->slices3, streams, kPlanStreams));   // every job's H digits
     GAIN_TRY(join());
@@ -4365,37 +4412,7 @@ gain_status plan_enqueue(gain_plan P) {
         GAIN_CUDA(cudaEventRecordWithFlags(P->ev[4], st, cudaEventRecordExternal));
     }
     // ---- stage 5: FP64 refinement of the amplitudes
-    GAIN_TRY(fork());
-    for (int q = 0; q < nj; ++q) {
-        PlanJob& J = *P->jobs[q];
-        PairLayout& L = *J.L;
-        const gain_pair_job* j = &J.job;
-        cudaStream_t sq = stream_of(q);
-        const Eig& EF = *e->eig[{j->jindF, j->gammaF}];
-        split::RefineAmpArgs ra;
-        ra.flags = J.flags2.p;
-        ra.nflags = P->counters.p + 2 * q + 1;
-        ra.max_flags = J.cap2;
-        ra.U = EF.d.p;
-        ra.nsize = EF.nsize;
-        ra.col_level = J.d_upper.p;
-        ra.colpos = L.general ? L.d_ident.p : L.d_colposF.p;
-        ra.H = L.general ? J.Hsym.p : J.H.p;
-        ra.ldh = J.K2;
-        ra.h_inerr = J.Hst.inerr.p;
-        ra.eH = J.Hst.e.p;
-        ra.amp = J.amp.p;
-        ra.lda = J.Nupad;
-        ra.bnd = J.ampbnd.p;
-        ra.ldb = J.Nupad;
-        ra.tol = (P->has_opts && P->opts.tol > 0) ? P->opts.tol : 4.5e-9;
-        ra.absmax = P->ull.p + 4 * q + 2;
-        ra.amp_floor = std::sqrt((P->has_opts && P->opts.s_floor > 0) ? P->opts.s_floor : 1e-10);
-        ra.uncertified = P->ull.p + 4 * q;
-        ra.uncertified_weak = P->ull.p + 4 * q + 3;
-        GAIN_CUDA(split::launch_refine_amp(ra, std::min(4 * e->num_sms, std::max(1, J.cap2 / 8)), sq));
-    }
-    GAIN_TRY(join());
+    GAIN_CUDA(split::launch_refine_amp_grouped(P->refine2.p, nj, 4 * e->num_sms, st));
     GAIN_CUDA(cudaEventRecordWithFlags(P->ev[5], st, cudaEventRecordExternal));
     GAIN_CUDA(cudaMemcpyAsync(P->rb, P->counters.p, sizeof(unsigned int) * 2 * nj, cudaMemcpyDeviceToHost, st));
     GAIN_CUDA(cudaMemcpyAsync(P->rb + 8 * (size_t)nj, P->ull.p, sizeof(unsigned long long) * 4 * nj,
@@ -4414,7 +4431,16 @@ gain_status plan_build(gain_plan P) {
         GAIN_TRY(P->counters.alloc(2 * nj));
         GAIN_TRY(P->ull.alloc(4 * nj));
         GAIN_TRY(P->err.alloc(1));
+        P->nrowerr = 0;
+        for (auto& J : P->jobs) P->nrowerr += J->Bpad;
+        GAIN_TRY(P->rowerr.alloc(P->nrowerr));
+        float* re = P->rowerr.p;
+        for (auto& J : P->jobs) {
+            J->rowerr = re;
+            re += J->Bpad;
+        }
         GAIN_TRY(plan_build_groups(P));
+        GAIN_TRY(plan_build_refinement(P));
         return plan_build_slices(P);
     };
     // the residue form unless the options (or the autotuner) name digits, or its planes and

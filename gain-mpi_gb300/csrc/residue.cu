@@ -684,12 +684,11 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_residue_slice_grouped(const S
 }
 
 // ------------------------------------------------------------------- reconstruction
-constexpr int kCrtThreads = 128, kCrtCols = 4 * kCrtThreads, kCrtRows = 4;
-// Rows per block: four share their column statistics' loads once that still leaves every SM
-// several blocks; fewer outputs take one row each (the four rows run one after another).
-__host__ __device__ __forceinline__ int crt_rows(const CrtArgs& a) {
-    return (long)a.rows * ((a.cols + kCrtCols - 1) / kCrtCols) >= 4096 ? kCrtRows : 1;
-}
+constexpr int kCrtThreads = 128, kCrtCols = 4 * kCrtThreads;
+// Threads of a block that share a row (four columns each): rows of few columns leave room for two
+// or four rows side by side.
+__host__ __device__ __forceinline__ int crt_width(int cols) { return cols <= 128 ? 32 : cols <= 256 ? 64 : kCrtThreads; }
+__host__ __device__ __forceinline__ int crt_col_blocks(int cols) { return (cols + kCrtCols - 1) / kCrtCols; }
 
 // Bits of the double nearest (ties up) to F 2^-80 M 2^E0: F a signed 80-bit integer in three words
 // (w2, w1, 16 bits w0), M = m_mant 2^(m_exp - 63), E = m_exp - 126 + E0; *mag = |value| 2^-es as a
@@ -735,17 +734,16 @@ __device__ __forceinline__ unsigned long long crt_bits(uint32_t w0, uint32_t w1,
     return sign | (((unsigned long long)(be - 1) << 52) + q);   // q's leading bit, or its carry, adds to the exponent
 }
 
-// Four columns per thread, crt_rows rows per block.  Per output: C / M = sum_i r_i / m_i mod 1 as
+// Four columns per thread, a.nrow rows per block.  Per output: C / M = sum_i r_i / m_i mod 1 as
 // an 80-bit fixed-point sum (three multiply-adds per modulus, carries combined at the end), then value, certified bound and flag.  Reads the residues once
 // (2 bytes per modulus) and writes 8 (12 with bounds) bytes per output.  NM: the number of
 // moduli, 0 for any; all of a row's residues are loaded before the first is used.
-// Measured: 24.6 M outputs 220 us (0.14 ms at the copy bandwidth; the rest is integer issue),
-// 96-bit sums and 64-bit finalisation 237, four loads at a time 330; 50 x 600 outputs 7 us, four
-// rows to a block there 20.
+// Measured: 24.6 M outputs 185 us (0.14 ms at the copy bandwidth; the rest is integer issue), 330
+// with rolled loads, 96-bit sums, 64-bit finalisation and block-wide row sums; 50 x 600 outputs 6 us,
+// with four rows to a block there 20; the 16 M outputs of a 52-pair plan 140 us, one row to a block 172.
 template <bool G, int NM>
 __global__ void __launch_bounds__(kCrtThreads) k_crt(const CrtArgs a0, const CrtGroups gs) {
     __shared__ CrtArgs sa;
-    __shared__ float red_f[kCrtThreads / 32][kCrtRows];
     __shared__ unsigned long long red_m[kCrtThreads / 32];
     const int tid = threadIdx.x;
     int blk = (int)blockIdx.x;
@@ -763,23 +761,20 @@ __global__ void __launch_bounds__(kCrtThreads) k_crt(const CrtArgs a0, const Crt
     }
     if (G) __syncthreads();
     const CrtArgs& a = G ? sa : a0;
-    const int ncb = (a.cols + kCrtCols - 1) / kCrtCols;
-    const int nrow = crt_rows(a);
+    const int ncb = crt_col_blocks(a.cols), width = crt_width(a.cols);
     const int rb = blk / ncb, cb = blk - rb * ncb;
-    const int c = cb * kCrtCols + 4 * tid;
+    const int lane = tid & 31, warp = tid >> 5;
+    const int c = cb * kCrtCols + 4 * (tid & (width - 1));   // a warp lies in one row
     const int nmod = NM ? NM : a.nmod;
-    const int lr0 = rb * nrow, lr1 = min(lr0 + nrow, a.rows);
+    const int lr1 = min((rb + 1) * a.nrow, a.rows);
     unsigned long long vmax = 0ull;
-    float re[kCrtRows];
-#pragma unroll
-    for (int rr = 0; rr < kCrtRows; ++rr) re[rr] = 0.0f;
     if (c < a.cols) {
         const int4 eB4 = *reinterpret_cast<const int4*>(a.B.e + c);
         const float4 lB4 = *reinterpret_cast<const float4*>(a.B.l2 + c), dB4 = *reinterpret_cast<const float4*>(a.B.dn + c);
         const int eB[4] = {eB4.x, eB4.y, eB4.z, eB4.w};
         const float l2B[4] = {lB4.x, lB4.y, lB4.z, lB4.w}, dqB[4] = {dB4.x, dB4.y, dB4.z, dB4.w};
 #pragma unroll 1
-        for (int lr = lr0; lr < lr1; ++lr) {
+        for (int lr = rb * a.nrow + tid / width; lr < lr1; lr += kCrtThreads / width) {
             const int r = a.row0 + lr;
             const uint2* src = reinterpret_cast<const uint2*>(a.res + (long)lr * a.ldr + c);
             uint32_t s0[4] = {0, 0, 0, 0}, s2[4] = {0, 0, 0, 0};   // s0: 16 x 25 bits; s2 wraps (mod 1)
@@ -845,21 +840,13 @@ __global__ void __launch_bounds__(kCrtThreads) k_crt(const CrtArgs a0, const Crt
             o[0] = make_double2(vout[0], vout[1]);
             o[1] = make_double2(vout[2], vout[3]);
             if (a.bnd) *reinterpret_cast<float4*>(a.bnd + (long)r * a.ldb + c) = make_float4(bout[0], bout[1], bout[2], bout[3]);
-            const int rr = lr - lr0;
-#pragma unroll
-            for (int q = 0; q < kCrtRows; ++q)
-                if (q == rr) re[q] = rowerr2;
+            if (a.rowerr2) {   // (columns is a multiple of 128: whole warps are here together)
+                for (int o = 16; o > 0; o >>= 1) rowerr2 = __fadd_ru(rowerr2, __shfl_xor_sync(0xffffffffu, rowerr2, o));
+                if (lane == 0 && rowerr2 > 0.0f) atomicAdd(&a.rowerr2[r], rowerr2 * 1.0001f);   // (the atomics round to nearest)
+            }
         }
     }
-    // per block: warp partials, then one atomic per row (or per block)
-    const int lane = tid & 31, warp = tid >> 5;
-    if (a.rowerr2) {
-#pragma unroll
-        for (int rr = 0; rr < kCrtRows; ++rr) {
-            for (int o = 16; o > 0; o >>= 1) re[rr] = __fadd_ru(re[rr], __shfl_xor_sync(0xffffffffu, re[rr], o));
-            if (lane == 0) red_f[warp][rr] = re[rr];
-        }
-    }
+    // the largest value: warp maxima, one atomic per block that raises it
     if (a.absmax) {
         for (int o = 16; o > 0; o >>= 1) {
             const unsigned long long y = __shfl_xor_sync(0xffffffffu, vmax, o);
@@ -868,11 +855,6 @@ __global__ void __launch_bounds__(kCrtThreads) k_crt(const CrtArgs a0, const Crt
         if (lane == 0) red_m[warp] = vmax;
     }
     __syncthreads();
-    if (a.rowerr2 && tid < nrow) {
-        float t = 0.0f;
-        for (int w = 0; w < kCrtThreads / 32; ++w) t = __fadd_ru(t, red_f[w][tid]);
-        if (t > 0.0f) atomicAdd(&a.rowerr2[a.row0 + lr0 + tid], t * 1.0001f);   // (the atomics round to nearest)
-    }
     if (a.absmax && tid == 0) {
         for (int w = 1; w < kCrtThreads / 32; ++w) vmax = red_m[w] > vmax ? red_m[w] : vmax;
         if (vmax > *(volatile unsigned long long*)a.absmax) atomicMax(a.absmax, vmax);
@@ -942,8 +924,19 @@ void crt_constants(CrtArgs* a) {
 }
 
 int crt_blocks(const CrtArgs& a) {
-    const int n = crt_rows(a);
-    return ((a.cols + kCrtCols - 1) / kCrtCols) * ((a.rows + n - 1) / n);
+    return crt_col_blocks(a.cols) * ((a.rows + a.nrow - 1) / a.nrow);
+}
+
+// Blocks go over several rows (sharing the column statistics, and a grouped launch's look-up of the
+// block's arguments) once that leaves every SM plenty of blocks.
+void crt_set_rows(CrtArgs* a, int n) {
+    long base = 0;
+    for (int q = 0; q < n; ++q) {
+        a[q].nrow = kCrtThreads / crt_width(a[q].cols);
+        base += crt_blocks(a[q]);
+    }
+    const int k = (int)std::max(1l, std::min(8l, base / 4864));
+    for (int q = 0; q < n; ++q) a[q].nrow *= k;
 }
 
 cudaError_t launch_residue_gemm(const CUtensorMap& tmA, const CUtensorMap& tmB, const ResGemmArgs& a, int num_sms,
@@ -993,7 +986,9 @@ cudaError_t launch_residue_gemm_grouped(const ResGemmArgs& a, int units, cudaStr
                 : cudaLaunchKernelEx(&cfg, k_residue_gemm<false, true>, unused, unused, a);
 }
 
-cudaError_t launch_crt(const CrtArgs& a, cudaStream_t st) {
+cudaError_t launch_crt(const CrtArgs& a0, cudaStream_t st) {
+    CrtArgs a = a0;
+    crt_set_rows(&a, 1);
     const int nb = crt_blocks(a);
     if (nb <= 0) return cudaSuccess;
     if (a.nmod == 13) k_crt<false, 13><<<nb, kCrtThreads, 0, st>>>(a, CrtGroups{});

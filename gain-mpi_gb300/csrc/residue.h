@@ -75,7 +75,8 @@ struct CrtArgs {
     int nmod, bits;
     int row0;              // output row of residue row 0
     int rows;              // residue rows to reconstruct
-    int cols;              // columns to reconstruct (a multiple of 4)
+    int cols;              // columns to reconstruct (a multiple of 128)
+    int nrow;              // rows per block (crt_set_rows; launch_crt sets it)
     int cols_valid;        // columns that are flagged and counted
     RowStats A, B;
     double* out;
@@ -97,6 +98,8 @@ struct CrtArgs {
 // m_mant, m_exp and c_fix of a set of nmod moduli at `bits` fraction bits
 void crt_constants(CrtArgs* a);
 cudaError_t launch_crt(const CrtArgs& a, cudaStream_t st);
+// Rows per block (nrow) of n reconstructions in one launch, and the blocks of one of them.
+void crt_set_rows(CrtArgs* a, int n);
 int crt_blocks(const CrtArgs& a);
 // args[g] (device memory) runs on blocks offs[g] <= b < offs[g + 1]
 struct CrtGroups {

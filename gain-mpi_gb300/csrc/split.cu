@@ -1062,7 +1062,17 @@ __global__ void k_wait_selftest(unsigned long long limit_ns, int* err) {
 }
 
 // ------------------------------------------------------------------- refinement
-__global__ void k_refine_h(const RefineHArgs a) {
+// k_refine_*_grouped: the entries of several jobs' lists, list after list.  Usually all are empty:
+// a warp looks at 32 counters at a time.
+template <class A, class F>
+__device__ __forceinline__ void refine_jobs(const A* __restrict__ a, int n, F refine) {
+    const int lane = threadIdx.x & 31;
+    for (int q0 = 0; q0 < n; q0 += 32) {
+        unsigned int filled = __ballot_sync(0xffffffffu, q0 + lane < n && *a[min(q0 + lane, n - 1)].nflags != 0u);
+        for (; filled; filled &= filled - 1u) refine(a[q0 + __ffs((int)filled) - 1]);
+    }
+}
+__device__ __forceinline__ void refine_h(const RefineHArgs& a) {
     const int lane = threadIdx.x & 31;
     const int gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int nw = (gridDim.x * blockDim.x) >> 5;
@@ -1096,7 +1106,12 @@ __global__ void k_refine_h(const RefineHArgs a) {
     }
 }
 
-__global__ void k_refine_amp(const RefineAmpArgs a) {
+__global__ void k_refine_h(const RefineHArgs a) { refine_h(a); }
+__global__ void k_refine_h_grouped(const RefineHArgs* __restrict__ a, int n) {
+    refine_jobs(a, n, [](const RefineHArgs& x) { refine_h(x); });
+}
+
+__device__ __forceinline__ void refine_amp(const RefineAmpArgs& a) {
     const int lane = threadIdx.x & 31;
     const int gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int nw = (gridDim.x * blockDim.x) >> 5;
@@ -1134,6 +1149,11 @@ __global__ void k_refine_amp(const RefineAmpArgs a) {
             }
         }
     }
+}
+
+__global__ void k_refine_amp(const RefineAmpArgs a) { refine_amp(a); }
+__global__ void k_refine_amp_grouped(const RefineAmpArgs* __restrict__ a, int n) {
+    refine_jobs(a, n, [](const RefineAmpArgs& x) { refine_amp(x); });
 }
 
 }  // namespace
@@ -1344,6 +1364,18 @@ cudaError_t launch_band(const BandArgs& a, cudaStream_t st) {
 
 cudaError_t launch_refine_h(const RefineHArgs& a, int max_blocks, cudaStream_t st) {
     k_refine_h<<<max_blocks, 256, 0, st>>>(a);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_refine_h_grouped(const RefineHArgs* a, int n, int blocks, cudaStream_t st) {
+    if (n <= 0) return cudaSuccess;
+    k_refine_h_grouped<<<blocks, 256, 0, st>>>(a, n);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_refine_amp_grouped(const RefineAmpArgs* a, int n, int blocks, cudaStream_t st) {
+    if (n <= 0) return cudaSuccess;
+    k_refine_amp_grouped<<<blocks, 256, 0, st>>>(a, n);
     return cudaGetLastError();
 }
 

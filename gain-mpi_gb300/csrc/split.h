@@ -221,6 +221,8 @@ struct RefineHArgs {
     float* rowerr2;
 };
 cudaError_t launch_refine_h(const RefineHArgs& a, int max_blocks, cudaStream_t st);
+// the same for n jobs' lists in one launch (a: device memory)
+cudaError_t launch_refine_h_grouped(const RefineHArgs* a, int n, int blocks, cudaStream_t st);
 
 // FP64 recomputation of flagged amplitudes.
 struct RefineAmpArgs {
@@ -246,6 +248,7 @@ struct RefineAmpArgs {
     unsigned long long* uncertified_weak;  // below it
 };
 cudaError_t launch_refine_amp(const RefineAmpArgs& a, int max_blocks, cudaStream_t st);
+cudaError_t launch_refine_amp_grouped(const RefineAmpArgs* a, int n, int blocks, cudaStream_t st);
 
 }  // namespace split
 }  // namespace gain

@@ -307,9 +307,9 @@ gain_status gain_run_plan(gain_engine* engines, int n_engines, const gain_pair_j
  *                                                                kernel; jobs of one block
  *                                                                share its digits)
  *   ONE persistent grouped tensor-core launch of the first GEMM over the tiles of all jobs
- *   per-job FP64 refinement of H (concurrent streams), then the digits of all jobs' H
+ *   FP64 refinement of every job's H (one launch), then the digits of all jobs' H
  *   ONE persistent grouped tensor-core launch of the second GEMM over all jobs' tiles
- *   per-job FP64 refinement of the amplitudes                   (concurrent streams)
+ *   FP64 refinement of every job's amplitudes                  (one launch)
  * captured once into a CUDA graph and replayed by gain_plan_run.  The tiles of each grouped
  * launch are dealt to the persistent CTAs in list order, each to the first free one, with
  * the jobs with the costliest tiles (k-blocks x digit products) first, so block pairs of

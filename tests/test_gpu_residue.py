@@ -132,3 +132,33 @@ def test_scales_and_zero_rows(built_lib):
     eng.run_pair(0, 0, 1, 1, lo, up, gainls.PATH_SPLIT)
     got = eng.fetch_amp()
     assert np.max(np.abs(got - np.ldexp(ref, -1060))) <= 2.0 ** -1074 * 64 * vI.shape[1]
+
+
+@pytest.mark.gpu
+def test_plan_refines_flagged_entries_of_every_job(built_lib, monkeypatch):
+    """A first GEMM of 40 bits: no H entry certifies FP64-grade, so every job's list is full.  The
+    plan's one refinement launch recomputes what the single runs' do, and both agree with the
+    plain FP64 path as an FP64 H and a 48-bit second GEMM must (see above)."""
+    import gainls
+    import synth
+    p = synth.make_problem(20, [1, 2, 3], "c4")
+    eng = gainls.Engine(JMAX, p.nsym, 1)
+    gainls.upload_problem(eng, p)
+    filt = gainls.make_filters([1.0] * 4, p.isym_pairs, p.igamma_pair, p.sym_degen, (0.0, 5000.0), (-1e9, 1e9),
+                               (-1e9, 1e9), 0.0, 3)
+    table = gainls.state_table(p.st_energy, p.st_J, p.st_jind, p.st_gamma, p.st_ndeg, p.st_ilevel)
+    jobs = gainls.plan_pairs(filt, table)
+    monkeypatch.setenv("GAINLS_GEMM1_BITS", "40")
+    plan = gainls.Plan(eng, jobs)
+    ps, js, st = plan.run()
+    assert st == gainls.OK and all(j["inexact"] > 0 for j in js)
+    for q, job in enumerate(jobs):
+        one = eng.run_pair(*job, gainls.PATH_SPLIT)
+        assert one["inexact"] == js[q]["inexact"]
+        eng.run_pair(*job, gainls.PATH_PLAIN_FP64)
+        ref = eng.fetch_amp().copy()
+        N = p.blocks[(job[2], job[3])].vecs.shape[1]
+        mrow = np.sqrt(15.0) * np.sqrt((p.dipole ** 2).sum(axis=(0, 1))).max()
+        tol = (4 * np.sqrt(N) * 2.0 ** -48) * np.sqrt(N) * mrow + np.sqrt(N) * (3 * N + 64) * 2.0 ** -52 * mrow
+        assert np.max(np.abs(plan.amp(q) - ref)) <= tol
+    plan.close()
