@@ -11,6 +11,7 @@
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
+#include <limits>
 #include <map>
 #include <mutex>
 #include <queue>
@@ -325,6 +326,9 @@ struct gain_engine_s {
     gain::DevArray<long long> ovrIdx;
     gain::DevArray<double> ovrVal;
     gain::DevArray<double> pow10;   // 10^k, k = -300..300, correctly rounded (C library strtod)
+    gain::DevArray<unsigned long long> textMant;   // the conversions' table of powers of ten
+    gain::DevArray<gain::TextArgs::Patch> textPatch;
+    gain::DevArray<double> rowFactor;
     long long intensity_host = 0;
     long launches = 0;          // kernels this engine has launched (split path and band builds)
     void* readback = nullptr;   // page-locked area of a run's counter readbacks
@@ -1966,6 +1970,16 @@ LineParams line_params(const gain_line_params* prm, int jI, int jF, bool with_in
     p.thresh = prm->thresh;
     p.freq_lo = prm->freq_lo;
     p.freq_hi = prm->freq_hi;
+    // the bits of non-negative doubles are ordered as the doubles; a NaN limit passes nothing
+    auto bits = [](double x) {
+        long long b;
+        memcpy(&b, &x, sizeof b);
+        return b;
+    };
+    constexpr long long kNone = std::numeric_limits<long long>::max();
+    p.nu_lo = std::isnan(p.freq_lo) ? kNone : bits(std::max(p.freq_lo, 1e-40));
+    p.nu_hi = p.freq_hi > 0 ? bits(p.freq_hi) : -1;
+    p.a_lo = std::isnan(p.thresh) ? kNone : p.thresh > 0 ? bits(p.thresh) : 0;
     p.with_intensity = with_intensity;
     p.nslot = 0;
     p.ndegI = 1;
@@ -3442,7 +3456,11 @@ gain_status lines_text(gain_engine e, const gain_line_params* prm, const double*
     GAIN_TRY(thresh_certify(e, prm, lp, amp, ld));
     GAIN_TRY(e->textLens.alloc(n));
     GAIN_TRY(e->textBlocks.alloc(nb + 3));
-    GAIN_TRY(e->textBlocks.zero(st, nb + 3));
+    if (!e->textMant.p) {
+        int count = 0;
+        const unsigned long long* mant = text_pow10(&count);
+        GAIN_TRY(e->textMant.upload(mant, count));
+    }
     TextArgs t;
     t.rows = rows;
     t.cols = cols;
@@ -3458,6 +3476,7 @@ gain_status lines_text(gain_engine e, const gain_line_params* prm, const double*
     t.gammaI = gammaI;
     t.gammaF = gammaF;
     t.with_amps = (flags & GAIN_TEXT_AMPLITUDES) != 0;
+    t.row_factor = nullptr;
     t.lens = e->textLens.p;
     t.block_bytes = e->textBlocks.p;
     t.nkeep = e->textBlocks.p + nb + 1;
@@ -3467,6 +3486,10 @@ gain_status lines_text(gain_engine e, const gain_line_params* prm, const double*
     t.nhard = nullptr;
     t.hard_cap = 0;
     t.pow10 = nullptr;
+    t.mant = e->textMant.p;
+    // an intensity without a sign always fills its 16 characters: A, 2J+1, exp, 1 - exp(-beta nu)
+    // and Q are not negative, so only the spin weight decides
+    t.signed_intensity = lp.with_intensity && !(lp.gnsF >= 0.0);
     t.ovr_idx = nullptr;
     t.ovr_val = nullptr;
     t.n_ovr = 0;
@@ -3481,76 +3504,105 @@ gain_status lines_text(gain_engine e, const gain_line_params* prm, const double*
             GAIN_TRY(e->pow10.upload(pw));
         }
         t.pow10 = e->pow10.p;
+        GAIN_TRY(e->rowFactor.alloc(rows));
+        t.row_factor = e->rowFactor.p;
         GAIN_TRY(e->hardLines.alloc(kHardCap));
         GAIN_TRY(e->hardCount.alloc(1));
-        GAIN_TRY(e->hardCount.zero(st, 1));
         t.hard = e->hardLines.p;
         t.nhard = e->hardCount.p;
         t.hard_cap = kHardCap;
     }
-    GAIN_CUDA(launch_text_len(t, st));
     std::vector<unsigned long long> offs(nb + 3);   // block offsets, text size, lines, largest block
-    unsigned int nhard = 0;
-    GAIN_CUDA(cudaMemcpyAsync(offs.data(), e->textBlocks.p, sizeof(unsigned long long) * (nb + 3),
-                              cudaMemcpyDeviceToHost, st));
-    if (t.nhard) GAIN_CUDA(cudaMemcpyAsync(&nhard, t.nhard, sizeof nhard, cudaMemcpyDeviceToHost, st));
-    GAIN_CUDA(cudaStreamSynchronize(st));
+    std::vector<TextArgs::HardLine> hl;
+    std::vector<TextArgs::Patch> patches;
+    unsigned long long total = 0;
+    bool copy = false;
     e->intensity_host = 0;
-    if (nhard > 0) {
-        // Output.cpp:101-102 on the host, with this host's exp, for the lines whose printed
-        // intensity the device's exp could change; both passes then print these values
-        if (nhard > (unsigned)kHardCap)
-            return set_error(GAIN_ERR_UNSUPPORTED, "%u lines need the host's intensity (at most %d)", nhard, kHardCap);
-        std::vector<TextArgs::HardLine> hl(nhard);
-        GAIN_CUDA(cudaMemcpy(hl.data(), e->hardLines.p, sizeof(TextArgs::HardLine) * nhard, cudaMemcpyDeviceToHost));
-        std::sort(hl.begin(), hl.end(), [](const TextArgs::HardLine& a, const TextArgs::HardLine& b) {
-            return a.idx < b.idx;
-        });
-        std::vector<long long> oi(nhard);
-        std::vector<double> ov(nhard);
-        bool relen = false;
-        for (unsigned int k = 0; k < nhard; ++k) {
-            oi[k] = hl[k].idx;
-            ov[k] = host_intensity(lp, hl[k].A, hl[k].nu, hl[k].eI);
-            char b1[64], b2[64];
-            relen = relen || snprintf(b1, sizeof b1, "%16.9E", hl[k].I) != snprintf(b2, sizeof b2, "%16.9E", ov[k]);
+    for (bool again = true; again;) {   // at most twice: with the host's values no line is listed
+        again = false;
+        GAIN_TRY(e->textBlocks.zero(st, nb + 3));
+        if (t.hard) GAIN_TRY(e->hardCount.zero(st, 1));
+        GAIN_CUDA(launch_text_len(t, st));
+        GAIN_CUDA(cudaMemcpyAsync(offs.data(), e->textBlocks.p, sizeof(unsigned long long) * (nb + 3),
+                                  cudaMemcpyDeviceToHost, st));
+        GAIN_CUDA(cudaStreamSynchronize(st));
+        total = offs[nb];
+        const unsigned long long largest = offs[nb + 2];
+        GAIN_TRY(e->text.alloc(total ? total : 1));
+        t.text = e->text.p;
+        t.text_size = total;
+        copy = out && cap >= total;
+        // parts of at least 64 blocks (about 6 MB of text) on average, at most 8; they grow from
+        // the first on, whose formatting is all that the copies wait for
+        const long nparts = copy ? std::max(1L, std::min(8L, nb / 64)) : 1;
+        for (long part = 0; part < nparts; ++part) {
+            const long b0 = nb * part * part / (nparts * nparts);
+            const long b1 = nb * (part + 1) * (part + 1) / (nparts * nparts);
+            GAIN_CUDA(launch_text_write(t, largest, b0, b1, st));
+            if (copy) {
+                const unsigned long long o0 = offs[b0], o1 = b1 < nb ? offs[b1] : total;
+                GAIN_CUDA(cudaEventRecord(e->ev[8], st));
+                GAIN_CUDA(cudaStreamWaitEvent(e->stc, e->ev[8], 0));
+                if (o1 > o0)
+                    GAIN_CUDA(cudaMemcpyAsync(out + o0, e->text.p + o0, o1 - o0, cudaMemcpyDeviceToHost, e->stc));
+            }
         }
-        GAIN_TRY(e->ovrIdx.upload(oi));
-        GAIN_TRY(e->ovrVal.upload(ov));
-        t.ovr_idx = e->ovrIdx.p;
-        t.ovr_val = e->ovrVal.p;
-        t.n_ovr = (int)nhard;
-        e->intensity_host = nhard;
-        if (relen) {   // a field length changed (an exponent of three digits, say): lengths again
-            t.hard = nullptr;
-            GAIN_TRY(e->textBlocks.zero(st, nb + 3));
-            GAIN_CUDA(launch_text_len(t, st));
-            GAIN_CUDA(cudaMemcpyAsync(offs.data(), e->textBlocks.p, sizeof(unsigned long long) * (nb + 3),
-                                      cudaMemcpyDeviceToHost, st));
+        if (t.hard) {
+            unsigned int nhard = 0;
+            GAIN_CUDA(cudaMemcpyAsync(&nhard, t.nhard, sizeof nhard, cudaMemcpyDeviceToHost, st));
             GAIN_CUDA(cudaStreamSynchronize(st));
+            if (nhard > (unsigned)kHardCap) {
+                if (copy) GAIN_CUDA(cudaStreamSynchronize(e->stc));
+                return set_error(GAIN_ERR_UNSUPPORTED, "%u lines need the host's intensity (at most %d)", nhard,
+                                 kHardCap);
+            }
+            // Output.cpp:101-102 on the host, with this host's exp, for the lines whose printed
+            // intensity the device's exp could change; the text then holds these values
+            hl.resize(nhard);
+            patches.resize(nhard);
+            if (nhard > 0)
+                GAIN_CUDA(cudaMemcpyAsync(hl.data(), e->hardLines.p, sizeof(TextArgs::HardLine) * nhard,
+                                          cudaMemcpyDeviceToHost, st));
+            GAIN_CUDA(cudaStreamSynchronize(st));
+            for (unsigned int k = 0; k < nhard; ++k) {
+                char b[64];
+                const int len = gain_format_value(b, sizeof b, host_intensity(lp, hl[k].A, hl[k].nu, hl[k].eI), 'E', 16, 9);
+                again = again || len != hl[k].len;
+                patches[k].pos = hl[k].pos;
+                patches[k].len = len;
+                memcpy(patches[k].s, b, std::min((size_t)len, sizeof patches[k].s));
+            }
+            e->intensity_host = nhard;
+            if (!again && nhard > 0) {
+                GAIN_TRY(e->textPatch.upload(patches));
+                GAIN_CUDA(launch_text_patch(e->text.p, total, e->textPatch.p, (int)nhard, st));
+            }
+        }
+        GAIN_CUDA(cudaStreamSynchronize(st));
+        if (copy) GAIN_CUDA(cudaStreamSynchronize(e->stc));
+        if (again) {   // a field length changed (an exponent of three digits after a sign): once more
+            std::sort(hl.begin(), hl.end(), [](const TextArgs::HardLine& a, const TextArgs::HardLine& b) {
+                return a.idx < b.idx;
+            });
+            std::vector<long long> oi;
+            std::vector<double> ov;
+            for (const TextArgs::HardLine& h : hl) {
+                oi.push_back(h.idx);
+                ov.push_back(host_intensity(lp, h.A, h.nu, h.eI));
+            }
+            GAIN_TRY(e->ovrIdx.upload(oi));
+            GAIN_TRY(e->ovrVal.upload(ov));
+            t.ovr_idx = e->ovrIdx.p;
+            t.ovr_val = e->ovrVal.p;
+            t.n_ovr = (int)oi.size();
+            t.hard = nullptr;
+            patches.clear();
         }
     }
-    const unsigned long long total = offs[nb], lines = offs[nb + 1], largest = offs[nb + 2];
+    if (copy)
+        for (const TextArgs::Patch& q : patches) memcpy(out + q.pos, q.s, (size_t)q.len);
     if (text_bytes) *text_bytes = total;
-    if (n_lines) *n_lines = (long long)lines;
-    GAIN_TRY(e->text.alloc(total ? total : 1));
-    t.text = e->text.p;
-    t.text_size = total;
-    const bool copy = out && cap >= total;
-    // parts of at least 64 blocks (about 6 MB of text) each, at most 8
-    const long nparts = copy ? std::max(1L, std::min(8L, nb / 64)) : 1;
-    for (long part = 0; part < nparts; ++part) {
-        const long b0 = nb * part / nparts, b1 = nb * (part + 1) / nparts;
-        GAIN_CUDA(launch_text_write(t, largest, b0, b1, st));
-        if (copy) {
-            const unsigned long long o0 = offs[b0], o1 = b1 < nb ? offs[b1] : total;
-            GAIN_CUDA(cudaEventRecord(e->ev[8], st));
-            GAIN_CUDA(cudaStreamWaitEvent(e->stc, e->ev[8], 0));
-            if (o1 > o0) GAIN_CUDA(cudaMemcpyAsync(out + o0, e->text.p + o0, o1 - o0, cudaMemcpyDeviceToHost, e->stc));
-        }
-    }
-    GAIN_CUDA(cudaStreamSynchronize(st));
-    if (copy) GAIN_CUDA(cudaStreamSynchronize(e->stc));
+    if (n_lines) *n_lines = (long long)offs[nb + 1];
     e->text_bytes = total;
     e->have_text = true;
     if (out && !copy)
@@ -3608,10 +3660,14 @@ gain_status gain_format_values_device(const double* values, long long n, int con
     DevArray<double> v;
     DevArray<char> o;
     DevArray<int> l;
+    DevArray<unsigned long long> m;
+    int count = 0;
+    const unsigned long long* mant = text_pow10(&count);
     GAIN_TRY(v.upload(values, (size_t)n));
+    GAIN_TRY(m.upload(mant, (size_t)count));
     GAIN_TRY(o.alloc((size_t)n * stride));
     GAIN_TRY(l.alloc((size_t)n));
-    GAIN_CUDA(launch_format_values(n, v.p, conv, width, prec, o.p, stride, l.p, nullptr));
+    GAIN_CUDA(launch_format_values(n, v.p, conv, width, prec, m.p, o.p, stride, l.p, nullptr));
     GAIN_CUDA(cudaMemcpy(out, o.p, (size_t)n * stride, cudaMemcpyDeviceToHost));
     GAIN_CUDA(cudaMemcpy(lens, l.p, sizeof(int) * (size_t)n, cudaMemcpyDeviceToHost));
     return GAIN_OK;

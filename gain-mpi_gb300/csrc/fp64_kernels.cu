@@ -452,7 +452,10 @@ k_lines(int rows, int cols, const double* __restrict__ amp, long ld,
         kept += v.keep;
         if (S) S[idx] = v.ls;
         if (A) A[idx] = v.A;
-        if (I) I[idx] = v.I;
+        if (I) {
+            double e2;
+            I[idx] = p.with_intensity ? line_intensity(v, line_row_factor(eI[r], p), p, &e2) : 0.0;
+        }
         if (keep) keep[idx] = (unsigned char)v.keep;
     }
     for (int o = 16; o > 0; o >>= 1) kept += __shfl_xor_sync(0xffffffffu, kept, o);

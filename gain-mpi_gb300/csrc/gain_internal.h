@@ -159,6 +159,8 @@ struct LineParams {
     double acoef_2jI1;   // ACOEF * (2 jI + 1), the first product of Output.cpp:93
     double cmcoef, gnsF, two_jF1;
     double beta, zpe, q_part, thresh, freq_lo, freq_hi;
+    // the same limits on the bits of nu and A (line_eval): nu_lo <= nu <= nu_hi, a_lo <= A
+    long long nu_lo, nu_hi, a_lo;
     int with_intensity;
     // Degenerate states (Output.cpp:78-91): nslot > 0 sums amp^2 over the listed component
     // slots (idegF outer, idegI inner, those passing DegeneracyFilter), divides by ndegI and,
@@ -188,23 +190,29 @@ struct TextArgs {
     LineParams p;
     const int *levI, *levF;                // printed level indices (0-based) of rows / columns
     int jI, jF, gammaI, gammaF, with_amps;
+    double* row_factor;                    // [rows]: line_row_factor of each row, left by the length pass
     uint32_t* lens;                        // [rows*cols] text length of each line (0: not written)
     unsigned long long* block_bytes;       // [text_blocks + 3]: block offsets, the total, -, the largest block
     unsigned long long* nkeep;             // lines written
     char* text;
     unsigned long long text_size;          // bytes of text (the write pass stays inside)
     // Intensity column: lines whose printed intensity could differ from the host C library's
-    // (the device exp and the host exp may differ in the last bits) are listed by the length
-    // pass; the host evaluates their intensity with its own exp and both passes then print
-    // those values (ovr_idx sorted, n_ovr entries)
-    struct HardLine { long long idx; double A, nu, eI, I; };
+    // (the device exp and the host exp may differ in the last bits) are listed by the write
+    // pass with the place of their text; the host evaluates their intensity with its own exp
+    // and its text replaces the device's.  Where a length depends on the intensity
+    // (signed_intensity, a negative spin weight) and the host's differs, the passes run again
+    // with the host's values (ovr_idx sorted, n_ovr entries).
+    struct HardLine { long long idx; double A, nu, eI; unsigned long long pos; int len; };
     HardLine* hard;                        // may be null (no collection)
     const double* pow10;                   // [601]: pow10[k + 300] = 10^k correctly rounded
+    const unsigned long long* mant;        // the conversions' table (text_pow10)
     unsigned int* nhard;
-    int hard_cap;
+    int hard_cap, signed_intensity;
     const long long* ovr_idx;
     const double* ovr_val;
     int n_ovr;
+    // a replaced field: len characters at text + pos
+    struct Patch { unsigned long long pos; int len; char s[20]; };
 };
 long text_blocks(long lines);
 cudaError_t launch_text_len(const TextArgs& t, cudaStream_t st);     // lens, offsets, total, nkeep
@@ -212,7 +220,12 @@ cudaError_t launch_text_len(const TextArgs& t, cudaStream_t st);     // lens, of
 // blocks [b0, b1) of the text
 cudaError_t launch_text_write(const TextArgs& t, unsigned long long max_block_bytes, long b0, long b1,
                               cudaStream_t st);
-cudaError_t launch_format_values(long n, const double* vals, int conv, int width, int prec, char* out,
-                                 int stride, int* lens, cudaStream_t st);
+cudaError_t launch_text_patch(char* text, unsigned long long text_size, const TextArgs::Patch* patches, int n,
+                              cudaStream_t st);
+// the conversions' table of powers of ten (host memory, *count entries)
+const unsigned long long* text_pow10(int* count);
+cudaError_t launch_format_values(long n, const double* vals, int conv, int width, int prec,
+                                 const unsigned long long* mant, char* out, int stride, int* lens,
+                                 cudaStream_t st);
 
 }  // namespace gain

@@ -10,14 +10,22 @@
 // remainder was dropped), and round that half to even.  %E picks the exponent X from
 // floor(log2 y) log10(2) and corrects it until the 1+prec digit significand lies in
 // [10^prec, 10^(prec+1)) -- the exponent printf prints, which is fixed after rounding.
+//
+// Nearly every conversion takes a short way to the same digits: %f below 2^33 is exact in 128
+// bits; %E multiplies by the leading 64 bits of the power of ten (make_pow10) and keeps the
+// digits when the product's error, less than two units of its upper word, cannot reach a
+// rounding boundary.  What is left (ties among it, about one value in 10^8 at ten digits) and
+// values outside those ranges take the big integers.
 #pragma once
 #include <cstdint>
 #include <cstring>
 
 #if defined(__CUDACC__)
 #define GAIN_HD __host__ __device__ __forceinline__
+#define GAIN_HD_CALL static __host__ __device__ __noinline__   // the long ways, off the fast path
 #else
 #define GAIN_HD inline
+#define GAIN_HD_CALL static
 #endif
 
 namespace gain {
@@ -188,23 +196,94 @@ struct Sink {
     GAIN_HD void spaces(int k) {
         for (int i = 0; i < k; ++i) put(' ');
     }
-    GAIN_HD void digits(uint64_t v, int width) {   // exactly width digits, zero-padded
-        char t[20];
-        for (int i = width - 1; i >= 0; --i) {
-            t[i] = (char)('0' + v % 10u);
-            v /= 10u;
+    // the last `width` <= 9 digits of v < 10^9, zero-padded: v / 10^8 as 32.32 fixed point (2^57 /
+    // 10^8 rounded up, and one unit up: the digits of every v < 10^9 come out exact), then digit by
+    // digit from the fraction, without a division
+    GAIN_HD void digits9(uint32_t v, int width) {
+        uint64_t f = (((uint64_t)v * 1441151881u) >> 25) + 1u;
+#pragma unroll
+        for (int i = 9; i > 0; --i) {
+            if (i <= width) put((char)('0' + (uint32_t)(f >> 32)));
+            f = (uint64_t)(uint32_t)f * 10u;
         }
-        for (int i = 0; i < width; ++i) put(t[i]);
+    }
+    GAIN_HD void digits(uint64_t v, int width) {   // exactly width digits, zero-padded; v < 10^width
+        if (width > 18) {
+            digits9((uint32_t)(v / 1000000000000000000ull), width - 18);
+            v %= 1000000000000000000ull;
+            width = 18;
+        }
+        if (width > 9) {
+            digits9((uint32_t)(v / 1000000000u), width - 9);
+            v %= 1000000000u;
+            width = 9;
+        }
+        digits9((uint32_t)v, width);
     }
 };
 
 GAIN_HD int ndigits(uint64_t v) {
     int d = 1;
-    while (v >= 10u) {
-        v /= 10u;
-        ++d;
+    while (v >= 1000000000u) {
+        v /= 1000000000u;
+        d += 9;
     }
-    return d;
+    const uint32_t u = (uint32_t)v;
+    return d + (u >= 10u) + (u >= 100u) + (u >= 1000u) + (u >= 10000u) + (u >= 100000u) + (u >= 1000000u) +
+           (u >= 10000000u) + (u >= 100000000u);
+}
+
+GAIN_HD uint64_t mulhi64(uint64_t a, uint64_t b) {
+#if defined(__CUDA_ARCH__)
+    return __umul64hi(a, b);
+#else
+    return (uint64_t)(((unsigned __int128)a * b) >> 64);
+#endif
+}
+
+// mant[k - kPow10Min] = floor(10^k 2^(63 - floor(log2 10^k))): the leading 64 bits of 10^k.
+constexpr int kPow10Min = -330, kPow10Max = 345, kPow10Count = kPow10Max - kPow10Min + 1;
+GAIN_HD int pow10_log2(int k) { return (int)(((long long)k * 1741647) >> 19); }   // floor(k log2 10), |k| <= 1233
+inline void make_pow10(uint64_t* mant) {
+    for (int k = kPow10Min; k <= kPow10Max; ++k) {
+        Big b;
+        const int e = pow10_log2(k);
+        big_set(b, 1);
+        if (k < 0) big_shl(b, 63 - e);
+        for (int j = k; j > 0; j -= 9) big_mul(b, j >= 9 ? 1000000000u : pow10_32(j));
+        for (int j = -k; j > 0; j -= 9) big_div(b, j >= 9 ? 1000000000u : pow10_32(j));
+        if (k >= 0) {
+            if (e >= 63) big_shr(b, e - 63);
+            else big_shl(b, 63 - e);
+        }
+        mant[k - kPow10Min] = big_u64(b);
+    }
+}
+
+// D = x 10^k rounded to an integer, ties to even, for x = m 2^e with 0 < m < 2^53, where the
+// leading 64 bits of 10^k decide it; *margin then holds the distance of x 10^k from the nearest
+// half-integer (to 10^-6 relative, 10^-7 absolute for D < 2^35).  False when they do not.
+GAIN_HD bool scaled_round_fast(uint64_t m, int e, int k, const uint64_t* mant, uint64_t* D, float* margin) {
+    if (k < kPow10Min || k > kPow10Max) return false;
+    const int z = clz64(m);
+    // x 10^k = (hi + d) 2^-s, 0 <= d < 2
+    const uint64_t hi = mulhi64(m << z, mant[k - kPow10Min]);
+    const int s = -(e - z + pow10_log2(k) + 1);
+    if (s < 2 || s > 63) return false;
+    const uint64_t half = 1ull << (s - 1), frac = hi & ((half << 1) - 1ull);
+    const bool up = frac > half;
+    *D = (hi >> s) + (up ? 1u : 0u);
+    *margin = (float)(up ? frac - half : half - frac) / (float)half * 0.5f;
+    return up || frac + 2u < half;
+}
+
+// The same by big integers; false when D does not fit 64 bits.
+GAIN_HD_CALL bool scaled_round_u64(uint64_t m, int e, int k, uint64_t* D) {
+    Big q;
+    scaled_round(m, e, k, q);
+    if (q.n > 2) return false;
+    *D = big_u64(q);
+    return true;
 }
 
 // "%<width>d"
@@ -217,32 +296,34 @@ GAIN_HD void put_d(Sink& s, int v, int width) {
     s.digits(a, nd);
 }
 
-// "%<width>.<prec>E", prec <= 17
-GAIN_HD void put_E(Sink& s, double x, int width, int prec) {
+// "%<width>.<prec>E", prec <= 17.  mant: the table of make_pow10 (NULL: big integers only).
+// *margin (optional): how far the value lies from the nearest other rounding, in units of the
+// last digit printed; 0 when the short way did not decide the digits or they are next to a power of ten.
+GAIN_HD void put_E(Sink& s, double x, int width, int prec, const uint64_t* mant, float* margin = nullptr) {
     const Parts p = decompose(x);
+    if (margin) *margin = 0.0f;
     if (p.nan || p.inf) {
         s.spaces(width - 3 - (p.neg ? 1 : 0));
         if (p.neg) s.put('-');
         s.puts(p.nan ? "NAN" : "INF");
         return;
     }
+    uint64_t lo = 1;
+    for (int i = 0; i < prec; ++i) lo *= 10u;
     uint64_t D = 0;
     int X = 0;
     if (p.m != 0) {
         const int e2 = p.e + 63 - clz64(p.m);   // floor(log2 |x|)
         const int t = e2 * 78913;               // 78913 / 2^18 ~ log10(2)
         X = t >= 0 ? (t >> 18) : -((-t + 262143) >> 18);
-        uint64_t lo = 1;
-        for (int i = 0; i < prec; ++i) lo *= 10u;
         const uint64_t hi = lo * 10u;
         for (int it = 0; it < 6; ++it) {
-            Big q;
-            scaled_round(p.m, p.e, prec - X, q);
-            if (q.n > 2) {
+            float mg = 0.0f;
+            if ((!mant || !scaled_round_fast(p.m, p.e, prec - X, mant, &D, &mg)) &&
+                !scaled_round_u64(p.m, p.e, prec - X, &D)) {
                 ++X;
                 continue;
             }
-            D = big_u64(q);
             if (D >= hi) {
                 ++X;
                 continue;
@@ -251,11 +332,10 @@ GAIN_HD void put_E(Sink& s, double x, int width, int prec) {
                 --X;
                 continue;
             }
+            if (margin && D > lo + 2u && D + 3u < hi) *margin = mg;
             break;
         }
     }
-    uint64_t lo = 1;
-    for (int i = 0; i < prec; ++i) lo *= 10u;
     const int ax = X < 0 ? -X : X;
     const int xd = ax >= 100 ? 3 : 2;
     const int len = (p.neg ? 1 : 0) + 1 + (prec ? 1 + prec : 0) + 2 + xd;
@@ -271,20 +351,13 @@ GAIN_HD void put_E(Sink& s, double x, int width, int prec) {
     s.digits((uint64_t)ax, xd);
 }
 
-// "%<width>.<prec>f", prec <= 9
-GAIN_HD void put_F(Sink& s, double x, int width, int prec) {
-    const Parts p = decompose(x);
-    if (p.nan || p.inf) {
-        s.spaces(width - 3 - (p.neg ? 1 : 0));
-        if (p.neg) s.put('-');
-        s.puts(p.nan ? "nan" : "inf");
-        return;
-    }
+// The digits of |x| = m 2^e for %.<prec>f by big integers.
+GAIN_HD_CALL void put_F_big(Sink& s, uint64_t m, int e, bool neg, int width, int prec) {
     Big q;
     q.n = 0;
-    if (p.m != 0) scaled_round(p.m, p.e, prec, q);
+    if (m != 0) scaled_round(m, e, prec, q);
     const uint32_t frac = prec ? big_div(q, pow10_32(prec)) : 0u;
-    const int sign = p.neg ? 1 : 0;
+    const int sign = neg ? 1 : 0;
     if (q.n <= 2) {   // integer part below 2^64
         const uint64_t ip = big_u64(q);
         const int nd = ndigits(ip);
@@ -304,6 +377,49 @@ GAIN_HD void put_F(Sink& s, double x, int width, int prec) {
     if (prec) {
         s.put('.');
         s.digits(frac, prec);
+    }
+}
+
+// "%<width>.<prec>f", prec <= 9
+GAIN_HD void put_F(Sink& s, double x, int width, int prec) {
+    const Parts p = decompose(x);
+    if (p.nan || p.inf) {
+        s.spaces(width - 3 - (p.neg ? 1 : 0));
+        if (p.neg) s.put('-');
+        s.puts(p.nan ? "nan" : "inf");
+        return;
+    }
+    // |x| < 2^33: q = x 10^prec rounded, from the 128-bit product m 10^prec = hi 2^64 + lo < 2^83.
+    // 20 <= sh = -e there; from sh = 64 on the result is below 2^19.
+    const int sh = -p.e;
+    if (p.m != 0 && p.e + 63 - clz64(p.m) > 32) return put_F_big(s, p.m, p.e, p.neg, width, prec);
+    const uint32_t f = pow10_32(prec);
+    const uint64_t hi = mulhi64(p.m, f), lo = p.m * f;
+    uint64_t q = 0, rem = 0, half = 1;   // remainder and half a unit, in 2^-sh (2^(64 - sh) past 64)
+    bool sticky = false;
+    if (sh < 64) {
+        q = (lo >> sh) | (hi << (64 - sh));
+        rem = lo & ((1ull << sh) - 1ull);
+        half = 1ull << (sh - 1);
+    } else if (sh == 64) {
+        q = hi;
+        rem = lo;
+        half = 1ull << 63;
+    } else if (sh < 128) {
+        q = hi >> (sh - 64);
+        rem = hi & ((1ull << (sh - 64)) - 1ull);
+        half = 1ull << (sh - 65);
+        sticky = lo != 0;
+    }
+    q += rem > half || (rem == half && (sticky || (q & 1u))) ? 1u : 0u;
+    const uint64_t ip = q / f;
+    const int nd = ndigits(ip), sign = p.neg ? 1 : 0;
+    s.spaces(width - sign - nd - (prec ? 1 + prec : 0));
+    if (sign) s.put('-');
+    s.digits(ip, nd);
+    if (prec) {
+        s.put('.');
+        s.digits(q - ip * f, prec);
     }
 }
 
@@ -329,7 +445,7 @@ GAIN_HD int len_E(double x, int width, int prec) {
     }
     if (body < 0) {
         Sink c{nullptr, 0, 0};
-        put_E(c, x, 0, prec);
+        put_E(c, x, 0, prec, nullptr);
         body = (int)c.n;
     }
     return body > width ? body : width;
@@ -343,9 +459,8 @@ GAIN_HD int len_F(double x, int width, int prec) {
     if (p.nan || p.inf) {
         body = 3 + (p.neg ? 1 : 0);
     } else {
-        const double a = x < 0 ? -x : x;
-        if (a < 9007199254740992.0) {
-            const uint64_t ip = (uint64_t)a;
+        if (p.e <= 0) {
+            const uint64_t ip = p.e > -64 ? p.m >> -p.e : 0;
             const int nd = ndigits(ip);
             if (ndigits(ip + 1) == nd) body = (p.neg ? 1 : 0) + nd + (prec ? 1 + prec : 0);
         }
@@ -366,9 +481,11 @@ struct LineFields {
     int with_intensity;
     const double* amps;   // linestrength components (output_linestrengths), namp of them
     int namp;
+    const uint64_t* mant;   // the table of make_pow10 (NULL: the big integers everywhere)
 };
 
-GAIN_HD void put_line(Sink& s, const LineFields& f) {
+// *pos and *margin (optional): where the intensity's text begins, and its rounding margin.
+GAIN_HD void put_line(Sink& s, const LineFields& f, long* pos = nullptr, float* margin = nullptr) {
     put_F(s, f.nu, 12, 6);
     s.put(' ');
     put_d(s, f.indexF + 1, 8);
@@ -383,17 +500,18 @@ GAIN_HD void put_line(Sink& s, const LineFields& f) {
     s.put(' ');
     put_d(s, f.gammaI + 1, 4);
     s.put(' ');
-    put_E(s, f.A, 16, 9);
+    put_E(s, f.A, 16, 9, f.mant);
     s.put(' ');
     if (f.with_intensity) {
-        put_E(s, f.intensity, 16, 9);
+        if (pos) *pos = s.n;
+        put_E(s, f.intensity, 16, 9, f.mant, margin);
         s.put(' ');
     }
     if (f.amps && f.namp > 0) {
         s.puts("[ ");
         for (int i = 0; i < f.namp; ++i) {
             s.put(' ');
-            put_E(s, f.amps[i], 16, 9);
+            put_E(s, f.amps[i], 16, 9, f.mant);
         }
         s.puts(" ] ");
     }

@@ -2,16 +2,23 @@
 // as Output::OutputLinestrength prints it (BaseClasses/Output.cpp:99-111), compacted into one
 // contiguous buffer in row-major (lower state, then upper state) order.
 //
-// Three launches over the rows x cols lines, 1024 lines per block (256 threads x 4 lines):
-//   k_text_len    S/A/I of each line (line_eval), its text length (0 when not written) and
+// Three launches over the rows x cols lines, 1024 lines per block:
+//   k_text_len    S and A of each line (line_eval), its text length (0 when not written) and
 //                 the block's byte total; the lengths come from the value ranges where those
 //                 fix them and from the conversion itself elsewhere (wide %f fields,
-//                 three-digit exponents), so they equal what the write pass writes;
+//                 three-digit exponents), so they equal what the write pass writes.  The
+//                 intensity's field is 16 characters wide whatever its value (it has no sign),
+//                 so its two exponentials are left to the write pass, which runs beside the
+//                 copy of the text to the host;
 //   k_text_offs   exclusive scan of the block totals, the total and the largest block;
 //   k_text_write  the block-local scan of the lengths; each thread formats its lines into
 //                 shared memory, placed at the block's output offset modulo 16, and the block
 //                 copies its text out in aligned 16-byte stores (whole L2 sectors, no partial
 //                 writes).  A block whose text does not fit shared memory writes directly.
+// 3.6 million lines with the intensity column, GB300, under ncu: the length pass 61 us (385 with
+// the intensity's exponentials, big-integer lengths and FP64 comparisons in it; FP64 pipe), the
+// text 650 us in eight launches, all but the first (49 us) beside the copy to the host; into
+// page-locked memory 1.14 ms in all (1.91 before), which the copy bounds.
 #include <atomic>
 
 #include "gain_internal.h"
@@ -21,7 +28,11 @@
 namespace gain {
 namespace {
 
-constexpr int kTextThreads = 256, kTextItems = 4, kTextSpan = kTextThreads * kTextItems;
+// One line per thread of the write pass: a block's conversions are a serial chain of some
+// thousand instructions per line, which four lines per thread make four times as long.
+constexpr int kTextSpan = 1024, kTextThreads = kTextSpan;
+// The length pass has little to do per line and no need of neighbouring lines.
+constexpr int kLenThreads = 256;
 constexpr int kStageMax = 200 * 1024;   // shared-memory staging of one block's text
 
 // Could the printed intensity (%16.9E: ten significant digits) of a line whose device value
@@ -62,17 +73,20 @@ __device__ __forceinline__ double intensity_of(const TextArgs& t, long idx, doub
     return lo < t.n_ovr && t.ovr_idx[lo] == idx ? t.ovr_val[lo] : v_dev;
 }
 
+__device__ __forceinline__ int line_row(const TextArgs& t, long idx) {
+    return (unsigned long)idx <= 0xffffffffu ? (int)((unsigned)idx / (unsigned)t.cols) : (int)(idx / t.cols);
+}
+
 // The fields of line idx; false when the line is not written.  a_out receives the printed
-// amplitudes (kMaxDegSlots at most); eI_out / e2_out (optional) the lower energy and the
-// exp(-beta nu) of the intensity.
-__device__ __forceinline__ bool line_fields(const TextArgs& t, long idx, double* a_out, fmt::LineFields& f,
-                                            double* eI_out = nullptr, double* e2_out = nullptr) {
-    const int r = (int)(idx / t.cols), c = (int)(idx - (long)r * t.cols);
+// amplitudes (kMaxDegSlots at most).  INTENSITY: the intensity too, with *e2 the exp(-beta nu)
+// it used and row_factor the row's factor (NULL: computed here).
+template <bool INTENSITY>
+__device__ __forceinline__ bool line_fields(const TextArgs& t, long idx, const double* row_factor, double* a_out,
+                                            fmt::LineFields& f, double* e2) {
+    const int r = line_row(t, idx), c = (int)(idx - (long)r * t.cols);
     const long off = (long)r * t.ld + c;
     const LineVals v = line_eval(t.amp, off, t.eI[r], t.eF[c], t.p);
     if (!v.keep) return false;
-    if (eI_out) *eI_out = t.eI[r];
-    if (e2_out) *e2_out = v.e2;
     int namp = 1;
     if (t.p.nslot == 0) {
         a_out[0] = t.amp[off];
@@ -82,7 +96,11 @@ __device__ __forceinline__ bool line_fields(const TextArgs& t, long idx, double*
     }
     f.nu = v.nu;
     f.A = v.A;
-    f.intensity = (t.p.with_intensity && t.n_ovr > 0) ? intensity_of(t, idx, v.I) : v.I;
+    f.intensity = 0.0;
+    if (INTENSITY) {
+        f.intensity = line_intensity(v, row_factor ? row_factor[r] : line_row_factor(t.eI[r], t.p), t.p, e2);
+        if (t.n_ovr > 0) f.intensity = intensity_of(t, idx, f.intensity);
+    }
     f.indexF = t.levF[c];
     f.jF = t.jF;
     f.gammaF = t.gammaF;
@@ -92,31 +110,51 @@ __device__ __forceinline__ bool line_fields(const TextArgs& t, long idx, double*
     f.with_intensity = t.p.with_intensity;
     f.amps = t.with_amps ? a_out : nullptr;
     f.namp = namp;
+    f.mant = (const uint64_t*)t.mant;
     return true;
 }
 
-__device__ __forceinline__ long line_text(const TextArgs& t, long idx, fmt::Sink& s) {
+// Line idx as text at s; text0: the text offset of s.p[0].
+__device__ __forceinline__ void line_write(const TextArgs& t, long idx, fmt::Sink& s, unsigned long long text0) {
     double a[kMaxDegSlots];
     fmt::LineFields f;
-    if (!line_fields(t, idx, a, f)) return 0;
-    const long n0 = s.n;
-    fmt::put_line(s, f);
-    return s.n - n0;
+    double e2 = 0.0;
+    if (!t.p.with_intensity) {
+        if (line_fields<false>(t, idx, nullptr, a, f, &e2)) fmt::put_line(s, f);
+        return;
+    }
+    if (!line_fields<true>(t, idx, t.row_factor, a, f, &e2)) return;
+    long pos = 0;
+    float margin = 0.0f;
+    fmt::put_line(s, f, &pos, &margin);
+    if (!t.hard) return;
+    // Most lines are far from a boundary, and the conversion's own margin says so: the allowance
+    // of intensity_hard in single precision (x below 10^10), with room for the rounding of both
+    // margins (2^-52 10^10 there).  The rest is decided there.
+    const float q = (float)e2 / (float)(1.0 - e2);
+    const float room = 1e10f * 0x1p-52f * (44.0f + 8.0f * q);
+    if (e2 < 0.999 && fabs(f.intensity) >= 1e-289 && fabs(f.intensity) <= 1e289 && room < 0.1f &&
+        margin > 1.01f * room + 1e-5f)
+        return;
+    if (intensity_hard(f.intensity, e2, t.pow10)) {
+        const unsigned int k = atomicAdd(t.nhard, 1u);
+        if ((int)k < t.hard_cap)
+            t.hard[k] = TextArgs::HardLine{(long long)idx, f.A, f.nu, t.eI[line_row(t, idx)],
+                                           text0 + (unsigned long long)pos, fmt::len_E(f.intensity, 16, 9)};
+    }
 }
 
 __device__ __forceinline__ long line_length(const TextArgs& t, long idx) {
     double a[kMaxDegSlots];
     fmt::LineFields f;
-    double eI = 0.0, e2 = 0.0;
-    if (!line_fields(t, idx, a, f, &eI, &e2)) return 0;
-    if (t.hard && t.p.with_intensity && intensity_hard(f.intensity, e2, t.pow10)) {
-        const unsigned int k = atomicAdd(t.nhard, 1u);
-        if ((int)k < t.hard_cap) t.hard[k] = TextArgs::HardLine{(long long)idx, f.A, f.nu, eI, f.intensity};
-    }
+    double e2 = 0.0;
+    if (t.signed_intensity ? !line_fields<true>(t, idx, nullptr, a, f, &e2)
+                           : !line_fields<false>(t, idx, nullptr, a, f, &e2))
+        return 0;
     return fmt::line_len(f);
 }
 
-// Block-wide exclusive scan of one value per thread (256 threads); returns the prefix and
+// Block-wide exclusive scan of one value per thread (kTextThreads threads); returns the prefix and
 // sets *total.
 __device__ __forceinline__ unsigned long long block_exclusive_scan(unsigned long long v, unsigned long long* total) {
     __shared__ unsigned long long warp_sum[kTextThreads / 32];
@@ -141,22 +179,40 @@ __device__ __forceinline__ unsigned long long block_exclusive_scan(unsigned long
     return before + x - v;
 }
 
-__global__ void __launch_bounds__(kTextThreads) k_text_len(TextArgs t) {
+__global__ void __launch_bounds__(kLenThreads) k_text_len(TextArgs t) {
+    __shared__ unsigned long long warp_sum[kLenThreads / 32];
+    __shared__ unsigned int warp_kept[kLenThreads / 32];
     const long total = (long)t.rows * t.cols;
-    const long base = (long)blockIdx.x * kTextSpan + (long)threadIdx.x * kTextItems;
-    unsigned long long sum = 0, kept = 0;
-    for (int i = 0; i < kTextItems; ++i) {
-        const long idx = base + i;
+    const long base = (long)blockIdx.x * kTextSpan + threadIdx.x;
+    unsigned long long sum = 0;
+    unsigned int kept = 0;
+    for (int i = 0; i < kTextSpan / kLenThreads; ++i) {
+        const long idx = base + i * kLenThreads;
         if (idx >= total) break;
         const long n = line_length(t, idx);
         t.lens[idx] = (uint32_t)n;
         sum += (unsigned long long)n;
         kept += n > 0;
     }
-    unsigned long long all, nk;
-    block_exclusive_scan(sum, &all);
-    block_exclusive_scan(kept, &nk);
+    if (t.row_factor) {
+        for (long r = (long)blockIdx.x * kLenThreads + threadIdx.x; r < t.rows; r += (long)gridDim.x * kLenThreads)
+            t.row_factor[r] = line_row_factor(t.eI[r], t.p);
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+        sum += __shfl_xor_sync(0xffffffffu, sum, o);
+        kept += __shfl_xor_sync(0xffffffffu, kept, o);
+    }
+    if ((threadIdx.x & 31) == 0) {
+        warp_sum[threadIdx.x >> 5] = sum;
+        warp_kept[threadIdx.x >> 5] = kept;
+    }
+    __syncthreads();
     if (threadIdx.x == 0) {
+        unsigned long long all = 0, nk = 0;
+        for (int w = 0; w < kLenThreads / 32; ++w) {
+            all += warp_sum[w];
+            nk += warp_kept[w];
+        }
         t.block_bytes[blockIdx.x] = all;
         if (nk) atomicAdd(t.nkeep, nk);
     }
@@ -165,14 +221,24 @@ __global__ void __launch_bounds__(kTextThreads) k_text_len(TextArgs t) {
 // Exclusive scan of nblocks block totals in place; block_bytes[nblocks] = the text size,
 // block_bytes[nblocks + 2] = the largest block total.
 __global__ void __launch_bounds__(kTextThreads) k_text_offs(unsigned long long* block_bytes, long nblocks) {
+    constexpr int kPer = 4;
     unsigned long long carry = 0, mx = 0;
-    for (long b0 = 0; b0 < nblocks; b0 += kTextThreads) {
-        const long b = b0 + threadIdx.x;
-        const unsigned long long v = b < nblocks ? block_bytes[b] : 0ull;
-        mx = v > mx ? v : mx;
+    for (long b0 = 0; b0 < nblocks; b0 += kTextThreads * kPer) {
+        const long b = b0 + (long)threadIdx.x * kPer;
+        unsigned long long v[kPer], sum = 0;
+#pragma unroll
+        for (int k = 0; k < kPer; ++k) {
+            v[k] = b + k < nblocks ? block_bytes[b + k] : 0ull;
+            mx = v[k] > mx ? v[k] : mx;
+            sum += v[k];
+        }
         unsigned long long all;
-        const unsigned long long pre = block_exclusive_scan(v, &all);
-        if (b < nblocks) block_bytes[b] = carry + pre;
+        unsigned long long pre = carry + block_exclusive_scan(sum, &all);
+#pragma unroll
+        for (int k = 0; k < kPer; ++k) {
+            if (b + k < nblocks) block_bytes[b + k] = pre;
+            pre += v[k];
+        }
         carry += all;
     }
     for (int o = 16; o > 0; o >>= 1) {
@@ -188,20 +254,14 @@ __global__ void __launch_bounds__(kTextThreads) k_text_write_staged(TextArgs t, 
     extern __shared__ __align__(16) char stage[];
     const long blk = block0 + blockIdx.x;
     const long total = (long)t.rows * t.cols;
-    const long base = blk * kTextSpan + (long)threadIdx.x * kTextItems;
-    unsigned long long mine = 0;
-    for (int i = 0; i < kTextItems; ++i)
-        if (base + i < total) mine += t.lens[base + i];
+    const long idx = blk * kTextSpan + threadIdx.x;
+    const unsigned long long mine = idx < total ? t.lens[idx] : 0u;
     unsigned long long all;
     const unsigned long long pre = block_exclusive_scan(mine, &all);
     const unsigned long long D = t.block_bytes[blk];
     const int pad = (int)(D & 15u);
     fmt::Sink s{stage + pad + pre, 0, (long)(all - pre)};
-    for (int i = 0; i < kTextItems; ++i) {
-        const long idx = base + i;
-        if (idx >= total) break;
-        if (t.lens[idx]) line_text(t, idx, s);
-    }
+    if (mine) line_write(t, idx, s, D + pre);
     __syncthreads();
     // stage[pad + j] -> text[D + j], j < all, both 16-byte aligned from j = head on
     const unsigned long long lim = t.text_size > D ? t.text_size - D : 0ull;
@@ -220,42 +280,60 @@ __global__ void __launch_bounds__(kTextThreads) k_text_write_staged(TextArgs t, 
 __global__ void __launch_bounds__(kTextThreads) k_text_write(TextArgs t, long block0) {
     const long blk = block0 + blockIdx.x;
     const long total = (long)t.rows * t.cols;
-    const long base = blk * kTextSpan + (long)threadIdx.x * kTextItems;
-    unsigned long long mine = 0;
-    for (int i = 0; i < kTextItems; ++i)
-        if (base + i < total) mine += t.lens[base + i];
+    const long idx = blk * kTextSpan + threadIdx.x;
+    const unsigned long long mine = idx < total ? t.lens[idx] : 0u;
     unsigned long long all;
     const unsigned long long pre = block_exclusive_scan(mine, &all);
     const unsigned long long off = t.block_bytes[blk] + pre;   // bounded by the text size
     fmt::Sink s{t.text + off, 0, (long)(t.text_size > off ? t.text_size - off : 0)};
-    for (int i = 0; i < kTextItems; ++i) {
-        const long idx = base + i;
-        if (idx >= total) break;
-        if (t.lens[idx]) line_text(t, idx, s);
-    }
+    if (mine) line_write(t, idx, s, off);
+}
+
+// One replaced field per 32 threads.
+__global__ void k_text_patch(char* text, unsigned long long text_size, const TextArgs::Patch* __restrict__ patches,
+                             int n) {
+    const int i = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5), j = threadIdx.x & 31;
+    if (i >= n) return;
+    const unsigned long long at = patches[i].pos + j;
+    if (j < patches[i].len && at < text_size) text[at] = patches[i].s[j];
 }
 
 // One conversion per value: out[i * stride ...] holds the text of vals[i], lens[i] its length.
 __global__ void k_format_values(long n, const double* __restrict__ vals, int conv, int width, int prec,
-                                char* __restrict__ out, int stride, int* __restrict__ lens) {
+                                const uint64_t* __restrict__ mant, char* __restrict__ out, int stride, int* __restrict__ lens) {
     const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     fmt::Sink c{nullptr, 0, 0};
-    if (conv == 'E') fmt::put_E(c, vals[i], width, prec); else fmt::put_F(c, vals[i], width, prec);
+    if (conv == 'E') fmt::put_E(c, vals[i], width, prec, mant); else fmt::put_F(c, vals[i], width, prec);
     lens[i] = (int)c.n;
     if (c.n > stride) return;
     fmt::Sink s{out + i * (long)stride, 0, stride};
-    if (conv == 'E') fmt::put_E(s, vals[i], width, prec); else fmt::put_F(s, vals[i], width, prec);
+    if (conv == 'E') fmt::put_E(s, vals[i], width, prec, mant); else fmt::put_F(s, vals[i], width, prec);
+}
+
+// The table of make_pow10, made once (thread-safe initialisation of a function-local static).
+const uint64_t* pow10_table() {
+    struct Table {
+        uint64_t mant[fmt::kPow10Count];
+        Table() { fmt::make_pow10(mant); }
+    };
+    static const Table t;
+    return t.mant;
 }
 
 }  // namespace
+
+const unsigned long long* text_pow10(int* count) {
+    *count = fmt::kPow10Count;
+    return (const unsigned long long*)pow10_table();
+}
 
 long text_blocks(long lines) { return (lines + kTextSpan - 1) / kTextSpan; }
 
 cudaError_t launch_text_len(const TextArgs& t, cudaStream_t st) {
     const long nb = text_blocks((long)t.rows * t.cols);
     if (nb <= 0) return cudaSuccess;
-    k_text_len<<<(unsigned)nb, kTextThreads, 0, st>>>(t);
+    k_text_len<<<(unsigned)nb, kLenThreads, 0, st>>>(t);
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     k_text_offs<<<1, kTextThreads, 0, st>>>(t.block_bytes, nb);
@@ -285,10 +363,19 @@ cudaError_t launch_text_write(const TextArgs& t, unsigned long long max_block_by
     return cudaGetLastError();
 }
 
-cudaError_t launch_format_values(long n, const double* vals, int conv, int width, int prec, char* out, int stride,
-                                 int* lens, cudaStream_t st) {
+cudaError_t launch_text_patch(char* text, unsigned long long text_size, const TextArgs::Patch* patches, int n,
+                              cudaStream_t st) {
     if (n <= 0) return cudaSuccess;
-    k_format_values<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(n, vals, conv, width, prec, out, stride, lens);
+    k_text_patch<<<(unsigned)((n + 7) / 8), 256, 0, st>>>(text, text_size, patches, n);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_format_values(long n, const double* vals, int conv, int width, int prec,
+                                 const unsigned long long* mant, char* out, int stride, int* lens,
+                                 cudaStream_t st) {
+    if (n <= 0) return cudaSuccess;
+    k_format_values<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(n, vals, conv, width, prec, (const uint64_t*)mant, out,
+                                                                 stride, lens);
     return cudaGetLastError();
 }
 
@@ -313,6 +400,7 @@ int gain_format_line_native(char* buf, size_t cap, double nu, int indexF, int jF
     f.with_intensity = with_intensity;
     f.amps = amps;
     f.namp = namp;
+    f.mant = gain::pow10_table();
     gain::fmt::Sink c{nullptr, 0, 0};
     gain::fmt::put_line(c, f);
     if ((size_t)c.n >= cap) return -(int)c.n;
@@ -337,16 +425,17 @@ long gain_line_length_native(double nu, int indexF, int jF, int gammaF, int inde
     f.with_intensity = with_intensity;
     f.amps = amps;
     f.namp = namp;
+    f.mant = nullptr;
     return gain::fmt::line_len(f);
 }
 
 int gain_format_value(char* buf, size_t cap, double x, int conv, int width, int prec) {
     if (!buf || cap == 0 || (conv != 'E' && conv != 'f') || prec < 0 || prec > (conv == 'E' ? 17 : 9)) return 0;
     gain::fmt::Sink c{nullptr, 0, 0};
-    if (conv == 'E') gain::fmt::put_E(c, x, width, prec); else gain::fmt::put_F(c, x, width, prec);
+    if (conv == 'E') gain::fmt::put_E(c, x, width, prec, gain::pow10_table()); else gain::fmt::put_F(c, x, width, prec);
     if ((size_t)c.n >= cap) return -(int)c.n;
     gain::fmt::Sink s{buf, 0, (long)cap - 1};
-    if (conv == 'E') gain::fmt::put_E(s, x, width, prec); else gain::fmt::put_F(s, x, width, prec);
+    if (conv == 'E') gain::fmt::put_E(s, x, width, prec, gain::pow10_table()); else gain::fmt::put_F(s, x, width, prec);
     buf[s.n] = 0;
     return (int)s.n;
 }
