@@ -19,7 +19,7 @@ LIBDIR = os.path.join(HERE, "lib")
 LIB = os.path.join(LIBDIR, "libgainls.so")
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 SOURCES = ["engine.cpp", "threej.cpp", "states.cpp", "fp64_kernels.cu", "split.cu", "residue.cu", "noalloc.cu", "adjoint.cu", "linetext.cu", "trove.cpp"]
-HEADERS = ["gain_internal.h", "split.h", "residue.h", "tcgen05.cuh", "linefmt.h", "linemath.cuh"]
+HEADERS = ["gain_internal.h", "split.h", "residue.h", "tcgen05.cuh", "follow.cuh", "linefmt.h", "linemath.cuh"]
 
 
 def nvcc() -> str:

@@ -8,6 +8,7 @@
 
 #include <cuda_bf16.h>
 
+#include "follow.cuh"
 #include "gain_internal.h"
 #include "tcgen05.cuh"
 
@@ -676,6 +677,7 @@ __device__ __forceinline__ void residue_rows(const SliceArgs& a0, const SliceGro
 // thread cost resident blocks and gained nothing (0.96 to 1.03 over 2 to 5 blocks).
 template <int NT>
 __global__ void __launch_bounds__(NT, 1024 / NT) k_residue_slice(const SliceArgs a) {
+    follow_wait();
     residue_rows<false, NT, NT == 256 ? 8 : 4>(a, SliceGroups{});
 }
 template <int NT>
@@ -747,6 +749,7 @@ __global__ void __launch_bounds__(kCrtThreads) k_crt(const CrtArgs a0, const Crt
     __shared__ unsigned long long red_m[kCrtThreads / 32];
     const int tid = threadIdx.x;
     int blk = (int)blockIdx.x;
+    follow_next();
     if (G) {
         int lo = 0, hi = gs.n - 1;
         while (lo < hi) {
@@ -1007,9 +1010,8 @@ cudaError_t launch_crt_grouped(const CrtGroups& g, cudaStream_t st) {
 // slicing: twice the rows in flight for the same threads).
 cudaError_t launch_residue_slice(const SliceArgs& a, cudaStream_t st) {
     if (a.nrows <= 0) return cudaSuccess;
-    if (a.kpad <= kShortRow) k_residue_slice<128><<<a.nrows, 128, 0, st>>>(a);
-    else k_residue_slice<256><<<a.nrows, 256, 0, st>>>(a);
-    return cudaGetLastError();
+    return a.kpad <= kShortRow ? launch_following(k_residue_slice<128>, (unsigned)a.nrows, 128, st, a)
+                               : launch_following(k_residue_slice<256>, (unsigned)a.nrows, 256, st, a);
 }
 
 cudaError_t launch_residue_slice_grouped(const SliceGroups& g, bool short_rows, cudaStream_t st) {

@@ -6,6 +6,7 @@
 
 #include <cuda_bf16.h>
 
+#include "follow.cuh"
 #include "gain_internal.h"
 #include "residue.h"
 #include "tcgen05.cuh"
@@ -1106,7 +1107,11 @@ __device__ __forceinline__ void refine_h(const RefineHArgs& a) {
     }
 }
 
-__global__ void k_refine_h(const RefineHArgs a) { refine_h(a); }
+__global__ void k_refine_h(const RefineHArgs a) {
+    follow_next();
+    follow_wait();
+    refine_h(a);
+}
 __global__ void k_refine_h_grouped(const RefineHArgs* __restrict__ a, int n) {
     refine_jobs(a, n, [](const RefineHArgs& x) { refine_h(x); });
 }
@@ -1151,7 +1156,10 @@ __device__ __forceinline__ void refine_amp(const RefineAmpArgs& a) {
     }
 }
 
-__global__ void k_refine_amp(const RefineAmpArgs a) { refine_amp(a); }
+__global__ void k_refine_amp(const RefineAmpArgs a) {
+    follow_wait();
+    refine_amp(a);
+}
 __global__ void k_refine_amp_grouped(const RefineAmpArgs* __restrict__ a, int n) {
     refine_jobs(a, n, [](const RefineAmpArgs& x) { refine_amp(x); });
 }
@@ -1363,8 +1371,7 @@ cudaError_t launch_band(const BandArgs& a, cudaStream_t st) {
 }
 
 cudaError_t launch_refine_h(const RefineHArgs& a, int max_blocks, cudaStream_t st) {
-    k_refine_h<<<max_blocks, 256, 0, st>>>(a);
-    return cudaGetLastError();
+    return launch_following(k_refine_h, (unsigned)max_blocks, 256, st, a);
 }
 
 cudaError_t launch_refine_h_grouped(const RefineHArgs* a, int n, int blocks, cudaStream_t st) {
@@ -1385,8 +1392,7 @@ cudaError_t launch_wait_selftest(unsigned long long limit_ns, int* err, cudaStre
 }
 
 cudaError_t launch_refine_amp(const RefineAmpArgs& a, int max_blocks, cudaStream_t st) {
-    k_refine_amp<<<max_blocks, 256, 0, st>>>(a);
-    return cudaGetLastError();
+    return launch_following(k_refine_amp, (unsigned)max_blocks, 256, st, a);
 }
 
 }  // namespace split
