@@ -358,6 +358,7 @@ struct gain_engine_s {
     unsigned int* counters() const { return (unsigned int*)words.p; }   // [0] nflags1 [1] nflags2
     unsigned long long* ull() const { return words.p + 2; }   // [0] uncertified [2] amp max [3] uncertified weak
     int* err() const { return (int*)(words.p + 6); }
+    unsigned long long* span(int gemm) const { return words.p + 8 + 2 * (gemm - 1); }   // ResGemmArgs::span
     // page-locked area the run's small uploads (level lists, tile lists) are read from by one
     // kernel; stage_busy: a launched kernel may still be reading it
     char* stage = nullptr;
@@ -385,7 +386,7 @@ namespace gain {
 namespace {
 
 constexpr int kMaxFlags = 1 << 22;
-constexpr int kRunWords = 8;
+constexpr int kRunWords = 12;
 
 gain_status check_engine(gain_engine e) {
     if (!e) return set_error(GAIN_ERR_INVALID_ARG, "engine is NULL");
@@ -1282,7 +1283,7 @@ ResiduePlan residue_plan(gain_engine e, const std::vector<std::vector<ColumnRang
 // set here).  d_tiles: P.tiles on the device.
 gain_status residue_gemm(gain_engine e, const CUtensorMap& tmA, const CUtensorMap& tmB, const ResiduePlan& P,
                          const split::ResTile* d_tiles, const cudaEvent_t* waits, int B, int Bpad, bool pair,
-                         split::CrtArgs crt, int* err, cudaEvent_t ev_done) {
+                         split::CrtArgs crt, int* err, unsigned long long* span) {
     cudaStream_t st = e->st;
     const int panel = residue_panel(pair ? 2 * split::BM : split::BM);
     split::ResGemmArgs g;
@@ -1292,6 +1293,7 @@ gain_status residue_gemm(gain_engine e, const CUtensorMap& tmA, const CUtensorMa
     g.ldr = crt.ldr;
     g.plane = (long)P.rows0 * crt.ldr;
     g.err = err;
+    g.span = span;
     for (int m0 = 0; m0 < Bpad; m0 += panel) {
         const bool last = m0 + panel >= Bpad;
         g.m_base = m0;
@@ -1304,7 +1306,6 @@ gain_status residue_gemm(gain_engine e, const CUtensorMap& tmA, const CUtensorMa
             GAIN_CUDA(split::launch_residue_gemm(tmA, tmB, g, e->num_sms, st, pair));
             ++e->launches;
         }
-        if (last && ev_done) GAIN_CUDA(cudaEventRecord(ev_done, st));
         crt.res = e->res.p;
         crt.plane = g.plane;
         crt.row0 = m0;
@@ -1657,7 +1658,7 @@ gain_status run_split(gain_engine e, const gain_pair_job* j, int dI, int dF, con
         g1.cols_valid = L.fpad;
         g1.err = e->err();
         g1.fuse = fuse1;
-        if (piece == 0) GAIN_CUDA(cudaEventRecord(e->ev[2], st));
+        if (!res && piece == 0) GAIN_CUDA(cudaEventRecord(e->ev[2], st));
         if (res) {
             split::CrtArgs c1;
             memset(&c1, 0, sizeof c1);
@@ -1688,7 +1689,7 @@ gain_status run_split(gain_engine e, const gain_pair_job* j, int dI, int dF, con
             }
             res_flops += rp1.flops;
             GAIN_TRY(residue_gemm(e, tmV, L.tmBandPair, rp1, e->rtiles1.p, nullptr, B, Bpad, pair, c1,
-                                  e->err(), piece == npieces - 1 ? e->ev[3] : nullptr));
+                                  e->err(), e->span(1)));
         } else {
             if (!t1.empty()) {
                 GAIN_CUDA(split::launch_gemm(tmV, pair ? L.tmBandPair : L.tmBand, g1, e->num_sms, st, pair));
@@ -1811,7 +1812,7 @@ gain_status run_split(gain_engine e, const gain_pair_job* j, int dI, int dF, con
     g2.err = e->err();
     g2.bnd = e->ampbnd.p;
     g2.ldb = Nupad;
-    GAIN_CUDA(cudaEventRecord(e->ev[4], st));
+    if (!res) GAIN_CUDA(cudaEventRecord(e->ev[4], st));
     if (res) {
         split::CrtArgs c2;
         memset(&c2, 0, sizeof c2);
@@ -1836,7 +1837,7 @@ gain_status run_split(gain_engine e, const gain_pair_job* j, int dI, int dF, con
         split::crt_constants(&c2);
         const cudaEvent_t waits[2] = {nullptr, e->ev[7]};
         res_flops += rp2.flops;
-        GAIN_TRY(residue_gemm(e, tmH, tmU, rp2, e->rtiles2.p, waits, B, Bpad, pair, c2, e->err(), e->ev[5]));
+        GAIN_TRY(residue_gemm(e, tmH, tmU, rp2, e->rtiles2.p, waits, B, Bpad, pair, c2, e->err(), e->span(2)));
     } else if (Nu2 > 0) {
         // tiles are upper-block-major: those of the first half (n0 < Nu2) come first
         int n1 = 0;
@@ -1880,7 +1881,7 @@ gain_status run_split(gain_engine e, const gain_pair_job* j, int dI, int dF, con
     GAIN_CUDA(cudaEventRecord(e->ev[1], st));
 
     unsigned int cnt[4];
-    unsigned long long unc[4];
+    unsigned long long unc[4], spans[4];
     int errw = 0;
     {   // the run's counters through one page-locked area
         if (!e->readback) GAIN_CUDA(cudaMallocHost(&e->readback, 128));
@@ -1891,6 +1892,7 @@ gain_status run_split(gain_engine e, const gain_pair_job* j, int dI, int dF, con
         memcpy(cnt, rb, sizeof cnt);
         memcpy(unc, rb + 16, sizeof unc);
         memcpy(&errw, rb + 48, sizeof errw);
+        memcpy(spans, rb + 64, sizeof spans);
     }
     e->amp_rows = B;
     e->amp_cols = Nu;
@@ -1904,8 +1906,13 @@ gain_status run_split(gain_engine e, const gain_pair_job* j, int dI, int dF, con
         memset(stats, 0, sizeof *stats);
         float ms = 0.f, g1ms = 0.f, g2ms = 0.f;
         cudaEventElapsedTime(&ms, e->ev[0], e->ev[1]);
-        cudaEventElapsedTime(&g1ms, e->ev[2], e->ev[3]);
-        cudaEventElapsedTime(&g2ms, e->ev[4], e->ev[5]);
+        if (res) {
+            g1ms = (float)((double)(spans[1] - ~spans[0]) * 1e-6);
+            g2ms = (float)((double)(spans[3] - ~spans[2]) * 1e-6);
+        } else {
+            cudaEventElapsedTime(&g1ms, e->ev[2], e->ev[3]);
+            cudaEventElapsedTime(&g2ms, e->ev[4], e->ev[5]);
+        }
         stats->device_ms = ms;
         stats->gemm1_ms = g1ms;
         stats->gemm2_ms = g2ms;

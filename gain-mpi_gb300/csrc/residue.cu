@@ -202,6 +202,9 @@ k_residue_gemm(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     else __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tmem_holder;
+    follow_next();
+    follow_wait();
+    if (a.span && threadIdx.x == 0) atomicMax(&a.span[0], ~globaltimer());
 
     // The unit's items (unit, unit + nunits, ...) alternate between two streams, one per
     // accumulator; every role walks both in the same order.
@@ -475,6 +478,7 @@ k_residue_gemm(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     // and write its TMEM) have drained
     if (PAIR) cluster_sync_all();
     else __syncthreads();
+    if (a.span && threadIdx.x == 0) atomicMax(&a.span[1], globaltimer());
     if (warp == 1) {
         tc_fence_after();
         if (PAIR) tmem_dealloc_pair(tmem, 2 * ACC_COLS);
@@ -750,6 +754,7 @@ __global__ void __launch_bounds__(kCrtThreads) k_crt(const CrtArgs a0, const Crt
     const int tid = threadIdx.x;
     int blk = (int)blockIdx.x;
     follow_next();
+    follow_wait();
     if (G) {
         int lo = 0, hi = gs.n - 1;
         while (lo < hi) {
@@ -956,13 +961,15 @@ cudaError_t launch_residue_gemm(const CUtensorMap& tmA, const CUtensorMap& tmB, 
     cfg.blockDim = dim3(NTHREADS);
     cfg.dynamicSmemBytes = kSmemBytes;
     cfg.stream = st;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = 2;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = 2;
+    attr[1].val.clusterDim.y = 1;
+    attr[1].val.clusterDim.z = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = pair ? 1 : 0;
+    cfg.numAttrs = pair ? 2 : 1;
     return pair ? cudaLaunchKernelEx(&cfg, k_residue_gemm<true, false>, tmA, tmB, a)
                 : cudaLaunchKernelEx(&cfg, k_residue_gemm<false, false>, tmA, tmB, a);
 }
@@ -994,9 +1001,8 @@ cudaError_t launch_crt(const CrtArgs& a0, cudaStream_t st) {
     crt_set_rows(&a, 1);
     const int nb = crt_blocks(a);
     if (nb <= 0) return cudaSuccess;
-    if (a.nmod == 13) k_crt<false, 13><<<nb, kCrtThreads, 0, st>>>(a, CrtGroups{});
-    else k_crt<false, 0><<<nb, kCrtThreads, 0, st>>>(a, CrtGroups{});
-    return cudaGetLastError();
+    return a.nmod == 13 ? launch_following(k_crt<false, 13>, (unsigned)nb, kCrtThreads, st, a, CrtGroups{})
+                        : launch_following(k_crt<false, 0>, (unsigned)nb, kCrtThreads, st, a, CrtGroups{});
 }
 
 cudaError_t launch_crt_grouped(const CrtGroups& g, cudaStream_t st) {

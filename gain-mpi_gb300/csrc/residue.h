@@ -53,6 +53,10 @@ struct ResGemmArgs {
     uint16_t* res;         // residues in [0, m_i): res[i * plane + row * ldr + col]
     long plane, ldr;
     int* err;              // device error word (0 ok, else timeout code)
+    // optional: the launch's span on the global timer (ns), as maxima over the CTAs from zero:
+    // span[0] the complement of the first start, span[1] the last end.  (An event between two
+    // kernels costs a short run about 2 us, and the next kernel cannot be launched behind it.)
+    unsigned long long* span;
 };
 
 struct alignas(128) ResGroup {
