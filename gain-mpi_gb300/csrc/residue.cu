@@ -212,6 +212,8 @@ k_residue_gemm(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         ResTile tl;
         int it;    // the item (>= nitems: none left)
         int kb;    // its next k-block
+        int w;     // the accumulator
+        uint32_t chunks;   // the stream's chunks so far
     };
     auto load_item = [&](Stream& x) {   // the first filled slot from x.it on
         for (; x.it < nitems; x.it += 2 * nunits) {
@@ -231,22 +233,29 @@ k_residue_gemm(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     auto load_work = [&](Stream& x) {
         for (load_item(x); x.it < nitems && x.tl.nkb <= 0; load_item(x)) x.it += 2 * nunits;
     };
-    Stream str[2];
-    str[0].it = unit;
-    str[1].it = unit + nunits;
+    // x runs next, y after it: the roles swap the two instead of indexing or unrolling over them,
+    // so that their code exists once (a short launch fetches it cold)
+    Stream x, y;
+    x.it = unit;
+    x.w = 0;
+    y.it = unit + nunits;
+    y.w = 1;
+    x.chunks = y.chunks = 0;
+    auto swap_streams = [&]() {
+        const Stream t = x;
+        x = y;
+        y = t;
+    };
 
     if (warp == 0) {
         // ---------------- TMA producer
         if (lane == 0) {
             uint32_t stage = 0, phase = 0, issued_mask = 0, last_par = 0;
             bool ok = true;
-            load_work(str[0]);
-            load_work(str[1]);
-            while (ok && (str[0].it < nitems || str[1].it < nitems)) {
-#pragma unroll
-                for (int w = 0; w < 2; ++w) {
-                    Stream& x = str[w];
-                    if (x.it >= nitems || !ok) continue;
+            load_work(x);
+            load_work(y);
+            for (; ok && (x.it < nitems || y.it < nitems); swap_streams()) {
+                if (x.it < nitems) {
                     const ResTile& tl = x.tl;
                     const CUtensorMap* mapA = GROUPED ? &a.groups[tl.group].tmA : &tmA;
                     const CUtensorMap* mapB = GROUPED ? &a.groups[tl.group].tmB : &tmB;
@@ -307,23 +316,20 @@ k_residue_gemm(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     } else if (warp == 1) {
         // ---------------- MMA issuer (one thread; of the first CTA of a pair)
         if (lane == 0 && rank == 0) {
-            uint32_t stage = 0, phase = 0, acc_cnt[2] = {0, 0};
+            uint32_t stage = 0, phase = 0;
             bool ok = true, any = false;
-            load_work(str[0]);
-            load_work(str[1]);
-            while (ok && (str[0].it < nitems || str[1].it < nitems)) {
-#pragma unroll
-                for (int w = 0; w < 2; ++w) {
-                    Stream& x = str[w];
-                    if (x.it >= nitems || !ok) continue;
+            load_work(x);
+            load_work(y);
+            for (; ok && (x.it < nitems || y.it < nitems); swap_streams()) {
+                if (x.it < nitems) {
                     // the accumulator's last chunk has been reduced (or its residues stored)
-                    if (!mbar_wait(smem_u32(&accempty[w]), (acc_cnt[w] & 1) ^ 1, abort_flag, a.err, 2)) {
+                    if (!mbar_wait(smem_u32(&accempty[x.w]), (x.chunks & 1) ^ 1, abort_flag, a.err, 2)) {
                         ok = false;
                         break;
                     }
                     tc_fence_after();
                     const uint32_t idesc = idesc_of(PAIR, x.tl.ncols);
-                    const uint32_t d = tmem + w * ACC_COLS;
+                    const uint32_t d = tmem + x.w * ACC_COLS;
                     const int end = x.kb + kChunkBlocks < x.tl.nkb ? x.kb + kChunkBlocks : x.tl.nkb;
                     for (int kb = x.kb; kb < end; kb += KS) {
                         const int nk = end - kb < KS ? end - kb : KS;
@@ -353,9 +359,9 @@ k_residue_gemm(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                         if (++stage == NST) { stage = 0; phase ^= 1; }
                     }
                     if (!ok) break;
-                    if (PAIR) mma_commit_pair(smem_u32(&accfull[w]), (uint16_t)3);
-                    else mma_commit(smem_u32(&accfull[w]));
-                    ++acc_cnt[w];
+                    if (PAIR) mma_commit_pair(smem_u32(&accfull[x.w]), (uint16_t)3);
+                    else mma_commit(smem_u32(&accfull[x.w]));
+                    ++x.chunks;
                     x.kb = end;
                     if (end >= x.tl.nkb) {
                         x.it += 2 * nunits;
@@ -422,23 +428,19 @@ k_residue_gemm(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                 x.it += 2 * nunits;
             }
         };
-        uint32_t acc_cnt[2] = {0, 0};
         bool ok = true;
-        load_chunks(str[0]);
-        load_chunks(str[1]);
-        while (ok && (str[0].it < nitems || str[1].it < nitems)) {
-#pragma unroll
-            for (int w = 0; w < 2; ++w) {
-                Stream& x = str[w];
-                if (x.it >= nitems || !ok) continue;
+        load_chunks(x);
+        load_chunks(y);
+        for (; ok && (x.it < nitems || y.it < nitems); swap_streams()) {
+            if (x.it < nitems) {
                 const float m = c_tab.m[x.tl.mod], inv = c_tab.inv[x.tl.mod];
                 const int npc = x.tl.ncols / 64;   // 32-column pieces of this warp (2 or 4)
-                if (!mbar_wait(smem_u32(&accfull[w]), acc_cnt[w] & 1, abort_flag, a.err, 5)) {
+                if (!mbar_wait(smem_u32(&accfull[x.w]), x.chunks & 1, abort_flag, a.err, 5)) {
                     ok = false;
                     break;
                 }
                 tc_fence_after();
-                const uint32_t t0 = tmem + lane_off + w * ACC_COLS + (uint32_t)(half * (x.tl.ncols / 2));
+                const uint32_t t0 = tmem + lane_off + x.w * ACC_COLS + (uint32_t)(half * (x.tl.ncols / 2));
                 x.kb += kChunkBlocks;
                 const bool last = x.kb >= x.tl.nkb;
                 uint32_t o[64];   // (last chunk) packed residues: stored after the accumulator is released
@@ -463,9 +465,9 @@ k_residue_gemm(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                 // The warp's accesses to the accumulator are complete.  (The arrival is relaxed: the
                 // fences order the TMEM accesses, and nothing else is handed over.  A release at
                 // cluster scope waited for this warp's global stores: 1800 clocks a chunk.)
-                if (lane == 0) mbar_arrive_relaxed(PAIR ? cluster_map(smem_u32(&accempty[w]), 0) : smem_u32(&accempty[w]));
+                if (lane == 0) mbar_arrive_relaxed(PAIR ? cluster_map(smem_u32(&accempty[x.w]), 0) : smem_u32(&accempty[x.w]));
                 if (last) store(x.tl, o);
-                ++acc_cnt[w];
+                ++x.chunks;
                 if (last) {
                     x.it += 2 * nunits;
                     load_chunks(x);
