@@ -443,23 +443,34 @@ k_residue_gemm(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                 const uint32_t t0 = tmem + lane_off + x.w * ACC_COLS + (uint32_t)(half * (x.tl.ncols / 2));
                 x.kb += kChunkBlocks;
                 const bool last = x.kb >= x.tl.nkb;
+                auto reduce = [&](int p, uint32_t (&v)[32]) {   // 32 columns at a time
+                    tmem_ld32(t0 + p * 32, v);
+                    tmem_wait_ld();
+#pragma unroll
+                    for (int j = 0; j < 32; j += 2)
+                        unpack2(mod_balanced2(pack2(__uint_as_float(v[j]), __uint_as_float(v[j + 1])), pack2(inv, inv),
+                                              pack2(-m, -m)),
+                                v[j], v[j + 1]);
+                };
                 uint32_t o[64];   // (last chunk) packed residues: stored after the accumulator is released
+                if (last) {
 #pragma unroll
-                for (int p = 0; p < 4; ++p) {   // 32 columns at a time
-                    if (p < npc) {
-                        uint32_t v[32];
-                        tmem_ld32(t0 + p * 32, v);
-                        tmem_wait_ld();
-#pragma unroll
-                        for (int j = 0; j < 32; j += 2)
-                            unpack2(mod_balanced2(pack2(__uint_as_float(v[j]), __uint_as_float(v[j + 1])),
-                                                  pack2(inv, inv), pack2(-m, -m)),
-                                    v[j], v[j + 1]);
-                        if (last) pack(v, m, o + 16 * p);
-                        else tmem_st32(t0 + p * 32, v);
+                    for (int p = 0; p < 4; ++p) {
+                        if (p < npc) {
+                            uint32_t v[32];
+                            reduce(p, v);
+                            pack(v, m, o + 16 * p);
+                        }
                     }
+                } else {
+#pragma unroll 1
+                    for (int p = 0; p < npc; ++p) {
+                        uint32_t v[32];
+                        reduce(p, v);
+                        tmem_st32(t0 + p * 32, v);
+                    }
+                    tmem_wait_st();
                 }
-                if (!last) tmem_wait_st();
                 tc_fence_before();
                 __syncwarp();
                 // The warp's accesses to the accumulator are complete.  (The arrival is relaxed: the

@@ -162,3 +162,25 @@ def test_plan_refines_flagged_entries_of_every_job(built_lib, monkeypatch):
         tol = (4 * np.sqrt(N) * 2.0 ** -48) * np.sqrt(N) * mrow + np.sqrt(N) * (3 * N + 64) * 2.0 ** -52 * mrow
         assert np.max(np.abs(plan.amp(q) - ref)) <= tol
     plan.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("rows,cols", [(1, 1), (100, 130), (129, 257), (300, 500), (520, 700), (700, 770)])
+def test_items_shared_by_both_accumulators(built_lib, rows, cols, monkeypatch):
+    """Inner lengths of two to four chunks and one to five items a unit: a unit's odd item is
+    accumulated by both of its accumulators.  The residues are the same integers however they are
+    summed, so every amplitude equals the whole block's bits."""
+    import gainls
+    import synth
+    p = synth.make_problem(310, [5, 6], "c4", blocks=[(5, 0), (6, 1)])
+    eng = gainls.Engine(JMAX, p.nsym, 1)
+    gainls.upload_problem(eng, p)
+    nI, nF = p.blocks[(0, 0)].vecs.shape[0], p.blocks[(1, 1)].vecs.shape[0]
+    assert nI >= 700 and nF >= 2 * 384 + 1
+    eng.run_pair(0, 0, 1, 1, np.arange(nI, dtype=np.int32), np.arange(nF, dtype=np.int32), gainls.PATH_SPLIT)
+    whole = eng.fetch_amp().copy()
+    lo, up = np.arange(rows, dtype=np.int32), np.arange(cols, dtype=np.int32)
+    for pair in ("1", "0"):
+        monkeypatch.setenv("GAINLS_GEMM_PAIR", pair)
+        eng.run_pair(0, 0, 1, 1, lo, up, gainls.PATH_SPLIT)
+        assert np.array_equal(eng.fetch_amp(), whole[:rows, :cols])
