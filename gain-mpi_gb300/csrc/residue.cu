@@ -551,11 +551,15 @@ __device__ __forceinline__ void residue_rows(const SliceArgs& a0, const SliceGro
                     top(v[u].y);
                 }
             }
-#pragma unroll 4
-            for (; c < n2; c += NT) {
-                const ulonglong2 v = __ldg(s2 + c);
-                top(v.x);
-                top(v.y);
+            {   // the rest (a short row: all of it), loads first as well
+                ulonglong2 v[8];
+#pragma unroll
+                for (int u = 0; u < 8; ++u) v[u] = c + u * NT < n2 ? __ldg(s2 + c + u * NT) : make_ulonglong2(0ull, 0ull);
+#pragma unroll
+                for (int u = 0; u < 8; ++u) {
+                    top(v[u].x);
+                    top(v[u].y);
+                }
             }
             if ((a.ncols & 1) && tid == 0) top(src[a.ncols - 1]);
         } else {
@@ -692,14 +696,14 @@ __device__ __forceinline__ void residue_rows(const SliceArgs& a0, const SliceGro
 // 1.04.  Neither the stores (one plane stored instead of 13: 0.95), the residues' arithmetic (none:
 // 0.91) nor the search for the maximum (none: 0.88) bounds it alone; more loads in flight per
 // thread cost resident blocks and gained nothing (0.96 to 1.03 over 2 to 5 blocks).
-template <int NT>
+template <int NT, int COLS>
 __global__ void __launch_bounds__(NT, 1024 / NT) k_residue_slice(const SliceArgs a) {
     follow_wait();
-    residue_rows<false, NT, NT == 256 ? 8 : 4>(a, SliceGroups{});
+    residue_rows<false, NT, COLS>(a, SliceGroups{});
 }
-template <int NT>
+template <int NT, int COLS>
 __global__ void __launch_bounds__(NT, 1024 / NT) k_residue_slice_grouped(const SliceGroups gs) {
-    residue_rows<true, NT, NT == 256 ? 8 : 4>(SliceArgs{}, gs);
+    residue_rows<true, NT, COLS>(SliceArgs{}, gs);
 }
 
 // ------------------------------------------------------------------- reconstruction
@@ -1025,18 +1029,26 @@ cudaError_t launch_crt_grouped(const CrtGroups& g, cudaStream_t st) {
     return cudaGetLastError();
 }
 
-// Rows of at most 4096 destination columns take 128 threads, longer ones 256 (as the digit
-// slicing: twice the rows in flight for the same threads).
+// Rows of at most 4096 destination columns take 128 threads of four columns, longer ones 256 of eight
+// (as the digit slicing: twice the rows in flight for the same threads).  Where such rows are too
+// few to fill the chip with 128 threads each, a row is a chain of passes on a few warps of a
+// nearly idle SM: 256 or 512 threads then share it.
+constexpr long kFullThreads = 152 * 1024 * 3 / 4;
 cudaError_t launch_residue_slice(const SliceArgs& a, cudaStream_t st) {
     if (a.nrows <= 0) return cudaSuccess;
-    return a.kpad <= kShortRow ? launch_following(k_residue_slice<128>, (unsigned)a.nrows, 128, st, a)
-                               : launch_following(k_residue_slice<256>, (unsigned)a.nrows, 256, st, a);
+    const unsigned rows = (unsigned)a.nrows;
+    if (a.kpad > kShortRow) return launch_following(k_residue_slice<256, 8>, rows, 256, st, a);
+    int nt = 128;
+    while (nt < 512 && (long)rows * nt < kFullThreads && 4 * nt < a.kpad) nt *= 2;
+    return nt == 128   ? launch_following(k_residue_slice<128, 4>, rows, 128, st, a)
+           : nt == 256 ? launch_following(k_residue_slice<256, 4>, rows, 256, st, a)
+                       : launch_following(k_residue_slice<512, 4>, rows, 512, st, a);
 }
 
 cudaError_t launch_residue_slice_grouped(const SliceGroups& g, bool short_rows, cudaStream_t st) {
     if (g.rows <= 0 || g.n <= 0) return cudaSuccess;
-    if (short_rows) k_residue_slice_grouped<128><<<g.rows, 128, 0, st>>>(g);
-    else k_residue_slice_grouped<256><<<g.rows, 256, 0, st>>>(g);
+    if (short_rows) k_residue_slice_grouped<128, 4><<<g.rows, 128, 0, st>>>(g);
+    else k_residue_slice_grouped<256, 8><<<g.rows, 256, 0, st>>>(g);
     return cudaGetLastError();
 }
 
