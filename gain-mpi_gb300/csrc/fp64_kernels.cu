@@ -444,19 +444,33 @@ k_lines(int rows, int cols, const double* __restrict__ amp, long ld,
         double* __restrict__ S, double* __restrict__ A, double* __restrict__ I,
         unsigned char* __restrict__ keep, unsigned long long* nkeep) {
     __shared__ unsigned int warp_kept[8];
+    __shared__ double row_factor[256];
     const long total = (long)rows * cols;
     unsigned int kept = 0;
-    for (long idx = (long)blockIdx.x * blockDim.x + threadIdx.x; idx < total; idx += (long)gridDim.x * blockDim.x) {
-        const int r = (int)(idx / cols), c = (int)(idx - (long)r * cols);
-        const LineVals v = line_eval(amp, (long)r * ld + c, eI[r], eF[c], p);
-        kept += v.keep;
-        if (S) S[idx] = v.ls;
-        if (A) A[idx] = v.A;
-        if (I) {
-            double e2;
-            I[idx] = p.with_intensity ? line_intensity(v, line_row_factor(eI[r], p), p, &e2) : 0.0;
+    for (long base = (long)blockIdx.x * 256; base < total; base += (long)gridDim.x * 256) {
+        const int r0 = (int)(base / cols);
+        const unsigned int at = (unsigned int)(base - (long)r0 * cols) + threadIdx.x;   // column, from row r0's first
+        const int k = (int)(at / (unsigned int)cols), r = r0 + k, c = (int)(at - (unsigned int)k * cols);
+        const long idx = base + threadIdx.x;
+        LineVals v;
+        if (idx < total) v = line_eval(amp, (long)r * ld + c, eI[r], eF[c], p);
+        if (I && p.with_intensity) {   // the rows' exponentials once per block and row
+            const unsigned int last = (at - threadIdx.x + 255u) / (unsigned int)cols;   // rows in these 256 lines, less one
+            if (threadIdx.x <= last && r0 + (int)threadIdx.x < rows)
+                row_factor[threadIdx.x] = line_row_factor(eI[r0 + threadIdx.x], p);
+            __syncthreads();
         }
-        if (keep) keep[idx] = (unsigned char)v.keep;
+        if (idx < total) {
+            kept += v.keep;
+            if (S) S[idx] = v.ls;
+            if (A) A[idx] = v.A;
+            if (I) {
+                double e2;
+                I[idx] = p.with_intensity ? line_intensity(v, row_factor[k], p, &e2) : 0.0;
+            }
+            if (keep) keep[idx] = (unsigned char)v.keep;
+        }
+        if (I && p.with_intensity) __syncthreads();
     }
     for (int o = 16; o > 0; o >>= 1) kept += __shfl_xor_sync(0xffffffffu, kept, o);
     if ((threadIdx.x & 31) == 0) warp_kept[threadIdx.x >> 5] = kept;
