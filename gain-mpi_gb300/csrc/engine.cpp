@@ -139,21 +139,28 @@ struct Inflation {
     std::vector<std::unique_ptr<GammaMaps>> maps;
 };
 
+// Parts of an asynchronous vector upload at most.  A run works on each part's upper states while
+// the next one arrives, so what follows the copy is the work of the last part.
+constexpr int kUploadParts = 4;
+
 struct Eig {
     int nlevels = 0, nsize = 0;
     DevArray<double> d;
     // recorded on the copy stream after an asynchronous upload; every consumer's stream waits
     // on it before reading d (NULL until the first asynchronous upload)
     cudaEvent_t ready = nullptr;
-    // the copy runs in two parts: rows [0, head_rows) are in place when ready_head fires
-    cudaEvent_t ready_head = nullptr;
-    int head_rows = 0;
+    // the copy runs in parts: rows [0, part_rows[k]) are in place when part[k] fires, k < nparts,
+    // and all of them when `ready` does
+    cudaEvent_t part[kUploadParts - 1] = {};
+    int part_rows[kUploadParts - 1] = {};
+    int nparts = 0;
     Eig() = default;
     Eig(const Eig&) = delete;
     Eig& operator=(const Eig&) = delete;
     ~Eig() {
         if (ready) cudaEventDestroy(ready);
-        if (ready_head) cudaEventDestroy(ready_head);
+        for (cudaEvent_t v : part)
+            if (v) cudaEventDestroy(v);
     }
 };
 
@@ -271,6 +278,7 @@ struct gain_engine_s {
     bool lines_pending = false;     // gain_pair_lines_async copies still in flight
     long long* lines_nout = nullptr;   // their caller's n_lines
     cudaEvent_t ev[10] = {};
+    cudaEvent_t ev_upper[gain::kUploadParts] = {};   // each part of the upper rows sliced
     // orders an asynchronous upload after the engine work that reads eigenvectors: recorded
     // at the end of every run (runs, plans, adjoints and line recomputations return only when
     // their work is done), so an upload need not wait for line kernels queued after a run
@@ -1438,22 +1446,32 @@ gain_status run_split(gain_engine e, const gain_pair_job* j, int dI, int dF, con
     auto band_digits = [&]() -> gain_status { return layout_band_digits(e, L, p1x, st); };
     GAIN_TRY(band_digits());
 
-    // While the upper vectors are still arriving in two parts, the upper side runs in two
-    // halves: the first half's digits and amplitude GEMM start when the first part lands.
-    int Nu2 = 0;
+    // While the upper vectors are still arriving in parts, the upper side runs part by part: each
+    // one's digits and amplitude GEMM start when its rows have landed.  uparts[k]: the part's first
+    // upper state and the event it waits for; a part takes the leading states whose rows arrive
+    // with it, in whole tiles.
+    struct UpperPart { int first; cudaEvent_t wait; };
+    std::vector<UpperPart> uparts;
     bool arriving = false;
-    if (EF.ready && EF.ready_head && EF.head_rows > 0 && Nu >= 2 * split::BN) {
+    if (EF.ready && EF.nparts > 0 && Nu >= 2 * split::BN) {
         const cudaError_t q = cudaEventQuery(EF.ready);
         if (q == cudaErrorNotReady) (void)cudaGetLastError();   // not an error: the copy is in flight
         const char* halves = getenv("GAINLS_UPPER_HALVES");     // "force": also after the copy landed
         arriving = q == cudaErrorNotReady || (halves && std::string(halves) == "force");
     }
-    if (arriving) {
-        const int cand = (Nupad / split::BN + 1) / 2 * split::BN;   // the upper blocks halved, rounded up
-        bool in_head = true;
-        for (int u = 0; u < cand && in_head; ++u) in_head = j->upper_levels[u] < EF.head_rows;
-        if (in_head) Nu2 = cand;
+    int first = 0;
+    for (int k = 0; arriving && k < EF.nparts; ++k) {
+        if (!res && k != EF.nparts / 2) continue;   // digit products: two halves
+        int u = first;
+        while (u < Nu && j->upper_levels[u] < EF.part_rows[k]) ++u;
+        u = u / (2 * split::BN) * (2 * split::BN);
+        if (u <= first) continue;
+        uparts.push_back({first, EF.part[k]});
+        first = u;
     }
+    if (first < Nu) uparts.push_back({first, EF.ready});
+    const int nup = (int)uparts.size();
+    auto upper_end = [&](int k) { return k + 1 < nup ? uparts[k + 1].first : Nu; };
     GAIN_TRY(e->words.alloc(kRunWords));
     GAIN_TRY(e->rowerr.alloc(Bpad));
     ResiduePlan rp1, rp2;
@@ -1472,8 +1490,7 @@ gain_status run_split(gain_engine e, const gain_pair_job* j, int dI, int dF, con
         }
         const int nkb2 = K2 / split::BK;
         std::vector<std::vector<ColumnRange>> parts;
-        if (Nu2 > 0) parts = {{{0, Nu2, 0, nkb2}}, {{Nu2, Nupad, 0, nkb2}}};
-        else parts = {{{0, Nupad, 0, nkb2}}};
+        for (int k = 0; k < nup; ++k) parts.push_back({{uparts[k].first, k + 1 < nup ? upper_end(k) : Nupad, 0, nkb2}});
         rp2 = residue_plan(e, parts, Bpad, pair, p2.slices);
         GAIN_TRY(up.add(e->rtiles2, rp2.tiles.data(), rp2.tiles.size()));
     }
@@ -1708,14 +1725,11 @@ gain_status run_split(gain_engine e, const gain_pair_job* j, int dI, int dF, con
                              0, r0);
             };
             GAIN_CUDA(cudaStreamWaitEvent(e->st2, e->ev[6], 0));
-            if (Nu2 > 0) {
-                GAIN_CUDA(cudaStreamWaitEvent(e->st2, EF.ready_head, 0));
-                GAIN_TRY(slice_upper(0, Nu2));
-                GAIN_CUDA(cudaEventRecord(e->ev[9], e->st2));
+            for (int k = 0; k < nup; ++k) {
+                if (uparts[k].wait) GAIN_CUDA(cudaStreamWaitEvent(e->st2, uparts[k].wait, 0));
+                GAIN_TRY(slice_upper(uparts[k].first, upper_end(k)));
+                GAIN_CUDA(cudaEventRecord(e->ev_upper[k], e->st2));
             }
-            if (EF.ready) GAIN_CUDA(cudaStreamWaitEvent(e->st2, EF.ready, 0));
-            GAIN_TRY(slice_upper(Nu2, Nu));
-            GAIN_CUDA(cudaEventRecord(e->ev[7], e->st2));
         }
         // inexact first-GEMM entries recomputed in FP64
         split::RefineHArgs rh;
@@ -1759,7 +1773,7 @@ gain_status run_split(gain_engine e, const gain_pair_job* j, int dI, int dF, con
     GAIN_TRY(slice(e, Hs, K2, nullptr, B, L.general ? L.nsymF : L.fpad, nullptr, nullptr, K2, Bpad, e->Hdig.p, p2,
                    e->Hst, true, e->rowerr.p, e->Vst.e.p, st));
     // the upper digits the (first) amplitude GEMM reads
-    GAIN_CUDA(cudaStreamWaitEvent(st, Nu2 > 0 ? e->ev[9] : e->ev[7], 0));
+    GAIN_CUDA(cudaStreamWaitEvent(st, e->ev_upper[0], 0));
     if (!split::make_digit_map(&tmH, e->Hdig.p, K2, Bpad, p2.slices) ||
         !split::make_digit_map(&tmU, e->Udig.p, K2, Nupad, p2.slices, pair || res ? split::BN / 2 : split::BM))
         return set_error(GAIN_ERR_CUDA, "cuTensorMapEncodeTiled failed (second GEMM digits)");
@@ -1777,7 +1791,7 @@ gain_status run_split(gain_engine e, const gain_pair_job* j, int dI, int dF, con
             t.nkb = K2 / split::BK;
             t2.push_back(t);
         }
-    row_grouped(t2, mstep, [&](const split::Tile& t) { return Nu2 > 0 && t.n0 >= Nu2 ? 1 : 0; });
+    row_grouped(t2, mstep, [&](const split::Tile& t) { return nup > 1 && t.n0 >= uparts[1].first ? 1 : 0; });
     const std::vector<split::Prod> pr2 = res ? std::vector<split::Prod>() : make_prods(p2);
     if (!res) {
         GAIN_TRY(e->tiles2.upload(t2));
@@ -1835,19 +1849,18 @@ gain_status run_split(gain_engine e, const gain_pair_job* j, int dI, int dF, con
         c2.nflags = g2.nflags;
         c2.max_flags = max_flags;
         split::crt_constants(&c2);
-        const cudaEvent_t waits[2] = {nullptr, e->ev[7]};
         res_flops += rp2.flops;
-        GAIN_TRY(residue_gemm(e, tmH, tmU, rp2, e->rtiles2.p, waits, B, Bpad, pair, c2, e->err(), e->span(2)));
-    } else if (Nu2 > 0) {
-        // tiles are upper-block-major: those of the first half (n0 < Nu2) come first
+        GAIN_TRY(residue_gemm(e, tmH, tmU, rp2, e->rtiles2.p, e->ev_upper, B, Bpad, pair, c2, e->err(), e->span(2)));
+    } else if (nup > 1) {
+        // tiles are upper-block-major: those of the first half come first
         int n1 = 0;
-        while (n1 < (int)t2.size() && t2[n1].n0 < Nu2) ++n1;
+        while (n1 < (int)t2.size() && t2[n1].n0 < uparts[1].first) ++n1;
         split::GemmArgs ga = g2, gb = g2;
         ga.ntiles = n1;
         gb.tiles = e->tiles2.p + n1;
         gb.ntiles = (int)t2.size() - n1;
         GAIN_CUDA(split::launch_gemm(tmH, tmU, ga, e->num_sms, st, pair));
-        GAIN_CUDA(cudaStreamWaitEvent(st, e->ev[7], 0));
+        GAIN_CUDA(cudaStreamWaitEvent(st, e->ev_upper[nup - 1], 0));
         GAIN_CUDA(split::launch_gemm(tmH, tmU, gb, e->num_sms, st, pair));
         e->launches += 2;
     } else {
@@ -2043,6 +2056,8 @@ void destroy_engine(gain_engine e) {
     if (e->std2h) cudaStreamSynchronize(e->std2h);
     for (auto& ev : e->ev)
         if (ev) cudaEventDestroy(ev);
+    for (auto& ev : e->ev_upper)
+        if (ev) cudaEventDestroy(ev);
     if (e->ev_up) cudaEventDestroy(e->ev_up);
     if (e->ev_lines) cudaEventDestroy(e->ev_lines);
     if (e->ev_lines_d2h) cudaEventDestroy(e->ev_lines_d2h);
@@ -2168,6 +2183,7 @@ gain_status gain_engine_create(int device, int jmax, int nsym, int maxdeg, gain_
     GAIN_CUDA(cudaEventCreateWithFlags(&e->ev_lines, cudaEventDisableTiming));
     GAIN_CUDA(cudaEventCreateWithFlags(&e->ev_lines_d2h, cudaEventDisableTiming));
     for (auto& ev : e->ev) GAIN_CUDA(cudaEventCreate(&ev));
+    for (auto& ev : e->ev_upper) GAIN_CUDA(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
     GAIN_CUDA(cudaEventCreateWithFlags(&e->ev_up, cudaEventDisableTiming));
     std::vector<double> t((size_t)(jmax + 1) * (jmax + 1) * 9);
     threej_table_host(jmax, t.data());
@@ -2378,7 +2394,7 @@ gain_status gain_upload_eigvecs(gain_engine e, int jind, int gamma, int nlevels,
     auto& slot = e->eig[{jind, gamma}];
     if (!slot) slot.reset(new Eig());
     if (slot->ready) GAIN_CUDA(cudaEventSynchronize(slot->ready));   // an asynchronous copy into it
-    slot->head_rows = 0;
+    slot->nparts = 0;
     slot->nlevels = nlevels;
     slot->nsize = nsize;
     GAIN_TRY(slot->d.alloc((size_t)nlevels * nsize));
@@ -2419,7 +2435,8 @@ gain_status gain_upload_eigvecs_async(gain_engine e, int jind, int gamma, int nl
     auto& slot = e->eig[{jind, gamma}];
     if (!slot) slot.reset(new Eig());
     if (!slot->ready) GAIN_CUDA(cudaEventCreateWithFlags(&slot->ready, cudaEventDisableTiming));
-    if (!slot->ready_head) GAIN_CUDA(cudaEventCreateWithFlags(&slot->ready_head, cudaEventDisableTiming));
+    for (cudaEvent_t& v : slot->part)
+        if (!v) GAIN_CUDA(cudaEventCreateWithFlags(&v, cudaEventDisableTiming));
     GAIN_CUDA(cudaEventSynchronize(slot->ready));   // a previous asynchronous copy into it
     slot->nlevels = nlevels;
     slot->nsize = nsize;
@@ -2428,19 +2445,22 @@ gain_status gain_upload_eigvecs_async(gain_engine e, int jind, int gamma, int nl
     // joined to the first before each run ends)
     if (!e->ev_up_fresh) GAIN_CUDA(cudaEventRecord(e->ev_up, e->st));   // after all queued work
     GAIN_CUDA(cudaStreamWaitEvent(e->stc, e->ev_up, 0));
-    // two parts: a run can start on the upper states of the first part while the second
-    // is still arriving
-    // (the head ends on a multiple of 128 rows, where the run's upper halves split)
-    const int head = nlevels >= 512 ? std::min(nlevels - 1, round_up(nlevels / 2, 128)) : 0;
-    if (head > 0) {
-        GAIN_CUDA(cudaMemcpyAsync(slot->d.p, vecs, sizeof(double) * (size_t)head * nsize, cudaMemcpyHostToDevice,
-                                  e->stc));
-        GAIN_CUDA(cudaEventRecord(slot->ready_head, e->stc));
+    // equal parts of at least 256 rows, ending on whole 256-column tiles: a run starts on the upper
+    // states of a part while the next is still arriving
+    const int parts = std::max(1, std::min(kUploadParts, nlevels / 256));
+    slot->nparts = 0;
+    for (int k = 0, r0 = 0; k < parts && r0 < nlevels; ++k) {
+        const int r1 = k + 1 < parts ? ((int)((long)nlevels * (k + 1) / parts) + 128) / 256 * 256 : nlevels;
+        if (r1 <= r0) continue;
+        GAIN_CUDA(cudaMemcpyAsync(slot->d.p + (size_t)r0 * nsize, vecs + (size_t)r0 * nsize,
+                                  sizeof(double) * (size_t)(r1 - r0) * nsize, cudaMemcpyHostToDevice, e->stc));
+        if (r1 < nlevels) {
+            GAIN_CUDA(cudaEventRecord(slot->part[slot->nparts], e->stc));
+            slot->part_rows[slot->nparts++] = r1;
+        }
+        r0 = r1;
     }
-    GAIN_CUDA(cudaMemcpyAsync(slot->d.p + (size_t)head * nsize, vecs + (size_t)head * nsize,
-                              sizeof(double) * (size_t)(nlevels - head) * nsize, cudaMemcpyHostToDevice, e->stc));
     GAIN_CUDA(cudaEventRecord(slot->ready, e->stc));
-    slot->head_rows = head;
     return GAIN_OK;
 }
 

@@ -184,3 +184,33 @@ def test_items_shared_by_both_accumulators(built_lib, rows, cols, monkeypatch):
         monkeypatch.setenv("GAINLS_GEMM_PAIR", pair)
         eng.run_pair(0, 0, 1, 1, lo, up, gainls.PATH_SPLIT)
         assert np.array_equal(eng.fetch_amp(), whole[:rows, :cols])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("order", ["all", "half", "reversed", "late"])
+def test_upper_vectors_arriving_in_parts(built_lib, order, monkeypatch):
+    """An asynchronous upload in several parts, the upper side run part by part
+    (GAINLS_UPPER_HALVES=force: also when the copy has landed): leading states, in whole tiles,
+    with each part; lists that do not ascend or lie in the last part wait for it.  The same bits as
+    after one synchronous upload."""
+    import torch
+    import gainls
+    import synth
+    p = synth.make_problem(345, [5, 6], "c4", blocks=[(5, 0), (6, 1)])
+    eng = gainls.Engine(JMAX, p.nsym, 1)
+    gainls.upload_problem(eng, p)
+    nI, vu = p.blocks[(0, 0)].vecs.shape[0], p.blocks[(1, 1)].vecs
+    n = vu.shape[0]
+    assert n >= 1024
+    up = {"all": np.arange(n), "half": np.arange(0, n, 2), "reversed": np.arange(n)[::-1],
+          "late": np.arange(n - 300, n)}[order].astype(np.int32)
+    lo = np.arange(0, nI, 3, dtype=np.int32)
+    eng.run_pair(0, 0, 1, 1, lo, up, gainls.PATH_SPLIT)
+    one = eng.fetch_amp().copy()
+    pin = torch.empty(vu.shape, dtype=torch.float64, pin_memory=True).numpy()
+    pin[...] = vu
+    monkeypatch.setenv("GAINLS_UPPER_HALVES", "force")
+    eng.upload_eigvecs_async(1, 1, pin)
+    st = eng.run_pair(0, 0, 1, 1, lo, up, gainls.PATH_SPLIT)
+    assert st["kernel_launches"] == {"all": 16, "half": 12, "reversed": 10, "late": 10}[order]
+    assert np.array_equal(eng.fetch_amp(), one)
