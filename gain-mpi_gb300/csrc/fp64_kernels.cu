@@ -156,6 +156,18 @@ __device__ __forceinline__ double hls_sum(double acc, const HlsTerm* list, int n
 // has one K block's primitives (a few thousand at most): small blocks spread their chains over
 // the SMs, the block's other threads share in forming the terms.
 constexpr int kDropThreads = 128, kDropF = 32;
+// Its loads should not lengthen a chain that is alone on its SM: the first warp only runs the
+// chains, the other three copy the dipole (terms of the list x the 32 functions) into shared
+// memory two tiles ahead of it.  What is left is the latency of 900 dependent FP64 operations:
+// 8 to 32 functions and 128 to 512 threads a block, and longer lists, all take the same time.
+// 32 upper states of J = 10 -> 11 (12 launches of 1200 outputs): 1075 us when the chain loaded the
+// dipole itself, 1034 so.
+constexpr int kDropTile = 16, kDropBufs = 3;
+
+__device__ __forceinline__ void copy8_async(double* dst, const double* src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src)
+                 : "memory");
+}
 
 __global__ void __launch_bounds__(kDropThreads)
 k_hls_kblock(int dimenF, int dimenI, int jI, int jF, int kF, const int* __restrict__ tauI,
@@ -166,9 +178,11 @@ k_hls_kblock(int dimenF, int dimenI, int jI, int jF, int kF, const int* __restri
              const double* __restrict__ threej, double* __restrict__ half_ls, int jmax,
              int dip_stride) {
     __shared__ HlsLists L;
-    const int f = blockIdx.x * kDropF + threadIdx.x;
+    __shared__ double tile[kDropBufs][kDropTile][kDropF];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int f = blockIdx.x * kDropF + lane;   // the function of the lane, in every warp
     const int irootF = startF_idx + f;
-    const bool inF = (int)threadIdx.x < kDropF && f < dimenF;
+    const bool inF = f < dimenF;
     int icF = 0, tF = 0;
     if (inF) {
         icF = icorrF[irootF];
@@ -190,13 +204,38 @@ k_hls_kblock(int dimenF, int dimenI, int jI, int jF, int kF, const int* __restri
                 t = tauI[startI + i];
                 ic = icorrI[startI + i];
             },
-            [&](int n) {
-                if (valid) acc = hls_sum(acc, L.term[tF], n, mu);
+            [&](int n) {   // every warp of the block takes part
+                const HlsTerm* list = L.term[tF];
+                auto fetch = [&](int t) {   // tile t into its buffer; an empty group past the end
+                    if (warp > 0 && valid)
+                        for (int i = warp - 1; i < kDropTile; i += kDropThreads / 32 - 1)
+                            if (t * kDropTile + i < n)
+                                copy8_async(&tile[t % kDropBufs][i][lane], mu + list[t * kDropTile + i].off);
+                    asm volatile("cp.async.commit_group;" ::: "memory");
+                };
+                const int nt = (n + kDropTile - 1) / kDropTile;
+                fetch(0);
+                fetch(1);
+                for (int t = 0; t < nt; ++t) {
+                    asm volatile("cp.async.wait_group 1;" ::: "memory");
+                    __syncthreads();   // tile t has landed, and tile t - 1's buffer is free
+                    fetch(t + 2);
+                    if (warp > 0) continue;
+                    const double(*m)[kDropF] = tile[t % kDropBufs];
+                    const HlsTerm* l = list + t * kDropTile;
+                    if ((t + 1) * kDropTile <= n) {
+#pragma unroll
+                        for (int k = 0; k < kDropTile; ++k) acc = __fma_rn(l[k].v, m[k][lane], acc);
+                    } else {
+                        for (int k = 0; t * kDropTile + k < n; ++k) acc = __fma_rn(l[k].v, m[k][lane], acc);
+                    }
+                }
+                asm volatile("cp.async.wait_group 0;" ::: "memory");
             });
         startI += kbs;
         if (startI >= dimenI) break;
     }
-    if (valid) half_ls[irootF] = __dmul_rn(acc, parity_sign((kF % 3) * tF));
+    if (valid && warp == 0) half_ls[irootF] = __dmul_rn(acc, parity_sign((kF % 3) * tF));
 }
 
 // ---------------------------------------------------------------------------------------
