@@ -6,7 +6,7 @@ functions) -> J'=11 class 1 (12000 functions); the 2000 lowest lower states (all
 per step.  Synthetic, seeded inputs stand in for the TROVE checkpoints.
 
 One step = the split-precision tensor-core path over the whole block pair starting from
-FP64 inputs resident in HBM: digit slicing of both eigenvector sets, the rotational-dipole
+FP64 inputs resident in HBM: residue planes of both eigenvector sets, the rotational-dipole
 band GEMM, the amplitude GEMM, FP64 refinement of uncertified lines.  `e2e` runs the same
 step through the C ABI from pinned host buffers: upload of both eigenvector sets, the run,
 and the device-to-host read of S and A.
@@ -630,7 +630,7 @@ def adjoint_check(args):
                                    "tensor_flops": tc_flops,
                                    "tensor_tflops": tc_flops / (chain_ms["split_tensor_core"] * 1e-3) / 1e12,
                                    "peak_bf16_tflops": _peak("bf16_tflops"),
-                                   "digits": "48 bits (8-bit digits x 6, exact FP32 accumulation)"},
+                                   "precision": "operands of 48 bits, 13 or more moduli, exact"},
            "split_forward_gradient_max_err_over_max_grad": split_vs_fp64,
            "fp32_gradient_max_err_over_max_grad": fp32_vs_fp64,
            "fp32_fd_median_rel_err": float(np.median(rel32)), "fp32_fd_p99_rel_err": float(np.quantile(rel32, 0.99)),

@@ -1,6 +1,8 @@
-// Split-precision (Ozaki-style) tensor-core path: internal interface.
+// Split-precision tensor-core path: internal interface.  What runs by default is the residue form
+// (residue.h); this file also holds balanced digits (Ozaki scheme I), which explicit digit
+// options take, and devices without room for the residue planes.
 //
-// Every FP64 operand row x is written as x = 2^e (sum_{i<s} d_i 2^{-(i+1) beta} + r),
+// In digit form every FP64 operand row x is written as x = 2^e (sum_{i<s} d_i 2^{-(i+1) beta} + r),
 // |r| <= 2^{-s beta - 1}, with balanced integer digits d_i (|d_0| <= 2^beta,
 // |d_i| <= 2^{beta-1}) stored as BF16 (exact for beta <= 8).  A product of two rows is
 // sum over digit pairs (i, j), i + j < s, of an integer dot product computed exactly by

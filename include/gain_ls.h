@@ -261,10 +261,11 @@ typedef enum {
     GAIN_ADJOINT_FP32 = 1,   /* G, dL/dH, dL/dh, the lower vectors and the dL/dmu sums in FP32; the
                                 FP64 amplitudes, eigenvectors and expansion tables are rounded to
                                 FP32 as they are read; dL_dmu is still accumulated in double */
-    GAIN_ADJOINT_SPLIT = 2   /* both products on the tensor cores as digit GEMMs (the split
-                                path's Ozaki digits, 48 bits, exact accumulation, FP64
-                                recombination; entries whose exactness certificate fails are
-                                recomputed in FP64): dL/dH = G U over the upper states, and the
+    GAIN_ADJOINT_SPLIT = 2   /* both products on the tensor cores in the split path's residue
+                                form (operands of 48 bits, exact products; balanced digits where
+                                the device cannot hold the residue planes, entries whose
+                                exactness certificate fails then recomputed in FP64):
+                                dL/dH = G U over the upper states, and the
                                 batched outer product dL/dM = sum_b dh_b v_b^T over the band of
                                 the rotational-dipole matrix (|K_I - K_F| <= 1, or all K in the
                                 rotational-symmetry form), then the FP64 scatter into dL/dmu.
@@ -303,16 +304,16 @@ gain_status gain_run_plan(gain_engine* engines, int n_engines, const gain_pair_j
  * main.cpp:238-342's loop over (J'', Gamma'') -> (J', Gamma') pairs and their lower states;
  * no counterpart in the reference, which launches per lower state and per transition,
  * BaseClasses/GpuManager.cpp:645-746).  The split path of every job runs as
- *   the digits of all jobs' lower and upper eigenvectors        (one launch per slicing
- *                                                                kernel; jobs of one block
- *                                                                share its digits)
+ *   the operand planes (residues, or digits with a digit        (one launch per slicing
+ *   configuration) of all jobs' lower and upper eigenvectors     kernel; jobs of one block
+ *                                                                share its planes)
  *   ONE persistent grouped tensor-core launch of the first GEMM over the tiles of all jobs
- *   FP64 refinement of every job's H (one launch), then the digits of all jobs' H
+ *   FP64 refinement of every job's H (one launch), then the planes of all jobs' H
  *   ONE persistent grouped tensor-core launch of the second GEMM over all jobs' tiles
  *   FP64 refinement of every job's amplitudes                  (one launch)
  * captured once into a CUDA graph and replayed by gain_plan_run.  The tiles of each grouped
  * launch are dealt to the persistent CTAs in list order, each to the first free one, with
- * the jobs with the costliest tiles (k-blocks x digit products) first, so block pairs of
+ * the jobs with the costliest tiles first, so block pairs of
  * very uneven sizes share one launch.  Each job keeps its own device buffers; the engine's
  * uploads (bases, expansion tables, dipole, eigenvectors) must hold every job's inputs.  Jobs are non-degenerate (components 0, 0) with a single dipole
  * piece.  After gain_plan_run, gain_plan_select makes one job's amplitudes the engine's last
@@ -324,11 +325,11 @@ gain_status gain_run_plan(gain_engine* engines, int n_engines, const gain_pair_j
 typedef struct gain_plan_s* gain_plan;
 
 /* gain_plan_create flags */
-#define GAIN_PLAN_AUTOTUNE 1   /* choose the tile shape (CTA pairs or single CTAs) and, per size
-                                  class of the second GEMM's inner dimension, its digit
-                                  configuration (8-bit x 6 or 7-bit x 7) by timing the plan's
-                                  candidates on first use; the choice is cached per plan shape
-                                  for the process */
+#define GAIN_PLAN_AUTOTUNE 1   /* choose the tile shape (CTA pairs or single CTAs) by timing the
+                                  plan's candidates on first use; the choice is cached per plan
+                                  shape for the process.  A plan that runs on digits also chooses,
+                                  per size class of the second GEMM's inner dimension, 8-bit x 6 or
+                                  7-bit x 7 */
 
 typedef struct gain_plan_stats {
     double device_ms;            /* the graph replay (CUDA events around it) */
@@ -341,19 +342,22 @@ typedef struct gain_plan_stats {
     int kernel_launches;         /* kernel nodes among them */
     int gemm1_tiles, gemm2_tiles;/* tiles of the two grouped launches (empty slots excluded) */
     int units;                   /* persistent CTAs (CTA pairs) of each grouped launch */
-    int pair;                    /* 1: 256 x 128 tiles on CTA pairs; 0: 128 x 128 tiles */
+    int pair;                    /* 1: tiles of 256 rows on CTA pairs; 0: of 128 rows */
     int captures;                /* graph captures so far */
     int tuned;                   /* 1: the configuration came from the autotuner */
     double tune_ms;              /* wall time the autotuner spent (first use) */
     double tensor_flops;         /* BF16 MMA flops of the two grouped launches (whole tiles) */
-    int beta2[4], slices2[4];    /* second-GEMM digits per size class of its inner dimension K:
-                                    K <= 2048, <= 8192, <= 16384, above (0: class absent) */
-    double digits_ms;            /* before the first GEMM: expansions and eigenvector digits */
-    double middle_ms;            /* between the GEMMs: refinement of H, contraction, H digits */
-    double refine_ms;            /* after the second GEMM: refinement of the amplitudes */
-    int shared_lower;            /* jobs reading another job's lower digits (same lower block,
-                                    levels, layout and first-GEMM digits) */
-    int shared_upper;            /* jobs reading another job's upper digits */
+    int beta2[4], slices2[4];    /* second GEMM per size class of its inner dimension K (K <= 2048,
+                                    <= 8192, <= 16384, above; 0: class absent): digit bits and
+                                    digits, or 8 and the number of moduli */
+    double digits_ms;            /* before the first GEMM: expansions and eigenvector planes */
+    double middle_ms;            /* between the GEMMs: reconstruction and refinement of H,
+                                    contraction, H planes */
+    double refine_ms;            /* after the second GEMM: reconstruction and refinement of the
+                                    amplitudes */
+    int shared_lower;            /* jobs reading another job's lower planes (same lower block,
+                                    levels, layout and first-GEMM configuration) */
+    int shared_upper;            /* jobs reading another job's upper planes */
 } gain_plan_stats;
 
 gain_status gain_plan_create(gain_engine e, const gain_pair_job* jobs, int n_jobs, const gain_split_opts* opts,
