@@ -1472,13 +1472,13 @@ gain_status run_split(gain_engine e, const gain_pair_job* j, int dI, int dF, con
     if (first < Nu) uparts.push_back({first, EF.ready});
     const int nup = (int)uparts.size();
     auto upper_end = [&](int k) { return k + 1 < nup ? uparts[k + 1].first : Nu; };
-    GAIN_TRY(e->words.alloc(kRunWords));
+    GAIN_TRY(e->words.alloc(kRunWords + 1));   // and the count of k_refine_amp's finished blocks
     GAIN_TRY(e->rowerr.alloc(Bpad));
     ResiduePlan rp1, rp2;
     Staging up;
     GAIN_TRY(up.add(e->d_lower, j->lower_levels, B));
     GAIN_TRY(up.add(e->d_upper, j->upper_levels, Nu));
-    GAIN_TRY(up.add(e->words.p, nullptr, sizeof(unsigned long long) * kRunWords));
+    GAIN_TRY(up.add(e->words.p, nullptr, sizeof(unsigned long long) * (kRunWords + 1)));
     GAIN_TRY(up.add(e->rowerr.p, nullptr, sizeof(float) * Bpad));
     if (res) {
         if (npieces == 1) {
@@ -1889,6 +1889,11 @@ gain_status run_split(gain_engine e, const gain_pair_job* j, int dI, int dF, con
     ra.amp_floor = std::sqrt((opts && opts->s_floor > 0) ? opts->s_floor : 1e-10);
     ra.uncertified = e->ull();
     ra.uncertified_weak = e->ull() + 3;
+    if (!e->readback) GAIN_CUDA(cudaMallocHost(&e->readback, 128));
+    ra.words = e->words.p;
+    ra.host = (unsigned long long*)e->readback;
+    ra.nwords = kRunWords;
+    ra.done = (unsigned int*)(e->words.p + kRunWords);
     GAIN_CUDA(split::launch_refine_amp(ra, 4 * e->num_sms, st));
     ++e->launches;
     GAIN_CUDA(cudaEventRecord(e->ev[1], st));
@@ -1896,10 +1901,8 @@ gain_status run_split(gain_engine e, const gain_pair_job* j, int dI, int dF, con
     unsigned int cnt[4];
     unsigned long long unc[4], spans[4];
     int errw = 0;
-    {   // the run's counters through one page-locked area
-        if (!e->readback) GAIN_CUDA(cudaMallocHost(&e->readback, 128));
-        char* rb = (char*)e->readback;
-        GAIN_CUDA(cudaMemcpyAsync(rb, e->words.p, sizeof(unsigned long long) * kRunWords, cudaMemcpyDeviceToHost, st));
+    {   // the run's counters, stored by the last kernel
+        const char* rb = (const char*)e->readback;
         GAIN_CUDA(cudaStreamSynchronize(st));
         e->stage_busy = false;
         memcpy(cnt, rb, sizeof cnt);

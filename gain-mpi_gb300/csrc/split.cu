@@ -1159,6 +1159,19 @@ __device__ __forceinline__ void refine_amp(const RefineAmpArgs& a) {
 __global__ void k_refine_amp(const RefineAmpArgs a) {
     follow_wait();
     refine_amp(a);
+    if (!a.host) return;
+    __shared__ bool last;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        last = atomicAdd(a.done, 1u) == gridDim.x - 1;
+        __threadfence();
+    }
+    __syncthreads();
+    if (last && (int)threadIdx.x < a.nwords) {
+        a.host[threadIdx.x] = __ldcg(a.words + threadIdx.x);
+        __threadfence_system();
+    }
 }
 __global__ void k_refine_amp_grouped(const RefineAmpArgs* __restrict__ a, int n) {
     refine_jobs(a, n, [](const RefineAmpArgs& x) { refine_amp(x); });

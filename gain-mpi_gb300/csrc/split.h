@@ -248,6 +248,12 @@ struct RefineAmpArgs {
     double amp_floor;                    // sqrt(s_floor): certification domain |amp| >= floor*max
     unsigned long long* uncertified;     // in the domain
     unsigned long long* uncertified_weak;  // below it
+    // optional: the run's counter block, which the last block to finish stores to page-locked host
+    // memory (a copy behind the kernel costs a short run about 5 us); *done counts the blocks
+    const unsigned long long* words;
+    unsigned long long* host;
+    int nwords;
+    unsigned int* done;
 };
 cudaError_t launch_refine_amp(const RefineAmpArgs& a, int max_blocks, cudaStream_t st);
 cudaError_t launch_refine_amp_grouped(const RefineAmpArgs* a, int n, int blocks, cudaStream_t st);
