@@ -45,7 +45,8 @@ __device__ __forceinline__ void rot_factor(int kI, int kF, int tauI, int tauF, i
 // reference skips them: the other symmetry classes' primitives) are left out of the list.
 // Measured (GB300): the drop-in kernel 526 -> 60 us for 1200 outputs of 900 non-zero terms each
 // (32 outputs per block instead of 128, and the dipole loads run ahead of the chain), the plain
-// path's 480 -> 88 us for 8 x 3000 outputs of 1200 terms (53 us at the FP64 rate).
+// path's 480 -> 88 us for 8 x 3000 outputs of 1200 terms (53 us at the FP64 rate), and 68 us of a
+// launch of 32 x 3000.
 struct HlsTerm {
     double v;    // weight: vector x 1/sqrt(2) x 3j x coefficient x sign
     long off;    // the lower function's row of the dipole component it couples through
@@ -403,9 +404,14 @@ __global__ void k_expand_levels(int dimen, int igamma, int maxcoeff, int ideg, i
 constexpr int kGemvBatch = 8;
 __global__ void __launch_bounds__(256)
 k_gemv_batch(int nrows, int n, const double* __restrict__ U, long ldu, const int* __restrict__ levels,
-             const double* __restrict__ x, long ldx, int nb, double* __restrict__ out, long ldo) {
-    const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+             const double* __restrict__ x, long ldx, int nall, double* __restrict__ out, long ldo) {
+    // neighbouring blocks: the same upper states with the next kGemvBatch lower ones
+    const int groups = (nall + kGemvBatch - 1) / kGemvBatch, group = blockIdx.x % groups;
+    const int warp = ((blockIdx.x / groups) * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
+    const int nb = min(kGemvBatch, nall - group * kGemvBatch);
+    x += (long)group * kGemvBatch * ldx;
+    out += (long)group * kGemvBatch * ldo;
     if (warp >= nrows) return;
     const double* row = U + (long)levels[warp] * ldu;
     double acc[kGemvBatch];
@@ -778,8 +784,9 @@ cudaError_t launch_expand_levels(int dimen, int igamma, int maxcoeff, int ideg, 
 cudaError_t launch_gemv_batch(int nrows, int n, const double* U, long ldu, const int* levels, const double* x,
                               long ldx, int nbatch, double* out, long ldo, cudaStream_t st) {
     if (nrows <= 0 || nbatch <= 0) return cudaSuccess;
-    if (nbatch > kGemvBatch) return cudaErrorInvalidValue;
-    k_gemv_batch<<<(nrows + 7) / 8, 256, 0, st>>>(nrows, n, U, ldu, levels, x, ldx, nbatch, out, ldo);
+    const long blocks = (long)((nrows + 7) / 8) * ((nbatch + kGemvBatch - 1) / kGemvBatch);
+    if (blocks > 0x7fffffffl) return cudaErrorInvalidValue;
+    k_gemv_batch<<<(unsigned)blocks, 256, 0, st>>>(nrows, n, U, ldu, levels, x, ldx, nbatch, out, ldo);
     return cudaGetLastError();
 }
 

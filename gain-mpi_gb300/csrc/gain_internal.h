@@ -125,8 +125,12 @@ cudaError_t launch_expand_levels(int dimen, int igamma, int maxcoeff, int ideg, 
                                  const float* vecs, long ldv, const int* levels, float* prim, long ldp,
                                  int nbatch, cudaStream_t st);
 
-// out[b*ldo + u] = sum_f U[level[u]*ldu + f] * x[b*ldx + f], u < nrows, b < nbatch <= 8
-constexpr int kPlainBatch = 8;
+// out[b*ldo + u] = sum_f U[level[u]*ldu + f] * x[b*ldx + f], u < nrows, b < nbatch
+// Lower states per launch of the plain path.  Its kernels are FP64 chains, of which an SM needs six
+// or more in flight; eight states left two or three blocks to an SM, unevenly.  96 lower x 3000
+// upper states of 3000 functions: 3264 us with eight, 2543 with 32 (per eight states the half line
+// strengths 88 -> 68 us, the products with the upper vectors 165 -> 135, 53 and 132 at the FP64 rate).
+constexpr int kPlainBatch = 32;
 cudaError_t launch_gemv_batch(int nrows, int n, const double* U, long ldu, const int* levels, const double* x,
                               long ldx, int nbatch, double* out, long ldo, cudaStream_t st);
 
