@@ -277,7 +277,7 @@ struct gain_engine_s {
     gain::DevArray<unsigned long long> lcnt;
     bool lines_pending = false;     // gain_pair_lines_async copies still in flight
     long long* lines_nout = nullptr;   // their caller's n_lines
-    cudaEvent_t ev[10] = {};
+    cudaEvent_t ev[8] = {};
     cudaEvent_t ev_upper[gain::kUploadParts] = {};   // each part of the upper rows sliced
     // orders an asynchronous upload after the engine work that reads eigenvectors: recorded
     // at the end of every run (runs, plans, adjoints and line recomputations return only when
@@ -3571,8 +3571,8 @@ gain_status lines_text(gain_engine e, const gain_line_params* prm, const double*
             GAIN_CUDA(launch_text_write(t, largest, b0, b1, st));
             if (copy) {
                 const unsigned long long o0 = offs[b0], o1 = b1 < nb ? offs[b1] : total;
-                GAIN_CUDA(cudaEventRecord(e->ev[8], st));
-                GAIN_CUDA(cudaStreamWaitEvent(e->stc, e->ev[8], 0));
+                GAIN_CUDA(cudaEventRecord(e->ev[7], st));
+                GAIN_CUDA(cudaStreamWaitEvent(e->stc, e->ev[7], 0));
                 if (o1 > o0)
                     GAIN_CUDA(cudaMemcpyAsync(out + o0, e->text.p + o0, o1 - o0, cudaMemcpyDeviceToHost, e->stc));
             }

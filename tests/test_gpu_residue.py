@@ -166,10 +166,10 @@ def test_plan_refines_flagged_entries_of_every_job(built_lib, monkeypatch):
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("rows,cols", [(1, 1), (100, 130), (129, 257), (300, 500), (520, 700), (700, 770)])
-def test_items_shared_by_both_accumulators(built_lib, rows, cols, monkeypatch):
-    """Inner lengths of two to four chunks and one to five items a unit: a unit's odd item is
-    accumulated by both of its accumulators.  The residues are the same integers however they are
-    summed, so every amplitude equals the whole block's bits."""
+def test_any_number_of_items_gives_the_same_bits(built_lib, rows, cols, monkeypatch):
+    """Inner lengths of two to four chunks and one to five items a unit, odd and even: the items
+    alternate between the accumulators, and the last one of an odd number runs alone.  The residues
+    are the same integers whatever the tiles, so every amplitude equals the whole block's bits."""
     import gainls
     import synth
     p = synth.make_problem(310, [5, 6], "c4", blocks=[(5, 0), (6, 1)])
