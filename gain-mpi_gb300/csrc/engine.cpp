@@ -1538,10 +1538,14 @@ gain_status run_split(gain_engine e, const gain_pair_job* j, int dI, int dF, con
         e->zkey_U = kU;
     }
 
-    // The upper slicing runs on the second stream from here on.  It cannot share SMs with the
-    // first GEMM (the GEMM's 256-register warps fill two SM sub-partitions' register files),
-    // so it overlaps the lower slicing and precedes the GEMM.
-    GAIN_CUDA(cudaEventRecord(e->ev[6], st));
+    // The upper slicing (second stream) cannot share SMs with the first GEMM, whose registers fill
+    // them.  A long one overlaps the lower slicing and precedes the GEMM (2000 x 12 000 outputs: 7.0
+    // ms; behind the GEMM, beside the reconstruction and the slicing of H, 7.15); a short one
+    // follows the GEMM, so the lower slicing has the chip to itself and directly follows the
+    // run's first kernel (50 x 600: 99.7 us against 102.5, 640 x 900 167 against 171, 1000 x 6000
+    // the same either way).
+    const bool fork_first = (long)Nu * K2 > (1l << 25);
+    if (fork_first) GAIN_CUDA(cudaEventRecord(e->ev[6], st));
 
     // ---- lower vectors -> digits in the padded lower layout (expanded to primitives first
     // when the expansion mixes them)
@@ -1675,6 +1679,7 @@ gain_status run_split(gain_engine e, const gain_pair_job* j, int dI, int dF, con
         g1.cols_valid = L.fpad;
         g1.err = e->err();
         g1.fuse = fuse1;
+        if (piece == 0 && !fork_first) GAIN_CUDA(cudaEventRecord(e->ev[6], st));
         if (!res && piece == 0) GAIN_CUDA(cudaEventRecord(e->ev[2], st));
         if (res) {
             split::CrtArgs c1;
