@@ -3,6 +3,7 @@
 // the needed upper functions, transpose expansion, GEMV against resident upper vectors) and
 // the S / A / I line assembly.
 #include <algorithm>
+#include <utility>
 
 #include <cooperative_groups.h>
 
@@ -263,7 +264,9 @@ __global__ void k_expand(int dimen, int igamma, int maxcoeff, int ideg, int sdeg
 // calls on any streams are independent).  At n = 13 800: 11 us on one CTA, 7 on the cluster; one
 // CTA reads about 0.1 TB/s however long the vectors are.
 // Deterministic: element i always belongs to thread i mod the launch's threads, partials are
-// added in a fixed order.
+// added in a fixed order.  A block may touch another's shared memory only once that block has
+// started: every thread arrives at the cluster's barrier on entry and waits for it before the
+// partial sums are stored, so that the loads hide the wait.
 constexpr int kDotThreads = 1024, kDotCtas = 8, kDotSmall = 4096;
 
 template <bool CLUSTER>
@@ -271,6 +274,8 @@ __global__ void __launch_bounds__(kDotThreads) k_dot(int n, const double* __rest
                                                      const double* __restrict__ y, double* result) {
     __shared__ double red[32];
     __shared__ double part[kDotCtas];
+    cg::cluster_group::arrival_token started;
+    if (CLUSTER) started = cg::this_cluster().barrier_arrive();
     const long step = CLUSTER ? kDotThreads * kDotCtas : kDotThreads;
     long i = (CLUSTER ? (long)blockIdx.x * kDotThreads : 0l) + threadIdx.x;
     double acc = 0.0;
@@ -292,6 +297,7 @@ __global__ void __launch_bounds__(kDotThreads) k_dot(int n, const double* __rest
     for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
     if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = acc;
     __syncthreads();
+    if (CLUSTER) cg::this_cluster().barrier_wait(std::move(started));
     if (threadIdx.x < 32) {
         acc = red[threadIdx.x];
         for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);

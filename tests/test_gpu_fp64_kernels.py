@@ -73,3 +73,24 @@ def test_dot_one_block_and_cluster(built_lib, n):
     assert got[0] == got[1] and np.isnan(got[2])
     ref = oracle.dot(x[:n], y[:n], oracle.DD) if n else 0.0
     assert abs(got[0] - ref) <= (n + 1) * 2.0 ** -53 * np.sum(np.abs(x[:n] * y[:n]))
+
+
+@pytest.mark.parametrize("n", [4097, 5000, 8193])
+def test_cluster_dots_back_to_back_on_several_streams(built_lib, n):
+    """The shortest sums on the cluster: most of its blocks have no element and reach the exchange of
+    the partial sums at once, while other launches keep the chip busy.  Every launch gives the
+    bits of the first."""
+    import torch
+    import gainls
+    rng = np.random.default_rng(n)
+    dx, dy = _dev(rng.standard_normal(n)), _dev(rng.standard_normal(n))
+    res = torch.full((4, 400), np.nan, dtype=torch.float64, device="cuda")
+    streams = [torch.cuda.Stream() for _ in range(4)]
+    for s in streams:
+        s.wait_stream(torch.cuda.current_stream())
+    for k in range(res.shape[1]):
+        for q, s in enumerate(streams):
+            gainls.dot(n, dx.data_ptr(), dy.data_ptr(), res[q, k:].data_ptr(), s.cuda_stream)
+    torch.cuda.synchronize()
+    got = res.cpu().numpy().view(np.uint64)
+    assert np.all(got == got[0, 0]) and np.isfinite(res[0, 0].item())
