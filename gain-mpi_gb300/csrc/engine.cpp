@@ -1902,6 +1902,9 @@ gain_status run_split(gain_engine e, const gain_pair_job* j, int dI, int dF, con
     GAIN_CUDA(split::launch_refine_amp(ra, 4 * e->num_sms, st));
     ++e->launches;
     GAIN_CUDA(cudaEventRecord(e->ev[1], st));
+    // the caller may change the uploaded vectors once the run returns: a run that reads leading
+    // parts only waits for the rest of the copy too
+    if (EF.ready && nup > 0 && uparts.back().wait != EF.ready) GAIN_CUDA(cudaStreamWaitEvent(st, EF.ready, 0));
 
     unsigned int cnt[4];
     unsigned long long unc[4], spans[4];

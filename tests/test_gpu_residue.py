@@ -214,3 +214,33 @@ def test_upper_vectors_arriving_in_parts(built_lib, order, monkeypatch):
     st = eng.run_pair(0, 0, 1, 1, lo, up, gainls.PATH_SPLIT)
     assert st["kernel_launches"] == {"all": 16, "half": 12, "reversed": 10, "late": 10}[order]
     assert np.array_equal(eng.fetch_amp(), one)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("lead", [256, 512])
+def test_a_run_returns_after_the_whole_asynchronous_copy(built_lib, lead):
+    """Leading upper states that whole parts of an asynchronous upload hold: the run needs none of
+    the rest, but the caller may change the vectors once it returns, so the rest (270 MB here,
+    over a millisecond) has to be in place then."""
+    import torch
+    import gainls
+    import synth
+    p = synth.make_problem(345, [5, 6], "c4", blocks=[(5, 0), (6, 1)])
+    eng = gainls.Engine(JMAX, p.nsym, 1)
+    gainls.upload_problem(eng, p)
+    nsize, n = p.blocks[(1, 1)].vecs.shape[1], 40000
+    pin = torch.empty((n, nsize), dtype=torch.float64, pin_memory=True)
+    pin.normal_(generator=torch.Generator().manual_seed(1))
+    lo, tail = np.arange(3, dtype=np.int32), np.arange(n - 256, n, dtype=np.int32)
+    up = np.arange(lead, dtype=np.int32)
+    pin = pin.numpy()
+    eng.upload_eigvecs(1, 1, pin)
+    eng.run_pair(0, 0, 1, 1, lo, tail, gainls.PATH_SPLIT)
+    want = eng.fetch_amp().copy()
+    eng.run_pair(0, 0, 1, 1, lo, up, gainls.PATH_SPLIT)     # (the layout and buffers are there)
+    eng.upload_eigvecs(1, 1, np.zeros_like(pin))
+    eng.upload_eigvecs_async(1, 1, pin)
+    eng.run_pair(0, 0, 1, 1, lo, up, gainls.PATH_SPLIT)
+    pin[-64:] = 0.0
+    eng.run_pair(0, 0, 1, 1, lo, tail, gainls.PATH_SPLIT)
+    np.testing.assert_array_equal(eng.fetch_amp(), want)
