@@ -1210,6 +1210,41 @@ struct ColumnRange {
     int n0, n1, a_k0, nkb;
 };
 
+// One attempt to place the buffers of the residue form, whose planes take about twice the digits'
+// memory: first the bytes they are short of are counted and compared with what the device has
+// left (a digit run of a size without room makes no attempt, and keeps its buffers), then they
+// are allocated.  GAINLS_RESIDUE_BYTES limits the new memory of an attempt, to exercise the way
+// back to digits on small cases.
+struct ResidueRoom {
+    size_t grow = 0, held = 0;   // new bytes, and those freed for them
+    size_t left = std::numeric_limits<size_t>::max();
+    ResidueRoom() {
+        if (const char* s = getenv("GAINLS_RESIDUE_BYTES")) left = (size_t)strtoull(s, nullptr, 10);
+    }
+    template <class T>
+    gain_status count(const DevArray<T>& d, size_t n) {
+        if (d.p && n <= d.n) return GAIN_OK;
+        grow += sizeof(T) * n;
+        held += sizeof(T) * d.n;
+        return GAIN_OK;
+    }
+    bool fits() const {
+        size_t free_bytes = 0, total = 0;
+        if (!grow || cudaMemGetInfo(&free_bytes, &total) != cudaSuccess) return true;
+        return grow <= free_bytes + held;
+    }
+    template <class T>
+    gain_status alloc(DevArray<T>& d, size_t n) {
+        if (d.p && n <= d.n) return GAIN_OK;
+        if (sizeof(T) * n > left) {
+            d.release();
+            return set_error(GAIN_ERR_OOM, "residue form: more than GAINLS_RESIDUE_BYTES");
+        }
+        left -= sizeof(T) * n;
+        return d.alloc(n);
+    }
+};
+
 // Tiles of `rows` output rows over the column ranges, column by column: 256 columns wide on CTA
 // pairs (where a range has them), 128 otherwise.
 void residue_tiles(const std::vector<ColumnRange>& cols, int rows, int mstep, bool wide, std::vector<split::ResTile>& out) {
@@ -1421,19 +1456,42 @@ gain_status run_split(gain_engine e, const gain_pair_job* j, int dI, int dF, con
     const int Nu = j->nupper, Nupad = round_up(Nu, split::BN);
     SplitParams p1x, p2;
     bool res = residues_wanted(opts);
+    // the residue form's planes and panel of residues, each passed to `take` with its size
+    auto planes = [&](auto&& take) -> gain_status {
+        const size_t panel = (size_t)std::min(Bpad, residue_panel(mstep));
+        GAIN_TRY(take(e->Vdig, (size_t)p1x.slices * Bpad * L.kpadI));
+        GAIN_TRY(take(e->Hdig, (size_t)p2.slices * Bpad * K2));
+        GAIN_TRY(take(e->Udig, (size_t)p2.slices * Nupad * K2));
+        GAIN_TRY(take(L.bandDig, (size_t)p1x.slices * L.fpad * L.W));
+        return take(e->res, std::max(panel * L.fpad * p1x.slices, panel * Nupad * p2.slices));
+    };
+    auto drop_planes = [&]() {
+        (void)cudaGetLastError();
+        e->Vdig.release();
+        e->Hdig.release();
+        e->Udig.release();
+        e->res.release();
+        L.bandDig.release();
+        L.dig = {};
+        e->zkey_V.clear();   // (another buffer may get an old one's address)
+        e->zkey_H.clear();
+        e->zkey_U.clear();
+    };
     if (res) {
         p1x = residue_params1(L);
         p2 = residue_params2(K2);
         res = digits_supported(p1x, p2);
-        const size_t panel = (size_t)std::min(Bpad, residue_panel(mstep));
-        if (res && (e->Vdig.alloc((size_t)p1x.slices * Bpad * L.kpadI) || e->Hdig.alloc((size_t)p2.slices * Bpad * K2) ||
-                    e->Udig.alloc((size_t)p2.slices * Nupad * K2) || L.bandDig.alloc((size_t)p1x.slices * L.fpad * L.W) ||
-                    e->res.alloc(std::max(panel * L.fpad * p1x.slices, panel * Nupad * p2.slices)))) {
-            (void)cudaGetLastError();
-            clear_error();
-            e->res.release();
-            L.dig = {};
-            res = false;
+        if (res) {
+            ResidueRoom room;
+            (void)planes([&](auto& d, size_t n) { return room.count(d, n); });
+            const bool tried = room.fits();
+            if (tried && !L.digits_are(p1x)) L.dig = {};   // (its planes may move)
+            if (!tried || planes([&](auto& d, size_t n) { return room.alloc(d, n); }) != GAIN_OK) {
+                if (tried) drop_planes();   // what was enlarged
+                e->res.release();
+                clear_error();
+                res = false;
+            }
         }
     }
     if (!res) {

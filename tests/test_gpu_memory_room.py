@@ -1,0 +1,74 @@
+"""The residue form's planes take about twice the memory of the digits'.  Where they do not fit,
+the run takes digits with the memory a digit run has: an allocation that fails at any point
+(GAINLS_RESIDUE_BYTES limits the new memory of an attempt) leaves nothing behind."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+JMAX = 11
+LIMITS = [0] + [(1 << k) + (1 << (k - 1)) * h for k in range(17, 28) for h in (0, 1)]
+
+
+def _problem():
+    import synth
+    return synth.make_problem(120, [5, 6], "c4", blocks=[(5, 0), (6, 1)])
+
+
+def _engine(p):
+    import gainls
+    eng = gainls.Engine(JMAX, p.nsym, 1)
+    gainls.upload_problem(eng, p)
+    return eng
+
+
+def _job(p):
+    return (0, 0, 1, 1, np.arange(p.blocks[(0, 0)].vecs.shape[0], dtype=np.int32),
+            np.arange(p.blocks[(1, 1)].vecs.shape[0], dtype=np.int32))
+
+
+def _free():
+    import torch
+    torch.cuda.synchronize()
+    return torch.cuda.mem_get_info()[0]
+
+
+def test_pair_runs_on_digits_where_the_residue_planes_do_not_fit(built_lib, monkeypatch):
+    """Limits from nothing to more than the attempt takes: every run gives the bits of a digit run or
+    of the residue form, a digit run has the memory of one that never tried, and the same engine
+    takes the residue form once there is room."""
+    import gainls
+    p = _problem()
+    job = _job(p)
+    _engine(p).run_pair(*job, gainls.PATH_SPLIT)    # (the context and the modules are loaded)
+
+    def run(eng, **kw):
+        st = eng.run_pair(*job, gainls.PATH_SPLIT, **kw)
+        assert st["status"] == gainls.OK
+        return st["products2"], eng.fetch_amp().copy()
+
+    eng = _engine(p)
+    before = _free()
+    n_dig, digits = run(eng, slices=6)     # the digits a run without room takes
+    used = before - _free()
+    n_res, residues = run(eng)
+    assert (n_dig, n_res) == (21, 13)
+    del eng
+    seen = set()
+    for limit in LIMITS:
+        eng = _engine(p)
+        monkeypatch.setenv("GAINLS_RESIDUE_BYTES", str(limit))
+        before = _free()
+        n, amp = run(eng)
+        seen.add(n)
+        assert np.array_equal(amp, residues if n == n_res else digits)
+        if n == n_dig:
+            assert before - _free() <= used + (4 << 20)
+            # a digit run, the failing attempt, and digits again in what may be the same addresses
+            assert np.array_equal(run(eng, slices=6)[1], digits)
+            assert np.array_equal(run(eng)[1], digits)
+        monkeypatch.delenv("GAINLS_RESIDUE_BYTES")
+        n, amp = run(eng)
+        assert n == n_res and np.array_equal(amp, residues)
+        del eng
+    assert seen == {n_dig, n_res}
