@@ -1415,6 +1415,18 @@ struct Staging {
     }
 };
 
+// The planes of the engine's last split run (none is needed once the run has returned).
+void drop_split_planes(gain_engine e) {
+    (void)cudaGetLastError();
+    e->Vdig.release();
+    e->Hdig.release();
+    e->Udig.release();
+    e->res.release();
+    e->zkey_V.clear();   // (another buffer may get an old one's address)
+    e->zkey_H.clear();
+    e->zkey_U.clear();
+}
+
 gain_status run_split(gain_engine e, const gain_pair_job* j, int dI, int dF, const gain_split_opts* opts,
                       gain_stats* stats) {
     GammaMaps* mI = gamma_maps(e, j->jindI, j->gammaI, dI);
@@ -1454,28 +1466,35 @@ gain_status run_split(gain_engine e, const gain_pair_job* j, int dI, int dF, con
     const int mstep = pair ? 2 * split::BM : split::BM;
     const int Bpad = round_up(B, mstep);
     const int Nu = j->nupper, Nupad = round_up(Nu, split::BN);
+    if (L.general && B > 65535)
+        return set_error(GAIN_ERR_UNSUPPORTED, "split path with a mixing expansion: at most 65535 lower states per run");
     SplitParams p1x, p2;
     bool res = residues_wanted(opts);
-    // the residue form's planes and panel of residues, each passed to `take` with its size
-    auto planes = [&](auto&& take) -> gain_status {
+    // everything of size that the run allocates, each passed to `take` with its size: the planes,
+    // the residue form's panel, and the outputs of either form (a form is chosen only when all
+    // of it has its place)
+    auto buffers = [&](auto&& take) -> gain_status {
         const size_t panel = (size_t)std::min(Bpad, residue_panel(mstep));
         GAIN_TRY(take(e->Vdig, (size_t)p1x.slices * Bpad * L.kpadI));
         GAIN_TRY(take(e->Hdig, (size_t)p2.slices * Bpad * K2));
         GAIN_TRY(take(e->Udig, (size_t)p2.slices * Nupad * K2));
-        GAIN_TRY(take(L.bandDig, (size_t)p1x.slices * L.fpad * L.W));
-        return take(e->res, std::max(panel * L.fpad * p1x.slices, panel * Nupad * p2.slices));
+        if (!L.digits_are(p1x)) GAIN_TRY(take(L.bandDig, (size_t)p1x.slices * L.fpad * L.W));
+        if (res) GAIN_TRY(take(e->res, std::max(panel * L.fpad * p1x.slices, panel * Nupad * p2.slices)));
+        GAIN_TRY(take(e->H, (size_t)Bpad * L.fpad));
+        if (npieces > 1) GAIN_TRY(take(e->acc, (size_t)Bpad * L.fpad));
+        if (L.general) {
+            GAIN_TRY(take(e->primI, (size_t)B * e->bases[j->jindI].dimen));
+            GAIN_TRY(take(e->Hsym, (size_t)Bpad * K2));
+        }
+        GAIN_TRY(take(e->amp, (size_t)Bpad * Nupad));
+        GAIN_TRY(take(e->ampbnd, (size_t)Bpad * Nupad));
+        GAIN_TRY(take(e->flags1, (size_t)kMaxFlags));
+        return take(e->flags2, (size_t)kMaxFlags);
     };
     auto drop_planes = [&]() {
-        (void)cudaGetLastError();
-        e->Vdig.release();
-        e->Hdig.release();
-        e->Udig.release();
-        e->res.release();
+        drop_split_planes(e);
         L.bandDig.release();
         L.dig = {};
-        e->zkey_V.clear();   // (another buffer may get an old one's address)
-        e->zkey_H.clear();
-        e->zkey_U.clear();
     };
     if (res) {
         p1x = residue_params1(L);
@@ -1483,10 +1502,10 @@ gain_status run_split(gain_engine e, const gain_pair_job* j, int dI, int dF, con
         res = digits_supported(p1x, p2);
         if (res) {
             ResidueRoom room;
-            (void)planes([&](auto& d, size_t n) { return room.count(d, n); });
+            (void)buffers([&](auto& d, size_t n) { return room.count(d, n); });
             const bool tried = room.fits();
             if (tried && !L.digits_are(p1x)) L.dig = {};   // (its planes may move)
-            if (!tried || planes([&](auto& d, size_t n) { return room.alloc(d, n); }) != GAIN_OK) {
+            if (!tried || buffers([&](auto& d, size_t n) { return room.alloc(d, n); }) != GAIN_OK) {
                 if (tried) drop_planes();   // what was enlarged
                 e->res.release();
                 clear_error();
@@ -1499,6 +1518,17 @@ gain_status run_split(gain_engine e, const gain_pair_job* j, int dI, int dF, con
         p2 = choose_params(K2, opts, 48, 8);
     }
     if (!digits_supported(p1x, p2)) return set_error(GAIN_ERR_INVALID_ARG, "unsupported digit configuration");
+    if (!res) {
+        auto place = [&]() {
+            if (!L.digits_are(p1x)) L.dig = {};
+            return buffers([](auto& d, size_t n) { return d.alloc(n); });
+        };
+        if (place() != GAIN_OK) {   // once more without the planes that earlier runs of other sizes left
+            drop_planes();
+            clear_error();
+            GAIN_TRY(place());
+        }
+    }
 
     // band digits (cached per digit configuration)
     auto band_digits = [&]() -> gain_status { return layout_band_digits(e, L, p1x, st); };
@@ -1553,8 +1583,6 @@ gain_status run_split(gain_engine e, const gain_pair_job* j, int dI, int dF, con
         GAIN_TRY(up.add(e->rtiles2, rp2.tiles.data(), rp2.tiles.size()));
     }
     GAIN_TRY(up.launch(e, st));
-    GAIN_TRY(e->flags1.alloc(kMaxFlags));
-    GAIN_TRY(e->flags2.alloc(kMaxFlags));
     // capacity of the refinement lists (GAINLS_MAX_FLAGS lowers it, to exercise the overflow
     // handling on small cases)
     int max_flags = kMaxFlags;
@@ -1566,11 +1594,8 @@ gain_status run_split(gain_engine e, const gain_pair_job* j, int dI, int dF, con
     const size_t vdig = (size_t)p1x.slices * Bpad * L.kpadI;
     const size_t hdig = (size_t)p2.slices * Bpad * K2;
     const size_t udig = (size_t)p2.slices * Nupad * K2;
-    GAIN_TRY(e->Vdig.alloc(vdig));
     GAIN_TRY(e->Vst.alloc(Bpad, p1x.stat_chunks(), false));
-    GAIN_TRY(e->Hdig.alloc(hdig));
     GAIN_TRY(e->Hst.alloc(Bpad, p2.stat_chunks(), true));
-    GAIN_TRY(e->Udig.alloc(udig));
     GAIN_TRY(e->Ust.alloc(Nupad, p2.stat_chunks(), false));
     if (res) {   // the residue slicing writes whole rows, and padding rows reach no output that is read
         e->zkey_V.clear();
@@ -1608,11 +1633,8 @@ gain_status run_split(gain_engine e, const gain_pair_job* j, int dI, int dF, con
     // ---- lower vectors -> digits in the padded lower layout (expanded to primitives first
     // when the expansion mixes them)
     const Basis& bIs = e->bases[j->jindI];
-    if (L.general && B > 65535)
-        return set_error(GAIN_ERR_UNSUPPORTED, "split path with a mixing expansion: at most 65535 lower states per run");
     if (L.general) {
         Inflation& iI = e->infl[j->jindI];
-        GAIN_TRY(e->primI.alloc((size_t)B * bIs.dimen));
         GAIN_TRY(e->iota.alloc(B));
         {
             std::vector<int> io(B);
@@ -1643,11 +1665,7 @@ gain_status run_split(gain_engine e, const gain_pair_job* j, int dI, int dF, con
     const std::vector<split::Prod> pr1 = res ? std::vector<split::Prod>() : make_prods(p1x, fuse1);
     if (!res) GAIN_TRY(e->prods1.upload(pr1));
     double res_flops = 0.0;
-    GAIN_TRY(e->H.alloc((size_t)Bpad * L.fpad));
-    if (npieces > 1) {
-        GAIN_TRY(e->acc.alloc((size_t)Bpad * L.fpad));
-        GAIN_TRY(e->acc.zero(st, (size_t)Bpad * L.fpad));
-    }
+    if (npieces > 1) GAIN_TRY(e->acc.zero(st, (size_t)Bpad * L.fpad));
     const Basis& bFs = e->bases[j->jindF];
     std::vector<split::Tile> t1;
     // first-GEMM refinement counts of the pieces before the last (the counter restarts per piece)
@@ -1823,7 +1841,6 @@ gain_status run_split(gain_engine e, const gain_pair_job* j, int dI, int dF, con
     // ---- mixing expansion: H_sym = H_prim T_F (FP64), row error bounds carried over
     const double* Hs = e->H.p;
     if (L.general) {
-        GAIN_TRY(e->Hsym.alloc((size_t)Bpad * K2));
         GAIN_CUDA(launch_contract_rowerr(B, e->H.p, L.fpad, L.fpad, e->rowerr.p, e->Vst.e.p, L.sigmaF, L.gamF, st));
         ++e->launches;
         GAIN_CUDA(launch_contract(L.nsymF, L.d_cF_ptr.p, L.d_cF_col.p, L.d_cF_val.p, e->H.p, L.fpad, e->Hsym.p, K2, B,
@@ -1860,8 +1877,6 @@ gain_status run_split(gain_engine e, const gain_pair_job* j, int dI, int dF, con
         GAIN_TRY(e->tiles2.upload(t2));
         GAIN_TRY(e->prods2.upload(pr2));
     }
-    GAIN_TRY(e->amp.alloc((size_t)Bpad * Nupad));
-    GAIN_TRY(e->ampbnd.alloc((size_t)Bpad * Nupad));
     split::GemmArgs g2;
     memset(&g2, 0, sizeof g2);
     g2.tiles = e->tiles2.p;
@@ -3142,8 +3157,15 @@ gain_status gain_run_pair_component(gain_engine e, const gain_pair_job* job, int
     if (e->deg_job != key) {
         e->deg_job.clear();
         e->deg_filled = 0;
-        GAIN_TRY(e->deg_amp.alloc((size_t)md * md * n));
-        GAIN_TRY(e->deg_bnd.alloc((size_t)md * md * n));
+        auto slots = [&]() -> gain_status {
+            GAIN_TRY(e->deg_amp.alloc((size_t)md * md * n));
+            return e->deg_bnd.alloc((size_t)md * md * n);
+        };
+        if (slots() != GAIN_OK) {   // the run's planes have done their work
+            drop_split_planes(e);
+            clear_error();
+            GAIN_TRY(slots());
+        }
         e->deg_job = key;
     }
     const int slot = idegI + idegF * md;

@@ -64,11 +64,39 @@ def test_pair_runs_on_digits_where_the_residue_planes_do_not_fit(built_lib, monk
         assert np.array_equal(amp, residues if n == n_res else digits)
         if n == n_dig:
             assert before - _free() <= used + (4 << 20)
-            # a digit run, the failing attempt, and digits again in what may be the same addresses
+            # a digit run, then another attempt, in what may be the same addresses; the outputs have
+            # their place by now, so the attempt may succeed
             assert np.array_equal(run(eng, slices=6)[1], digits)
-            assert np.array_equal(run(eng)[1], digits)
+            n, amp = run(eng)
+            assert np.array_equal(amp, residues if n == n_res else digits)
         monkeypatch.delenv("GAINLS_RESIDUE_BYTES")
         n, amp = run(eng)
         assert n == n_res and np.array_equal(amp, residues)
         del eng
     assert seen == {n_dig, n_res}
+
+
+@pytest.mark.parametrize("rule,nv,jv", [("c4", 120, (5, 6)), ("c4m", 75, (3, 4))])
+def test_a_form_is_chosen_with_room_for_its_outputs(built_lib, rule, nv, jv, monkeypatch):
+    """Room for the planes but not for what is written next to them (the refinement lists of 2 x 32 MB
+    are the last to be placed): digits, as without room for the planes."""
+    import gainls
+    import synth
+    p = synth.make_problem(nv, list(jv), rule, blocks=[(jv[0], 0), (jv[1], 1)])
+    job = _job(p)
+    warm = _engine(p)
+    warm.run_pair(*job, gainls.PATH_SPLIT, slices=6)
+    digits = warm.fetch_amp().copy()
+    eng = _engine(p)
+    before = _free()
+    assert eng.run_pair(*job, gainls.PATH_SPLIT)["products2"] == 13
+    residues, used = eng.fetch_amp().copy(), before - _free()
+    for short in (16 << 20, 48 << 20, 80 << 20):
+        eng = _engine(p)
+        monkeypatch.setenv("GAINLS_RESIDUE_BYTES", str(max(used - short, 0)))
+        st = eng.run_pair(*job, gainls.PATH_SPLIT)
+        assert st["status"] == gainls.OK and st["products2"] == 21
+        assert np.array_equal(eng.fetch_amp(), digits)
+        monkeypatch.delenv("GAINLS_RESIDUE_BYTES")
+        assert eng.run_pair(*job, gainls.PATH_SPLIT)["products2"] == 13
+        assert np.array_equal(eng.fetch_amp(), residues)
