@@ -1122,11 +1122,49 @@ gain_status slice(gain_engine e, const double* src, long ld, const int* src_rows
     return GAIN_OK;
 }
 
+// One attempt to place the buffers of the residue form, whose planes take about twice the digits'
+// memory: first the bytes they are short of are counted and compared with what the device has
+// left (a digit run of a size without room makes no attempt, and keeps its buffers), then they
+// are allocated.  GAINLS_RESIDUE_BYTES limits the new memory of an attempt, to exercise the way
+// back to digits on small cases.
+struct ResidueRoom {
+    size_t grow = 0, held = 0;   // new bytes, and those freed for them
+    size_t left = std::numeric_limits<size_t>::max();
+    ResidueRoom() {
+        if (const char* s = getenv("GAINLS_RESIDUE_BYTES")) left = (size_t)strtoull(s, nullptr, 10);
+    }
+    template <class T>
+    gain_status count(const DevArray<T>& d, size_t n) {
+        if (d.p && n <= d.n) return GAIN_OK;
+        grow += sizeof(T) * n;
+        held += sizeof(T) * d.n;
+        return GAIN_OK;
+    }
+    bool fits() const {
+        size_t free_bytes = 0, total = 0;
+        if (!grow || cudaMemGetInfo(&free_bytes, &total) != cudaSuccess) return true;
+        return grow <= free_bytes + held;
+    }
+    template <class T>
+    gain_status alloc(DevArray<T>& d, size_t n) {
+        if (d.p && n <= d.n) return GAIN_OK;
+        if (sizeof(T) * n > left) {
+            d.release();
+            return set_error(GAIN_ERR_OOM, "residue form: more than GAINLS_RESIDUE_BYTES");
+        }
+        left -= sizeof(T) * n;
+        return d.alloc(n);
+    }
+};
+
 // The band digits of layout L for the first GEMM's digit configuration p1 (kept until the
 // configuration or the band changes) and their tensor maps.
-gain_status layout_band_digits(gain_engine e, PairLayout& L, const SplitParams& p1, cudaStream_t st) {
+gain_status layout_band_digits(gain_engine e, PairLayout& L, const SplitParams& p1, cudaStream_t st,
+                               ResidueRoom* room = nullptr) {
     if (!L.digits_are(p1)) {
-        GAIN_TRY(L.bandDig.alloc((size_t)p1.slices * L.fpad * L.W));
+        L.dig = {};   // the old planes go with the allocation, whether it succeeds or not
+        const size_t n = (size_t)p1.slices * L.fpad * L.W;
+        GAIN_TRY(room ? room->alloc(L.bandDig, n) : L.bandDig.alloc(n));
         GAIN_TRY(L.bandStats.alloc(L.fpad, p1.stat_chunks(), false));
         if (!p1.bits) {   // every row and column of the residue planes is written
             GAIN_TRY(L.bandDig.zero(st, (size_t)p1.slices * L.fpad * L.W));
@@ -1208,41 +1246,6 @@ bool digits_supported(const SplitParams& p1, const SplitParams& p2) {
 // Columns [n0, n1) of a GEMM that share their inner range (k-blocks [a_k0 / BK, + nkb) of A).
 struct ColumnRange {
     int n0, n1, a_k0, nkb;
-};
-
-// One attempt to place the buffers of the residue form, whose planes take about twice the digits'
-// memory: first the bytes they are short of are counted and compared with what the device has
-// left (a digit run of a size without room makes no attempt, and keeps its buffers), then they
-// are allocated.  GAINLS_RESIDUE_BYTES limits the new memory of an attempt, to exercise the way
-// back to digits on small cases.
-struct ResidueRoom {
-    size_t grow = 0, held = 0;   // new bytes, and those freed for them
-    size_t left = std::numeric_limits<size_t>::max();
-    ResidueRoom() {
-        if (const char* s = getenv("GAINLS_RESIDUE_BYTES")) left = (size_t)strtoull(s, nullptr, 10);
-    }
-    template <class T>
-    gain_status count(const DevArray<T>& d, size_t n) {
-        if (d.p && n <= d.n) return GAIN_OK;
-        grow += sizeof(T) * n;
-        held += sizeof(T) * d.n;
-        return GAIN_OK;
-    }
-    bool fits() const {
-        size_t free_bytes = 0, total = 0;
-        if (!grow || cudaMemGetInfo(&free_bytes, &total) != cudaSuccess) return true;
-        return grow <= free_bytes + held;
-    }
-    template <class T>
-    gain_status alloc(DevArray<T>& d, size_t n) {
-        if (d.p && n <= d.n) return GAIN_OK;
-        if (sizeof(T) * n > left) {
-            d.release();
-            return set_error(GAIN_ERR_OOM, "residue form: more than GAINLS_RESIDUE_BYTES");
-        }
-        left -= sizeof(T) * n;
-        return d.alloc(n);
-    }
 };
 
 // Tiles of `rows` output rows over the column ranges, column by column: 256 columns wide on CTA
@@ -3937,7 +3940,7 @@ struct gain_plan_s {
 
 namespace {
 // Buffers, layout, digit configuration and tensor maps of one job (before any capture).
-gain_status plan_prepare_job(gain_plan P, PlanJob& J) {
+gain_status plan_prepare_job(gain_plan P, PlanJob& J, ResidueRoom* room) {
     gain_engine e = P->e;
     const gain_pair_job* j = &J.job;
     cudaStream_t st = e->st;
@@ -3964,7 +3967,7 @@ gain_status plan_prepare_job(gain_plan P, PlanJob& J) {
         P->residues_unsupported = P->residues;
         return set_error(GAIN_ERR_INVALID_ARG, "unsupported digit configuration");
     }
-    GAIN_TRY(layout_band_digits(e, L, J.p1, st));
+    GAIN_TRY(layout_band_digits(e, L, J.p1, st, room));
     const Basis& bI = e->bases[j->jindI];
     const Eig& EI = *e->eig[{j->jindI, j->gammaI}];
     const Eig& EF = *e->eig[{j->jindF, j->gammaF}];
@@ -4014,8 +4017,9 @@ gain_status plan_prepare_job(gain_plan P, PlanJob& J) {
     const size_t vdig = J.lowner < 0 ? (size_t)J.p1.slices * J.Bpad * L.kpadI : 0;
     const size_t hdig = (size_t)J.p2.slices * J.Bpad * J.K2;
     const size_t udig = J.uowner < 0 ? (size_t)J.p2.slices * J.Nupad * J.K2 : 0;
+    auto place = [room](auto& d, size_t n) { return room ? room->alloc(d, n) : d.alloc(n); };
     if (J.lowner < 0) {
-        GAIN_TRY(J.Vdig.alloc(vdig));
+        GAIN_TRY(place(J.Vdig, vdig));
         GAIN_TRY(J.Vst.alloc(J.Bpad, J.p1.stat_chunks(), false));
         if (!P->residues) {   // (residue planes and the statistics that are read are written whole)
             GAIN_TRY(J.Vdig.zero(st, vdig));
@@ -4025,14 +4029,14 @@ gain_status plan_prepare_job(gain_plan P, PlanJob& J) {
         J.Vdig.release();
         J.Vst = StatsDev();
     }
-    GAIN_TRY(J.Hdig.alloc(hdig));
+    GAIN_TRY(place(J.Hdig, hdig));
     GAIN_TRY(J.Hst.alloc(J.Bpad, J.p2.stat_chunks(), true));
     if (!P->residues) {
         GAIN_TRY(J.Hdig.zero(st, hdig));
         GAIN_TRY(J.Hst.zero(st, J.Bpad, J.p2.chunks, true));
     }
     if (J.uowner < 0) {
-        GAIN_TRY(J.Udig.alloc(udig));
+        GAIN_TRY(place(J.Udig, udig));
         GAIN_TRY(J.Ust.alloc(J.Nupad, J.p2.stat_chunks(), false));
         if (!P->residues) {
             GAIN_TRY(J.Udig.zero(st, udig));
@@ -4042,9 +4046,9 @@ gain_status plan_prepare_job(gain_plan P, PlanJob& J) {
         J.Udig.release();
         J.Ust = StatsDev();
     }
-    GAIN_TRY(J.H.alloc((size_t)J.Bpad * L.fpad));
-    GAIN_TRY(J.amp.alloc((size_t)J.Bpad * J.Nupad));
-    GAIN_TRY(J.ampbnd.alloc((size_t)J.Bpad * J.Nupad));
+    GAIN_TRY(place(J.H, (size_t)J.Bpad * L.fpad));
+    GAIN_TRY(place(J.amp, (size_t)J.Bpad * J.Nupad));
+    GAIN_TRY(place(J.ampbnd, (size_t)J.Bpad * J.Nupad));
     GAIN_TRY(J.flags1.alloc(J.cap1));
     GAIN_TRY(J.flags2.alloc(J.cap2));
     GAIN_TRY(J.d_lower.upload(J.lower));
@@ -4158,7 +4162,7 @@ gain_status plan_launch_slices(const std::vector<gain_plan_s::SliceBatch>& batch
 
 // The residue form of plan_build_groups: per job and GEMM an operand group, its (tile, modulus)
 // items and the reconstruction of its outputs.
-gain_status plan_build_residue_groups(gain_plan P) {
+gain_status plan_build_residue_groups(gain_plan P, ResidueRoom* room) {
     gain_engine e = P->e;
     const int mstep = P->pair ? 2 * split::BM : split::BM;
     P->units = P->pair ? e->num_sms / 2 : e->num_sms;
@@ -4170,7 +4174,7 @@ gain_status plan_build_residue_groups(gain_plan P) {
         const PlanJob& J = *P->jobs[q];
         off[q + 1] = off[q] + (size_t)J.Bpad * std::max((size_t)J.L->fpad * J.p1.slices, (size_t)J.Nupad * J.p2.slices);
     }
-    GAIN_TRY(P->res.alloc(off[nj]));
+    GAIN_TRY(room->alloc(P->res, off[nj]));
     std::vector<split::ResGroup> g1(nj), g2(nj);
     std::vector<split::CrtArgs> a1(nj), a2(nj);
     std::vector<int> o1(nj + 1, 0), o2(nj + 1, 0);
@@ -4308,8 +4312,8 @@ gain_status plan_residue_gemm(gain_plan P, const split::ResGroup* groups, const 
 }
 
 // Groups and schedules of both grouped launches.
-gain_status plan_build_groups(gain_plan P) {
-    if (P->residues) return plan_build_residue_groups(P);
+gain_status plan_build_groups(gain_plan P, ResidueRoom* room) {
+    if (P->residues) return plan_build_residue_groups(P, room);
     gain_engine e = P->e;
     const int mstep = P->pair ? 2 * split::BM : split::BM;
     P->units = P->pair ? e->num_sms / 2 : e->num_sms;
@@ -4601,7 +4605,8 @@ gain_status plan_build(gain_plan P) {
     P->drop_graph();
     const int nj = (int)P->jobs.size();
     auto prepare = [&]() -> gain_status {
-        for (auto& J : P->jobs) GAIN_TRY(plan_prepare_job(P, *J));
+        ResidueRoom attempt, *room = P->residues ? &attempt : nullptr;
+        for (auto& J : P->jobs) GAIN_TRY(plan_prepare_job(P, *J, room));
         GAIN_TRY(P->counters.alloc(2 * nj));
         GAIN_TRY(P->ull.alloc(4 * nj));
         GAIN_TRY(P->err.alloc(1));
@@ -4613,7 +4618,7 @@ gain_status plan_build(gain_plan P) {
             J->rowerr = re;
             re += J->Bpad;
         }
-        GAIN_TRY(plan_build_groups(P));
+        GAIN_TRY(plan_build_groups(P, room));
         GAIN_TRY(plan_build_refinement(P));
         return plan_build_slices(P);
     };
@@ -4631,9 +4636,18 @@ gain_status plan_build(gain_plan P) {
             J->Vdig.release();
             J->Hdig.release();
             J->Udig.release();
+            if (J->L) {
+                J->L->bandDig.release();
+                J->L->dig = {};
+            }
         }
         clear_error();
         ps = prepare();
+        if (ps == GAIN_ERR_OOM) {   // once more without what the engine's single runs keep
+            drop_split_planes(e);
+            clear_error();
+            ps = prepare();
+        }
     }
     GAIN_TRY(ps);
     if (!P->rb) GAIN_CUDA(cudaMallocHost(&P->rb, 40 * (size_t)nj + 64));

@@ -100,3 +100,45 @@ def test_a_form_is_chosen_with_room_for_its_outputs(built_lib, rule, nv, jv, mon
         monkeypatch.delenv("GAINLS_RESIDUE_BYTES")
         assert eng.run_pair(*job, gainls.PATH_SPLIT)["products2"] == 13
         assert np.array_equal(eng.fetch_amp(), residues)
+
+
+def test_plan_runs_on_digits_where_the_residue_planes_do_not_fit(built_lib, monkeypatch):
+    """A digit run leaves its band planes with the block pair; a plan's attempt at the residue form
+    then replaces them and fails at any of its allocations.  The plan runs on digits made anew:
+    every job has the bits of a digit plan, or of the residue form where all of it fits."""
+    import gainls
+    import synth
+    p = synth.make_problem(40, [1, 2, 3], "c4")
+    filt = gainls.make_filters([1.0] * 4, p.isym_pairs, p.igamma_pair, p.sym_degen, (0.0, 5000.0), (-1e9, 1e9),
+                               (-1e9, 1e9), 0.0, 3)
+    table = gainls.state_table(p.st_energy, p.st_J, p.st_jind, p.st_gamma, p.st_ndeg, p.st_ilevel)
+    jobs = gainls.plan_pairs(filt, table)
+
+    def run(eng, **kw):
+        plan = gainls.Plan(eng, jobs, **kw)
+        ps, _, st = plan.run()
+        amps = [plan.amp(q) for q in range(len(jobs))]
+        plan.close()
+        assert st == gainls.OK
+        return ps["slices2"][0], amps
+
+    def same(a, b):
+        return all(np.array_equal(x, y) for x, y in zip(a, b))
+
+    eng = _engine(p)
+    n_dig, digits = run(eng, slices=6)
+    n_res, residues = run(eng)
+    assert (n_dig, n_res) == (6, 13)
+    seen = set()
+    for limit in LIMITS:
+        eng = _engine(p)
+        for job in jobs:
+            eng.run_pair(*job, gainls.PATH_SPLIT, slices=6)
+        monkeypatch.setenv("GAINLS_RESIDUE_BYTES", str(limit))
+        n, amps = run(eng)
+        monkeypatch.delenv("GAINLS_RESIDUE_BYTES")
+        seen.add(n)
+        assert same(amps, residues if n == n_res else digits)
+        assert same(run(eng)[1], residues)
+        del eng
+    assert seen == {n_dig, n_res}
