@@ -2626,21 +2626,51 @@ gain_status adjoint_split_chain(gain_engine e, const gain_pair_job* job, int dI,
     // device cannot hold them, else 48-bit digits.
     SplitParams pA = residue_params(kAdjSplitBits, Nuk), pB = residue_params(kAdjSplitBits, Bk);
     const int panel1 = std::min(Bpad, residue_panel(pair ? 2 * BM : BM)), panel2 = std::min(Fpad, residue_panel(BM));
+    const int cap = kMaxFlags;
     bool res = pA.slices && pB.slices;
-    if (res && (e->adjs_dig[0].alloc((size_t)pA.slices * Bpad * Nuk) || e->adjs_dig[1].alloc((size_t)pA.slices * NtFpad * Nuk) ||
-                e->adjs_dig[2].alloc((size_t)pB.slices * Fpad * Bk) || e->adjs_dig[3].alloc((size_t)pB.slices * ldM * Bk) ||
-                e->res.alloc(std::max((size_t)panel1 * NtFpad * pA.slices, (size_t)panel2 * ldM * pB.slices)))) {
+    // everything of size, as in run_split: the form is chosen with room for all of it
+    auto buffers = [&](auto&& take) -> gain_status {
+        GAIN_TRY(take(e->adjs_dig[0], (size_t)pA.slices * Bpad * Nuk));
+        GAIN_TRY(take(e->adjs_dig[1], (size_t)pA.slices * NtFpad * Nuk));
+        GAIN_TRY(take(e->adjs_dig[2], (size_t)pB.slices * Fpad * Bk));
+        GAIN_TRY(take(e->adjs_dig[3], (size_t)pB.slices * ldM * Bk));
+        if (res)
+            GAIN_TRY(take(e->res, std::max((size_t)panel1 * NtFpad * pA.slices, (size_t)panel2 * ldM * pB.slices)));
+        GAIN_TRY(take(e->adjs_UT, (size_t)NtFpad * Nuk));
+        GAIN_TRY(take(e->adjs_dH, (size_t)Bpad * NtFpad));
+        GAIN_TRY(take(e->adj_dh, (size_t)B * bF.dimen));
+        GAIN_TRY(take(e->adj_vp, (size_t)B * bI.dimen));
+        GAIN_TRY(take(e->adjs_dhT, (size_t)Fpad * Bk));
+        GAIN_TRY(take(e->adjs_vpT, (size_t)ldM * Bk));
+        GAIN_TRY(take(e->adjs_dM, (size_t)Fpad * ldM));
+        return take(e->adjs_flags, (size_t)cap);
+    };
+    auto drop_planes = [&]() {
         (void)cudaGetLastError();
-        clear_error();
-        e->res.release();
-        res = false;
+        for (auto& d : e->adjs_dig) d.release();
+    };
+    if (res) {
+        ResidueRoom room;
+        (void)buffers([&](auto& d, size_t n) { return room.count(d, n); });
+        const bool tried = room.fits();
+        if (!tried || buffers([&](auto& d, size_t n) { return room.alloc(d, n); }) != GAIN_OK) {
+            if (tried) drop_planes();
+            e->res.release();
+            clear_error();
+            res = false;
+        }
     }
     if (!res) {
         pA = choose_params(Nuk, nullptr, kAdjSplitBits, 8);
         pB = choose_params(Bk, nullptr, kAdjSplitBits, 8);
+        auto place = [&]() { return buffers([](auto& d, size_t n) { return d.alloc(n); }); };
+        if (place() != GAIN_OK) {   // once more without what other sizes and the forward runs left
+            drop_planes();
+            drop_split_planes(e);
+            clear_error();
+            GAIN_TRY(place());
+        }
     }
-    const int cap = kMaxFlags;
-    GAIN_TRY(e->adjs_flags.alloc(cap));
     GAIN_TRY(e->adjs_cnt.alloc(2));
     GAIN_TRY(e->adjs_err.alloc(1));
 
@@ -2701,7 +2731,6 @@ gain_status adjoint_split_chain(gain_engine e, const gain_pair_job* job, int dI,
     auto planes = [&](int k, const SplitParams& p, const double* src, long ld, int nrows, int ncols, int kpad,
                       int rows_pad) -> gain_status {
         const size_t n = (size_t)p.slices * rows_pad * kpad;
-        GAIN_TRY(e->adjs_dig[k].alloc(n));
         GAIN_TRY(e->adjs_st[k].alloc(rows_pad, p.stat_chunks(), false));
         if (!res) {
             GAIN_TRY(e->adjs_dig[k].zero(st, n));
@@ -2770,11 +2799,9 @@ gain_status adjoint_split_chain(gain_engine e, const gain_pair_job* job, int dI,
         return GAIN_OK;
     };
     // ---- dH = G U: A = G rows (inner: upper states), B = U^T rows (upper symmetric functions)
-    GAIN_TRY(e->adjs_UT.alloc((size_t)NtFpad * Nuk));
     GAIN_CUDA(launch_gather_t(NtFpad, Nu, Nuk, EF.d.p, EF.nsize, e->d_upper.p, e->adjs_umap.p, e->adjs_UT.p, st));
     GAIN_TRY(planes(0, pA, G, Nu, B, Nu, Nuk, Bpad));
     GAIN_TRY(planes(1, pA, e->adjs_UT.p, Nuk, NtFpad, Nuk, Nuk, NtFpad));
-    GAIN_TRY(e->adjs_dH.alloc((size_t)Bpad * NtFpad));
     if (res) {
         CUtensorMap ta, tb;
         GAIN_TRY(maps(&ta, &tb, 0, 1, pA, Nuk, Bpad, NtFpad));
@@ -2788,8 +2815,6 @@ gain_status adjoint_split_chain(gain_engine e, const gain_pair_job* job, int dI,
                                      NtFpad, 2 * e->num_sms, st));
     }
     // ---- dh = T_F dH, vp = T_I v (primitive spaces)
-    GAIN_TRY(e->adj_dh.alloc((size_t)B * bF.dimen));
-    GAIN_TRY(e->adj_vp.alloc((size_t)B * bI.dimen));
     double* dh = e->adj_dh.p;
     double* vp = e->adj_vp.p;
     GAIN_CUDA(launch_expand_levels(iF.dimen, job->gammaF, iF.maxcoeff, dF, iF.sdeg[job->gammaF], NtF, iF.dijterms.p,
@@ -2799,13 +2824,10 @@ gain_status adjoint_split_chain(gain_engine e, const gain_pair_job* job, int dI,
                                    iI.dijterms.p, iI.dicontr.p, iI.dN[job->gammaI]->p, iI.drepres[job->gammaI]->p,
                                    EI.d.p, EI.nsize, e->d_lower.p, vp, bI.dimen, B, st));
     // ---- dM = dh^T vp on the band: A = dh^T rows (upper positions), B = vp^T rows (lower)
-    GAIN_TRY(e->adjs_dhT.alloc((size_t)Fpad * Bk));
-    GAIN_TRY(e->adjs_vpT.alloc((size_t)ldM * Bk));
     GAIN_CUDA(launch_gather_t(Fpad, B, Bk, dh, bF.dimen, nullptr, e->adjs_fmap.p, e->adjs_dhT.p, st));
     GAIN_CUDA(launch_gather_t(ldM, B, Bk, vp, bI.dimen, nullptr, e->adjs_imap.p, e->adjs_vpT.p, st));
     GAIN_TRY(planes(2, pB, e->adjs_dhT.p, Bk, Fpad, Bk, Bk, Fpad));
     GAIN_TRY(planes(3, pB, e->adjs_vpT.p, Bk, ldM, Bk, Bk, ldM));
-    GAIN_TRY(e->adjs_dM.alloc((size_t)Fpad * ldM));
     if (res) {
         CUtensorMap ta, tb;
         GAIN_TRY(maps(&ta, &tb, 2, 3, pB, Bk, Fpad, ldM));

@@ -142,3 +142,43 @@ def test_plan_runs_on_digits_where_the_residue_planes_do_not_fit(built_lib, monk
         assert same(run(eng)[1], residues)
         del eng
     assert seen == {n_dig, n_res}
+
+
+def test_adjoint_runs_on_digits_where_the_residue_form_does_not_fit(built_lib, monkeypatch):
+    """The tensor-core adjoint at the same limits: the gradient of the FP64 chain to 1e-9 of its
+    largest component (what either form is held to), and on digits the memory of one that never
+    tried."""
+    import gainls
+    import synth
+    p = synth.make_problem(75, [4, 5], "c4", blocks=[(4, 0), (5, 1)])
+    job = _job(p)
+    w = np.random.default_rng(5).standard_normal((len(job[4]), len(job[5])))
+    g64 = _engine(p).adjoint(*job, w, np.zeros(p.dipole.size))
+
+    def run(eng):     # (behind a plain run: the forward is not part of it)
+        eng.run_pair(*job, gainls.PATH_PLAIN_FP64)
+        g = eng.adjoint(*job, w, np.zeros(p.dipole.size), precision="split")
+        assert np.max(np.abs(g - g64)) <= 1e-9 * np.abs(g64).max()
+        return eng.last_adjoint_stats.tensor_flops
+
+    before = _free()
+    eng = _engine(p)
+    f_res, used_res = run(eng), before - _free()
+    del eng
+    forms, used_dig = set(), None
+    for limit in LIMITS + [used_res - (20 << 20)]:
+        before = _free()
+        eng = _engine(p)
+        monkeypatch.setenv("GAINLS_RESIDUE_BYTES", str(limit))
+        f, used = run(eng), before - _free()
+        monkeypatch.delenv("GAINLS_RESIDUE_BYTES")
+        if limit == 0:
+            assert f != f_res
+            f_dig, used_dig = f, used
+        assert f in (f_dig, f_res)
+        if f == f_dig:
+            assert used <= used_dig + (4 << 20)
+        forms.add(f)
+        assert run(eng) == f_res
+        del eng
+    assert forms == {f_dig, f_res} and f == f_dig    # (the last limit ends in the list of 32 MB)
