@@ -2846,17 +2846,19 @@ gain_status adjoint_split_chain(gain_engine e, const gain_pair_job* job, int dI,
             g.tiles = e->rtiles1.p + rt2_at + pn[0];
             g.ntiles = pn[1];
             GAIN_CUDA(split::launch_residue_gemm(ta, tb, g, e->num_sms, st, false));
-            // the panel's columns (entries outside its rows' bands are never read)
+            // the panel's columns in whole blocks of 128 (bands start on blocks of 64; entries outside
+            // the rows' bands are never read)
+            const int col0 = pn[2] / BN * BN, col1 = round_up(pn[3], BN);
             split::CrtArgs c = c0;
-            c.res = g.res + pn[2];
+            c.res = g.res + col0;
             c.plane = g.plane;
             c.row0 = g.m_base;
             c.rows = std::min(panel2, Fpad - g.m_base);
-            c.cols = pn[3] - pn[2];
-            c.B.e += pn[2];
-            c.B.l2 += pn[2];
-            c.B.dn += pn[2];
-            c.out += pn[2];
+            c.cols = col1 - col0;
+            c.B.e += col0;
+            c.B.l2 += col0;
+            c.B.dn += col0;
+            c.out += col0;
             GAIN_CUDA(split::launch_crt(c, st));
             fl += 2.0 * pn[1] * BM * BN * (double)Bk * pB.slices;
         }

@@ -1014,6 +1014,7 @@ cudaError_t launch_residue_gemm_grouped(const ResGemmArgs& a, int units, cudaStr
 }
 
 cudaError_t launch_crt(const CrtArgs& a0, cudaStream_t st) {
+    if (a0.cols % 128) return cudaErrorInvalidValue;   // (the kernel's warps lie whole in a row)
     CrtArgs a = a0;
     crt_set_rows(&a, 1);
     const int nb = crt_blocks(a);

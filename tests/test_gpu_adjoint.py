@@ -173,3 +173,21 @@ def test_tensor_core_adjoint_degenerate(built_lib):
     gtc = eng.adjoint(0, 2, 1, 2, lo, up, w, np.zeros(p.dipole.size), precision="split", filters=f)
     assert np.max(np.abs(gtc - g64)) <= 1e-9 * np.abs(g64).max()
     eng.close()
+
+
+@pytest.mark.parametrize("nv,jv", [(37, (10, 9)), (40, (9, 10))])
+def test_tensor_core_adjoint_bands_that_start_off_the_tiles(built_lib, nv, jv):
+    """Lower K blocks of one 64-function block each (K = 0 of less), two panels of 1024 upper rows: the
+    second panel's bands start at column 448 and end at 640 or 768, so that neither its first
+    column nor its width is a multiple of 128.  The gradient of the FP64 chain, as above."""
+    import gainls
+    import synth
+    p = synth.make_problem(nv, list(jv), "c4", blocks=[(jv[0], 0), (jv[1], 1)])
+    eng = gainls.Engine(JMAX, p.nsym, 1)
+    gainls.upload_problem(eng, p)
+    lo = list(range(p.blocks[(0, 0)].vecs.shape[0]))
+    up = list(range(p.blocks[(1, 1)].vecs.shape[0]))
+    w = np.random.default_rng(nv).standard_normal((len(lo), len(up)))
+    g64 = eng.adjoint(0, 0, 1, 1, lo, up, w, np.zeros(p.dipole.size))
+    gtc = eng.adjoint(0, 0, 1, 1, lo, up, w, np.zeros(p.dipole.size), precision="split")
+    assert np.max(np.abs(gtc - g64)) <= 1e-9 * np.abs(g64).max()
