@@ -1216,22 +1216,26 @@ SplitParams residue_params(int bits, int K) {
     return p;
 }
 
-// First GEMM in residue form.  Its certificate (every H entry within the FP64 bound of its dot
-// product) needs 53 - log2(W + 64) + 6 bits as the digits do; the moduli that holds are then
-// filled: the fraction bits that the same number of moduli still holds, at most 52 (beyond
-// that the FP64 output's own rounding is all that is left).  At W = 3072: 49 bits, 13 moduli.
+// The bits that the digits of a configuration hold; the residue form holds no fewer.
+int digit_bits(const SplitParams& d) { return std::min(split::kResMaxBits, d.slices * d.beta); }
+
+// First GEMM in residue form: the bits that its digits hold (56 at band widths below 960 and, with
+// rotational symmetry, 1984; 49 or 48 above), then the moduli filled: the fraction bits that the
+// same number of moduli still holds, at most 52 (beyond that the FP64 output's own rounding is all
+// that is left).  At W = 3072: 49 bits, 13 moduli; at W = 256 to 959: 56 bits, 15.
 SplitParams residue_params1(const PairLayout& L) {
-    int bits = (int)std::ceil(53.0 - std::log2((double)L.W + 64.0) + 6.0);
-    bits = std::max(46, std::min(52, bits));
     if (const char* b1 = getenv("GAINLS_GEMM1_BITS"))
         return residue_params(std::max(40, std::min(split::kResMaxBits, atoi(b1))), L.W);
+    int bits = digit_bits(gemm1_params(L, nullptr));
     SplitParams p = residue_params(bits, L.W);
     while (p.slices && bits < 52 && split::residue_moduli(bits + 1, L.W) == p.slices) p = residue_params(++bits, L.W);
     return p;
 }
 
-// Second GEMM in residue form: 48 bits, as the digits keep, with no product dropped.
-SplitParams residue_params2(int K2) { return residue_params(48, K2); }
+// A product of inner length K in residue form with the bits that digits of `bits` bits hold: 48 of
+// the second GEMM, 49 where its digits are of 7 bits (K above 19 660).
+SplitParams residue_params_as(int bits, int K) { return residue_params(digit_bits(choose_params(K, nullptr, bits, 8)), K); }
+SplitParams residue_params2(int K2) { return residue_params_as(48, K2); }
 
 // The residue form serves runs that leave the digit configuration open.
 bool residues_wanted(const gain_split_opts* o) { return !(o && (o->beta || o->slices || o->kchunks)); }
@@ -1455,9 +1459,9 @@ gain_status run_split(gain_engine e, const gain_pair_job* j, int dI, int dF, con
     // through ||dH||_2 ||u||_2; every entry must certify FP64-grade), see gemm1_params.
     // Second GEMM: 48 bits (8-bit digits in up to MAX_CHUNKS chunks, else 7 x 7 bits);
     // options (beta, slices, kchunks) apply to it.
-    // Both GEMMs take the residue form (residue.h: 13 products each at these precisions, against
-    // 28 and 21 digit products) unless the options name a digit configuration or the device
-    // cannot hold its planes (26 bytes per operand entry, the digits' 12 to 16).  Residues
+    // Both GEMMs take the residue form (residue.h: 13 products each, 15 in a narrow first GEMM,
+    // against 28 to 36 and 21 digit products) unless the options name a digit configuration or the
+    // device cannot hold its planes (26 to 30 bytes per operand entry, the digits' 12 to 16).  Residues
     // against digits on GB300: 7.8 / 13.5 ms at 2000 x 12 000 of 11 000 x 12 000 functions, 0.27 /
     // 0.40 ms at 550 x 1200, 0.17 / 0.33 ms at 50 x 600; errors against FP64 1.8e-14 / 6.3e-14.
     const int K2 = L.general ? L.ntpad : L.fpad;   // inner dimension of the second GEMM
@@ -2624,7 +2628,7 @@ gain_status adjoint_split_chain(gain_engine e, const gain_pair_job* job, int dI,
 
     // Operand planes: residues (residue.h: 13 products, exact for any operands) unless the
     // device cannot hold them, else 48-bit digits.
-    SplitParams pA = residue_params(kAdjSplitBits, Nuk), pB = residue_params(kAdjSplitBits, Bk);
+    SplitParams pA = residue_params_as(kAdjSplitBits, Nuk), pB = residue_params_as(kAdjSplitBits, Bk);
     const int panel1 = std::min(Bpad, residue_panel(pair ? 2 * BM : BM)), panel2 = std::min(Fpad, residue_panel(BM));
     const int cap = kMaxFlags;
     bool res = pA.slices && pB.slices;

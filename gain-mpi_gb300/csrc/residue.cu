@@ -1019,14 +1019,20 @@ cudaError_t launch_crt(const CrtArgs& a0, cudaStream_t st) {
     crt_set_rows(&a, 1);
     const int nb = crt_blocks(a);
     if (nb <= 0) return cudaSuccess;
-    return a.nmod == 13 ? launch_following(k_crt<false, 13>, (unsigned)nb, kCrtThreads, st, a, CrtGroups{})
-                        : launch_following(k_crt<false, 0>, (unsigned)nb, kCrtThreads, st, a, CrtGroups{});
+    const auto k = a.nmod == 13   ? k_crt<false, 13>
+                   : a.nmod == 14 ? k_crt<false, 14>
+                   : a.nmod == 15 ? k_crt<false, 15>
+                                  : k_crt<false, 0>;
+    return launch_following(k, (unsigned)nb, kCrtThreads, st, a, CrtGroups{});
 }
 
 cudaError_t launch_crt_grouped(const CrtGroups& g, cudaStream_t st) {
     if (g.blocks <= 0 || g.n <= 0) return cudaSuccess;
-    if (g.nmod == 13) k_crt<true, 13><<<g.blocks, kCrtThreads, 0, st>>>(CrtArgs{}, g);
-    else k_crt<true, 0><<<g.blocks, kCrtThreads, 0, st>>>(CrtArgs{}, g);
+    const auto k = g.nmod == 13   ? k_crt<true, 13>
+                   : g.nmod == 14 ? k_crt<true, 14>
+                   : g.nmod == 15 ? k_crt<true, 15>
+                                  : k_crt<true, 0>;
+    k<<<g.blocks, kCrtThreads, 0, st>>>(CrtArgs{}, g);
     return cudaGetLastError();
 }
 

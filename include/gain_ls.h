@@ -208,9 +208,10 @@ typedef struct gain_pair_job {
  * whose exact-accumulation certificate fails) are recomputed in FP64.  Every amplitude is
  * therefore within tol or within the reference FP64 method's own worst-case bound. */
 /* With beta, slices and kchunks all 0 both GEMMs run in residue form (one BF16 product per
- * modulus, the exact product of operands rounded to 48 bits, 49 to 52 in the first GEMM;
- * Ozaki scheme II), unless the device cannot hold its operand planes; naming any of the three
- * takes balanced digits (Ozaki scheme I). */
+ * modulus, the exact product of operands rounded to no fewer bits than the default digits hold:
+ * 48 in the second GEMM, 49 above an inner length of 19 660; 48 to 56 in the first by its inner
+ * length, 56 below 960; Ozaki scheme II), unless the device cannot hold its operand planes
+ * and outputs; naming any of the three takes balanced digits (Ozaki scheme I). */
 typedef struct gain_split_opts {
     double tol;       /* relative tolerance on each amplitude (0 -> 4.5e-9, so that
                          S = amp^2 meets 1e-8) */

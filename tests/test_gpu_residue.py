@@ -244,3 +244,22 @@ def test_a_run_returns_after_the_whole_asynchronous_copy(built_lib, lead):
     pin[-64:] = 0.0
     eng.run_pair(0, 0, 1, 1, lo, tail, gainls.PATH_SPLIT)
     np.testing.assert_array_equal(eng.fetch_amp(), want)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("name", ["c4", "c4r", "full", "c4m"])
+def test_narrow_bands_keep_the_bits_of_their_digits(problems, name, monkeypatch):
+    """First GEMMs of band widths below 960: their digits hold 8 x 7 = 56 bits of each operand, and
+    the residue form holds as many, so a run without options is the run of 56 bits."""
+    import gainls
+    p, eng, (gI, gF) = problems[name]
+    lo = np.arange(p.blocks[(0, gI)].vecs.shape[0], dtype=np.int32)
+    up = np.arange(p.blocks[(1, gF)].vecs.shape[0], dtype=np.int32)
+    dig = eng.run_pair(0, gI, 1, gF, lo, up, gainls.PATH_SPLIT, slices=6)
+    assert dig["beta1"] * dig["slices1"] == 56
+    st = eng.run_pair(0, gI, 1, gF, lo, up, gainls.PATH_SPLIT)
+    amp = eng.fetch_amp().copy()
+    monkeypatch.setenv("GAINLS_GEMM1_BITS", "56")
+    want = eng.run_pair(0, gI, 1, gF, lo, up, gainls.PATH_SPLIT)
+    assert st["slices1"] == want["slices1"] in (14, 15)
+    assert np.array_equal(amp, eng.fetch_amp())
