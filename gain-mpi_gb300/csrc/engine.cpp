@@ -1224,8 +1224,11 @@ int digit_bits(const SplitParams& d) { return std::min(split::kResMaxBits, d.sli
 // same number of moduli still holds, at most 52 (beyond that the FP64 output's own rounding is all
 // that is left).  At W = 3072: 49 bits, 13 moduli; at W = 256 to 959: 56 bits, 15.
 SplitParams residue_params1(const PairLayout& L) {
-    if (const char* b1 = getenv("GAINLS_GEMM1_BITS"))
-        return residue_params(std::max(40, std::min(split::kResMaxBits, atoi(b1))), L.W);
+    if (const char* b1 = getenv("GAINLS_GEMM1_BITS")) {
+        SplitParams p = residue_params(std::max(40, std::min(62, atoi(b1))), L.W);
+        if (p.bits > split::kResMaxBits) p.slices = 0;   // more than the planes hold: left to the digits
+        return p;
+    }
     int bits = digit_bits(gemm1_params(L, nullptr));
     SplitParams p = residue_params(bits, L.W);
     while (p.slices && bits < 52 && split::residue_moduli(bits + 1, L.W) == p.slices) p = residue_params(++bits, L.W);

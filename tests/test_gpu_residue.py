@@ -263,3 +263,22 @@ def test_narrow_bands_keep_the_bits_of_their_digits(problems, name, monkeypatch)
     want = eng.run_pair(0, gI, 1, gF, lo, up, gainls.PATH_SPLIT)
     assert st["slices1"] == want["slices1"] in (14, 15)
     assert np.array_equal(amp, eng.fetch_amp())
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("name", ["c4", "c4r"])
+@pytest.mark.parametrize("bits", [56, 57, 62])
+def test_more_bits_than_the_planes_hold_are_left_to_the_digits(problems, name, bits, monkeypatch):
+    """GAINLS_GEMM1_BITS above 56: a run without options answers as one with a digit configuration
+    does, here a refusal (9 x 7 or 8 x 8 bits do not fit the recombination), and a plan too."""
+    import gainls
+    p, eng, (gI, gF) = problems[name]
+    lo, up = np.arange(5, dtype=np.int32), np.arange(7, dtype=np.int32)
+    monkeypatch.setenv("GAINLS_GEMM1_BITS", str(bits))
+    got = [eng.run_pair(0, gI, 1, gF, lo, up, gainls.PATH_SPLIT, raise_on_error=False, **kw)["status"]
+           for kw in (dict(), dict(slices=6))]
+    assert got[0] == got[1] == (gainls.OK if bits <= 56 else gainls.ERR_INVALID_ARG)
+    for kw in (dict(), dict(slices=6)) if bits > 56 else ():
+        with pytest.raises(gainls.GainError) as err:    # (a plan prepares its jobs when it is made)
+            gainls.Plan(eng, [(0, gI, 1, gF, lo, up)], **kw)
+        assert err.value.status == gainls.ERR_INVALID_ARG
