@@ -452,7 +452,9 @@ gain_status gain_pair_lines_text(gain_engine e, const gain_line_params* prm, con
 /* gain_pair_lines_text with the text copied into out as it is formed: the copy of each
  * part overlaps the formatting of the next (page-locked out for that overlap).  cap must
  * hold the whole text; otherwise nothing is copied, *text_bytes holds its size and the call
- * returns GAIN_ERR_INVALID_ARG (the text stays on the device for gain_fetch_lines_text). */
+ * returns GAIN_ERR_INVALID_ARG (the text stays on the device for gain_fetch_lines_text).  A call
+ * with GAIN_TEXT_INTENSITY that needs the host's intensity for more than 1048576 lines returns
+ * GAIN_ERR_UNSUPPORTED; parts of the text are then already in out, whose contents are of no use. */
 gain_status gain_pair_lines_text_host(gain_engine e, const gain_line_params* prm, const double* energiesI,
                                       const double* energiesF, int jI, int jF, int gammaI, int gammaF,
                                       int flags, char* out, unsigned long long cap,
